@@ -40,7 +40,7 @@ def build(ref=True):
     """Compile the restatement (and, when the reference tree is present, the
     reference engine driver)."""
     subprocess.check_call(["make", "-s", "-C", HERE, "restate"])
-    if ref and os.path.isdir(reference_dir()):
+    if ref and os.path.isdir(os.path.join(reference_dir(), "storage_engine", "src")):
         subprocess.check_call(["make", "-s", "-C", HERE, "ref", "REF=" + reference_dir()])
 
 
