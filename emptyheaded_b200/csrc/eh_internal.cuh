@@ -41,6 +41,8 @@ struct TrieView {
   const int32_t* head_index;  // [n_nodes] value -> head position, -1 if absent
   const uint64_t* off;        // [n_head + 1] child set i = vals[off[i] .. off[i+1])
   const uint32_t* vals;       // [rows] sorted within each set
+  const uint32_t* up;         // symmetric relation: [n_head] first element of set i above head[i] (index into
+                              // vals, the set's end if none); null otherwise
   const uint8_t* layout;      // [n_head + 1] EH_LAYOUT_*; entry n_head is the head set
   const SetAux* aux;          // [n_head + 1]
   const uint64_t* bs_words;   // range-bitset words
@@ -84,6 +86,7 @@ struct eh_trie {
   eh::DevBuf<uint32_t> rev_src;   // head position of a for entry k
   eh::DevBuf<uint64_t> rev_wpre;  // exclusive prefix of entry work, rev_entries + 1 values
   uint64_t rev_entries = 0, rev_pairs = 0;
+  eh::DevBuf<uint32_t> up;        // DIR_SYM: per head entry, first element above it (TrieView::up)
   // With learned layouts: the cost model's predicted SM cycles of every
   // staged set's work (0 for sets never staged), and their sum over the
   // probes; the planner cuts work items by predicted cycles instead of
@@ -101,6 +104,7 @@ struct eh_trie {
     v.head_index = head_index.p;
     v.off = off.p;
     v.vals = vals.p;
+    v.up = up.p;
     v.layout = layout.p;
     v.aux = aux.p;
     v.bs_words = bs_words.p;

@@ -171,6 +171,34 @@ __host__ __device__ __forceinline__ uint32_t zbits_words(uint32_t W, uint32_t le
   return 2 * groups + 2 * (len < W ? len : W);
 }
 
+// The part of N(b) the plans stage.  On a symmetric relation every row a->b
+// runs with a < b and only candidates above b, so only N(b)'s elements above b
+// can match: t.up[b] is the first of them, found once at build.  With ids in
+// degree order that part is short even for a hub (Chung-Lu 2^21: sets of up to
+// 630,714 elements, a few hundred of them above their own id), so it is staged in
+// shared memory where the whole set had to be searched in global memory
+// (lollipop there 36.6 -> 11.8 ms, barbell on 2^16 nodes 2.5 -> 1.5 ms).  Other relations stage the whole set.  No
+// row of the reverse level has a b without such elements.
+struct StagedRange {
+  uint64_t s0;   // first element in vals
+  uint32_t len;
+};
+__device__ __forceinline__ StagedRange staged_range(const TrieView& t, uint32_t b) {
+  const uint64_t s0 = t.up ? (uint64_t)__ldg(t.up + b) : t.off[b];
+  return StagedRange{s0, (uint32_t)(t.off[b + 1] - s0)};
+}
+// the same part of a range bitset: from the word of its first element on
+__device__ __forceinline__ SetAux staged_bits(const TrieView& t, uint32_t b, const StagedRange& sr) {
+  SetAux a = t.aux[b];
+  if (t.up && sr.len) {
+    const uint32_t skip = (__ldg(t.vals + sr.s0) >> 6) - a.start;
+    a.off += skip;
+    a.start += skip;
+    a.n -= skip;
+  }
+  return a;
+}
+
 // Work of head entry b is staged in one of two classes: per warp (N(b)
 // fits a warp's shared region, or must be probed in global memory) or per
 // block (N(b) needs more than a warp's region but fits the block's: every
@@ -178,13 +206,15 @@ __host__ __device__ __forceinline__ uint32_t zbits_words(uint32_t W, uint32_t le
 // holds `warps` times a warp item's work.
 __device__ __forceinline__ uint32_t staged_words(const TrieView& t, uint32_t b, uint32_t warp_words) {
   const uint8_t l = t.layout[b];
+  const StagedRange sr = staged_range(t, b);
   if (l == EH_LAYOUT_RANGE_BITSET) {
-    const uint32_t raw = 2u * t.aux[b].n;
+    const uint32_t words = staged_bits(t, b, sr).n;
+    const uint32_t raw = 2u * words;
     if (raw <= warp_words) return raw;
-    const uint32_t z = zbits_words(t.aux[b].n, (uint32_t)(t.off[b + 1] - t.off[b]));
+    const uint32_t z = zbits_words(words, sr.len);
     return z <= warp_words ? z : raw;  // compressed in a warp, or raw across a block
   }
-  if (l == EH_LAYOUT_UINTEGER) return (uint32_t)(t.off[b + 1] - t.off[b]);
+  if (l == EH_LAYOUT_UINTEGER) return sr.len;
   return 0xffffffffu;  // block bitsets are probed in global memory
 }
 
@@ -379,7 +409,7 @@ struct Sink {
   int wmode;                  // P_SLIST (position by search) or P_SBITS (position by rank)
   const uint32_t* wlist;      // P_SLIST: the staged list, wn elements
   const uint64_t* wwords;     // P_SBITS: the staged words, wn of them from word wstart
-  const uint32_t* wrank;      // P_SBITS: elements before each staged word
+  const uint32_t* wrank;      // P_SBITS: staged elements before each staged word
   uint32_t wstart, wn;
 };
 
@@ -728,9 +758,10 @@ __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_
                                          bool zlist = false) {
   const uint32_t lane = lane_id();
   const uint8_t layout = t.layout[hb];
-  const SetAux a = t.aux[hb];
-  const uint64_t s0 = t.off[hb];
-  const uint32_t len = (uint32_t)(t.off[hb + 1] - s0);
+  const StagedRange sr = staged_range(t, hb);
+  const uint64_t s0 = sr.s0;
+  const uint32_t len = sr.len;
+  const SetAux a = layout == EH_LAYOUT_RANGE_BITSET ? staged_bits(t, hb, sr) : t.aux[hb];
   if (layout == EH_LAYOUT_RANGE_BITSET) {
     st.start = a.start;
     st.n = a.n;
@@ -841,9 +872,10 @@ __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_
 __device__ __forceinline__ int stage_set_block(const TrieView& t, uint32_t hb, uint32_t* sm, int cap_words,
                                                Staged& st) {
   const uint8_t layout = t.layout[hb];
-  const SetAux a = t.aux[hb];
-  const uint64_t s0 = t.off[hb];
-  const uint32_t len = (uint32_t)(t.off[hb + 1] - s0);
+  const StagedRange sr = staged_range(t, hb);
+  const uint64_t s0 = sr.s0;
+  const uint32_t len = sr.len;
+  const SetAux a = layout == EH_LAYOUT_RANGE_BITSET ? staged_bits(t, hb, sr) : t.aux[hb];
   if (layout == EH_LAYOUT_RANGE_BITSET) {
     st.start = a.start;
     st.n = a.n;
@@ -980,8 +1012,8 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict_
     } else {
       mode = stage_set(t, item.hb, sm, cap_words, st, kMode == MODE_COUNT);
     }
-    const uint64_t b0 = t.off[item.hb];
-    const uint32_t blen = (uint32_t)(t.off[item.hb + 1] - b0);
+    const StagedRange sr = staged_range(t, item.hb);
+    const uint32_t blen = sr.len;
     if (kMode == MODE_ANNOT && r.dir == DIR_SYM && (mode == P_SLIST || mode == P_SBITS)) {
       // per-element counters after the staged structure, if they fit
       const uint32_t used = mode == P_SLIST ? st.n : 3 * st.n;  // list, or words (2 per) + ranks
@@ -993,8 +1025,11 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict_
         sk.wstart = st.start;
         if (mode == P_SBITS) {
           uint32_t* rk = sm + 2 * st.n;
-          const uint32_t* grk = t.bs_rank + t.aux[item.hb].off;
-          for (uint32_t j = lane; j < st.n; j += 32) rk[j] = __ldg(grk + j);
+          // ranks within the staged part (the first word's may be negative,
+          // mod 2^32: it can hold elements before that part)
+          const uint32_t* grk = t.bs_rank + staged_bits(t, item.hb, sr).off;
+          const uint32_t before = (uint32_t)(sr.s0 - t.off[item.hb]);
+          for (uint32_t j = lane; j < st.n; j += 32) rk[j] = __ldg(grk + j) - before;
           sk.wrank = rk;
         }
         sk.wcnt = sm + used;
@@ -1021,7 +1056,7 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict_
       __syncwarp();
       for (uint32_t j = lane; j < blen; j += 32) {
         const uint32_t n = sk.wcnt[j];
-        if (n) atomicAdd(out.annot + __ldg(t.head_index + __ldg(t.vals + b0 + j)), 2ull * n);
+        if (n) atomicAdd(out.annot + __ldg(t.head_index + __ldg(t.vals + sr.s0 + j)), 2ull * n);
       }
     }
     if (kMode == MODE_ANNOT && r.dir == DIR_SYM && lane == 0 && c) atomicAdd(out.annot + item.hb, 2ull * c);
@@ -1031,7 +1066,8 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict_
     else __syncwarp();                 // the staged region is reused by the next item
     if (out.records && (block_phase ? threadIdx.x == 0 : lane == 0)) {
       const long long t1 = clock64();
-      const uint32_t len = blen;
+      const uint64_t b0 = t.off[item.hb];
+      const uint32_t len = (uint32_t)(t.off[item.hb + 1] - b0);
       const uint64_t pairs = r.rev_wpre[item.ke] - r.rev_wpre[item.kb];
       const uint32_t first = t.vals[b0], last = t.vals[b0 + len - 1];
       float* rec = out.records + 8 * (size_t)it;

@@ -459,7 +459,7 @@ static void update_bytes(eh_trie* t) {
                          t->layout.bytes() + t->aux.bytes() + t->bs_words.bytes() + t->bs_rank.bytes() +
                          t->bb_id.bytes() + t->bb_rank.bytes() + t->bb_words.bytes() + t->wedges.bytes() +
                          t->rev_off.bytes() + t->rev_lo.bytes() + t->rev_hi.bytes() + t->rev_src.bytes() +
-                         t->rev_wpre.bytes() + t->work_pred.bytes();
+                         t->rev_wpre.bytes() + t->work_pred.bytes() + t->up.bytes();
 }
 
 void trie_layout(eh_context* ctx, eh_trie* t, const eh_layout_config* cfg) {
@@ -666,6 +666,19 @@ __device__ __forceinline__ void rev_range(int dir, uint64_t e, uint64_t a_lo, ui
   else { lo = a_lo; hi = a_hi; }
 }
 
+// DIR_SYM: the first element of each set above its own head value
+__global__ void up_kernel(TrieView t, uint32_t* __restrict__ up) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < t.n_head; i += gridDim.x * blockDim.x) {
+    const uint32_t x = t.head[i];
+    uint64_t lo = t.off[i], hi = t.off[i + 1];
+    while (lo < hi) {
+      const uint64_t mid = (lo + hi) >> 1;
+      if (t.vals[mid] <= x) lo = mid + 1; else hi = mid;
+    }
+    up[i] = (uint32_t)lo;
+  }
+}
+
 // key = head position of b (sentinel for rows the plans never read),
 // payload = the row; rows arrive in row order, so a stable sort on the key
 // alone leaves each b's rows in row order
@@ -677,7 +690,8 @@ __global__ void rev_key_kernel(TrieView t, const uint32_t* __restrict__ seg, int
     const int32_t hb = t.head_index[b];
     uint64_t lo, hi;
     rev_range(dir, e, t.off[ha], t.off[ha + 1], lo, hi);
-    const bool keep = hb >= 0 && hi > lo && (dir != DIR_SYM || a < b);
+    // on a symmetric relation a row matters only while N(b) has elements above b
+    const bool keep = hb >= 0 && hi > lo && (dir != DIR_SYM || (a < b && t.up[hb] < t.off[hb + 1]));
     keys[e] = keep ? (uint32_t)hb : sentinel;
     rowid[e] = (uint32_t)e;
     if (keep) atomicAdd(&cnt[hb], 1u);
@@ -713,6 +727,7 @@ void trie_build_reverse(eh_context* ctx, eh_trie* t) {
   cudaStream_t s = ctx->stream;
   const int grid = num_sms() * 8;
   t->dir = DIR_GENERAL;
+  t->up.release();
   t->rev_entries = 0;
   t->rev_pairs = 0;
   t->rev_off.alloc(t->n_head + 1, s);
@@ -751,6 +766,11 @@ void trie_build_reverse(eh_context* ctx, eh_trie* t) {
     t->dir = (c[2] == 0 && c[3] == 0) ? DIR_SYM : DIR_GENERAL;
   }
   ph_dir.end();
+  if (t->dir == DIR_SYM) {
+    t->up.alloc(t->n_head, s);
+    up_kernel<<<grid, 256, 0, s>>>(t->view(), t->up.p);
+    EH_CHECK_LAUNCH();
+  }
   // group the rows a->b the plans read by b (stable: row order within b);
   // head positions are below 2^32, so 32-bit keys on bits_for(n_head) bits
   const int bh = bits_for(t->n_head);
