@@ -1,0 +1,469 @@
+// Row hit masks: which candidates of every row matched, as bits.
+//
+// For a row a->b the triangle plan intersects N(b) with the candidates of
+// N(a) beyond b.  hits_kernel runs exactly those intersections, on the same
+// work items and staged sets as triangle_kernel, and keeps every result as a
+// bit at the candidate's position in N(a) instead of only counting it.  The
+// rows of one a are then the adjacency matrix of its neighbourhood, and the
+// plans that read more than the count work on that matrix alone:
+//   4-clique     sum over set bits (i, j) of popc(row_i & row_j)
+//   annotation   (symmetric relation) row sums and column sums
+//   rows         the set bits in order are the sorted triangles of a
+//
+// Positions.  part(a) is what the plans read of N(a) (staged_range), d its
+// length.  On a relation that goes up, position i is element i of the part; on
+// one that goes down, element d - 1 - i; so a row at position i always has the
+// candidates i + 1 .. d - 1.  (A general relation has no such order: its
+// candidates are the whole N(a), and the plans run without masks.)
+// Layout.  W = ceil(d / 32) words per row.  Rows come in blocks of 32; block q
+// holds the words q .. W - 1 of its rows, word-major: word k of the 32 rows is
+// one 128-byte line, so a warp whose lanes hold 32 rows reads one line per
+// word.  The last block stores only its d - 32 (W - 1) rows.
+#pragma once
+
+#include "eh_internal.cuh"
+
+namespace eh {
+
+struct HitsView {
+  uint32_t* mask;         // words of every head entry of every graph, zero where nothing matched
+  const uint32_t* moff;   // [heads] first word of a head entry
+  const uint32_t* upre;   // [heads + 1] first work unit of a head entry (second pass); null: none
+  const uint32_t* gstart; // [graphs + 1] first head entry of a graph
+  uint32_t n_graphs;
+  uint32_t heads;         // of all graphs
+};
+
+__host__ __device__ __forceinline__ uint64_t hits_words(uint64_t d) {
+  if (d < 2) return 0;
+  const uint64_t W = (d + 31) / 32;
+  return 32 * (W * (W + 1) / 2 - 1) + (d - 32 * (W - 1));
+}
+// words before row block q; rows of a block (the stride between two words of a row)
+__device__ __forceinline__ uint32_t hits_block(uint32_t q, uint32_t W) { return 32 * (q * W - q * (q - 1) / 2); }
+__device__ __forceinline__ uint32_t hits_stride(uint32_t q, uint32_t W, uint32_t d) {
+  return q + 1 < W ? 32u : d - 32u * q;
+}
+
+// One batch of 32 rows at a time, a row per lane; a row of at least 32
+// candidates runs across the warp, a word per trip and four trips' candidates
+// loaded before any is probed; shorter ones are flattened over the lanes, and
+// each lane cuts its row's bits out of the trip's ballot (a short row's
+// candidates lie in at most two words).  Only non-zero words are written.
+template <int P>
+__device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, const RevView& r, uint32_t kb,
+                                         uint32_t ke, const uint32_t* __restrict__ moff,
+                                         uint32_t* __restrict__ mask, uint32_t shard_index, uint32_t shard_count) {
+  const uint32_t lane = lane_id();
+  const bool down = r.dir == DIR_DOWN;
+  for (uint32_t k0 = kb; k0 < ke; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    uint32_t len = 0, fe = 0;           // candidates; the element of the first one
+    uint32_t i = 0, base = 0, rs = 0;   // row position, first mask word, word stride
+    if (k < ke) {
+      const uint32_t lo = __ldg(r.rev_lo + k), hi = __ldg(r.rev_hi + k), src = __ldg(r.rev_src + k);
+      // shards split the heads a: each rank builds and reads the matrices of its own
+      if (shard_count == 1 || src % shard_count == shard_index) {
+        const StagedRange pr = staged_range(t, src);
+        const uint32_t d = pr.len, W = (d + 31) >> 5;
+        len = hi - lo;
+        i = d - 1 - len;
+        fe = down ? hi - 1 : lo;
+        const uint32_t q = i >> 5;
+        base = __ldg(moff + src) + hits_block(q, W) + (i & 31);
+        rs = hits_stride(q, W, d);
+      }
+    }
+    uint32_t rows = __ballot_sync(kFull, len >= 32);
+    const uint32_t rlen = len;
+    if (len >= 32) len = 0;
+    while (rows) {
+      const int j = __ffs(rows) - 1;
+      rows &= rows - 1;
+      const uint32_t ln = __shfl_sync(kFull, rlen, j), fj = __shfl_sync(kFull, fe, j);
+      const uint32_t ij = __shfl_sync(kFull, i, j) & 31u;
+      const uint32_t bj = __shfl_sync(kFull, base, j), rj = __shfl_sync(kFull, rs, j);
+      // candidate c of the row is bit (ij + 1 + c) & 31 of its word (ij + 1 + c) >> 5
+      const uint32_t skip = ij + 1, end = skip + ln;  // bit positions from the row's first word
+      for (uint32_t w0 = 0; 32 * w0 < end; w0 += 32) {
+        uint32_t mine = 0;
+        for (uint32_t u0 = 0; u0 < 32 && 32 * (w0 + u0) < end; u0 += 4) {
+          uint32_t v[4];
+          bool in[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const uint32_t p = 32 * (w0 + u0 + u) + lane;
+            in[u] = p >= skip && p < end;
+            v[u] = in[u] ? __ldg(t.vals + (down ? fj - (p - skip) : fj + (p - skip))) : 0u;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const uint32_t b = __ballot_sync(kFull, in[u] && probe<P>(st, v[u]));
+            if (lane == u0 + u) mine = b;
+          }
+        }
+        if (mine) mask[bj + (w0 + lane) * rj] = mine;
+      }
+    }
+    const uint32_t incl = warp_incl_scan(len);
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    const uint32_t excl = incl - len;
+    uint32_t acc = 0;  // the lane's short row, bit c = candidate c
+    for (uint32_t p = 0; p < total; p += 32 * kShortUnroll) {
+      uint32_t w[kShortUnroll];
+#pragma unroll
+      for (int u = 0; u < kShortUnroll; u++) {
+        const uint32_t q = p + 32 * u + lane;
+        const uint32_t j = owner_lane(incl, q);
+        const uint32_t fj = __shfl_sync(kFull, fe, j), exj = __shfl_sync(kFull, excl, j);
+        w[u] = q < total ? __ldg(t.vals + (down ? fj - (q - exj) : fj + (q - exj))) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < kShortUnroll; u++) {
+        const uint32_t p0 = p + 32 * u;
+        const uint32_t ball = __ballot_sync(kFull, p0 + lane < total && probe<P>(st, w[u]));
+        const uint32_t s = max(excl, p0), e = min(incl, p0 + 32);
+        if (s < e) {  // the row's candidates s - excl .. e - excl - 1 are bits s - p0 .. of the ballot
+          const uint32_t bits = (ball >> (s - p0)) & (0xffffffffu >> (32 - (e - s)));
+          acc |= bits << (s - excl);
+        }
+      }
+    }
+    if (acc) {
+      const uint64_t m = (uint64_t)acc << ((i & 31) + 1);
+      if ((uint32_t)m) mask[base] = (uint32_t)m;
+      if ((uint32_t)(m >> 32)) mask[base + rs] = (uint32_t)(m >> 32);
+    }
+  }
+}
+
+__global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const TrieView* __restrict__ views, const RevView* __restrict__ revs,
+                                                 const Item* __restrict__ items, uint32_t n_items, int cap_words,
+                                                 unsigned int* __restrict__ queue, HitsView hv, float* records,
+                                                 uint32_t shard_index, uint32_t shard_count) {
+  extern __shared__ uint32_t smem[];
+  const uint32_t lane = lane_id();
+  uint32_t* sm = smem + (size_t)(threadIdx.x >> 5) * cap_words;
+  for (;;) {
+    uint32_t it = 0;
+    if (lane == 0) it = atomicAdd(queue, 1u);
+    it = __shfl_sync(kFull, it, 0);
+    if (it >= n_items) break;
+    const Item item = items[it];
+    const TrieView t = views[item.g];
+    const RevView r = revs[item.g];
+    const uint32_t* moff = hv.moff + hv.gstart[item.g];
+    long long t0 = 0;
+    if (records && lane == 0) t0 = clock64();
+    Staged st;
+    const int mode = stage_set(t, item.hb, sm, cap_words, st, true);
+    switch (mode) {
+      case P_SBITS:
+        hit_rows<P_SBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        break;
+      case P_GBITS:
+        hit_rows<P_GBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        break;
+      case P_SLIST:
+        hit_rows<P_SLIST>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        break;
+      case P_GLIST:
+        hit_rows<P_GLIST>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        break;
+      case P_ZBITS:
+        hit_rows<P_ZBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        break;
+      default:
+        hit_rows<P_GBLOCK>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        break;
+    }
+    __syncwarp();  // the staged region is reused by the next item
+    if (records && lane == 0)
+      write_record(records + 8 * (size_t)it, t, r, item, mode, (float)(clock64() - t0));
+  }
+}
+
+// graph of global head entry gh
+__device__ __forceinline__ uint32_t hits_graph(const HitsView& hv, uint32_t gh) {
+  uint32_t lo = 0, hi = hv.n_graphs;  // first graph starting above gh
+  while (lo + 1 < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (hv.gstart[mid] <= gh) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+// global head entry of unit u: the last one whose units start at or before u
+__device__ __forceinline__ uint32_t hits_unit_head(const HitsView& hv, uint32_t u) {
+  uint32_t lo = 0, hi = hv.heads;  // first entry with upre > u, less one
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(hv.upre + mid) <= u) lo = mid + 1; else hi = mid;
+  }
+  return lo - 1;
+}
+
+// Work units of a head entry in the second pass.
+// 4-clique: parts of d > 32 elements, in (word, word, row) steps of which a
+// unit holds about kCliqueSteps; smaller parts are one row per lane and
+// have no units.  Annotation: one unit per word column.
+enum { HITS_CLIQUE = 0, HITS_ANNOT = 1, HITS_ROWS = 2 };
+constexpr uint64_t kCliqueSteps = 4096;
+__device__ __forceinline__ uint64_t hits_units(uint64_t d, int use) {
+  const uint64_t W = (d + 31) / 32;
+  if (use == HITS_ANNOT) return d >= 2 ? W : 0;
+  if (use == HITS_ROWS || d <= 32) return 0;
+  const uint64_t steps = 32 * (W * (W + 1) * (W + 2) / 6);
+  return min(d, (steps + kCliqueSteps - 1) / kCliqueSteps);
+}
+
+// mask words and second-pass units of every head entry; sums over all of them
+__global__ void hits_size_kernel(TrieView t, int use, uint32_t* __restrict__ words, uint32_t* __restrict__ units,
+                                 unsigned long long* __restrict__ sums) {
+  unsigned long long sw = 0, su = 0;
+  for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < t.n_head; a += gridDim.x * blockDim.x) {
+    const uint64_t d = staged_range(t, a).len;
+    const uint64_t w = hits_words(d), u = hits_units(d, use);
+    words[a] = (uint32_t)w;  // meaningful only while the sum stays below 2^32, which the host checks
+    units[a] = (uint32_t)u;
+    sw += w;
+    su += u;
+  }
+  sw = warp_sum(sw);
+  su = warp_sum(su);
+  if (lane_id() == 0) {
+    if (sw) atomicAdd(sums, sw);
+    if (su) atomicAdd(sums + 1, su);
+  }
+}
+
+// 4-cliques whose lowest vertex (highest, on a relation that goes down) has a
+// part of 3 to 32 elements: the matrix is one word per row, a row per lane.
+// Warps take 32 head entries at a time.
+__global__ void __launch_bounds__(256) clique_small_kernel(const TrieView* __restrict__ views, HitsView hv,
+                                                           unsigned long long* __restrict__ total) {
+  const uint32_t lane = lane_id();
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  unsigned long long acc = 0;
+  uint32_t cur_g = 0;
+  for (uint64_t h0 = 32ull * warp; h0 < hv.heads; h0 += 32ull * nwarps) {
+    const uint32_t gh = (uint32_t)h0 + lane;
+    uint32_t d = 0, mo = 0, g = 0;
+    if (gh < hv.heads) {
+      g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0;
+      const TrieView& t = views[g];
+      d = staged_range(t, gh - hv.gstart[g]).len;
+      mo = __ldg(hv.moff + gh);
+    }
+    uint32_t todo = __ballot_sync(kFull, d >= 3 && d <= 32);
+    while (todo) {
+      const int j = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint32_t dj = __shfl_sync(kFull, d, j), mj = __shfl_sync(kFull, mo, j), gj = __shfl_sync(kFull, g, j);
+      const uint32_t row = lane < dj ? __ldg(hv.mask + mj + lane) : 0u;
+      uint32_t set = __ballot_sync(kFull, row != 0);
+      if (gj != cur_g) {
+        acc = warp_sum(acc);
+        if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
+        acc = 0;
+        cur_g = gj;
+      }
+      uint32_t c = 0;
+      while (set) {
+        const int b = __ffs(set) - 1;
+        set &= set - 1;
+        const uint32_t rb = __shfl_sync(kFull, row, b);
+        if ((row >> b) & 1u) c += __popc(row & rb);
+      }
+      acc += c;
+    }
+  }
+  acc = warp_sum(acc);
+  if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
+}
+
+// 4-cliques of the larger parts.  A unit is the rows i = s, s + n, ... of one
+// matrix.  For a row i and a block q of 32 later positions, the lanes whose
+// bit of row i is set hold one row j each and AND it with row i word by word
+// (row i's word is the same for all lanes, the rows j are one 128-byte line
+// per word).  A warp takes four units in a row: they are mostly of one
+// matrix, which its L1 then holds.
+__global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restrict__ views, HitsView hv,
+                                                         uint32_t n_units, unsigned int* __restrict__ queue,
+                                                         unsigned long long* __restrict__ total) {
+  const uint32_t lane = lane_id();
+  unsigned long long acc = 0;
+  uint32_t cur_g = 0;
+  for (;;) {
+    uint32_t u0 = 0;
+    if (lane == 0) u0 = atomicAdd(queue, 4u);
+    u0 = __shfl_sync(kFull, u0, 0);
+    if (u0 >= n_units) break;
+    const uint32_t u1 = min(u0 + 4, n_units);
+    uint32_t gh = hits_unit_head(hv, u0);
+    for (uint32_t u = u0; u < u1; u++) {
+      while (__ldg(hv.upre + gh + 1) <= u) gh++;  // entries without units have equal bounds
+      const uint32_t g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0;
+      if (g != cur_g) {
+        acc = warp_sum(acc);
+        if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
+        acc = 0;
+        cur_g = g;
+      }
+      const uint32_t s = u - __ldg(hv.upre + gh), n = __ldg(hv.upre + gh + 1) - __ldg(hv.upre + gh);
+      const uint32_t d = staged_range(views[g], gh - hv.gstart[g]).len, W = (d + 31) >> 5;
+      const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
+      for (uint32_t i = s; i < d; i += n) {
+        const uint32_t qi = i >> 5, ri = hits_stride(qi, W, d);
+        const uint32_t* row = m + hits_block(qi, W) + (i & 31);
+        uint32_t c = 0;
+        for (uint32_t q = qi; q < W; q++) {
+          const uint32_t mine = __ldg(row + (q - qi) * ri);
+          if (!mine) continue;
+          const bool on = (mine >> lane) & 1u;
+          const uint32_t rq = hits_stride(q, W, d);
+          const uint32_t* rows = m + hits_block(q, W) + lane;  // read only where a bit, so a row, exists
+          for (uint32_t k = q; k < W; k += 4) {
+            uint32_t x[4], y[4];
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+              const bool in = k + v < W;
+              x[v] = in ? __ldg(row + (k + v - qi) * ri) : 0u;
+              y[v] = in && on ? __ldg(rows + (k + v - q) * rq) : 0u;
+            }
+#pragma unroll
+            for (int v = 0; v < 4; v++) c += __popc(x[v] & y[v]);
+          }
+        }
+        acc += c;
+      }
+    }
+  }
+  acc = warp_sum(acc);
+  if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
+}
+
+// 32 x 32 bits, row r in lane r's word -> column c in lane c's word
+__device__ __forceinline__ uint32_t transpose32(uint32_t x) {
+  const uint32_t lane = lane_id();
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const uint32_t y = __shfl_xor_sync(kFull, x, s);
+    x = (lane & s) ? ((x & ~m) | ((y >> s) & m)) : ((x & m) | ((y & m) << s));
+    m ^= m << (s >> 1);
+  }
+  return x;
+}
+
+// Annotation of a symmetric relation: every undirected triangle a < b < w
+// found once adds 2 (its two orderings) to T of each of its three vertices.
+// Unit k of a part is its word column k: the column sums of block column k
+// (how often position j is the third vertex) and the row sums of block k (how
+// often it is the second), one addition to T per element, and the row sums
+// once more to T[a].
+__global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv, uint32_t n_units,
+                                                         unsigned long long* __restrict__ T) {
+  const uint32_t lane = lane_id();
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  // consecutive units per warp: one search for the first head entry
+  const uint32_t per = (n_units + nwarps - 1) / nwarps;
+  const uint64_t b0 = (uint64_t)per * warp;
+  if (b0 >= n_units) return;
+  const uint32_t u0 = (uint32_t)b0, u1 = (uint32_t)min(b0 + per, (uint64_t)n_units);
+  uint32_t a = hits_unit_head(hv, u0);
+  for (uint32_t u = u0; u < u1; u++) {
+    while (__ldg(hv.upre + a + 1) <= u) a++;
+    const uint32_t k = u - __ldg(hv.upre + a);
+    const StagedRange pr = staged_range(t, a);
+    const uint32_t d = pr.len, W = (d + 31) >> 5;
+    const uint32_t* m = hv.mask + __ldg(hv.moff + a);
+    uint32_t col = 0, row = 0;
+    for (uint32_t q = 0; q <= k; q++) {
+      const uint32_t rq = hits_stride(q, W, d);
+      const uint32_t x = lane < rq ? __ldg(m + hits_block(q, W) + (k - q) * rq + lane) : 0u;
+      if (__any_sync(kFull, x != 0)) col += __popc(transpose32(x));
+    }
+    const uint32_t rk = hits_stride(k, W, d);
+    if (lane < rk)
+      for (uint32_t w = k; w < W; w++) row += __popc(__ldg(m + hits_block(k, W) + (w - k) * rk + lane));
+    if (col + row) {  // so the position is below d
+      const int32_t h = __ldg(t.head_index + __ldg(t.vals + pr.s0 + 32 * k + lane));
+      atomicAdd(T + h, 2ull * (col + row));
+    }
+    const uint32_t all = warp_sum(row);
+    if (lane == 0 && all) atomicAdd(T + a, 2ull * all);
+  }
+}
+
+// rows: triangles per relation row e = (a, position i); a warp per head entry
+// would starve on short parts, so a thread per row
+__device__ __forceinline__ uint32_t hits_position(int dir, const StagedRange& pr, uint64_t e) {
+  return dir == DIR_DOWN ? pr.len - 1 - (uint32_t)(e - pr.s0) : (uint32_t)(e - pr.s0);
+}
+__global__ void hits_row_count_kernel(TrieView t, int dir, HitsView hv, const uint32_t* __restrict__ seg,
+                                      uint64_t* __restrict__ cnt) {
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < t.rows; e += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t a = seg[e];
+    const StagedRange pr = staged_range(t, a);
+    uint32_t c = 0;
+    if (pr.len >= 2) {
+      const uint32_t d = pr.len, W = (d + 31) >> 5, i = hits_position(dir, pr, e), q = i >> 5;
+      const uint32_t rs = hits_stride(q, W, d);
+      const uint32_t* row = hv.mask + __ldg(hv.moff + a) + hits_block(q, W) + (i & 31);
+      for (uint32_t k = 0; k < W - q; k++) c += __popc(__ldg(row + k * rs));
+    }
+    cnt[e] = c;
+  }
+}
+// a warp per relation row with triangles: word by word, a lane per bit; the
+// relation's rows and the elements of a part are in ascending order, so the
+// triangles come out sorted by (a, b, c)
+__global__ void __launch_bounds__(256) hits_row_write_kernel(TrieView t, int dir, HitsView hv,
+                                                             const uint32_t* __restrict__ seg,
+                                                             const uint64_t* __restrict__ pos, uint64_t total,
+                                                             uint32_t* __restrict__ oa, uint32_t* __restrict__ ob,
+                                                             uint32_t* __restrict__ oc) {
+  const uint32_t lane = lane_id();
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint64_t e0 = 32ull * warp; e0 < t.rows; e0 += 32ull * nwarps) {
+    const uint64_t el = e0 + lane;
+    uint64_t p = 0, n = 0;
+    if (el < t.rows) {
+      p = pos[el];
+      n = (el + 1 < t.rows ? pos[el + 1] : total) - p;
+    }
+    uint32_t todo = __ballot_sync(kFull, n != 0);
+    while (todo) {
+      const int l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint64_t e = e0 + l;
+      uint64_t out = __shfl_sync(kFull, p, l);
+      const uint32_t a = __ldg(seg + e);
+      const StagedRange pr = staged_range(t, a);
+      const uint32_t d = pr.len, W = (d + 31) >> 5, i = hits_position(dir, pr, e), q = i >> 5;
+      const uint32_t rs = hits_stride(q, W, d);
+      const uint32_t* row = hv.mask + __ldg(hv.moff + a) + hits_block(q, W) + (i & 31);
+      const uint32_t va = __ldg(t.head + a), vb = __ldg(t.vals + e);
+      for (uint32_t kk = 0; kk < W - q; kk++) {
+        // ascending elements: positions descend on a relation that goes down
+        const uint32_t k = dir == DIR_DOWN ? W - q - 1 - kk : kk;
+        uint32_t x = __ldg(row + k * rs);
+        if (dir == DIR_DOWN) x = __brev(x);
+        if ((x >> lane) & 1u) {
+          const uint32_t bit = dir == DIR_DOWN ? 31 - lane : lane;
+          const uint32_t j = 32 * (q + k) + bit;
+          const uint64_t o = out + __popc(x & lanemask_lt());
+          oa[o] = va;
+          ob[o] = vb;
+          oc[o] = __ldg(t.vals + pr.s0 + (dir == DIR_DOWN ? d - 1 - j : j));
+        }
+        out += __popc(x);
+      }
+    }
+  }
+}
+
+}  // namespace eh

@@ -867,6 +867,23 @@ __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_
   return P_GLIST;
 }
 
+// One timing record of an item (eh_timing_records): warp-cycles spent on it
+// beside the staged set's features.
+__device__ __forceinline__ void write_record(float* rec, const TrieView& t, const RevView& r, const Item& item,
+                                             int mode, float cycles) {
+  const uint64_t b0 = t.off[item.hb];
+  const uint32_t len = (uint32_t)(t.off[item.hb + 1] - b0);
+  const uint32_t first = t.vals[b0], last = t.vals[b0 + len - 1];
+  rec[0] = (float)len;
+  rec[1] = (float)(r.rev_wpre[item.ke] - r.rev_wpre[item.kb]);
+  rec[2] = (float)len / (float)(last - first + 1);
+  rec[3] = (float)(last - first);
+  rec[4] = (float)t.layout[item.hb];
+  rec[5] = (float)mode;
+  rec[6] = __uint_as_float(item.hb);  // set id, bit pattern
+  rec[7] = cycles;
+}
+
 // stage_set for a block item: every thread of the block copies, into the
 // block's whole shared region (the caller synchronises the block after).
 __device__ __forceinline__ int stage_set_block(const TrieView& t, uint32_t hb, uint32_t* sm, int cap_words,
@@ -1064,22 +1081,9 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict_
     acc += c;
     if (block_phase) __syncthreads();  // every warp is done with the staged set
     else __syncwarp();                 // the staged region is reused by the next item
-    if (out.records && (block_phase ? threadIdx.x == 0 : lane == 0)) {
-      const long long t1 = clock64();
-      const uint64_t b0 = t.off[item.hb];
-      const uint32_t len = (uint32_t)(t.off[item.hb + 1] - b0);
-      const uint64_t pairs = r.rev_wpre[item.ke] - r.rev_wpre[item.kb];
-      const uint32_t first = t.vals[b0], last = t.vals[b0 + len - 1];
-      float* rec = out.records + 8 * (size_t)it;
-      rec[0] = (float)len;
-      rec[1] = (float)pairs;
-      rec[2] = (float)len / (float)(last - first + 1);
-      rec[3] = (float)(last - first);
-      rec[4] = (float)t.layout[item.hb];
-      rec[5] = (float)mode;
-      rec[6] = __uint_as_float(item.hb);  // set id, bit pattern
-      rec[7] = (float)(t1 - t0) * (block_phase ? (float)nwarps : 1.f);  // warp-cycles
-    }
+    if (out.records && (block_phase ? threadIdx.x == 0 : lane == 0))
+      write_record(out.records + 8 * (size_t)it, t, r, item, mode,
+                   (float)(clock64() - t0) * (block_phase ? (float)nwarps : 1.f));  // warp-cycles
   }
   if (lane == 0 && cur_g != 0xffffffffu && acc) atomicAdd(out.total + cur_g, acc);
   if (kMode == MODE_ANNOT) {  // every warp leaves the loop above; then flush the block's hot counts
@@ -1259,24 +1263,17 @@ __global__ void EH_TRI_LAUNCH_BOUNDS clique4_kernel(const TrieView* __restrict__
     }
     acc += warp_sum(c);
     __syncwarp();
-    if (out.records && lane == 0) {  // the same record as the triangle kernel's
-      const long long t1 = clock64();
-      const uint64_t b0 = t.off[item.hb];
-      const uint32_t len = (uint32_t)(t.off[item.hb + 1] - b0);
-      const uint32_t first = t.vals[b0], last = t.vals[b0 + len - 1];
-      float* rec = out.records + 8 * (size_t)it;
-      rec[0] = (float)len;
-      rec[1] = (float)(r.rev_wpre[item.ke] - r.rev_wpre[item.kb]);
-      rec[2] = (float)len / (float)(last - first + 1);
-      rec[3] = (float)(last - first);
-      rec[4] = (float)t.layout[item.hb];
-      rec[5] = (float)mode;
-      rec[6] = __uint_as_float(item.hb);
-      rec[7] = (float)(t1 - t0);
-    }
+    if (out.records && lane == 0)
+      write_record(out.records + 8 * (size_t)it, t, r, item, mode, (float)(clock64() - t0));
   }
   if (lane == 0 && cur_g != 0xffffffffu && acc) atomicAdd(out.total + cur_g, acc);
 }
+
+}  // namespace eh
+
+#include "eh_hits.cuh"
+
+namespace eh {
 
 // ------------------------------------------------- lollipop / barbell roots
 constexpr uint64_t kRootBig = 32768;  // barbell root: larger sets get grid-wide passes
@@ -1364,6 +1361,70 @@ struct Launch {
   float kernel_ms = 0;
 };
 
+// The hit masks of a prepared launch (eh_hits.cuh): where every head entry's
+// matrix and its second-pass units start, and the mask words.
+struct Hits {
+  bool on = false;
+  int use = 0;
+  uint64_t words = 0;
+  uint32_t units = 0, heads = 0, n = 0;
+  DevBuf<uint32_t> mask, moff, upre, gstart;
+  HitsView view() const { return HitsView{mask.p, moff.p, upre.p, gstart.p, n, heads}; }
+};
+// Masks hold a bit per candidate, so a relation in degree order needs far less
+// than its trie (R-MAT-22: 1.2 GB); past this many words (8 GB: a set of 300 K
+// elements read whole) the plans run without them.
+constexpr uint64_t kMaxHitWords = 1ull << 31;
+
+// false: the relation is general, or its masks are too large
+static bool plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int use, Hits& H) {
+  cudaStream_t s = ctx->stream;
+  uint64_t heads = 0;
+  std::vector<uint32_t> gstart(n + 1, 0);
+  for (uint32_t g = 0; g < n; g++) {
+    const int dir = tries[g]->dir;
+    if (dir == DIR_GENERAL || (use == HITS_ANNOT && dir != DIR_SYM) || (use == HITS_ROWS && dir == DIR_SYM))
+      return false;
+    heads += tries[g]->n_head;
+    if (heads >= (1ull << 32) - 1) return false;
+    gstart[g + 1] = (uint32_t)heads;
+  }
+  if (!heads) return false;
+  H.use = use;
+  H.n = n;
+  H.heads = (uint32_t)heads;
+  H.moff.alloc(heads, s);
+  H.upre.alloc(heads + 1, s);
+  H.gstart.alloc(n + 1, s);
+  DevBuf<unsigned long long> sums(2, s);
+  EH_CUDA(cudaMemsetAsync(sums.p, 0, 16, s));
+  EH_CUDA(cudaMemsetAsync(H.upre.p + heads, 0, 4, s));
+  EH_CUDA(cudaMemcpyAsync(H.gstart.p, gstart.data(), (n + 1) * 4, cudaMemcpyHostToDevice, s));
+  for (uint32_t g = 0; g < n; g++) {
+    const uint32_t nh = tries[g]->n_head;
+    if (!nh) continue;
+    const int grid = std::min(num_sms() * 4, ceil_div(nh, 256));
+    hits_size_kernel<<<grid, 256, 0, s>>>(tries[g]->view(), use, H.moff.p + gstart[g], H.upre.p + gstart[g], sums.p);
+    EH_CHECK_LAUNCH();
+  }
+  unsigned long long h[2];
+  EH_CUDA(cudaMemcpyAsync(h, sums.p, 16, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaStreamSynchronize(s));
+  if (h[0] > kMaxHitWords || h[1] >= kMaxHitWords) return false;
+  exclusive_scan<uint32_t>(H.moff.p, H.moff.p, heads, nullptr, s);
+  exclusive_scan<uint32_t>(H.upre.p, H.upre.p, heads + 1, nullptr, s);
+  try {
+    H.mask.alloc(h[0] ? h[0] : 1, s);
+  } catch (const Error& e) {
+    if (e.code != EH_ERR_OOM) throw;
+    return false;
+  }
+  H.words = h[0];
+  H.units = (uint32_t)h[1];
+  H.on = true;
+  return true;
+}
+
 // Runs the intersection kernel of `query` over the concatenated plans of
 // n graphs; results accumulate into d_total[g].
 // Everything a launch needs on the device, built once: the work plans of
@@ -1373,6 +1434,7 @@ struct Prepared {
   uint32_t n_items = 0;
   uint32_t n_bitems = 0;  // items[0, n_bitems) are block items
   uint64_t pairs = 0;
+  TrieView view0{};  // the first trie's view
   DevBuf<TrieView> dv;
   DevBuf<RevView> dr;
   DevBuf<unsigned int> q;
@@ -1385,6 +1447,7 @@ struct Prepared {
   const uint32_t* sel = nullptr;  // 4-clique selection bitmap (QueryOut::sel)
   DevBuf<uint32_t> gs;            // 4-clique global S buffers (ExecParams::s_cap)
   int32_t hot[kHot] = {-1, -1, -1, -1};  // annotation: largest sets (QueryOut::hot)
+  Hits hits;                      // the plan runs on hit masks
 };
 
 // head entry with the largest set, excluding `ex` (-1 unused): max over
@@ -1419,37 +1482,58 @@ static void hot_sets(eh_context* ctx, const eh_trie* t, int32_t* hot) {
   }
 }
 
+// 4-clique without hit masks: the warp's shared region holds the staged N(b) and S
+// (S <= the largest set) while that stays within 96 KB a block; beyond, S
+// moves to per-warp global buffers (L2-resident in practice) and the whole
+// region stages N(b).
+static void size_clique_staging(ExecParams& ep, uint32_t max_set) {
+  const int need = 2 * ((int)max_set + 1);
+  if ((size_t)std::max(ep.smem_words, need) * 4 * ep.warps <= 96 * 1024) {
+    if (ep.smem_words < need) ep.smem_words = (need + 1) & ~1;
+  } else {
+    ep.s_cap = max_set + 1;
+  }
+}
+
+// hits_use: run the plan on hit masks when they can be had (HITS_*; -1: never)
 static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query, ExecParams ep, bool annot,
-                    Prepared& P, bool block_items = false) {
+                    Prepared& P, bool block_items = false, int hits_use = -1) {
   cudaStream_t s = ctx->stream;
   P.query = query;
   P.annot = annot;
+  const bool hits = hits_use >= 0 && plan_hits(ctx, tries, n, hits_use, P.hits);
+  if (query == EH_QUERY_CLIQUE4 && !hits) {
+    uint32_t mx = 0;
+    for (uint32_t g = 0; g < n; g++) mx = std::max(mx, tries[g]->info.max_set);
+    size_clique_staging(ep, mx);
+  }
   // the launch shape first: the plan's classes depend on the staging capacity
   // the annotated pass stages more of N(b) by default: its matched elements
   // then count in shared memory (measured on Chung-Lu 2^23: 2048 words per
   // warp 234 ms, 1024 245 ms)
-  if (annot && !ep.smem_given) ep.smem_words = 2 * kDefaultSmemWords;
+  if (annot && !hits && !ep.smem_given) ep.smem_words = 2 * kDefaultSmemWords;
   P.threads = 32 * ep.warps;
   P.smem = (size_t)ep.smem_words * 4 * ep.warps;
   const void* kfn;
-  if (query == EH_QUERY_CLIQUE4) kfn = (const void*)clique4_kernel;
+  if (hits) kfn = (const void*)hits_kernel;
+  else if (query == EH_QUERY_CLIQUE4) kfn = (const void*)clique4_kernel;
   else if (annot) kfn = (const void*)triangle_kernel<MODE_ANNOT>;
   else kfn = (const void*)triangle_kernel<MODE_COUNT>;
   {
     size_t room = dynamic_smem_room(kfn);
     // the materializing pass launches MODE_MAT with the same shape
-    if (!annot && query != EH_QUERY_CLIQUE4)
+    if (!hits && !annot && query != EH_QUERY_CLIQUE4)
       room = std::min(room, dynamic_smem_room((const void*)triangle_kernel<MODE_MAT>));
     if (P.smem > room) {
       // shrink the per-warp region to what a block may hold (a staged set
       // that no longer fits is probed in global memory instead)
-      EH_REQUIRE(query != EH_QUERY_CLIQUE4, EH_ERR_UNSUPPORTED, "4-clique staging exceeds shared memory");
+      EH_REQUIRE(hits || query != EH_QUERY_CLIQUE4, EH_ERR_UNSUPPORTED, "4-clique staging exceeds shared memory");
       ep.smem_words = (int)((room / 4 / ep.warps) & ~(size_t)1);
       P.smem = (size_t)ep.smem_words * 4 * ep.warps;
     }
   }
   // block items only for the plain triangle COUNT
-  const bool blocks = block_items && query == EH_QUERY_TRIANGLE && !annot && ep.warps > 1 && !ep.no_block_items;
+  const bool blocks = block_items && !hits && query == EH_QUERY_TRIANGLE && !annot && ep.warps > 1 && !ep.no_block_items;
   PlanShape shape{ep.chunk, nullptr, 0.0, (uint32_t)ep.smem_words,
                    blocks ? (uint32_t)ep.smem_words * (uint32_t)ep.warps : 0u, (uint32_t)ep.warps};
   std::vector<Plan> plans(n);
@@ -1491,18 +1575,20 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     if ((reinterpret_cast<uintptr_t>(hv[g].vals) | reinterpret_cast<uintptr_t>(hv[g].bs_words)) & 15u)
       throw Error{EH_ERR_UNSUPPORTED, "trie arrays are not 16-byte aligned"};
   }
+  P.view0 = hv[0];
   P.dv.alloc(n, s);
   P.dr.alloc(n, s);
   P.q.alloc(2, s);
   EH_CUDA(cudaMemcpyAsync(P.dv.p, hv.data(), n * sizeof(TrieView), cudaMemcpyHostToDevice, s));
   EH_CUDA(cudaMemcpyAsync(P.dr.p, hr.data(), n * sizeof(RevView), cudaMemcpyHostToDevice, s));
-  if (query == EH_QUERY_CLIQUE4) set_smem_attr(clique4_kernel, P.smem);
+  if (hits) set_smem_attr(hits_kernel, P.smem);
+  else if (query == EH_QUERY_CLIQUE4) set_smem_attr(clique4_kernel, P.smem);
   else if (annot) set_smem_attr(triangle_kernel<MODE_ANNOT>, P.smem);
   else set_smem_attr(triangle_kernel<MODE_COUNT>, P.smem);
   const int per_sm = blocks_per_sm(kfn, P.threads, P.smem);
   const uint64_t units = (uint64_t)total_b + (total_items - total_b + ep.warps - 1) / ep.warps;
   P.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * per_sm, units));
-  if (annot && n == 1 && tries[0]->dir == DIR_SYM) hot_sets(ctx, tries[0], P.hot);
+  if (annot && !hits && n == 1 && tries[0]->dir == DIR_SYM) hot_sets(ctx, tries[0], P.hot);
   if (query == EH_QUERY_CLIQUE4 && ep.s_cap) {
     // one S buffer per resident warp, at most 2 GiB in all
     const uint64_t per_block = (uint64_t)ep.warps * ep.s_cap * 4;
@@ -1521,6 +1607,27 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
   if (!P.n_items) return;
   EH_CUDA(cudaMemsetAsync(P.q.p, 0, 8, s));
   const ExecParams& ep = P.ep;
+  if (P.hits.on) {
+    const Hits& H = P.hits;
+    const HitsView hv = H.view();
+    EH_CUDA(cudaMemsetAsync(H.mask.p, 0, H.words * 4, s));
+    hits_kernel<<<P.grid, P.threads, P.smem, s>>>(P.dv.p, P.dr.p, P.items.p, P.n_items, ep.smem_words, P.q.p, hv,
+                                                  d_records, ep.shard_index, ep.shard_count);
+    EH_CHECK_LAUNCH();
+    if (H.use == HITS_CLIQUE) {
+      clique_small_kernel<<<std::min(num_sms() * 8, ceil_div(H.heads, 256)), 256, 0, s>>>(P.dv.p, hv, d_total);
+      EH_CHECK_LAUNCH();
+      if (H.units) {
+        clique_big_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 32)), 256, 0, s>>>(P.dv.p, hv, H.units,
+                                                                                        P.q.p + 1, d_total);
+        EH_CHECK_LAUNCH();
+      }
+    } else if (H.use == HITS_ANNOT && H.units) {
+      annot_hits_kernel<<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, d_annot);
+      EH_CHECK_LAUNCH();
+    }
+    return;
+  }
   QueryOut out{ep.shard_index, ep.shard_count, ep.long_row, d_total, d_annot, d_records, P.q.p};
   out.n_bitems = P.n_bitems;
   out.bqueue = P.q.p + 1;
@@ -1540,19 +1647,6 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
 }
 
 // Plan + run + wait; the intersection kernel is timed with events.
-// 4-clique: the warp's shared region holds the staged N(b) and S
-// (S <= the largest set) while that stays within 96 KB a block; beyond, S
-// moves to per-warp global buffers (L2-resident in practice) and the whole
-// region stages N(b).
-static void size_clique_staging(ExecParams& ep, uint32_t max_set) {
-  const int need = 2 * ((int)max_set + 1);
-  if ((size_t)std::max(ep.smem_words, need) * 4 * ep.warps <= 96 * 1024) {
-    if (ep.smem_words < need) ep.smem_words = (need + 1) & ~1;
-  } else {
-    ep.s_cap = max_set + 1;
-  }
-}
-
 static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query, ExecParams ep,
                         bool annot, unsigned long long* d_total, unsigned long long* d_annot, float* d_records,
                         uint32_t* n_items_out, uint64_t* pairs_out, const uint32_t* sel = nullptr) {
@@ -1561,7 +1655,9 @@ static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n
   Prepared P;
   {
     TracePhase ph("query.prepare", s);
-    prepare(ctx, tries, n, query, ep, annot, P, true);
+    // selections weight cliques by their members: they run without masks
+    const int use = sel ? -1 : query == EH_QUERY_CLIQUE4 ? HITS_CLIQUE : annot ? HITS_ANNOT : -1;
+    prepare(ctx, tries, n, query, ep, annot, P, true, use);
   }
   P.sel = sel;
   L.launches = P.plan_launches;
@@ -1574,7 +1670,7 @@ static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n
     launch(ctx, P, d_total, d_annot, d_records);
   }
   EH_CUDA(cudaEventRecord(ctx->ev2, s));
-  L.launches += 1;
+  L.launches += P.hits.on ? (P.hits.use == HITS_CLIQUE && P.hits.units ? 3 : 2) : 1;
   EH_CUDA(cudaEventSynchronize(ctx->ev2));
   EH_CUDA(cudaEventElapsedTime(&L.kernel_ms, ctx->ev1, ctx->ev2));
   return L;
@@ -1724,11 +1820,6 @@ void query_count_batched(eh_context* ctx, const eh_trie* const* tries, uint32_t 
     EH_REQUIRE(tries[g]->ctx == ctx, EH_ERR_INVALID, "trie belongs to another context");
   }
   ExecParams ep = exec_params(cfg);
-  if (query == EH_QUERY_CLIQUE4) {
-    uint32_t mx = 0;
-    for (uint32_t g = 0; g < n; g++) mx = std::max(mx, tries[g]->info.max_set);
-    size_clique_staging(ep, mx);
-  }
   TracePhase ph_all("query.total", s);
   EH_CUDA(cudaEventRecord(ctx->ev0, s));
   DevBuf<unsigned long long> total(n, s);
@@ -1880,9 +1971,6 @@ void query_count_select(eh_context* ctx, const eh_trie* t, int query, uint32_t v
   ExecParams ep = exec_params(cfg);
   EH_REQUIRE(ep.shard_count == 1, EH_ERR_UNSUPPORTED, "selection plans run unsharded");
   const bool clique = query == EH_QUERY_CLIQUE4_SEL;
-  if (clique) {
-    size_clique_staging(ep, t->info.max_set);
-  }
   EH_CUDA(cudaEventRecord(ctx->ev0, s));
   DevBuf<unsigned long long> sums(4, s);  // partner sum, N(v) sum, partners, plan total
   EH_CUDA(cudaMemsetAsync(sums.p, 0, 32, s));
@@ -2029,6 +2117,47 @@ static void query_project_ab(eh_context* ctx, const eh_trie* t, uint32_t* ha, ui
   EH_CUDA(cudaStreamSynchronize(s));
 }
 
+// Oriented relations: the hit masks hold every triangle at its place in the
+// order (a, b, c), so the rows are counted per relation row, placed by a scan
+// and written in order; nothing is sorted.  false: no masks for this relation.
+static bool materialize_hits(eh_context* ctx, const eh_trie* t, const eh_exec_config* cfg, uint32_t* ha, uint32_t* hb,
+                             uint32_t* hc, uint64_t cap, uint64_t* n_rows) {
+  cudaStream_t s = ctx->stream;
+  ExecParams ep = exec_params(cfg);
+  ep.shard_index = 0;
+  ep.shard_count = 1;
+  Prepared P;
+  const eh_trie* ts[1] = {t};
+  prepare(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, false, P, false, HITS_ROWS);
+  if (!P.hits.on) return false;
+  *n_rows = 0;
+  if (!P.n_items) return true;
+  launch(ctx, P, nullptr, nullptr, nullptr);
+  DevBuf<uint32_t> seg(t->rows, s);
+  DevBuf<uint64_t> pos(t->rows, s), tot(1, s);
+  const int grid = num_sms() * 8;
+  seg_of_rows_kernel<<<grid, 256, 0, s>>>(t->off.p, t->n_head, seg.p);
+  hits_row_count_kernel<<<grid, 256, 0, s>>>(t->view(), t->dir, P.hits.view(), seg.p, pos.p);
+  EH_CHECK_LAUNCH();
+  exclusive_scan<uint64_t>(pos.p, pos.p, t->rows, tot.p, s);
+  uint64_t n = 0;
+  EH_CUDA(cudaMemcpyAsync(&n, tot.p, 8, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaStreamSynchronize(s));
+  *n_rows = n;
+  if (!n) return true;
+  EH_REQUIRE(cap >= n, EH_ERR_INVALID, "output columns hold fewer rows than the result");
+  EH_REQUIRE(n < (1ull << 32), EH_ERR_UNSUPPORTED, "materialized results hold fewer than 2^32 rows");
+  DevBuf<uint32_t> out(3 * n, s);
+  hits_row_write_kernel<<<grid, 256, 0, s>>>(t->view(), t->dir, P.hits.view(), seg.p, pos.p, n, out.p, out.p + n,
+                                             out.p + 2 * n);
+  EH_CHECK_LAUNCH();
+  EH_CUDA(cudaMemcpyAsync(ha, out.p, n * 4, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaMemcpyAsync(hb, out.p + n, n * 4, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaMemcpyAsync(hc, out.p + 2 * n, n * 4, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaStreamSynchronize(s));
+  return true;
+}
+
 void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_exec_config* cfg, int n_cols,
                        uint32_t* ha, uint32_t* hb, uint32_t* hc, uint64_t cap, uint64_t* n_rows) {
   cudaStream_t s = ctx->stream;
@@ -2039,6 +2168,7 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
     query_project_ab(ctx, t, ha, hb, cap, n_rows);
     return;
   }
+  if (ha && hb && hc && t->dir != DIR_SYM && materialize_hits(ctx, t, cfg, ha, hb, hc, cap, n_rows)) return;
   uint64_t n = 0;
   query_count(ctx, t, EH_QUERY_TRIANGLE, cfg, &n, nullptr);
   *n_rows = n;
@@ -2243,21 +2373,15 @@ eh_batch* batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n,
   EH_REQUIRE(query == EH_QUERY_TRIANGLE || query == EH_QUERY_CLIQUE4, EH_ERR_UNSUPPORTED,
              "batches run the triangle or 4-clique plan");
   ExecParams ep = exec_params(cfg);
-  uint32_t mx = 0;
-  for (uint32_t g = 0; g < n; g++) {
+  for (uint32_t g = 0; g < n; g++)
     EH_REQUIRE(tries[g] && tries[g]->ctx == ctx, EH_ERR_INVALID, "null trie or trie of another context");
-    if (query == EH_QUERY_CLIQUE4) {
-      mx = std::max(mx, tries[g]->info.max_set);
-    }
-  }
-  if (query == EH_QUERY_CLIQUE4) size_clique_staging(ep, mx);
   auto* b = new eh_batch();
   try {
     b->ctx = ctx;
     b->n = n;
     b->query = query;
     for (uint32_t g = 0; g < n; g++) b->dirs.push_back(tries[g]->dir);
-    prepare(ctx, tries, n, query, ep, false, b->P, true);
+    prepare(ctx, tries, n, query, ep, false, b->P, true, query == EH_QUERY_CLIQUE4 ? HITS_CLIQUE : -1);
     b->total.alloc(n, s);
     EH_CUDA(cudaMallocHost((void**)&b->host, n * sizeof(unsigned long long)));
     EH_CUDA(cudaStreamSynchronize(s));
