@@ -18,7 +18,8 @@
 // Layout.  W = ceil(d / 32) words per row.  Rows come in blocks of 32; block q
 // holds the words q .. W - 1 of its rows, word-major: word k of the 32 rows is
 // one 128-byte line, so a warp whose lanes hold 32 rows reads one line per
-// word.  The last block stores only its d - 32 (W - 1) rows.
+// word.  The last block stores its d - 32 (W - 1) rows, rounded up to a multiple
+// of 8: eight rows' words are always two 16-byte loads.
 #pragma once
 
 #include "eh_internal.cuh"
@@ -37,29 +38,55 @@ struct HitsView {
 __host__ __device__ __forceinline__ uint64_t hits_words(uint64_t d) {
   if (d < 2) return 0;
   const uint64_t W = (d + 31) / 32;
-  return 32 * (W * (W + 1) / 2 - 1) + (d - 32 * (W - 1));
+  return 32 * (W * (W + 1) / 2 - 1) + ((d - 32 * (W - 1) + 7) & ~7ull);
 }
 // words before row block q; rows of a block (the stride between two words of a row)
 __device__ __forceinline__ uint32_t hits_block(uint32_t q, uint32_t W) { return 32 * (q * W - q * (q - 1) / 2); }
 __device__ __forceinline__ uint32_t hits_stride(uint32_t q, uint32_t W, uint32_t d) {
-  return q + 1 < W ? 32u : d - 32u * q;
+  return q + 1 < W ? 32u : (d - 32u * q + 7) & ~7u;
 }
 
-// One batch of 32 rows at a time, a row per lane; a row of at least 32
-// candidates runs across the warp, a word per trip and four trips' candidates
-// loaded before any is probed; shorter ones are flattened over the lanes, and
-// each lane cuts its row's bits out of the trip's ballot (a short row's
-// candidates lie in at most two words).  Only non-zero words are written.
+// probe() for bit words, on their 32-bit halves: the pass is bound by
+// instruction issue, and a 64-bit variable shift takes several
+template <int P>
+__device__ __forceinline__ bool hit(const Staged& st, uint32_t w) {
+  if (P == P_SBITS || P == P_GBITS) {
+    const uint32_t idx = (w >> 5) - 2 * st.start;
+    if (idx >= 2 * st.n) return false;  // also below the first word (wraps)
+    const uint32_t* h = reinterpret_cast<const uint32_t*>(st.words) + idx;
+    return ((P == P_SBITS ? *h : __ldg(h)) >> (w & 31)) & 1u;
+  }
+  if (P == P_ZBITS) {
+    const uint32_t idx = (w >> 6) - st.start;
+    if (idx >= st.n) return false;
+    const uint2 g = st.pz[idx >> 5];
+    const uint32_t up = g.x >> (idx & 31);
+    if (!(up & 1u)) return false;
+    const uint32_t pos = g.y + __popc(g.x ^ (up << (idx & 31)));
+    return (reinterpret_cast<const uint32_t*>(st.words)[2 * pos + ((w >> 5) & 1u)] >> (w & 31)) & 1u;
+  }
+  return probe<P>(st, w) != 0;
+}
+
+// One batch of 32 rows at a time, a row per lane.  Rows of at least kTripRow
+// candidates run as trips: a trip is one mask word of one row, a bit per lane,
+// and the trips of all the batch's rows form one list, taken four at a time
+// (so a row need not fill four) with the four trips' candidates loaded before
+// any is probed.  Lane t keeps the word of trip t and writes it after 32
+// trips.  Shorter rows are flattened over the lanes, and each lane cuts its
+// row's bits out of the trip's ballot (a short row's candidates lie in at most
+// two words).  Only non-zero words are written.
+constexpr uint32_t kTripRow = 24;  // at most 32: a short row's hits are one register
 template <int P>
 __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, const RevView& r, uint32_t kb,
                                          uint32_t ke, const uint32_t* __restrict__ moff,
                                          uint32_t* __restrict__ mask, uint32_t shard_index, uint32_t shard_count) {
   const uint32_t lane = lane_id();
-  const bool down = r.dir == DIR_DOWN;
+  const uint32_t step = r.dir == DIR_DOWN ? 0xffffffffu : 1u;  // from one candidate's element to the next's
   for (uint32_t k0 = kb; k0 < ke; k0 += 32) {
     const uint32_t k = k0 + lane;
-    uint32_t len = 0, fe = 0;           // candidates; the element of the first one
-    uint32_t i = 0, base = 0, rs = 0;   // row position, first mask word, word stride
+    uint32_t len = 0, fe = 0;               // candidates; the element of the first one
+    uint32_t skip = 0, base = 0, rs = 0;    // bit of the first candidate in the row's words, first word, stride
     if (k < ke) {
       const uint32_t lo = __ldg(r.rev_lo + k), hi = __ldg(r.rev_hi + k), src = __ldg(r.rev_src + k);
       // shards split the heads a: each rank builds and reads the matrices of its own
@@ -67,61 +94,69 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
         const StagedRange pr = staged_range(t, src);
         const uint32_t d = pr.len, W = (d + 31) >> 5;
         len = hi - lo;
-        i = d - 1 - len;
-        fe = down ? hi - 1 : lo;
+        const uint32_t i = d - 1 - len;
+        fe = r.dir == DIR_DOWN ? hi - 1 : lo;
+        skip = (i & 31) + 1;
         const uint32_t q = i >> 5;
         base = __ldg(moff + src) + hits_block(q, W) + (i & 31);
         rs = hits_stride(q, W, d);
       }
     }
-    uint32_t rows = __ballot_sync(kFull, len >= 32);
-    const uint32_t rlen = len;
-    if (len >= 32) len = 0;
-    while (rows) {
-      const int j = __ffs(rows) - 1;
-      rows &= rows - 1;
-      const uint32_t ln = __shfl_sync(kFull, rlen, j), fj = __shfl_sync(kFull, fe, j);
-      const uint32_t ij = __shfl_sync(kFull, i, j) & 31u;
-      const uint32_t bj = __shfl_sync(kFull, base, j), rj = __shfl_sync(kFull, rs, j);
-      // candidate c of the row is bit (ij + 1 + c) & 31 of its word (ij + 1 + c) >> 5
-      const uint32_t skip = ij + 1, end = skip + ln;  // bit positions from the row's first word
-      for (uint32_t w0 = 0; 32 * w0 < end; w0 += 32) {
+    const bool is_long = len >= kTripRow;
+    if (__any_sync(kFull, is_long)) {
+      const uint32_t end = skip + len;      // bits skip .. end - 1 of the row's words
+      const uint32_t f0 = skip >> 5;        // a row at the end of its block has no candidate in its first word
+      const uint32_t nw = is_long ? ((end + 31) >> 5) - f0 : 0u;
+      const uint32_t incl = warp_incl_scan(nw);
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      const uint32_t word0 = f0 - (incl - nw);       // trip x of the list is word x + word0 of its row
+      const uint32_t elem0 = fe - step * skip;       // bit p of the row is element elem0 + step * p
+      for (uint32_t t0 = 0; t0 < total; t0 += 32) {
         uint32_t mine = 0;
-        for (uint32_t u0 = 0; u0 < 32 && 32 * (w0 + u0) < end; u0 += 4) {
+        for (uint32_t u0 = 0; u0 < 32 && t0 + u0 < total; u0 += 4) {
           uint32_t v[4];
-          bool in[4];
 #pragma unroll
           for (int u = 0; u < 4; u++) {
-            const uint32_t p = 32 * (w0 + u0 + u) + lane;
-            in[u] = p >= skip && p < end;
-            v[u] = in[u] ? __ldg(t.vals + (down ? fj - (p - skip) : fj + (p - skip))) : 0u;
+            const uint32_t x = min(t0 + u0 + u, total - 1);
+            const int j = __popc(__ballot_sync(kFull, incl <= x));
+            const uint32_t ej = __shfl_sync(kFull, elem0, j), lj = __shfl_sync(kFull, end, j);
+            const uint32_t p = 32 * (x + __shfl_sync(kFull, word0, j)) + lane;
+            v[u] = __ldg(t.vals + (ej + step * min(p, lj - 1)));  // bits outside the row are masked off below
           }
 #pragma unroll
           for (int u = 0; u < 4; u++) {
-            const uint32_t b = __ballot_sync(kFull, in[u] && probe<P>(st, v[u]));
+            const uint32_t b = __ballot_sync(kFull, hit<P>(st, v[u]));
             if (lane == u0 + u) mine = b;
           }
         }
-        if (mine) mask[bj + (w0 + lane) * rj] = mine;
+        const uint32_t x = min(t0 + lane, total - 1);
+        const uint32_t j = owner_lane(incl, x);
+        const uint32_t w = x + __shfl_sync(kFull, word0, j);
+        const uint32_t sj = __shfl_sync(kFull, skip, j), lj = __shfl_sync(kFull, end, j);
+        const uint32_t bj = __shfl_sync(kFull, base, j), rj = __shfl_sync(kFull, rs, j);
+        if (sj > 32 * w) mine &= 0xffffffffu << (sj - 32 * w);  // sj - 32 w < 32: the word holds a candidate
+        if (lj < 32 * w + 32) mine &= 0xffffffffu >> (32 * w + 32 - lj);
+        if (mine && t0 + lane < total) mask[bj + w * rj] = mine;
       }
+      if (is_long) len = 0;
     }
     const uint32_t incl = warp_incl_scan(len);
     const uint32_t total = __shfl_sync(kFull, incl, 31);
     const uint32_t excl = incl - len;
-    uint32_t acc = 0;  // the lane's short row, bit c = candidate c
+    const uint32_t elem0 = fe - step * excl;  // flattened pair q of the row is element elem0 + step * q
+    uint32_t acc = 0;                         // the lane's short row, bit c = candidate c
     for (uint32_t p = 0; p < total; p += 32 * kShortUnroll) {
       uint32_t w[kShortUnroll];
 #pragma unroll
       for (int u = 0; u < kShortUnroll; u++) {
-        const uint32_t q = p + 32 * u + lane;
+        const uint32_t q = min(p + 32 * u + lane, total - 1);
         const uint32_t j = owner_lane(incl, q);
-        const uint32_t fj = __shfl_sync(kFull, fe, j), exj = __shfl_sync(kFull, excl, j);
-        w[u] = q < total ? __ldg(t.vals + (down ? fj - (q - exj) : fj + (q - exj))) : 0u;
+        w[u] = __ldg(t.vals + (__shfl_sync(kFull, elem0, j) + step * q));
       }
 #pragma unroll
       for (int u = 0; u < kShortUnroll; u++) {
         const uint32_t p0 = p + 32 * u;
-        const uint32_t ball = __ballot_sync(kFull, p0 + lane < total && probe<P>(st, w[u]));
+        const uint32_t ball = __ballot_sync(kFull, hit<P>(st, w[u]));
         const uint32_t s = max(excl, p0), e = min(incl, p0 + 32);
         if (s < e) {  // the row's candidates s - excl .. e - excl - 1 are bits s - p0 .. of the ballot
           const uint32_t bits = (ball >> (s - p0)) & (0xffffffffu >> (32 - (e - s)));
@@ -130,7 +165,7 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
       }
     }
     if (acc) {
-      const uint64_t m = (uint64_t)acc << ((i & 31) + 1);
+      const uint64_t m = (uint64_t)acc << skip;
       if ((uint32_t)m) mask[base] = (uint32_t)m;
       if ((uint32_t)(m >> 32)) mask[base + rs] = (uint32_t)(m >> 32);
     }
@@ -203,17 +238,14 @@ __device__ __forceinline__ uint32_t hits_unit_head(const HitsView& hv, uint32_t 
 }
 
 // Work units of a head entry in the second pass.
-// 4-clique: parts of d > 32 elements, in (word, word, row) steps of which a
-// unit holds about kCliqueSteps; smaller parts are one row per lane and
-// have no units.  Annotation: one unit per word column.
+// 4-clique: eight rows of a part of d > 32 elements; smaller parts are one row
+// per lane and have no units.  Annotation: one unit per word column.
 enum { HITS_CLIQUE = 0, HITS_ANNOT = 1, HITS_ROWS = 2 };
-constexpr uint64_t kCliqueSteps = 4096;
 __device__ __forceinline__ uint64_t hits_units(uint64_t d, int use) {
   const uint64_t W = (d + 31) / 32;
   if (use == HITS_ANNOT) return d >= 2 ? W : 0;
   if (use == HITS_ROWS || d <= 32) return 0;
-  const uint64_t steps = 32 * (W * (W + 1) * (W + 2) / 6);
-  return min(d, (steps + kCliqueSteps - 1) / kCliqueSteps);
+  return (d + 7) / 8;
 }
 
 // mask words and second-pass units of every head entry; sums over all of them
@@ -282,12 +314,14 @@ __global__ void __launch_bounds__(256) clique_small_kernel(const TrieView* __res
   if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
 }
 
-// 4-cliques of the larger parts.  A unit is the rows i = s, s + n, ... of one
-// matrix.  For a row i and a block q of 32 later positions, the lanes whose
-// bit of row i is set hold one row j each and AND it with row i word by word
-// (row i's word is the same for all lanes, the rows j are one 128-byte line
-// per word).  A warp takes four units in a row: they are mostly of one
-// matrix, which its L1 then holds.
+// 4-cliques of the larger parts.  A unit is eight consecutive rows i of one
+// matrix.  For a block q of 32 later positions j, each lane holds the row of
+// one j and ANDs its words with the same words of the eight rows, of each row
+// i whose bit j is set.  Row j's word is one line per warp and serves all eight
+// rows, whose own words are two 16-byte loads, the same for all lanes; that
+// leaves AND, popcount and add per (i, j word) and makes the popcounts (16
+// lanes per clock) the bound.  A warp takes the four units of one row block in
+// a row: its L1 then holds the matrix.
 __global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restrict__ views, HitsView hv,
                                                          uint32_t n_units, unsigned int* __restrict__ queue,
                                                          unsigned long long* __restrict__ total) {
@@ -310,33 +344,33 @@ __global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restr
         acc = 0;
         cur_g = g;
       }
-      const uint32_t s = u - __ldg(hv.upre + gh), n = __ldg(hv.upre + gh + 1) - __ldg(hv.upre + gh);
       const uint32_t d = staged_range(views[g], gh - hv.gstart[g]).len, W = (d + 31) >> 5;
       const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
-      for (uint32_t i = s; i < d; i += n) {
-        const uint32_t qi = i >> 5, ri = hits_stride(qi, W, d);
-        const uint32_t* row = m + hits_block(qi, W) + (i & 31);
-        uint32_t c = 0;
-        for (uint32_t q = qi; q < W; q++) {
-          const uint32_t mine = __ldg(row + (q - qi) * ri);
-          if (!mine) continue;
-          const bool on = (mine >> lane) & 1u;
-          const uint32_t rq = hits_stride(q, W, d);
-          const uint32_t* rows = m + hits_block(q, W) + lane;  // read only where a bit, so a row, exists
-          for (uint32_t k = q; k < W; k += 4) {
-            uint32_t x[4], y[4];
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-              const bool in = k + v < W;
-              x[v] = in ? __ldg(row + (k + v - qi) * ri) : 0u;
-              y[v] = in && on ? __ldg(rows + (k + v - q) * rq) : 0u;
-            }
-#pragma unroll
-            for (int v = 0; v < 4; v++) c += __popc(x[v] & y[v]);
-          }
+      const uint32_t i0 = 8 * (u - __ldg(hv.upre + gh)), qi = i0 >> 5, ri = hits_stride(qi, W, d);
+      const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
+      uint32_t c = 0;  // below 2^32: masks of 2^31 words hold at most 2^26 (j word, row) steps per lane
+      for (uint32_t q = qi; q < W; q++) {
+        const uint4 ma = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri));
+        const uint4 mb = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri + 4));
+        if (!(ma.x | ma.y | ma.z | ma.w | mb.x | mb.y | mb.z | mb.w)) continue;
+        // all ones where the lane's position j = 32 q + lane is a hit of the row
+        const uint32_t on[8] = {0u - ((ma.x >> lane) & 1u), 0u - ((ma.y >> lane) & 1u), 0u - ((ma.z >> lane) & 1u),
+                                0u - ((ma.w >> lane) & 1u), 0u - ((mb.x >> lane) & 1u), 0u - ((mb.y >> lane) & 1u),
+                                0u - ((mb.z >> lane) & 1u), 0u - ((mb.w >> lane) & 1u)};
+        const uint32_t rq = hits_stride(q, W, d);
+        const uint32_t* jw = m + hits_block(q, W) + lane;
+        const bool has = lane < rq;
+#pragma unroll 2
+        for (uint32_t k = q; k < W; k++) {
+          const uint32_t y = has ? __ldg(jw + (k - q) * rq) : 0u;
+          const uint4 xa = __ldg(reinterpret_cast<const uint4*>(rows + (k - qi) * ri));
+          const uint4 xb = __ldg(reinterpret_cast<const uint4*>(rows + (k - qi) * ri + 4));
+          c += __popc(xa.x & y & on[0]) + __popc(xa.y & y & on[1]) + __popc(xa.z & y & on[2]) +
+               __popc(xa.w & y & on[3]) + __popc(xb.x & y & on[4]) + __popc(xb.y & y & on[5]) +
+               __popc(xb.z & y & on[6]) + __popc(xb.w & y & on[7]);
         }
-        acc += c;
       }
+      acc += c;
     }
   }
   acc = warp_sum(acc);
@@ -362,17 +396,25 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x) {
 // (how often position j is the third vertex) and the row sums of block k (how
 // often it is the second), one addition to T per element, and the row sums
 // once more to T[a].
+// The largest sets are in most matrices, and in a relation in degree order they
+// are the last head entries, neighbours in T: their additions would queue up on
+// a few L2 lines.  The last kHubs entries count in shared memory and are added
+// to T once per block.
+constexpr uint32_t kHubs = 4096;
 __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv, uint32_t n_units,
                                                          unsigned long long* __restrict__ T) {
+  __shared__ unsigned int hub[kHubs];
+  for (uint32_t i = threadIdx.x; i < kHubs; i += blockDim.x) hub[i] = 0;
+  __syncthreads();
+  const uint32_t hub0 = t.n_head > kHubs ? t.n_head - kHubs : 0;
   const uint32_t lane = lane_id();
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   // consecutive units per warp: one search for the first head entry
   const uint32_t per = (n_units + nwarps - 1) / nwarps;
   const uint64_t b0 = (uint64_t)per * warp;
-  if (b0 >= n_units) return;
-  const uint32_t u0 = (uint32_t)b0, u1 = (uint32_t)min(b0 + per, (uint64_t)n_units);
-  uint32_t a = hits_unit_head(hv, u0);
+  const uint32_t u0 = (uint32_t)min(b0, (uint64_t)n_units), u1 = (uint32_t)min(b0 + per, (uint64_t)n_units);
+  uint32_t a = u0 < u1 ? hits_unit_head(hv, u0) : 0;
   for (uint32_t u = u0; u < u1; u++) {
     while (__ldg(hv.upre + a + 1) <= u) a++;
     const uint32_t k = u - __ldg(hv.upre + a);
@@ -389,12 +431,17 @@ __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv
     if (lane < rk)
       for (uint32_t w = k; w < W; w++) row += __popc(__ldg(m + hits_block(k, W) + (w - k) * rk + lane));
     if (col + row) {  // so the position is below d
-      const int32_t h = __ldg(t.head_index + __ldg(t.vals + pr.s0 + 32 * k + lane));
-      atomicAdd(T + h, 2ull * (col + row));
+      const uint32_t h = (uint32_t)__ldg(t.head_index + __ldg(t.vals + pr.s0 + 32 * k + lane));
+      const uint32_t v = col + row;
+      if (h < hub0) atomicAdd(T + h, 2ull * v);
+      else if (atomicAdd(hub + (h - hub0), v) > 0xffffffffu - v) atomicAdd(T + h, 2ull << 32);  // wrapped
     }
     const uint32_t all = warp_sum(row);
     if (lane == 0 && all) atomicAdd(T + a, 2ull * all);
   }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < kHubs; i += blockDim.x)
+    if (hub[i]) atomicAdd(T + hub0 + i, 2ull * hub[i]);
 }
 
 // rows: triangles per relation row e = (a, position i); a warp per head entry

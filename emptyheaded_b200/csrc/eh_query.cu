@@ -821,6 +821,20 @@ __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_
   if (zlist && len >= 2) {
     const uint32_t first = __ldg(t.vals + s0), last = __ldg(t.vals + s0 + len - 1);
     const uint32_t W = (last >> 6) - (first >> 6) + 1;
+    if (2 * W <= (uint32_t)cap_words) {  // the whole bitmap fits: one load per probe, and quicker to build
+      const uint32_t start = first >> 6;
+      for (uint32_t j = lane; j < 2 * W; j += 32) sm[j] = 0u;
+      __syncwarp();
+      for (uint32_t j = lane; j < len; j += 32) {
+        const uint32_t v = __ldg(t.vals + s0 + j);
+        atomicOr(sm + ((v >> 5) - 2 * start), 1u << (v & 31));
+      }
+      __syncwarp();
+      st.words = reinterpret_cast<uint64_t*>(sm);
+      st.start = start;
+      st.n = W;
+      return P_SBITS;
+    }
     if (zbits_words(W, len) <= (uint32_t)cap_words) {
       const uint32_t groups = (W + 31) / 32, start = first >> 6;
       uint2* pz = reinterpret_cast<uint2*>(sm);
