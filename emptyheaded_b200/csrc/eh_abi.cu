@@ -183,6 +183,7 @@ eh_status eh_context_create(int device, eh_context** out) {
       EH_CUDA(cudaEventCreate(&c->ev0));
       EH_CUDA(cudaEventCreate(&c->ev1));
       EH_CUDA(cudaEventCreate(&c->ev2));
+      EH_CUDA(cudaEventCreate(&c->ev3));
     } catch (...) {
       delete c;
       throw;
@@ -197,9 +198,12 @@ eh_status eh_context_destroy(eh_context* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->annot) cudaFree(ctx->annot);
+    if (ctx->work) cudaFree(ctx->work);
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->ev2) cudaEventDestroy(ctx->ev2);
+    if (ctx->ev3) cudaEventDestroy(ctx->ev3);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->copy_stream) {
       cudaStreamSynchronize(ctx->copy_stream);

@@ -173,12 +173,14 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
 }
 
 __global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const TrieView* __restrict__ views, const RevView* __restrict__ revs,
-                                                 const Item* __restrict__ items, uint32_t n_items, int cap_words,
+                                                 const Item* __restrict__ items,
+                                                 const unsigned int* __restrict__ n_items_p, int cap_words,
                                                  unsigned int* __restrict__ queue, HitsView hv, float* records,
                                                  uint32_t shard_index, uint32_t shard_count) {
   extern __shared__ uint32_t smem[];
   const uint32_t lane = lane_id();
   uint32_t* sm = smem + (size_t)(threadIdx.x >> 5) * cap_words;
+  const uint32_t n_items = __ldg(n_items_p);
   for (;;) {
     uint32_t it = 0;
     if (lane == 0) it = atomicAdd(queue, 1u);
@@ -410,12 +412,15 @@ __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv
   const uint32_t lane = lane_id();
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  // consecutive units per warp: one search for the first head entry
-  const uint32_t per = (n_units + nwarps - 1) / nwarps;
-  const uint64_t b0 = (uint64_t)per * warp;
-  const uint32_t u0 = (uint32_t)min(b0, (uint64_t)n_units), u1 = (uint32_t)min(b0 + per, (uint64_t)n_units);
-  uint32_t a = u0 < u1 ? hits_unit_head(hv, u0) : 0;
-  for (uint32_t u = u0; u < u1; u++) {
+  // runs of consecutive units, so that few searches find the head entries,
+  // spread over the warps, so that the long rows of a range of ids are too
+  constexpr uint32_t kRun = 16;
+  uint32_t a = 0;
+  for (uint64_t v = 0;; v++) {
+    const uint64_t u64 = ((v / kRun) * nwarps + warp) * kRun + v % kRun;
+    if (u64 >= n_units) break;
+    const uint32_t u = (uint32_t)u64;
+    if (v % kRun == 0) a = hits_unit_head(hv, u);
     while (__ldg(hv.upre + a + 1) <= u) a++;
     const uint32_t k = u - __ldg(hv.upre + a);
     const StagedRange pr = staged_range(t, a);

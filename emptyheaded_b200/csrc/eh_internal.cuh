@@ -1,5 +1,6 @@
 // Internal types shared by the engine's translation units.
 #pragma once
+#include <mutex>
 #include <vector>
 
 #include "eh_common.cuh"
@@ -9,13 +10,20 @@ struct eh_context {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // host-to-device copies overlapped with work on `stream`
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
   // per-item timing records of the last recorded query (8 floats each)
   std::vector<float> timing_records;
   // the annotated triangle pass's per-head counters: a cudaMalloc'd buffer of
   // annot_cap entries kept across queries (see annot_buffer in eh_query.cu)
   unsigned long long* annot = nullptr;
   size_t annot_cap = 0;
+  // small memory kept from call to call (see workspace in eh_query.cu), used
+  // under the lock
+  unsigned char* work = nullptr;    // device
+  size_t work_cap = 0;
+  unsigned char* pinned = nullptr;  // host
+  size_t pinned_cap = 0;
+  std::recursive_mutex mu;
 };
 
 namespace eh {

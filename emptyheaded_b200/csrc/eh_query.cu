@@ -15,6 +15,8 @@
 // about `chunk_pairs` probes, pulled by warps of a persistent kernel from
 // an atomic queue, heaviest b first.
 #include <algorithm>
+#include <cstring>
+#include <exception>
 
 #include "eh_internal.cuh"
 
@@ -73,6 +75,7 @@ constexpr uint32_t kFlatClique = EH_FLAT_CLIQUE;  // 4-clique: S up to this size
 // autotuner (emptyheaded_b200/autotune.py) re-picks them per trie.
 constexpr int kDefaultSmemWords = 1024;  // per warp
 constexpr int kDefaultChunk = 32768;
+constexpr uint64_t kMinChunk = 4096;  // the smallest item the planner cuts by itself
 
 struct RevView {
   const uint64_t* rev_off;
@@ -95,6 +98,7 @@ struct ExecParams {
   uint32_t long_row;
   uint32_t s_cap;  // 4-clique: S buffers in global memory of this many words per warp (0: in shared memory)
   bool smem_given; // the caller chose smem_words
+  bool chunk_given;  // the caller chose chunk
   bool no_block_items;  // stage every N(b) per warp (no block items)
 };
 
@@ -102,7 +106,8 @@ static ExecParams exec_params(const eh_exec_config* cfg) {
   ExecParams p;
   p.warps = (cfg && cfg->warps_per_block > 0) ? cfg->warps_per_block : kDefaultWarps;
   p.smem_words = (cfg && cfg->smem_words > 0) ? cfg->smem_words : kDefaultSmemWords;
-  p.chunk = (cfg && cfg->chunk_pairs > 0) ? (uint32_t)cfg->chunk_pairs : (uint32_t)kDefaultChunk;
+  p.chunk_given = cfg && cfg->chunk_pairs > 0;
+  p.chunk = p.chunk_given ? (uint32_t)cfg->chunk_pairs : (uint32_t)kDefaultChunk;
   p.long_row = (cfg && cfg->long_row > 0) ? (uint32_t)cfg->long_row : kDefaultLongRow;
   p.shard_count = (cfg && cfg->shard_count > 1) ? (uint32_t)cfg->shard_count : 1u;
   p.shard_index = (cfg && cfg->shard_count > 1) ? (uint32_t)cfg->shard_index : 0u;
@@ -143,7 +148,7 @@ __device__ __forceinline__ uint64_t first_row_at(const uint64_t* __restrict__ wp
 // the first one at target i + 1 -- two independent searches over b's rows.
 // The work prefix is non-decreasing, so these are the bounds a serial cut of
 // b's items one after the other finds, at any number of items per entry.
-__global__ void plan_fill_kernel(RevView r, uint32_t nh, const uint32_t* __restrict__ nitems,
+__global__ void plan_fill_scratch_kernel(RevView r, uint32_t nh, const uint32_t* __restrict__ nitems,
                                  const uint32_t* __restrict__ ipos, uint32_t total, uint32_t g,
                                  Item* __restrict__ items) {
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
@@ -236,66 +241,175 @@ struct PlanShape {
   uint32_t warps;        // warps per block
 };
 
-__global__ void plan_split_kernel(TrieView t, RevView r, PlanShape ps, uint32_t* __restrict__ nw,
-                                  uint32_t* __restrict__ nb) {
-  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < t.n_head; b += gridDim.x * blockDim.x) {
-    const uint64_t w = r.rev_wpre[r.rev_off[b + 1]] - r.rev_wpre[r.rev_off[b]];
-    const uint32_t sw = staged_words(t, b, ps.warp_words);
-    const bool blk = ps.block_words && sw > ps.warp_words && sw <= ps.block_words && w >= kMinBlockWork;
-    const uint64_t mult = blk ? ps.warps : 1;
-    uint64_t n = 0;
-    if (w) {
-      if (ps.pred) {
-        n = (uint64_t)ceil((double)ps.pred[b] / (ps.unit * (double)mult));
-        n = max((uint64_t)1, min(n, (w + 63) / 64));
-      } else {
-        n = (w + ps.chunk * mult - 1) / (ps.chunk * mult);
-      }
-    }
-    nw[b] = blk ? 0u : (uint32_t)n;
-    nb[b] = blk ? (uint32_t)n : 0u;
+// Cost of a row beside its candidates, in candidates: a row of one candidate
+// takes its share of a batch's loads, scans and owner searches.  Without it an
+// item of a hub's one-candidate rows held 32,768 rows and ran alone at the end
+// (hit masks of Chung-Lu 2^20: SMs busy 56% of the kernel's time).
+#ifndef EH_ROW_COST
+#define EH_ROW_COST 8
+#endif
+constexpr uint32_t kRowCost = EH_ROW_COST;
+
+// the first row k in [k0, k1) before which rows and candidates cost at least
+// `target` (k1 if none)
+__device__ __forceinline__ uint64_t row_at_cost(const uint64_t* __restrict__ wpre, uint64_t k0, uint64_t k1,
+                                                uint64_t w0, uint64_t target) {
+  uint64_t lo = k0, hi = k1;
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) >> 1;
+    if (wpre[mid] - w0 + kRowCost * (mid - k0) < target) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// What a launch reads and writes beside the tries: the queues, the numbers of
+// items the planner made, the results.  One copy from pinned host memory sets
+// it up together with the views, one copy brings it back.
+// The queue heads have a 128-byte line of their own: every item pulled is an
+// atomic on it, and the warps read the rest (one line for all: triangle
+// R-MAT-22 8.61 -> 8.89 ms).
+struct Control {
+  unsigned int queue[2];   // warp items, block items (or second-pass units)
+  unsigned int pad0[30];
+  unsigned int items[2];   // warp items, block items
+  unsigned int pad1[30];
+  unsigned long long spare[2];  // a total nobody reads; the planner's total of a trie
+  // followed by unsigned long long total[n], then the views
+};
+
+// The plan of a trie, in three launches and without the host: how many items
+// each head entry gives (and the sums over tiles of kPlanTile entries), where
+// they go, and the items, one thread each.  The intersection kernel reads the
+// number of items from the control block.  Items lie in reverse head order
+// (ids are degree-ordered), so the queue starts at the heaviest b and small
+// items come last.  (Reserving the places by atomics in one launch put heavy
+// blocks behind light ones: triangle R-MAT-20 1.43 -> 1.7-2.5 ms.)
+// Shards take the items i of entry b with (b + i + g) % shard_count ==
+// shard_index.
+struct PlanArgs {
+  TrieView t;
+  RevView r;
+  PlanShape ps;
+  uint32_t g, shard_index, shard_count;
+  uint64_t* pos;    // [n_head] items (then places) of an entry: block items high, warp items low
+  uint64_t* tiles;  // [tiles] sums
+};
+constexpr uint32_t kPlanTile = 2048;
+
+// items of entry b over all shards
+__device__ __forceinline__ uint32_t plan_items(const PlanArgs& p, uint32_t b, uint64_t k0, uint64_t k1, bool& blk) {
+  blk = false;
+  if (k1 <= k0) return 0;
+  const uint64_t w = p.r.rev_wpre[k1] - p.r.rev_wpre[k0];
+  if (p.ps.block_words && w >= kMinBlockWork) {
+    const uint32_t sw = staged_words(p.t, b, p.ps.warp_words);
+    blk = sw > p.ps.warp_words && sw <= p.ps.block_words;
+  }
+  const uint64_t mult = blk ? p.ps.warps : 1;
+  if (p.ps.pred) {
+    const uint64_t m = (uint64_t)ceil((double)p.ps.pred[b] / (p.ps.unit * (double)mult));
+    return (uint32_t)max((uint64_t)1, min(m, (w + 63) / 64));
+  }
+  return (uint32_t)((w + kRowCost * (k1 - k0) + p.ps.chunk * mult - 1) / (p.ps.chunk * mult));
+}
+// this shard's first item of entry b
+__device__ __forceinline__ uint32_t plan_first(const PlanArgs& p, uint32_t b) {
+  return p.shard_count > 1 ? (p.shard_index + p.shard_count - (b + p.g) % p.shard_count) % p.shard_count : 0;
+}
+
+__global__ void __launch_bounds__(256) plan_split_kernel(PlanArgs p) {
+  __shared__ uint64_t s_warp[8];
+  uint64_t sum = 0;
+  for (uint32_t x = threadIdx.x; x < kPlanTile; x += 256) {
+    const uint64_t b = (uint64_t)blockIdx.x * kPlanTile + x;
+    if (b >= p.t.n_head) break;
+    bool blk;
+    const uint32_t n = plan_items(p, (uint32_t)b, p.r.rev_off[b], p.r.rev_off[b + 1], blk);
+    const uint32_t first = plan_first(p, (uint32_t)b);
+    const uint64_t mine = n > first ? (n - first + p.shard_count - 1) / p.shard_count : 0;
+    const uint64_t v = blk ? mine << 32 : mine;
+    p.pos[b] = v;
+    sum += v;
+  }
+  sum = warp_sum(sum);
+  if (lane_id() == 0) s_warp[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; i++) sum += s_warp[i];
+    p.tiles[blockIdx.x] = sum;
   }
 }
 
-struct Plan {
-  DevBuf<Item> items;  // block items first, then warp items
-  uint32_t n = 0;      // all items
-  uint32_t nb = 0;     // block items
-};
+// counts -> places in entry order; the totals to places[0..1] of ctl->spare
+__global__ void __launch_bounds__(256) plan_place_kernel(PlanArgs p, unsigned long long* __restrict__ total) {
+  __shared__ uint64_t s_warp[8], s_before;
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  uint64_t before = 0;  // sums of the tiles before this one
+  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += 256) before += p.tiles[i];
+  before = warp_sum(before);
+  if (lane == 0) s_warp[wid] = before;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; i++) before += s_warp[i];
+    s_before = before;
+  }
+  __syncthreads();
+  before = s_before;
+  const uint64_t b0 = (uint64_t)blockIdx.x * kPlanTile + 8 * threadIdx.x;
+  uint64_t v[8], sum = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    v[i] = b0 + i < p.t.n_head ? p.pos[b0 + i] : 0;
+    sum += v[i];
+  }
+  const uint64_t incl = warp_incl_scan(sum);
+  if (lane == 31) s_warp[wid] = incl;
+  __syncthreads();
+  for (uint32_t i = 0; i < wid; i++) before += s_warp[i];
+  uint64_t run = before + incl - sum;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    if (b0 + i < p.t.n_head) p.pos[b0 + i] = run;
+    run += v[i];
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 255) *total = run;
+}
 
-// returns the kernels it launched
-static uint32_t build_plan(eh_context* ctx, const eh_trie* t, const PlanShape& shape, uint32_t g, Plan& plan) {
-  cudaStream_t s = ctx->stream;
-  plan.n = plan.nb = 0;
-  if (!t->rev_entries) return 0;
-  RevView r{t->rev_off.p, t->rev_lo.p, t->rev_hi.p, t->rev_src.p, t->rev_wpre.p, t->dir};
-  PlanShape ps = shape;
-  if (!(t->work_pred.p && t->pred_per_probe > 0)) ps.pred = nullptr;
-  ps.unit = t->pred_per_probe * shape.chunk;
-  DevBuf<uint32_t> nw(t->n_head, s), nb(t->n_head, s), pw(t->n_head, s), pb(t->n_head, s), tot(2, s);
-  const int grid = num_sms() * 4;
-  TracePhase ph_split("plan.split+scan", s);
-  plan_split_kernel<<<grid, 256, 0, s>>>(t->view(), r, ps, nw.p, nb.p);
-  EH_CHECK_LAUNCH();
-  exclusive_scan<uint32_t>(nw.p, pw.p, t->n_head, tot.p, s);
-  exclusive_scan<uint32_t>(nb.p, pb.p, t->n_head, tot.p + 1, s);
-  uint32_t h[2] = {0, 0};
-  EH_CUDA(cudaMemcpyAsync(h, tot.p, 8, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaStreamSynchronize(s));
-  ph_split.end();
-  TracePhase ph_fill("plan.fill", s);
-  plan.nb = h[1];
-  plan.n = h[0] + h[1];
-  plan.items.alloc(plan.n ? plan.n : 1, s);
-  if (h[1]) {
-    plan_fill_kernel<<<grid, 256, 0, s>>>(r, t->n_head, nb.p, pb.p, h[1], g, plan.items.p);
-    EH_CHECK_LAUNCH();
+// One thread per item (warp items first): item q of a class belongs to the last
+// entry whose place is at or before q (entries without items share the next
+// one's place and are never found), and covers the rows from the first one at
+// its share of the entry's cost to the first one at the next share.  Items are
+// appended after those of the tries before (ctl->items, which the next
+// launch on the stream adds to).
+__global__ void __launch_bounds__(256) plan_fill_kernel(PlanArgs p, const unsigned long long* __restrict__ total,
+                                                        const Control* __restrict__ ctl, Item* __restrict__ items,
+                                                        Item* __restrict__ bitems) {
+  const uint32_t nw = (uint32_t)*total, nb = (uint32_t)(*total >> 32);
+  const uint32_t w0 = ctl->items[0], b0 = ctl->items[1];
+  for (uint64_t x = blockIdx.x * 256ull + threadIdx.x; x < (uint64_t)nw + nb; x += gridDim.x * 256ull) {
+    const bool cls = x >= nw;
+    const uint32_t q = cls ? (uint32_t)(x - nw) : (uint32_t)x;
+    uint32_t lo = 0, hi = p.t.n_head;  // first entry with its place above q
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      const uint64_t v = __ldg(p.pos + mid);
+      if ((cls ? (uint32_t)(v >> 32) : (uint32_t)v) <= q) lo = mid + 1; else hi = mid;
+    }
+    const uint32_t b = lo - 1;
+    const uint64_t v = p.pos[b];
+    const uint64_t k0 = p.r.rev_off[b], k1 = p.r.rev_off[b + 1];
+    bool blk;
+    const uint64_t m = plan_items(p, b, k0, k1, blk);
+    const uint64_t i = plan_first(p, b) + (uint64_t)(q - (cls ? (uint32_t)(v >> 32) : (uint32_t)v)) * p.shard_count;
+    const uint64_t wp = p.r.rev_wpre[k0], W = p.r.rev_wpre[k1] - wp + kRowCost * (k1 - k0);
+    const uint64_t kb = i ? row_at_cost(p.r.rev_wpre, k0, k1, wp, (W * i) / m) : k0;
+    const uint64_t ke = i + 1 < m ? row_at_cost(p.r.rev_wpre, k0, k1, wp, (W * (i + 1)) / m) : k1;
+    (cls ? bitems + b0 + (nb - 1 - q) : items + w0 + (nw - 1 - q))[0] = Item{b, (uint32_t)kb, (uint32_t)ke, p.g};
   }
-  if (h[0]) {
-    plan_fill_kernel<<<grid, 256, 0, s>>>(r, t->n_head, nw.p, pw.p, h[0], g, plan.items.p + h[1]);
-    EH_CHECK_LAUNCH();
-  }
-  return 1 + 2 * scan_launches(t->n_head) + (h[0] ? 1 : 0) + (h[1] ? 1 : 0);
+}
+__global__ void plan_append_kernel(const unsigned long long* __restrict__ total, Control* __restrict__ ctl) {
+  ctl->items[0] += (uint32_t)*total;
+  ctl->items[1] += (uint32_t)(*total >> 32);
 }
 
 
@@ -821,7 +935,10 @@ __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_
   if (zlist && len >= 2) {
     const uint32_t first = __ldg(t.vals + s0), last = __ldg(t.vals + s0 + len - 1);
     const uint32_t W = (last >> 6) - (first >> 6) + 1;
-    if (2 * W <= (uint32_t)cap_words) {  // the whole bitmap fits: one load per probe, and quicker to build
+    // a plain bitmap, one load per probe, where it fits and clearing it is not
+    // the larger part of building it (Chung-Lu 2^21, triangle: 3.87 -> 3.53 ms;
+    // sets of a few elements over hundreds of words stay compressed)
+    if (2 * W <= (uint32_t)cap_words && W <= 8 * len) {
       const uint32_t start = first >> 6;
       for (uint32_t j = lane; j < 2 * W; j += 32) sm[j] = 0u;
       __syncwarp();
@@ -949,12 +1066,13 @@ __device__ __forceinline__ uint64_t rows_of(int mode, const Staged& st, const Tr
 }
 
 struct QueryOut {
-  uint32_t shard_index, shard_count;  // this launch runs items shard_index + q * shard_count
   uint32_t long_row;                  // size-class boundary of rows (warp-wide vs flattened)
   unsigned long long* total;   // per graph results (one per trie)
   unsigned long long* annot;   // per head entry annotation or null
   float* records;              // per item timing records or null
-  unsigned int* queue;         // atomic queue head
+  unsigned int* queue;         // [2] atomic queue heads: warp items, block items
+  const unsigned int* n_items; // [2] warp items, block items
+  const Item* bitems;          // MODE_COUNT: the block items
   unsigned long long* item_counts;  // per item count x count_mult (materialize sizing) or null
   uint32_t count_mult;
   const unsigned long long* item_off;  // MODE_MAT: first output row of each item
@@ -963,15 +1081,13 @@ struct QueryOut {
   int32_t hot[kHot];           // MODE_ANNOT on a symmetric relation: largest sets' head entries, -1 if none
   uint32_t* gsbuf;             // 4-clique: per-warp S buffers in global memory (sets too large for
   uint32_t gcap;               //   shared memory), gcap words each; null: S in shared memory
-  uint32_t n_bitems;           // MODE_COUNT: items[0, n_bitems) are block items, the rest warp items
-  unsigned int* bqueue;        // atomic queue head of the block items
 };
 
 template <int kMode>
 __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict__ views,
                                                         const RevView* __restrict__ revs,
-                                                        const Item* __restrict__ items, uint32_t n_items,
-                                                        int cap_words, QueryOut out) {
+                                                        const Item* __restrict__ items, int cap_words,
+                                                        QueryOut out) {
   extern __shared__ uint32_t smem[];
   __shared__ unsigned int slot[kMaxWarps];  // MODE_MAT: rows written by the warp's item so far
   __shared__ unsigned long long hot_acc[kHot];
@@ -993,31 +1109,30 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict_
   // time from a block counter.  Then each warp pulls warp items on its own.
   __shared__ unsigned int s_q, s_next;
   const uint32_t nwarps = blockDim.x >> 5;
-  bool block_phase = kMode == MODE_COUNT && out.n_bitems > 0;
-  const uint32_t n_witems = n_items - (kMode == MODE_COUNT ? out.n_bitems : 0u);
+  const uint32_t n_witems = __ldg(out.n_items), n_bitems = kMode == MODE_COUNT ? __ldg(out.n_items + 1) : 0u;
+  bool block_phase = n_bitems != 0;
   for (;;) {
     uint32_t it;
     if (block_phase) {
       if (threadIdx.x == 0) {
-        s_q = atomicAdd(out.bqueue, 1u);
+        s_q = atomicAdd(out.queue + 1, 1u);
         s_next = 0;
       }
       __syncthreads();
-      const uint64_t bi64 = (uint64_t)out.shard_index + (uint64_t)s_q * out.shard_count;
-      if (bi64 >= out.n_bitems) {  // the same on every thread of the block
+      it = s_q;
+      if (it >= n_bitems) {  // the same on every thread of the block
         block_phase = false;
         continue;
       }
-      it = (uint32_t)bi64;
     } else {
       uint32_t q = 0;
       if (lane == 0) q = atomicAdd(out.queue, 1u);
-      q = __shfl_sync(kFull, q, 0);
-      const uint64_t it64 = (uint64_t)out.shard_index + (uint64_t)q * out.shard_count;
-      if (it64 >= n_witems) break;
-      it = (uint32_t)it64 + (kMode == MODE_COUNT ? out.n_bitems : 0u);
+      it = __shfl_sync(kFull, q, 0);
+      if (it >= n_witems) break;
     }
-    const Item item = items[it];
+    const Item item = block_phase ? out.bitems[it] : items[it];
+    if (block_phase) it += n_witems;  // records: the warp items', then the block items'
+
     if (item.g != cur_g) {  // flush the running count of the previous graph
       if (lane == 0 && cur_g != 0xffffffffu && acc) atomicAdd(out.total + cur_g, acc);
       acc = 0;
@@ -1234,8 +1349,8 @@ __device__ uint64_t clique_rows(const Staged& st, const TrieView& t, const RevVi
 
 __global__ void EH_TRI_LAUNCH_BOUNDS clique4_kernel(const TrieView* __restrict__ views,
                                                        const RevView* __restrict__ revs,
-                                                       const Item* __restrict__ items, uint32_t n_items,
-                                                       int cap_words, QueryOut out) {
+                                                       const Item* __restrict__ items, int cap_words,
+                                                       QueryOut out) {
   extern __shared__ uint32_t smem[];
   const uint32_t lane = lane_id();
   const uint32_t wid = threadIdx.x >> 5;
@@ -1246,13 +1361,12 @@ __global__ void EH_TRI_LAUNCH_BOUNDS clique4_kernel(const TrieView* __restrict__
   const uint32_t scap = out.gsbuf ? out.gcap : (uint32_t)half;
   unsigned long long acc = 0;
   uint32_t cur_g = 0xffffffffu;
+  const uint32_t n_items = __ldg(out.n_items);
   for (;;) {
-    uint32_t q = 0;
-    if (lane == 0) q = atomicAdd(out.queue, 1u);
-    q = __shfl_sync(kFull, q, 0);
-    const uint64_t it64 = (uint64_t)out.shard_index + (uint64_t)q * out.shard_count;
-    if (it64 >= n_items) break;
-    const uint32_t it = (uint32_t)it64;
+    uint32_t it = 0;
+    if (lane == 0) it = atomicAdd(out.queue, 1u);
+    it = __shfl_sync(kFull, it, 0);
+    if (it >= n_items) break;
     const Item item = items[it];
     if (item.g != cur_g) {
       if (lane == 0 && cur_g != 0xffffffffu && acc) atomicAdd(out.total + cur_g, acc);
@@ -1290,49 +1404,61 @@ __global__ void EH_TRI_LAUNCH_BOUNDS clique4_kernel(const TrieView* __restrict__
 namespace eh {
 
 // ------------------------------------------------- lollipop / barbell roots
-constexpr uint64_t kRootBig = 32768;  // barbell root: larger sets get grid-wide passes
+constexpr uint64_t kRootBig = 4096;  // barbell root: larger sets are shared by the whole grid
 
 // LollipopAgg root, order [a,d]: sum_a T(a) * |N(a)|
 // BarbellAgg root, order [a,x]: sum_a T(a) * sum_{x in N(a) ∩ head} T(x);
-// Tv = T by value (0 off the head): one random load per row instead of two
+// Tv = T by value (0 off the head): one random load per row instead of two.
+// A warp per set: a hub's 32 K elements in one warp took 0.53 ms of the 1.27
+// of a barbell on 2^16 nodes, so larger sets are left to root_big_kernel; and on
+// a symmetric relation the sum over rows (a,x) of T(a) T(x) is twice that over
+// the rows a < x.
 template <bool kBarbell>
 __global__ void root_kernel(TrieView t, const unsigned long long* __restrict__ T,
-                            const unsigned long long* __restrict__ Tv, unsigned long long* __restrict__ total) {
+                            const unsigned long long* __restrict__ Tv, unsigned long long* __restrict__ total,
+                            uint32_t* __restrict__ big, unsigned int* __restrict__ n_big) {
   const uint32_t lane = lane_id();
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   unsigned long long acc = 0;
-  for (uint32_t a = warp; a < t.n_head; a += nwarps) {
-    const unsigned long long ta = T[a];
-    if (!ta) continue;
-    if (kBarbell && t.off[a + 1] - t.off[a] > kRootBig) continue;  // root_big_kernel's
-    unsigned long long s = 0;
-    if (kBarbell) {
-      for (uint64_t e = t.off[a] + lane; e < t.off[a + 1]; e += 32) s += __ldg(Tv + __ldg(t.vals + e));
-      s = warp_sum(s);
-    } else {
-      s = t.off[a + 1] - t.off[a];
+  if (!kBarbell) {
+    for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < t.n_head; a += gridDim.x * blockDim.x)
+      acc += T[a] * (t.off[a + 1] - t.off[a]);
+    acc = warp_sum(acc);
+  } else {
+    for (uint32_t a = warp; a < t.n_head; a += nwarps) {
+      const unsigned long long ta = T[a];
+      if (!ta) continue;
+      const StagedRange r = staged_range(t, a);
+      if (r.len > kRootBig) {
+        if (lane == 0) big[atomicAdd(n_big, 1u)] = a;
+        continue;
+      }
+      unsigned long long s = 0;
+      for (uint32_t e = lane; e < r.len; e += 32) s += __ldg(Tv + __ldg(t.vals + r.s0 + e));
+      acc += ta * s;
     }
-    acc += ta * s;
+    acc = warp_sum(acc) * (t.up ? 2ull : 1ull);
   }
   if (lane == 0 && acc) atomicAdd(total, acc);
 }
 
-// the barbell root of one large set a, grid-wide
-__global__ void root_big_kernel(TrieView t, uint32_t a, const unsigned long long* __restrict__ T,
-                                const unsigned long long* __restrict__ Tv, unsigned long long* __restrict__ total) {
-  const unsigned long long ta = T[a];
-  unsigned long long s = 0;
-  for (uint64_t e = t.off[a] + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < t.off[a + 1];
-       e += (uint64_t)gridDim.x * blockDim.x)
-    s += __ldg(Tv + __ldg(t.vals + e));
-  s = warp_sum(s);
-  if (lane_id() == 0 && s) atomicAdd(total, ta * s);
-}
-
-__global__ void root_big_sets_kernel(TrieView t, uint32_t* __restrict__ idx, unsigned int* __restrict__ n) {
-  for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < t.n_head; a += gridDim.x * blockDim.x)
-    if (t.off[a + 1] - t.off[a] > kRootBig) idx[atomicAdd(n, 1u)] = a;
+// the barbell root of the large sets, each grid-wide
+__global__ void root_big_kernel(TrieView t, const uint32_t* __restrict__ big, const unsigned int* __restrict__ n_big,
+                                const unsigned long long* __restrict__ T, const unsigned long long* __restrict__ Tv,
+                                unsigned long long* __restrict__ total) {
+  unsigned long long acc = 0;
+  const unsigned int n = *n_big;
+  for (unsigned int k = 0; k < n; k++) {
+    const uint32_t a = big[k];
+    const StagedRange r = staged_range(t, a);
+    unsigned long long s = 0;
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < r.len; e += (uint64_t)gridDim.x * blockDim.x)
+      s += __ldg(Tv + __ldg(t.vals + r.s0 + e));
+    acc += T[a] * s;
+  }
+  acc = warp_sum(acc) * (t.up ? 2ull : 1ull);
+  if (lane_id() == 0 && acc) atomicAdd(total, acc);
 }
 
 __global__ void t_by_value_kernel(TrieView t, const unsigned long long* __restrict__ T,
@@ -1370,9 +1496,41 @@ static void set_smem_attr(K kernel, size_t smem) {
   EH_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 }
 
+// Small device and pinned host memory of a context, kept from call to call (a
+// caller holds the context's lock until its work is done): a query's plan and
+// control block.  Past kMaxWorkspace a call allocates and frees its own.  Not in
+// the stream-ordered pool: what a call took there goes back with it.
+constexpr size_t kMaxWorkspace = 64ull << 20;
+static unsigned char* workspace(eh_context* ctx, size_t bytes) {
+  if (bytes > kMaxWorkspace) return nullptr;
+  if (bytes > ctx->work_cap) {
+    EH_CUDA(cudaStreamSynchronize(ctx->stream));
+    const size_t want = std::min(kMaxWorkspace, std::max<size_t>(bytes + bytes / 2, 1u << 20));
+    void* p = nullptr;
+    if (cudaMalloc(&p, want) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (ctx->work) cudaFree(ctx->work);
+    ctx->work = (unsigned char*)p;
+    ctx->work_cap = want;
+  }
+  return ctx->work;
+}
+static unsigned char* pinned(eh_context* ctx, size_t bytes) {
+  if (bytes > ctx->pinned_cap) {
+    EH_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (ctx->pinned) EH_CUDA(cudaFreeHost(ctx->pinned));
+    ctx->pinned = nullptr;
+    ctx->pinned_cap = 0;
+    EH_CUDA(cudaMallocHost((void**)&ctx->pinned, 2 * bytes + 4096));
+    ctx->pinned_cap = 2 * bytes + 4096;
+  }
+  return ctx->pinned;
+}
+
 struct Launch {
   uint32_t launches = 0;
-  float kernel_ms = 0;
 };
 
 // The hit masks of a prepared launch (eh_hits.cuh): where every head entry's
@@ -1444,14 +1602,18 @@ static bool plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
 // Everything a launch needs on the device, built once: the work plans of
 // the tries concatenated into one queue, their views, the launch shape.
 struct Prepared {
-  DevBuf<Item> items;
-  uint32_t n_items = 0;
-  uint32_t n_bitems = 0;  // items[0, n_bitems) are block items
+  DevBuf<unsigned char> own;      // device arrays of a launch that outlives the call (a batch) or is large
+  Control* ctl = nullptr;         // control block, results, views, items: one piece of device memory
+  unsigned long long* total = nullptr;  // [n] results
+  TrieView view0{};               // the first trie's view
+  TrieView* dv = nullptr;
+  RevView* dr = nullptr;
+  Item* items = nullptr;          // warp items, at most cap_w
+  Item* bitems = nullptr;         // block items, at most cap_b
+  uint64_t cap_w = 0, cap_b = 0;
+  uint32_t n = 0;                 // tries
+  uint64_t entries = 0;           // rows of the tries' reverse levels: 0 means nothing to run
   uint64_t pairs = 0;
-  TrieView view0{};  // the first trie's view
-  DevBuf<TrieView> dv;
-  DevBuf<RevView> dr;
-  DevBuf<unsigned int> q;
   ExecParams ep{};
   size_t smem = 0;
   int grid = 1, threads = 32;
@@ -1462,6 +1624,7 @@ struct Prepared {
   DevBuf<uint32_t> gs;            // 4-clique global S buffers (ExecParams::s_cap)
   int32_t hot[kHot] = {-1, -1, -1, -1};  // annotation: largest sets (QueryOut::hot)
   Hits hits;                      // the plan runs on hit masks
+  size_t ctl_bytes() const { return sizeof(Control) + n * sizeof(unsigned long long); }  // what comes back
 };
 
 // head entry with the largest set, excluding `ex` (-1 unused): max over
@@ -1509,9 +1672,10 @@ static void size_clique_staging(ExecParams& ep, uint32_t max_set) {
   }
 }
 
-// hits_use: run the plan on hit masks when they can be had (HITS_*; -1: never)
+// hits_use: run the plan on hit masks when they can be had (HITS_*; -1: never).
+// keep: the launch outlives the call, so its device memory is its own.
 static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query, ExecParams ep, bool annot,
-                    Prepared& P, bool block_items = false, int hits_use = -1) {
+                    Prepared& P, bool block_items = false, int hits_use = -1, bool keep = false) {
   cudaStream_t s = ctx->stream;
   P.query = query;
   P.annot = annot;
@@ -1546,94 +1710,129 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
       P.smem = (size_t)ep.smem_words * 4 * ep.warps;
     }
   }
-  // block items only for the plain triangle COUNT
-  const bool blocks = block_items && !hits && query == EH_QUERY_TRIANGLE && !annot && ep.warps > 1 && !ep.no_block_items;
-  PlanShape shape{ep.chunk, nullptr, 0.0, (uint32_t)ep.smem_words,
-                   blocks ? (uint32_t)ep.smem_words * (uint32_t)ep.warps : 0u, (uint32_t)ep.warps};
-  std::vector<Plan> plans(n);
-  uint32_t total_items = 0, total_b = 0;
-  uint64_t pairs = 0;
-  for (uint32_t g = 0; g < n; g++) {
-    P.plan_launches += build_plan(ctx, tries[g], shape, g, plans[g]);
-    total_items += plans[g].n;
-    total_b += plans[g].nb;
-    pairs += tries[g]->rev_pairs;
-  }
-  P.n_items = total_items;
-  P.n_bitems = total_b;
-  P.pairs = pairs;
-  if (n == 1) {
-    P.items = std::move(plans[0].items);
-  } else {
-    // every graph's block items, then every graph's warp items
-    P.items.alloc(total_items ? total_items : 1, s);
-    uint32_t ob = 0, ow = total_b;
-    for (uint32_t g = 0; g < n; g++) {
-      const uint32_t nb = plans[g].nb, nw = plans[g].n - plans[g].nb;
-      if (nb)
-        EH_CUDA(cudaMemcpyAsync(P.items.p + ob, plans[g].items.p, nb * sizeof(Item), cudaMemcpyDeviceToDevice, s));
-      if (nw)
-        EH_CUDA(cudaMemcpyAsync(P.items.p + ow, plans[g].items.p + nb, nw * sizeof(Item), cudaMemcpyDeviceToDevice,
-                                s));
-      ob += nb;
-      ow += nw;
-    }
-  }
-  std::vector<TrieView> hv(n);
-  std::vector<RevView> hr(n);
-  for (uint32_t g = 0; g < n; g++) {
-    hv[g] = tries[g]->view();
-    hr[g] = rev_view(tries[g]);
-    // the intersection kernels read the values and the bitset words with
-    // 16-byte loads at 16-byte aligned indices
-    if ((reinterpret_cast<uintptr_t>(hv[g].vals) | reinterpret_cast<uintptr_t>(hv[g].bs_words)) & 15u)
-      throw Error{EH_ERR_UNSUPPORTED, "trie arrays are not 16-byte aligned"};
-  }
-  P.view0 = hv[0];
-  P.dv.alloc(n, s);
-  P.dr.alloc(n, s);
-  P.q.alloc(2, s);
-  EH_CUDA(cudaMemcpyAsync(P.dv.p, hv.data(), n * sizeof(TrieView), cudaMemcpyHostToDevice, s));
-  EH_CUDA(cudaMemcpyAsync(P.dr.p, hr.data(), n * sizeof(RevView), cudaMemcpyHostToDevice, s));
   if (hits) set_smem_attr(hits_kernel, P.smem);
   else if (query == EH_QUERY_CLIQUE4) set_smem_attr(clique4_kernel, P.smem);
   else if (annot) set_smem_attr(triangle_kernel<MODE_ANNOT>, P.smem);
   else set_smem_attr(triangle_kernel<MODE_COUNT>, P.smem);
   const int per_sm = blocks_per_sm(kfn, P.threads, P.smem);
-  const uint64_t units = (uint64_t)total_b + (total_items - total_b + ep.warps - 1) / ep.warps;
+  // block items only for the plain triangle COUNT
+  const bool blocks = block_items && !hits && query == EH_QUERY_TRIANGLE && !annot && ep.warps > 1 &&
+                      !ep.no_block_items;
+  // work of all tries, and how finely to cut it: the default item is
+  // kDefaultChunk, and smaller when that would leave resident warps without
+  // work (8 items for each)
+  uint64_t cost = 0, head_items = 0;
+  P.n = n;
+  for (uint32_t g = 0; g < n; g++) {
+    P.entries += tries[g]->rev_entries;
+    P.pairs += tries[g]->rev_pairs;
+    cost += tries[g]->rev_pairs + kRowCost * tries[g]->rev_entries;
+    head_items += std::min<uint64_t>(tries[g]->n_head, tries[g]->rev_entries);
+  }
+  if (!ep.chunk_given) {
+    const uint64_t slots = (uint64_t)num_sms() * per_sm * ep.warps;
+    ep.chunk = (uint32_t)std::min<uint64_t>(kDefaultChunk, std::max<uint64_t>(kMinChunk, cost / (8 * slots)));
+  }
+  PlanShape shape{ep.chunk, nullptr, 0.0, (uint32_t)ep.smem_words,
+                   blocks ? (uint32_t)ep.smem_words * (uint32_t)ep.warps : 0u, (uint32_t)ep.warps};
+  // items: at most one per entry with rows and one per chunk of work (with
+  // predicted costs: per chunk of probes, the sum of rounded-up shares; the
+  // slack covers their rounding)
+  P.cap_w = head_items + (cost / ep.chunk) + cost / ep.chunk / 64 + 64;
+  P.cap_b = blocks ? std::min<uint64_t>(P.cap_w, cost / ((uint64_t)ep.chunk * ep.warps) + cost / kMinBlockWork +
+                                                     cost / ep.chunk / 64 + 64)
+                   : 0;
+  EH_REQUIRE(P.cap_w < (1ull << 32), EH_ERR_UNSUPPORTED, "work plan of 2^32 items or more");
+  const size_t o_views = (P.ctl_bytes() + 127) & ~(size_t)127;
+  const size_t o_rev = o_views + n * sizeof(TrieView);
+  const size_t head_bytes = o_rev + n * sizeof(RevView);
+  uint32_t max_heads = 0;
+  for (uint32_t g = 0; g < n; g++) max_heads = std::max(max_heads, tries[g]->n_head);
+  const size_t o_pos = (head_bytes + 255) & ~(size_t)255;  // the planner's places and tile sums, trie by trie
+  const size_t o_items = o_pos + (((size_t)max_heads + max_heads / kPlanTile + 1) * 8 + 255 & ~(size_t)255);
+  const size_t bytes = o_items + (P.cap_w + P.cap_b) * sizeof(Item);
+  unsigned char* base = keep ? nullptr : workspace(ctx, bytes);
+  if (!base) {
+    P.own.alloc(bytes, s);
+    base = P.own.p;
+  }
+  P.ctl = reinterpret_cast<Control*>(base);
+  P.total = reinterpret_cast<unsigned long long*>(base + sizeof(Control));
+  P.dv = reinterpret_cast<TrieView*>(base + o_views);
+  P.dr = reinterpret_cast<RevView*>(base + o_rev);
+  P.items = reinterpret_cast<Item*>(base + o_items);
+  P.bitems = P.items + P.cap_w;
+  unsigned char* host = pinned(ctx, head_bytes);  // the last user of it has been waited for
+  memset(host, 0, o_views);
+  for (uint32_t g = 0; g < n; g++) {
+    const TrieView v = tries[g]->view();
+    const RevView r = rev_view(tries[g]);
+    memcpy(host + o_views + g * sizeof(TrieView), &v, sizeof(v));
+    memcpy(host + o_rev + g * sizeof(RevView), &r, sizeof(r));
+    // the intersection kernels read the values and the bitset words with
+    // 16-byte loads at 16-byte aligned indices
+    if ((reinterpret_cast<uintptr_t>(v.vals) | reinterpret_cast<uintptr_t>(v.bs_words)) & 15u)
+      throw Error{EH_ERR_UNSUPPORTED, "trie arrays are not 16-byte aligned"};
+    if (!g) P.view0 = v;
+  }
+  EH_CUDA(cudaMemcpyAsync(base, host, head_bytes, cudaMemcpyHostToDevice, s));
+  for (uint32_t g = 0; g < n; g++) {
+    const eh_trie* t = tries[g];
+    if (!t->rev_entries) continue;
+    // every shard of a plan on hit masks runs all the items: the masks split by head entry
+    PlanArgs pa{t->view(), rev_view(t), shape, g, hits ? 0 : ep.shard_index, hits ? 1 : ep.shard_count,
+                reinterpret_cast<uint64_t*>(base + o_pos), nullptr};
+    pa.tiles = pa.pos + t->n_head;
+    if (t->work_pred.p && t->pred_per_probe > 0) {
+      pa.ps.pred = t->work_pred.p;
+      pa.ps.unit = t->pred_per_probe * shape.chunk;
+    }
+    const int tiles = ceil_div(t->n_head, kPlanTile);
+    unsigned long long* total = &P.ctl->spare[1];
+    plan_split_kernel<<<tiles, 256, 0, s>>>(pa);
+    plan_place_kernel<<<tiles, 256, 0, s>>>(pa, total);
+    const uint64_t most = std::min<uint64_t>(t->n_head, t->rev_entries) +
+                          (t->rev_pairs + kRowCost * t->rev_entries) / ep.chunk;
+    plan_fill_kernel<<<(int)std::min<uint64_t>(num_sms() * 8, (most + 255) / 256), 256, 0, s>>>(pa, total, P.ctl,
+                                                                                              P.items, P.bitems);
+    plan_append_kernel<<<1, 1, 0, s>>>(total, P.ctl);
+    EH_CHECK_LAUNCH();
+    P.plan_launches += 4;
+  }
+  const uint64_t units = P.cap_b + (P.cap_w + ep.warps - 1) / ep.warps;
   P.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * per_sm, units));
   if (annot && !hits && n == 1 && tries[0]->dir == DIR_SYM) hot_sets(ctx, tries[0], P.hot);
-  if (query == EH_QUERY_CLIQUE4 && ep.s_cap) {
+  if (query == EH_QUERY_CLIQUE4 && !hits && ep.s_cap) {
     // one S buffer per resident warp, at most 2 GiB in all
     const uint64_t per_block = (uint64_t)ep.warps * ep.s_cap * 4;
     P.grid = std::max(1, (int)std::min<uint64_t>((uint64_t)P.grid, (2ull << 30) / per_block));
     P.gs.alloc((size_t)P.grid * ep.warps * ep.s_cap, s);
   }
   P.ep = ep;
-  EH_CUDA(cudaStreamSynchronize(s));  // host staging vectors go out of scope
 }
 
-// Enqueue one run of a prepared launch: reset the queue, run the persistent
-// kernel.  No host synchronisation: capturable in a CUDA graph.
+// Enqueue one run of a prepared launch; the first follows prepare directly, a
+// later one resets the queues.  No host synchronisation: capturable in a CUDA
+// graph.
 static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, unsigned long long* d_annot,
-                   float* d_records) {
+                   float* d_records, bool again = false) {
   cudaStream_t s = ctx->stream;
-  if (!P.n_items) return;
-  EH_CUDA(cudaMemsetAsync(P.q.p, 0, 8, s));
+  if (!P.entries) return;
+  if (again) EH_CUDA(cudaMemsetAsync(P.ctl->queue, 0, 8, s));
   const ExecParams& ep = P.ep;
   if (P.hits.on) {
     const Hits& H = P.hits;
     const HitsView hv = H.view();
     EH_CUDA(cudaMemsetAsync(H.mask.p, 0, H.words * 4, s));
-    hits_kernel<<<P.grid, P.threads, P.smem, s>>>(P.dv.p, P.dr.p, P.items.p, P.n_items, ep.smem_words, P.q.p, hv,
-                                                  d_records, ep.shard_index, ep.shard_count);
+    hits_kernel<<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, P.ctl->items, ep.smem_words,
+                                                  P.ctl->queue, hv, d_records, ep.shard_index, ep.shard_count);
     EH_CHECK_LAUNCH();
     if (H.use == HITS_CLIQUE) {
-      clique_small_kernel<<<std::min(num_sms() * 8, ceil_div(H.heads, 256)), 256, 0, s>>>(P.dv.p, hv, d_total);
+      clique_small_kernel<<<std::min(num_sms() * 8, ceil_div(H.heads, 256)), 256, 0, s>>>(P.dv, hv, d_total);
       EH_CHECK_LAUNCH();
       if (H.units) {
-        clique_big_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 32)), 256, 0, s>>>(P.dv.p, hv, H.units,
-                                                                                        P.q.p + 1, d_total);
+        clique_big_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 32)), 256, 0, s>>>(
+            P.dv, hv, H.units, P.ctl->queue + 1, d_total);
         EH_CHECK_LAUNCH();
       }
     } else if (H.use == HITS_ANNOT && H.units) {
@@ -1642,31 +1841,27 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
     }
     return;
   }
-  QueryOut out{ep.shard_index, ep.shard_count, ep.long_row, d_total, d_annot, d_records, P.q.p};
-  out.n_bitems = P.n_bitems;
-  out.bqueue = P.q.p + 1;
+  QueryOut out{ep.long_row, d_total, d_annot, d_records, P.ctl->queue, P.ctl->items, P.bitems};
   out.sel = P.sel;
   for (int k = 0; k < kHot; k++) out.hot[k] = P.hot[k];
   out.gsbuf = ep.s_cap ? P.gs.p : nullptr;
   out.gcap = ep.s_cap;
   if (P.query == EH_QUERY_CLIQUE4)
-    clique4_kernel<<<P.grid, P.threads, P.smem, s>>>(P.dv.p, P.dr.p, P.items.p, P.n_items, ep.smem_words, out);
+    clique4_kernel<<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, ep.smem_words, out);
   else if (P.annot)
-    triangle_kernel<MODE_ANNOT><<<P.grid, P.threads, P.smem, s>>>(P.dv.p, P.dr.p, P.items.p, P.n_items, ep.smem_words,
-                                                            out);
+    triangle_kernel<MODE_ANNOT><<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, ep.smem_words, out);
   else
-    triangle_kernel<MODE_COUNT><<<P.grid, P.threads, P.smem, s>>>(P.dv.p, P.dr.p, P.items.p, P.n_items, ep.smem_words,
-                                                             out);
+    triangle_kernel<MODE_COUNT><<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, ep.smem_words, out);
   EH_CHECK_LAUNCH();
 }
 
-// Plan + run + wait; the intersection kernel is timed with events.
+// Plan and run; nothing is waited for.  ev1 and ev2 bracket the intersection
+// kernels.  Results go to d_total (null: P.total; spare: nowhere that is read).
 static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query, ExecParams ep,
-                        bool annot, unsigned long long* d_total, unsigned long long* d_annot, float* d_records,
-                        uint32_t* n_items_out, uint64_t* pairs_out, const uint32_t* sel = nullptr) {
+                        bool annot, Prepared& P, unsigned long long* d_total, unsigned long long* d_annot,
+                        float* d_records, const uint32_t* sel = nullptr, bool spare = false) {
   cudaStream_t s = ctx->stream;
   Launch L;
-  Prepared P;
   {
     TracePhase ph("query.prepare", s);
     // selections weight cliques by their members: they run without masks
@@ -1675,19 +1870,36 @@ static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n
   }
   P.sel = sel;
   L.launches = P.plan_launches;
-  *n_items_out = P.n_items;
-  *pairs_out = P.pairs;
-  if (!P.n_items) return L;
   EH_CUDA(cudaEventRecord(ctx->ev1, s));
   {
     TracePhase ph("query.kernel", s);
-    launch(ctx, P, d_total, d_annot, d_records);
+    launch(ctx, P, spare ? P.ctl->spare : d_total ? d_total : P.total, d_annot, d_records);
   }
   EH_CUDA(cudaEventRecord(ctx->ev2, s));
-  L.launches += P.hits.on ? (P.hits.use == HITS_CLIQUE && P.hits.units ? 3 : 2) : 1;
-  EH_CUDA(cudaEventSynchronize(ctx->ev2));
-  EH_CUDA(cudaEventElapsedTime(&L.kernel_ms, ctx->ev1, ctx->ev2));
+  if (P.entries) L.launches += P.hits.on ? (P.hits.use == HITS_CLIQUE && P.hits.units ? 3 : 2) : 1;
   return L;
+}
+
+// The control block and results of a run, once everything before is done; the
+// query's device time.
+struct Returned {
+  const Control* ctl;
+  const unsigned long long* total;
+  uint64_t items;
+  float query_ms, kernel_ms;
+};
+static Returned finish(eh_context* ctx, const Prepared& P) {
+  cudaStream_t s = ctx->stream;
+  unsigned char* host = pinned(ctx, P.ctl_bytes());
+  EH_CUDA(cudaMemcpyAsync(host, P.ctl, P.ctl_bytes(), cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaEventRecord(ctx->ev3, s));
+  EH_CUDA(cudaEventSynchronize(ctx->ev3));
+  Returned r{reinterpret_cast<const Control*>(host),
+             reinterpret_cast<const unsigned long long*>(host + sizeof(Control)), 0, 0, 0};
+  r.items = (uint64_t)r.ctl->items[0] + r.ctl->items[1];
+  EH_CUDA(cudaEventElapsedTime(&r.query_ms, ctx->ev0, ctx->ev3));
+  if (P.entries) EH_CUDA(cudaEventElapsedTime(&r.kernel_ms, ctx->ev1, ctx->ev2));
+  return r;
 }
 
 // Algorithmic bytes of the triangle plan: both uint32 inputs of every
@@ -1695,12 +1907,12 @@ static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n
 // 4 * sum over rows (a,b) of (d(a) + d(b)) = 4 * (sum_a d(a)^2 + wedges).
 static uint64_t triangle_algorithmic_bytes(const eh_trie* t) { return 4 * (t->sum_sq_deg + t->total_wedges); }
 
-static void fill_stats(eh_query_stats* st, float query_ms, const Launch& L, uint32_t items, uint64_t pairs,
-                       uint64_t alg) {
+static void fill_stats(eh_query_stats* st, float query_ms, float kernel_ms, uint32_t launches, uint64_t items,
+                       uint64_t pairs, uint64_t alg) {
   if (!st) return;
   st->query_ms = query_ms;
-  st->kernel_ms = L.kernel_ms;
-  st->launches = L.launches;
+  st->kernel_ms = kernel_ms;
+  st->launches = launches;
   st->work_items = items;
   st->wedges = pairs;
   st->algorithmic_bytes = alg;
@@ -1717,7 +1929,7 @@ static uint32_t root_bag(eh_context* ctx, const eh_trie* t, int query, const uns
   if (!t->n_head) return 0;
   uint32_t launches = 0;
   if (query == EH_QUERY_LOLLIPOP) {
-    root_kernel<false><<<num_sms() * 8, 256, 0, s>>>(t->view(), T, nullptr, total);
+    root_kernel<false><<<num_sms() * 8, 256, 0, s>>>(t->view(), T, nullptr, total, nullptr, nullptr);
     EH_CHECK_LAUNCH();
     return 1;
   }
@@ -1729,26 +1941,19 @@ static uint32_t root_bag(eh_context* ctx, const eh_trie* t, int query, const uns
     Tv = tv.p;
     launches++;
   }
-  root_kernel<true><<<num_sms() * 8, 256, 0, s>>>(t->view(), T, Tv, total);
+  DevBuf<uint32_t> big;
+  const bool has_big = t->info.max_set > kRootBig;
+  if (has_big) {
+    big.alloc((size_t)t->n_head + 1, s);  // their number, then the entries
+    EH_CUDA(cudaMemsetAsync(big.p, 0, 4, s));
+  }
+  root_kernel<true><<<num_sms() * 8, 256, 0, s>>>(t->view(), T, Tv, total, big.p + 1, big.p);
   EH_CHECK_LAUNCH();
   launches++;
-  if (t->info.max_set > kRootBig) {
-    DevBuf<uint32_t> idx(t->n_head, s);
-    DevBuf<unsigned int> nb(1, s);
-    EH_CUDA(cudaMemsetAsync(nb.p, 0, 4, s));
-    root_big_sets_kernel<<<num_sms() * 4, 256, 0, s>>>(t->view(), idx.p, nb.p);
+  if (has_big) {
+    root_big_kernel<<<num_sms() * 4, 256, 0, s>>>(t->view(), big.p + 1, big.p, T, Tv, total);
     EH_CHECK_LAUNCH();
-    unsigned int hn = 0;
-    EH_CUDA(cudaMemcpyAsync(&hn, nb.p, 4, cudaMemcpyDeviceToHost, s));
-    EH_CUDA(cudaStreamSynchronize(s));
-    std::vector<uint32_t> big(hn);
-    if (hn) EH_CUDA(cudaMemcpyAsync(big.data(), idx.p, 4ull * hn, cudaMemcpyDeviceToHost, s));
-    EH_CUDA(cudaStreamSynchronize(s));
-    for (uint32_t a : big) {
-      root_big_kernel<<<num_sms() * 4, 256, 0, s>>>(t->view(), a, T, Tv, total);
-      EH_CHECK_LAUNCH();
-    }
-    launches += 1 + hn;
+    launches++;
   }
   return launches;
 }
@@ -1801,6 +2006,18 @@ void query_weighted_root(eh_context* ctx, const eh_trie* t, int query, const uin
   *result = h;
 }
 
+// A call that uses the context's workspace: one at a time per context, and a
+// failing one leaves none of its work in flight.
+struct Call {
+  eh_context* ctx;
+  std::lock_guard<std::recursive_mutex> lock;
+  int before;
+  explicit Call(eh_context* c) : ctx(c), lock(c->mu), before(std::uncaught_exceptions()) {}
+  ~Call() {
+    if (std::uncaught_exceptions() > before) cudaStreamSynchronize(ctx->stream);
+  }
+};
+
 // The annotated pass's per-head counters take one global atomic per hit
 // (2.8 G on Chung-Lu 2^23).  Measured on B200 (Chung-Lu 2^23 lollipop): with
 // the counters in the stream-ordered pool the pass ran at 243 or 184 ms
@@ -1834,47 +2051,34 @@ void query_count_batched(eh_context* ctx, const eh_trie* const* tries, uint32_t 
     EH_REQUIRE(tries[g]->ctx == ctx, EH_ERR_INVALID, "trie belongs to another context");
   }
   ExecParams ep = exec_params(cfg);
+  Call call(ctx);
   TracePhase ph_all("query.total", s);
   EH_CUDA(cudaEventRecord(ctx->ev0, s));
-  DevBuf<unsigned long long> total(n, s);
-  EH_CUDA(cudaMemsetAsync(total.p, 0, n * 8, s));
-  uint32_t items = 0;
-  uint64_t pairs = 0;
+  Prepared P;
   Launch L;
   DevBuf<float> rec;
   const bool record = cfg && cfg->record_timings && n == 1;
+  if (record) {
+    // one record per item; the plan size is known only after planning, so
+    // size for the worst case, as prepare does for the items; fixed chunks
+    ep.chunk_given = true;
+    const uint64_t cost = tries[0]->rev_pairs + kRowCost * tries[0]->rev_entries;
+    rec.alloc(8 * (tries[0]->n_head + 2 * (cost / ep.chunk + cost / ep.chunk / 32) + 256), s);
+  }
   if (query == EH_QUERY_TRIANGLE || query == EH_QUERY_CLIQUE4) {
-    float* recp = nullptr;
-    if (record) {
-      // one record per item; the plan size is known only after planning, so
-      // size for the worst case of one item per head entry plus splits
-      const uint64_t cap = tries[0]->n_head + tries[0]->rev_pairs / ep.chunk + 16;
-      rec.alloc(8 * cap, s);
-      recp = rec.p;
-    }
-    L = run_plans(ctx, tries, n, query, ep, false, total.p, nullptr, recp, &items, &pairs);
+    L = run_plans(ctx, tries, n, query, ep, false, P, nullptr, nullptr, rec.p);
   } else {
     EH_REQUIRE(n == 1, EH_ERR_UNSUPPORTED, "batched lollipop/barbell is not supported");
     const eh_trie* t = tries[0];
     EH_REQUIRE(ep.shard_count == 1, EH_ERR_UNSUPPORTED, "lollipop/barbell run unsharded");
-    float* recp = nullptr;
-    if (record) {  // the annotated triangle pass's items (the root bag is not logged)
-      rec.alloc(8 * (t->n_head + t->rev_pairs / ep.chunk + 16), s);
-      recp = rec.p;
-    }
     unsigned long long* T = annot_buffer(ctx, t->n_head ? t->n_head : 1);
-    DevBuf<unsigned long long> dummy(1, s);
     EH_CUDA(cudaMemsetAsync(T, 0, (t->n_head ? t->n_head : 1) * 8, s));
-    EH_CUDA(cudaMemsetAsync(dummy.p, 0, 8, s));
-    L = run_plans(ctx, tries, 1, EH_QUERY_TRIANGLE, ep, true, dummy.p, T, recp, &items, &pairs);
-    L.launches += root_bag(ctx, t, query, T, nullptr, total.p);
+    // the annotated pass (recorded), then the root bag over T into P.total
+    L = run_plans(ctx, tries, 1, EH_QUERY_TRIANGLE, ep, true, P, nullptr, T, rec.p, nullptr, true);
+    L.launches += root_bag(ctx, t, query, T, nullptr, P.total);
   }
-  std::vector<unsigned long long> h(n);
-  EH_CUDA(cudaMemcpyAsync(h.data(), total.p, n * 8, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaEventRecord(ctx->ev2, s));
-  EH_CUDA(cudaEventSynchronize(ctx->ev2));
-  float qms = 0;
-  EH_CUDA(cudaEventElapsedTime(&qms, ctx->ev0, ctx->ev2));
+  const Returned got = finish(ctx, P);
+  const unsigned long long* h = got.total;
   for (uint32_t g = 0; g < n; g++) {
     uint64_t v = h[g];
     const int dir = tries[g]->dir;
@@ -1885,13 +2089,14 @@ void query_count_batched(eh_context* ctx, const eh_trie* const* tries, uint32_t 
     results[g] = v;
   }
   if (record) {
-    ctx->timing_records.resize(8 * (size_t)items);
-    if (items)
-      EH_CUDA(cudaMemcpy(ctx->timing_records.data(), rec.p, 8 * (size_t)items * sizeof(float), cudaMemcpyDeviceToHost));
+    ctx->timing_records.resize(8 * (size_t)got.items);
+    if (got.items)
+      EH_CUDA(cudaMemcpy(ctx->timing_records.data(), rec.p, 8 * (size_t)got.items * sizeof(float),
+                         cudaMemcpyDeviceToHost));
   }
   uint64_t alg = 0;
   for (uint32_t g = 0; g < n; g++) alg += triangle_algorithmic_bytes(tries[g]);
-  fill_stats(stats, qms, L, items, pairs, alg);
+  fill_stats(stats, got.query_ms, got.kernel_ms, L.launches, got.items, P.pairs, alg);
 }
 
 void query_count(eh_context* ctx, const eh_trie* t, int query, const eh_exec_config* cfg, uint64_t* result,
@@ -1905,14 +2110,12 @@ void triangle_annotation(eh_context* ctx, const eh_trie* t, const eh_exec_config
   ExecParams ep = exec_params(cfg);
   ep.shard_index = 0;
   ep.shard_count = 1;
-  DevBuf<unsigned long long> dummy(1, s);
+  Call call(ctx);
   EH_CUDA(cudaMemsetAsync(annot_dev, 0, (t->n_head ? t->n_head : 1) * 8, s));
-  EH_CUDA(cudaMemsetAsync(dummy.p, 0, 8, s));
-  uint32_t items;
-  uint64_t pairs;
   const eh_trie* ts[1] = {t};
-  run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, true, dummy.p, (unsigned long long*)annot_dev, nullptr, &items,
-            &pairs);
+  Prepared P;
+  run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, true, P, nullptr, (unsigned long long*)annot_dev, nullptr, nullptr,
+            true);
   EH_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -1985,6 +2188,7 @@ void query_count_select(eh_context* ctx, const eh_trie* t, int query, uint32_t v
   ExecParams ep = exec_params(cfg);
   EH_REQUIRE(ep.shard_count == 1, EH_ERR_UNSUPPORTED, "selection plans run unsharded");
   const bool clique = query == EH_QUERY_CLIQUE4_SEL;
+  Call call(ctx);
   EH_CUDA(cudaEventRecord(ctx->ev0, s));
   DevBuf<unsigned long long> sums(4, s);  // partner sum, N(v) sum, partners, plan total
   EH_CUDA(cudaMemsetAsync(sums.p, 0, 32, s));
@@ -2010,32 +2214,34 @@ void query_count_select(eh_context* ctx, const eh_trie* t, int query, uint32_t v
   EH_CUDA(cudaStreamSynchronize(s));
   EH_REQUIRE(hv >= 0 || h[2] > 0, EH_ERR_INVALID,
              "selection value " + std::to_string(value) + " is not in the relation");
-  uint32_t items = 0;
-  uint64_t pairs = 0;
+  uint64_t items = 0, pairs = 0;
+  float kernel_ms = 0;
   const eh_trie* ts[1] = {t};
   uint64_t v = 0;
   if (h[2] > 0) {  // no partners: the selected bag is empty and so is the join
     if (clique) {
-      Launch K = run_plans(ctx, ts, 1, EH_QUERY_CLIQUE4, ep, false, sums.p + 3, nullptr, nullptr, &items, &pairs,
-                           bits.p);
-      L.launches += K.launches;
-      L.kernel_ms = K.kernel_ms;
-      EH_CUDA(cudaMemcpyAsync(h, sums.p, 32, cudaMemcpyDeviceToHost, s));
-      EH_CUDA(cudaStreamSynchronize(s));
-      v = h[3];
+      Prepared P;
+      L.launches += run_plans(ctx, ts, 1, EH_QUERY_CLIQUE4, ep, false, P, nullptr, nullptr, nullptr, bits.p).launches;
+      const Returned got = finish(ctx, P);
+      items = got.items;
+      pairs = P.pairs;
+      kernel_ms = got.kernel_ms;
+      v = got.total[0];
       if (t->dir == DIR_SYM) v *= 6ull;  // 3! orderings start at each selected member
     } else if (hv >= 0) {
-      DevBuf<unsigned long long> T(t->n_head, s), dummy(1, s);
+      DevBuf<unsigned long long> T(t->n_head, s);
       EH_CUDA(cudaMemsetAsync(T.p, 0, (size_t)t->n_head * 8, s));
-      EH_CUDA(cudaMemsetAsync(dummy.p, 0, 8, s));
       EH_CUDA(cudaMemsetAsync(sums.p, 0, 32, s));
-      Launch K = run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, true, dummy.p, T.p, nullptr, &items, &pairs);
+      Prepared P;
+      const Launch K = run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, true, P, nullptr, T.p, nullptr, nullptr, true);
       select_partners_kernel<<<sgrid, 256, 0, s>>>(t->view(), value, nullptr, T.p, sums.p);
       EH_CHECK_LAUNCH();
       L.launches += K.launches + 1;
-      L.kernel_ms = K.kernel_ms;
       EH_CUDA(cudaMemcpyAsync(h, sums.p, 32, cudaMemcpyDeviceToHost, s));
-      EH_CUDA(cudaStreamSynchronize(s));
+      const Returned got = finish(ctx, P);
+      items = got.items;
+      pairs = P.pairs;
+      kernel_ms = got.kernel_ms;
       v = (uint64_t)h[0] * (uint64_t)h[1];
     }
   }
@@ -2044,7 +2250,7 @@ void query_count_select(eh_context* ctx, const eh_trie* t, int query, uint32_t v
   float qms = 0;
   EH_CUDA(cudaEventElapsedTime(&qms, ctx->ev0, ctx->ev2));
   *result = v;
-  fill_stats(stats, qms, L, items, pairs, triangle_algorithmic_bytes(t));
+  fill_stats(stats, qms, kernel_ms, L.launches, items, pairs, triangle_algorithmic_bytes(t));
 }
 
 // ------------------------------------------------------------ materialize
@@ -2145,7 +2351,7 @@ static bool materialize_hits(eh_context* ctx, const eh_trie* t, const eh_exec_co
   prepare(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, false, P, false, HITS_ROWS);
   if (!P.hits.on) return false;
   *n_rows = 0;
-  if (!P.n_items) return true;
+  if (!P.entries) return true;
   launch(ctx, P, nullptr, nullptr, nullptr);
   DevBuf<uint32_t> seg(t->rows, s);
   DevBuf<uint64_t> pos(t->rows, s), tot(1, s);
@@ -2178,6 +2384,7 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   EH_REQUIRE(query == EH_QUERY_TRIANGLE, EH_ERR_UNSUPPORTED, "materialized output is built for the triangle plan");
   EH_REQUIRE(n_cols == 2 || n_cols == 3, EH_ERR_INVALID, "n_cols must be 3 (a,b,c) or 2 (projection on a,b)");
   EH_REQUIRE(t->ctx == ctx, EH_ERR_INVALID, "trie belongs to another context");
+  Call call(ctx);
   if (n_cols == 2) {
     query_project_ab(ctx, t, ha, hb, cap, n_rows);
     return;
@@ -2196,18 +2403,17 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   const eh_trie* ts[1] = {t};
   prepare(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, false, P);
   set_smem_attr(triangle_kernel<MODE_MAT>, P.smem);
-  DevBuf<unsigned long long> counts(P.n_items ? P.n_items : 1, s), offs(P.n_items ? P.n_items : 1, s),
-      total(1, s), rows(1, s);
-  EH_CUDA(cudaMemsetAsync(total.p, 0, 8, s));
+  unsigned int n_items = 0;
+  EH_CUDA(cudaMemcpyAsync(&n_items, P.ctl->items, 4, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaStreamSynchronize(s));
+  DevBuf<unsigned long long> counts(n_items ? n_items : 1, s), offs(n_items ? n_items : 1, s), rows(1, s);
   const uint32_t mult = t->dir == DIR_SYM ? 6u : 1u;
-  QueryOut out{0, 1, P.ep.long_row, total.p, nullptr, nullptr, P.q.p};
+  QueryOut out{P.ep.long_row, P.total, nullptr, nullptr, P.ctl->queue, P.ctl->items, P.bitems};
   out.item_counts = counts.p;
   out.count_mult = mult;
-  EH_CUDA(cudaMemsetAsync(P.q.p, 0, 8, s));
-  triangle_kernel<MODE_COUNT><<<P.grid, P.threads, P.smem, s>>>(P.dv.p, P.dr.p, P.items.p, P.n_items,
-                                                                P.ep.smem_words, out);
+  triangle_kernel<MODE_COUNT><<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, P.ep.smem_words, out);
   EH_CHECK_LAUNCH();
-  exclusive_scan<uint64_t>((const uint64_t*)counts.p, (uint64_t*)offs.p, P.n_items, (uint64_t*)rows.p, s);
+  exclusive_scan<uint64_t>((const uint64_t*)counts.p, (uint64_t*)offs.p, n_items, (uint64_t*)rows.p, s);
   uint64_t nr = 0;
   EH_CUDA(cudaMemcpyAsync(&nr, rows.p, 8, cudaMemcpyDeviceToHost, s));
   EH_CUDA(cudaStreamSynchronize(s));
@@ -2218,9 +2424,8 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   out.ma = ma.p;
   out.mb = mb.p;
   out.mc = mc.p;
-  EH_CUDA(cudaMemsetAsync(P.q.p, 0, 8, s));
-  triangle_kernel<MODE_MAT><<<P.grid, P.threads, P.smem, s>>>(P.dv.p, P.dr.p, P.items.p, P.n_items,
-                                                              P.ep.smem_words, out);
+  EH_CUDA(cudaMemsetAsync(P.ctl->queue, 0, 8, s));
+  triangle_kernel<MODE_MAT><<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, P.ep.smem_words, out);
   EH_CHECK_LAUNCH();
   // order by (a, b, c): stable sort by c, then stable sort by (a, b)
   const int grid = num_sms() * 8;
@@ -2282,13 +2487,12 @@ void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const 
   // carve the scratch
   const uint32_t nh = t->n_head;
   const uint64_t scan_elems = scan_scratch_elems(nh);
-  const size_t off_ctrl = 0;  // u32 queue, u32 unused, u64 total
+  const size_t off_ctrl = 0;  // u32 queue[2], u64 total, u32 items[2]
   const size_t off_tv = 256;
   const size_t off_rv = align256(off_tv + sizeof(TrieView));
   const size_t off_nitems = align256(off_rv + sizeof(RevView));
   const size_t off_ipos = align256(off_nitems + 4ull * nh);
-  const size_t off_tot = align256(off_ipos + 4ull * nh);
-  const size_t off_scan = align256(off_tot + 4);
+  const size_t off_scan = align256(off_ipos + 4ull * nh);
   const size_t off_items = align256(off_scan + 4ull * scan_elems);
   EH_REQUIRE(off_items <= bytes, EH_ERR_UNSUPPORTED,
              "trie too large for the allocation-free path: its planner needs " + std::to_string(off_items) +
@@ -2299,11 +2503,11 @@ void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const 
   RevView* dr = reinterpret_cast<RevView*>(scratch + off_rv);
   uint32_t* nitems = reinterpret_cast<uint32_t*>(scratch + off_nitems);
   uint32_t* ipos = reinterpret_cast<uint32_t*>(scratch + off_ipos);
-  uint32_t* tot = reinterpret_cast<uint32_t*>(scratch + off_tot);
+  uint32_t* tot = reinterpret_cast<uint32_t*>(scratch + off_ctrl + 16);  // items: warp items, no block items
   uint32_t* scan_tmp = reinterpret_cast<uint32_t*>(scratch + off_scan);
   Item* items = reinterpret_cast<Item*>(scratch + off_items);
   // the array keeps the previous call's contents: zero what must start at 0
-  EH_CUDA(cudaMemsetAsync(scratch + off_ctrl, 0, 16, s));
+  EH_CUDA(cudaMemsetAsync(scratch + off_ctrl, 0, 24, s));
   const TrieView hv = t->view();
   const RevView hr = rev_view(t);
   EH_CUDA(cudaMemcpyAsync(dv, &hv, sizeof(TrieView), cudaMemcpyHostToDevice, s));
@@ -2336,15 +2540,15 @@ void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const 
     gsbuf = reinterpret_cast<uint32_t*>(scratch + items_end);
   }
   if (n_items) {
-    plan_fill_kernel<<<pgrid, 256, 0, s>>>(hr, nh, nitems, ipos, n_items, 0, items);
+    plan_fill_scratch_kernel<<<pgrid, 256, 0, s>>>(hr, nh, nitems, ipos, n_items, 0, items);
     EH_CHECK_LAUNCH();
-    QueryOut out{0, 1, ep.long_row, total, nullptr, nullptr, queue};
+    QueryOut out{ep.long_row, total, nullptr, nullptr, queue, tot};
     out.gsbuf = gsbuf;
     out.gcap = ep.s_cap;
     if (clique)
-      clique4_kernel<<<grid, threads, smem, s>>>(dv, dr, items, n_items, ep.smem_words, out);
+      clique4_kernel<<<grid, threads, smem, s>>>(dv, dr, items, ep.smem_words, out);
     else
-      triangle_kernel<MODE_COUNT><<<grid, threads, smem, s>>>(dv, dr, items, n_items, ep.smem_words, out);
+      triangle_kernel<MODE_COUNT><<<grid, threads, smem, s>>>(dv, dr, items, ep.smem_words, out);
     EH_CHECK_LAUNCH();
   }
   unsigned long long h = 0;
@@ -2364,10 +2568,10 @@ void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const 
 struct eh_batch {
   eh_context* ctx = nullptr;
   eh::Prepared P;
-  eh::DevBuf<unsigned long long> total;
   unsigned long long* host = nullptr;  // pinned
   std::vector<int> dirs;
   uint32_t n = 0;
+  uint64_t items = 0;
   int query = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -2389,22 +2593,25 @@ eh_batch* batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n,
   ExecParams ep = exec_params(cfg);
   for (uint32_t g = 0; g < n; g++)
     EH_REQUIRE(tries[g] && tries[g]->ctx == ctx, EH_ERR_INVALID, "null trie or trie of another context");
+  Call call(ctx);
   auto* b = new eh_batch();
   try {
     b->ctx = ctx;
     b->n = n;
     b->query = query;
     for (uint32_t g = 0; g < n; g++) b->dirs.push_back(tries[g]->dir);
-    prepare(ctx, tries, n, query, ep, false, b->P, true, query == EH_QUERY_CLIQUE4 ? HITS_CLIQUE : -1);
-    b->total.alloc(n, s);
+    prepare(ctx, tries, n, query, ep, false, b->P, true, query == EH_QUERY_CLIQUE4 ? HITS_CLIQUE : -1, true);
+    unsigned int items[2] = {0, 0};
+    EH_CUDA(cudaMemcpyAsync(items, b->P.ctl->items, 8, cudaMemcpyDeviceToHost, s));
     EH_CUDA(cudaMallocHost((void**)&b->host, n * sizeof(unsigned long long)));
     EH_CUDA(cudaStreamSynchronize(s));
+    b->items = (uint64_t)items[0] + items[1];
     EH_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaError_t cap = cudaSuccess;
     try {
-      EH_CUDA(cudaMemsetAsync(b->total.p, 0, n * 8, s));
-      launch(ctx, b->P, b->total.p, nullptr, nullptr);
-      EH_CUDA(cudaMemcpyAsync(b->host, b->total.p, n * 8, cudaMemcpyDeviceToHost, s));
+      EH_CUDA(cudaMemsetAsync(b->P.total, 0, n * 8, s));
+      launch(ctx, b->P, b->P.total, nullptr, nullptr, true);
+      EH_CUDA(cudaMemcpyAsync(b->host, b->P.total, n * 8, cudaMemcpyDeviceToHost, s));
     } catch (...) {
       cudaGraph_t g = nullptr;
       cudaStreamEndCapture(s, &g);
@@ -2424,6 +2631,7 @@ eh_batch* batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n,
 void batch_run(eh_context* ctx, eh_batch* b, uint64_t* results, eh_query_stats* stats) {
   cudaStream_t s = ctx->stream;
   EH_REQUIRE(b->ctx == ctx, EH_ERR_INVALID, "batch belongs to another context");
+  Call call(ctx);
   EH_CUDA(cudaEventRecord(ctx->ev0, s));
   EH_CUDA(cudaGraphLaunch(b->exec, s));
   EH_CUDA(cudaEventRecord(ctx->ev2, s));
@@ -2439,7 +2647,7 @@ void batch_run(eh_context* ctx, eh_batch* b, uint64_t* results, eh_query_stats* 
     stats->query_ms = ms;
     stats->kernel_ms = ms;
     stats->launches = 1;
-    stats->work_items = b->P.n_items;
+    stats->work_items = b->items;
     stats->wedges = b->P.pairs;
     stats->algorithmic_bytes = 0;
   }
