@@ -1,5 +1,6 @@
 // Internal types shared by the engine's translation units.
 #pragma once
+#include <exception>
 #include <mutex>
 #include <vector>
 
@@ -137,6 +138,24 @@ struct eh_model {
 };
 
 namespace eh {
+
+// A call that uses the context's workspace: one at a time per context, and a
+// failing one leaves none of its work in flight.
+struct Call {
+  eh_context* ctx;
+  std::lock_guard<std::recursive_mutex> lock;
+  int before;
+  explicit Call(eh_context* c) : ctx(c), lock(c->mu), before(std::uncaught_exceptions()) {}
+  ~Call() {
+    if (std::uncaught_exceptions() > before) cudaStreamSynchronize(ctx->stream);
+  }
+};
+
+// Small memory of a context kept from call to call (eh_query.cu), used under a
+// Call; workspace is null past its limit or without memory
+unsigned char* workspace(eh_context* ctx, size_t bytes);
+unsigned char* pinned(eh_context* ctx, size_t bytes);
+
 
 // graph input pipeline (eh_graph.cu)
 void gen_er(cudaStream_t s, uint64_t seed, uint32_t n, uint64_t m, uint32_t* u, uint32_t* v);

@@ -16,7 +16,6 @@
 // an atomic queue, heaviest b first.
 #include <algorithm>
 #include <cstring>
-#include <exception>
 
 #include "eh_internal.cuh"
 
@@ -1501,7 +1500,7 @@ static void set_smem_attr(K kernel, size_t smem) {
 // control block.  Past kMaxWorkspace a call allocates and frees its own.  Not in
 // the stream-ordered pool: what a call took there goes back with it.
 constexpr size_t kMaxWorkspace = 64ull << 20;
-static unsigned char* workspace(eh_context* ctx, size_t bytes) {
+unsigned char* workspace(eh_context* ctx, size_t bytes) {
   if (bytes > kMaxWorkspace) return nullptr;
   if (bytes > ctx->work_cap) {
     EH_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1517,7 +1516,7 @@ static unsigned char* workspace(eh_context* ctx, size_t bytes) {
   }
   return ctx->work;
 }
-static unsigned char* pinned(eh_context* ctx, size_t bytes) {
+unsigned char* pinned(eh_context* ctx, size_t bytes) {
   if (bytes > ctx->pinned_cap) {
     EH_CUDA(cudaStreamSynchronize(ctx->stream));
     if (ctx->pinned) EH_CUDA(cudaFreeHost(ctx->pinned));
@@ -2005,18 +2004,6 @@ void query_weighted_root(eh_context* ctx, const eh_trie* t, int query, const uin
   EH_CUDA(cudaStreamSynchronize(s));
   *result = h;
 }
-
-// A call that uses the context's workspace: one at a time per context, and a
-// failing one leaves none of its work in flight.
-struct Call {
-  eh_context* ctx;
-  std::lock_guard<std::recursive_mutex> lock;
-  int before;
-  explicit Call(eh_context* c) : ctx(c), lock(c->mu), before(std::uncaught_exceptions()) {}
-  ~Call() {
-    if (std::uncaught_exceptions() > before) cudaStreamSynchronize(ctx->stream);
-  }
-};
 
 // The annotated pass's per-head counters take one global atomic per hit
 // (2.8 G on Chung-Lu 2^23).  Measured on B200 (Chung-Lu 2^23 lollipop): with
