@@ -78,10 +78,7 @@ struct eh_trie {
   eh::DevBuf<uint32_t> bb_id;
   eh::DevBuf<uint32_t> bb_rank;
   eh::DevBuf<uint64_t> bb_words;
-  // per head entry: sum over children v of d+(v) (wedge count), computed
-  // once per trie for planning the generic-join loops
-  eh::DevBuf<uint64_t> wedges;
-  uint64_t total_wedges = 0;
+  uint64_t total_wedges = 0;  // sum over rows (a,b) of |N(b)|
   uint64_t sum_sq_deg = 0;  // sum over head entries of |N(a)|^2
   // Direction of the relation, decided at build: every row goes up
   // (col0 < col1), every row goes down, the relation is symmetric, or none.

@@ -23,23 +23,125 @@ __global__ void pack_rows_kernel(const uint32_t* __restrict__ c0, const uint32_t
     keys[i] = ((uint64_t)c0[i] << b) | c1[i];
 }
 
-__global__ void head_flag_kernel(const uint64_t* __restrict__ keys, uint64_t n, int b, uint32_t* __restrict__ flag) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    flag[i] = (i == 0 || (keys[i] >> b) != (keys[i - 1] >> b)) ? 1u : 0u;
+// What the build has to know of its columns, in one pass: the largest value of
+// each, and whether a row is below the one before it.
+// Rows that arrive in order (an encoded relation, an exported one) are not
+// sorted again.
+struct ColumnStats {
+  unsigned int max0, max1, unsorted, pad;
+};
+__global__ void __launch_bounds__(256) column_stats_kernel(const uint32_t* __restrict__ c0,
+                                                           const uint32_t* __restrict__ c1, uint64_t n,
+                                                           ColumnStats* __restrict__ out) {
+  uint32_t m0 = 0, m1 = 0;
+  bool unsorted = false;
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+    const uint32_t a = c0[i], b = c1[i];
+    const uint32_t pa = i ? c0[i - 1] : 0u, pb = i ? c1[i - 1] : 0u;
+    m0 = max(m0, a);
+    m1 = max(m1, b);
+    unsorted |= pa > a || (pa == a && pb > b);  // nothing is below (0, 0)
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m0 = max(m0, __shfl_xor_sync(kFull, m0, o));
+    m1 = max(m1, __shfl_xor_sync(kFull, m1, o));
+  }
+  const bool u = __any_sync(kFull, unsorted);
+  if (lane_id() == 0) {
+    atomicMax(&out->max0, m0);
+    atomicMax(&out->max1, m1);
+    if (u) atomicOr(&out->unsorted, 1u);
+  }
 }
 
-__global__ void csr_kernel(const uint64_t* __restrict__ keys, uint64_t n, int b, const uint32_t* __restrict__ hpos,
-                           uint32_t* __restrict__ head, uint64_t* __restrict__ off, uint32_t* __restrict__ vals) {
-  const uint64_t mask = (1ull << b) - 1;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = keys[i];
-    vals[i] = (uint32_t)(k & mask);
-    if (i == 0 || (k >> b) != (keys[i - 1] >> b)) {
-      head[hpos[i]] = (uint32_t)(k >> b);
-      off[hpos[i]] = i;
+// Rows in order, from packed keys or straight from the columns.
+struct KeyRows {
+  const uint64_t* keys;
+  int b;
+  __device__ __forceinline__ uint32_t head(uint64_t i) const { return (uint32_t)(keys[i] >> b); }
+  __device__ __forceinline__ uint32_t val(uint64_t i) const { return (uint32_t)(keys[i] & ((1ull << b) - 1)); }
+};
+struct ColumnRows {
+  const uint32_t *c0, *c1;
+  __device__ __forceinline__ uint32_t head(uint64_t i) const { return c0[i]; }
+  __device__ __forceinline__ uint32_t val(uint64_t i) const { return c1[i]; }
+};
+// 1: a row not seen before it, 2: and of a new head value
+template <typename R>
+__device__ __forceinline__ uint32_t row_kind(const R& r, uint64_t i) {
+  if (i == 0) return 3;
+  if (r.head(i) != r.head(i - 1)) return 3;
+  return r.val(i) != r.val(i - 1) ? 1 : 0;
+}
+
+// CSR of ordered rows (repeats allowed) in two passes over them with a scan of
+// the tiles' counts (rows low, heads high) between: no flag or position per row
+// is stored.
+constexpr int kCsrThreads = 256, kCsrItems = 8, kCsrTile = kCsrThreads * kCsrItems;
+template <typename R>
+__global__ void __launch_bounds__(kCsrThreads) csr_count_kernel(R r, uint64_t n, uint64_t* __restrict__ tiles) {
+  __shared__ uint64_t tot[kCsrThreads / 32];
+  const uint64_t base = (uint64_t)blockIdx.x * kCsrTile;
+  uint32_t rows = 0, heads = 0;
+#pragma unroll
+  for (int k = 0; k < kCsrItems; k++) {
+    const uint64_t i = base + (uint64_t)k * kCsrThreads + threadIdx.x;
+    const uint32_t kind = i < n ? row_kind(r, i) : 0;
+    rows += kind & 1;
+    heads += kind >> 1;
+  }
+  uint64_t c = warp_sum((uint64_t)heads << 32 | rows);
+  if (lane_id() == 0) tot[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kCsrThreads / 32; w++) c += tot[w];
+    tiles[blockIdx.x] = c;
+  }
+}
+template <typename R>
+__global__ void __launch_bounds__(kCsrThreads) csr_write_kernel(R r, uint64_t n, const uint64_t* __restrict__ tiles,
+                                                                uint32_t* __restrict__ head, uint64_t* __restrict__ off,
+                                                                uint32_t* __restrict__ vals) {
+  __shared__ uint64_t cnt[kCsrItems * kCsrThreads / 32];  // per round and warp, in row order
+  const uint64_t base = (uint64_t)blockIdx.x * kCsrTile;
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  uint32_t hv[kCsrItems], vv[kCsrItems], rows[kCsrItems], heads[kCsrItems];
+#pragma unroll
+  for (int k = 0; k < kCsrItems; k++) {
+    const uint64_t i = base + (uint64_t)k * kCsrThreads + threadIdx.x;
+    const uint32_t kind = i < n ? row_kind(r, i) : 0;
+    hv[k] = i < n ? r.head(i) : 0;
+    vv[k] = i < n ? r.val(i) : 0;
+    rows[k] = __ballot_sync(kFull, kind & 1);
+    heads[k] = __ballot_sync(kFull, kind >> 1);
+    if (lane == 0) cnt[k * (kCsrThreads / 32) + wid] = (uint64_t)__popc(heads[k]) << 32 | __popc(rows[k]);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    static_assert(kCsrItems * kCsrThreads / 32 == 64, "two counts per lane");
+    const uint64_t a = cnt[2 * lane], b = cnt[2 * lane + 1];
+    const uint64_t incl = warp_incl_scan(a + b);
+    cnt[2 * lane] = incl - a - b;
+    cnt[2 * lane + 1] = incl - b;
+  }
+  __syncthreads();
+  const uint64_t t0 = tiles[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < kCsrItems; k++) {
+    const uint64_t at = t0 + cnt[k * (kCsrThreads / 32) + wid];
+    const uint64_t p = (uint32_t)at + __popc(rows[k] & lanemask_lt());
+    if ((rows[k] >> lane) & 1u) vals[p] = vv[k];
+    if ((heads[k] >> lane) & 1u) {
+      const uint32_t h = (uint32_t)(at >> 32) + __popc(heads[k] & lanemask_lt());
+      head[h] = hv[k];
+      off[h] = p;
     }
   }
 }
+__global__ void set_u64_kernel(uint64_t* p, uint64_t v) { *p = v; }
 
 __global__ void head_index_kernel(const uint32_t* __restrict__ head, uint32_t nh, int32_t* __restrict__ hidx) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) hidx[head[i]] = (int32_t)i;
@@ -266,23 +368,6 @@ __global__ void big_block_fill_kernel(SetSrc src, uint32_t i, const SetAux* __re
   }
 }
 
-// per head entry a: sum over children v in head of d+(v) (pairs the
-// triangle loop nest probes below a)
-__global__ void wedge_kernel(TrieView t, uint64_t* __restrict__ wedges) {
-  const uint32_t lane = lane_id();
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = warp; i < t.n_head; i += nwarps) {
-    uint64_t s = 0;
-    for (uint64_t j = t.off[i] + lane; j < t.off[i + 1]; j += 32) {
-      const int32_t h = t.head_index[t.vals[j]];
-      if (h >= 0) s += t.off[h + 1] - t.off[h];
-    }
-    s = warp_sum(s);
-    if (lane == 0) wedges[i] = s;
-  }
-}
-
 // red[0] = largest set, red[1] = sum of squared set sizes
 __global__ void set_size_stats_kernel(const uint64_t* __restrict__ off, uint32_t nh, unsigned long long* red) {
   unsigned long long mx = 0, sq = 0;
@@ -457,7 +542,7 @@ void build_layout_structs_public(eh_context* ctx, eh_trie* t) { build_layout_str
 static void update_bytes(eh_trie* t) {
   t->info.device_bytes = t->head.bytes() + t->head_index.bytes() + t->off.bytes() + t->vals.bytes() +
                          t->layout.bytes() + t->aux.bytes() + t->bs_words.bytes() + t->bs_rank.bytes() +
-                         t->bb_id.bytes() + t->bb_rank.bytes() + t->bb_words.bytes() + t->wedges.bytes() +
+                         t->bb_id.bytes() + t->bb_rank.bytes() + t->bb_words.bytes() +
                          t->rev_off.bytes() + t->rev_lo.bytes() + t->rev_hi.bytes() + t->rev_src.bytes() +
                          t->rev_wpre.bytes() + t->work_pred.bytes() + t->up.bytes();
 }
@@ -524,20 +609,10 @@ static void build_head_index(eh_context* ctx, eh_trie* t) {
   }
 }
 
-// wedges per head entry, their total, the largest set, sum of squared sizes
+// the largest set, sum of squared sizes
 static void build_stats(eh_context* ctx, eh_trie* t) {
   cudaStream_t s = ctx->stream;
   const int grid = num_sms() * 8;
-  t->wedges.alloc(t->n_head ? t->n_head : 1, s);
-  DevBuf<uint64_t> tot(1, s);
-  if (t->n_head) {
-    wedge_kernel<<<grid, 256, 0, s>>>(t->view(), t->wedges.p);
-    EH_CHECK_LAUNCH();
-    DevBuf<uint64_t> scratch(t->n_head, s);
-    exclusive_scan<uint64_t>(t->wedges.p, scratch.p, t->n_head, tot.p, s);
-    EH_CUDA(cudaMemcpyAsync(&t->total_wedges, tot.p, 8, cudaMemcpyDeviceToHost, s));
-  }
-  EH_CUDA(cudaStreamSynchronize(s));
   t->info.rows = t->rows;
   t->info.n_head = t->n_head;
   t->info.n_nodes = t->n_nodes;
@@ -568,39 +643,59 @@ void trie_build_from_csr(eh_context* ctx, eh_trie* t) {
   trie_build_reverse(ctx, t);
 }
 
+// head, off, vals from rows in order
+template <typename R>
+static void csr_from_rows(eh_context* ctx, eh_trie* t, R r, uint64_t n) {
+  cudaStream_t s = ctx->stream;
+  const unsigned tiles = (unsigned)((n + kCsrTile - 1) / kCsrTile);
+  DevBuf<uint64_t> cnt(tiles + 1, s);
+  csr_count_kernel<R><<<tiles, kCsrThreads, 0, s>>>(r, n, cnt.p);
+  EH_CHECK_LAUNCH();
+  exclusive_scan<uint64_t>(cnt.p, cnt.p, tiles, cnt.p + tiles, s);
+  uint64_t h = 0;
+  EH_CUDA(cudaMemcpyAsync(&h, cnt.p + tiles, 8, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaStreamSynchronize(s));
+  t->rows = (uint32_t)h;  // below 2^32 rows in all, so neither count carries
+  t->n_head = (uint32_t)(h >> 32);
+  t->head.alloc(t->n_head, s);
+  t->off.alloc((size_t)t->n_head + 1, s);
+  t->vals.alloc(t->rows, s);
+  csr_write_kernel<R><<<tiles, kCsrThreads, 0, s>>>(r, n, cnt.p, t->head.p, t->off.p, t->vals.p);
+  set_u64_kernel<<<1, 1, 0, s>>>(t->off.p + t->n_head, t->rows);
+  EH_CHECK_LAUNCH();
+}
+
 void trie_build(eh_context* ctx, const uint32_t* c0, const uint32_t* c1, uint64_t n, const eh_layout_config* cfg,
                 eh_trie* t) {
   cudaStream_t s = ctx->stream;
   const int grid = num_sms() * 8;
   EH_CUDA(cudaEventRecord(ctx->ev0, s));
-  const uint32_t m0 = n ? max_u32(c0, n, s) : 0, m1 = n ? max_u32(c1, n, s) : 0;
+  ColumnStats st{0, 0, 0, 0};
+  if (n) {
+    DevBuf<ColumnStats> d(1, s);
+    EH_CUDA(cudaMemsetAsync(d.p, 0, sizeof(ColumnStats), s));
+    column_stats_kernel<<<std::min(grid, ceil_div(n, 256)), 256, 0, s>>>(c0, c1, n, d.p);
+    EH_CHECK_LAUNCH();
+    EH_CUDA(cudaMemcpyAsync(&st, d.p, sizeof(st), cudaMemcpyDeviceToHost, s));
+    EH_CUDA(cudaStreamSynchronize(s));
+  }
+  const uint32_t m0 = st.max0, m1 = st.max1;
   const int b = bits_for(m1), ba = bits_for(m0);
   EH_REQUIRE(b + ba <= 64, EH_ERR_UNSUPPORTED, "value range too wide");
-  uint64_t r = 0;
   t->n_nodes = n ? std::max(m0, m1) + 1 : 0;
   if (n) {
     TracePhase ph("build.sort+csr", s);
-    DevBuf<uint64_t> keys(n, s), tmp(n, s);
-    pack_rows_kernel<<<grid, 256, 0, s>>>(c0, c1, n, b, keys.p);
-    EH_CHECK_LAUNCH();
-    radix_sort_u64(keys.p, tmp.p, n, b + ba, s);
-    r = unique_sorted_u64(keys.p, tmp.p, n, s);
-    DevBuf<uint32_t> hpos(r, s), nh(1, s);
-    head_flag_kernel<<<grid, 256, 0, s>>>(tmp.p, r, b, hpos.p);
-    EH_CHECK_LAUNCH();
-    exclusive_scan<uint32_t>(hpos.p, hpos.p, r, nh.p, s);
-    uint32_t n_head = 0;
-    EH_CUDA(cudaMemcpyAsync(&n_head, nh.p, 4, cudaMemcpyDeviceToHost, s));
-    EH_CUDA(cudaStreamSynchronize(s));
-    t->n_head = n_head;
-    t->rows = r;
-    t->head.alloc(n_head, s);
-    t->off.alloc(n_head + 1, s);
-    t->vals.alloc(r, s);
-    csr_kernel<<<grid, 256, 0, s>>>(tmp.p, r, b, hpos.p, t->head.p, t->off.p, t->vals.p);
-    EH_CHECK_LAUNCH();
-    EH_CUDA(cudaMemcpyAsync(t->off.p + n_head, &r, 8, cudaMemcpyHostToDevice, s));
-    EH_CUDA(cudaStreamSynchronize(s));  // &r is a host stack address
+    DevBuf<uint64_t> keys;
+    if (st.unsorted) {
+      DevBuf<uint64_t> tmp(n, s);
+      keys.alloc(n, s);
+      pack_rows_kernel<<<grid, 256, 0, s>>>(c0, c1, n, b, keys.p);
+      EH_CHECK_LAUNCH();
+      radix_sort_u64(keys.p, tmp.p, n, b + ba, s);
+      csr_from_rows(ctx, t, KeyRows{keys.p, b}, n);
+    } else {
+      csr_from_rows(ctx, t, ColumnRows{c0, c1}, n);
+    }
   } else {
     t->off.alloc(1, s);
     EH_CUDA(cudaMemsetAsync(t->off.p, 0, 8, s));
@@ -623,17 +718,11 @@ __global__ void seg_kernel(const uint64_t* __restrict__ off, uint32_t nh, uint32
     for (uint64_t e = off[i] + lane; e < off[i + 1]; e += 32) seg[e] = i;
 }
 
-// counts rows that are not "up" (b <= a), not "down" (b >= a), rows (a,b)
-// whose mirror (b,a) is absent, and self-loops
-template <bool kMirror>
-__global__ void direction_kernel(TrieView t, const uint32_t* __restrict__ seg, unsigned long long* __restrict__ cnt) {
-  unsigned long long not_up = 0, not_down = 0, no_mirror = 0, loops = 0;
+// counts rows (a,b) whose mirror (b,a) is absent
+__global__ void mirror_kernel(TrieView t, const uint32_t* __restrict__ seg, unsigned long long* __restrict__ cnt) {
+  unsigned long long no_mirror = 0;
   for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < t.rows; e += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t a = t.head[seg[e]], b = t.vals[e];
-    not_up += b <= a;
-    not_down += b >= a;
-    loops += a == b;
-    if (!kMirror) continue;
     const int32_t hb = t.head_index[b];
     bool found = false;
     if (hb >= 0) {
@@ -646,16 +735,8 @@ __global__ void direction_kernel(TrieView t, const uint32_t* __restrict__ seg, u
     }
     no_mirror += !found;
   }
-  not_up = warp_sum(not_up);
-  not_down = warp_sum(not_down);
   no_mirror = warp_sum(no_mirror);
-  loops = warp_sum(loops);
-  if (lane_id() == 0) {
-    atomicAdd(&cnt[0], not_up);
-    atomicAdd(&cnt[1], not_down);
-    atomicAdd(&cnt[2], no_mirror);
-    atomicAdd(&cnt[3], loops);
-  }
+  if (lane_id() == 0 && no_mirror) atomicAdd(&cnt[2], no_mirror);
 }
 
 // candidate range inside N(a) for row e = (a -> b), by direction
@@ -678,6 +759,63 @@ __global__ void up_kernel(TrieView t, uint32_t* __restrict__ up) {
     up[i] = (uint32_t)lo;
   }
 }
+
+// One pass over the rows [r0, r1): the largest value, the direction counts (cnt:
+// rows not going up, not going down, -, self-loops, then the pairs
+// sum |N(b)| over rows a->b), and the reverse level's keys as if every row went
+// up (the common case; they are made again when it does not).  Values at or
+// above n_alloc are outside the head index and match no head entry.
+// A hub b ends a large share of all rows and in degree order the hubs are the
+// last head entries: those kRowHubs count in shared memory first, or their
+// counters serialise in L2 (R-MAT-20: 417 us for the keys alone).
+constexpr uint32_t kRowHubs = 2048;
+constexpr int kRowThreads = 1024;
+__global__ void __launch_bounds__(kRowThreads) row_pass_kernel(TrieView t, uint64_t r0, uint64_t r1,
+                                                               const uint32_t* __restrict__ seg, uint32_t n_alloc,
+                                                               uint32_t sentinel, uint32_t* __restrict__ keys,
+                                                               uint32_t* __restrict__ rowid,
+                                                               uint32_t* __restrict__ per,
+                                                               unsigned int* __restrict__ vmax,
+                                                               unsigned long long* __restrict__ cnt) {
+  __shared__ uint32_t hub[kRowHubs];
+  for (uint32_t i = threadIdx.x; i < kRowHubs; i += kRowThreads) hub[i] = 0;
+  __syncthreads();
+  const uint32_t hub0 = t.n_head > kRowHubs ? t.n_head - kRowHubs : 0;
+  unsigned int mx = 0;
+  unsigned long long not_up = 0, not_down = 0, loops = 0, pairs = 0;
+  for (uint64_t e = r0 + (uint64_t)blockIdx.x * kRowThreads + threadIdx.x; e < r1;
+       e += (uint64_t)gridDim.x * kRowThreads) {
+    const uint32_t ha = seg[e];
+    const uint32_t a = t.head[ha], b = t.vals[e];
+    mx = max(mx, b);
+    not_up += b <= a;
+    not_down += b >= a;
+    loops += a == b;
+    const int32_t hb = b < n_alloc ? t.head_index[b] : -1;
+    if (hb >= 0) pairs += t.off[hb + 1] - t.off[hb];
+    const bool keep = hb >= 0 && e + 1 < t.off[ha + 1];
+    keys[e] = keep ? (uint32_t)hb : sentinel;
+    rowid[e] = (uint32_t)e;
+    if (keep) atomicAdd((uint32_t)hb < hub0 ? per + hb : hub + ((uint32_t)hb - hub0), 1u);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(kFull, mx, o));
+  not_up = warp_sum(not_up);
+  not_down = warp_sum(not_down);
+  loops = warp_sum(loops);
+  pairs = warp_sum(pairs);
+  if (lane_id() == 0) {
+    atomicMax(vmax, mx);
+    if (not_up) atomicAdd(&cnt[0], not_up);
+    if (not_down) atomicAdd(&cnt[1], not_down);
+    if (loops) atomicAdd(&cnt[3], loops);
+    if (pairs) atomicAdd(&cnt[4], pairs);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < kRowHubs; i += kRowThreads)
+    if (hub[i]) atomicAdd(per + hub0 + i, hub[i]);
+}
+static int row_pass_grid(uint64_t rows) { return std::max(1, std::min(num_sms() * 2, ceil_div(rows, kRowThreads))); }
 
 // key = head position of b (sentinel for rows the plans never read),
 // payload = the row; rows arrive in row order, so a stable sort on the key
@@ -730,6 +868,7 @@ void trie_build_reverse(eh_context* ctx, eh_trie* t) {
   t->up.release();
   t->rev_entries = 0;
   t->rev_pairs = 0;
+  t->total_wedges = 0;
   t->rev_off.alloc(t->n_head + 1, s);
   EH_CUDA(cudaMemsetAsync(t->rev_off.p, 0, (t->n_head + 1) * 8, s));
   if (!t->rows) {
@@ -742,24 +881,34 @@ void trie_build_reverse(eh_context* ctx, eh_trie* t) {
   TracePhase ph_dir("reverse.direction", s);
   seg_kernel<<<grid, 256, 0, s>>>(t->off.p, t->n_head, seg.p);
   EH_CHECK_LAUNCH();
-  // direction: up / down from one cheap pass; the mirror search only when
-  // the relation is neither
-  DevBuf<unsigned long long> cnt(4, s);
-  EH_CUDA(cudaMemsetAsync(cnt.p, 0, 32, s));
-  direction_kernel<false><<<grid, 256, 0, s>>>(t->view(), seg.p, cnt.p);
+  // group the rows a->b the plans read by b (stable: row order within b);
+  // head positions are below 2^32, so 32-bit keys on bits_for(n_head) bits
+  const int bh = bits_for(t->n_head);
+  const uint32_t sentinel = (uint32_t)((1ull << bh) - 1);  // above every head position
+  DevBuf<uint32_t> keys(t->rows, s), ktmp(t->rows, s);
+  DevBuf<uint32_t> rowid(t->rows, s), vtmp(t->rows, s);
+  DevBuf<uint32_t> per(t->n_head + 1, s);
+  DevBuf<unsigned long long> cnt(6, s);  // the last one: the largest value, not read here
+  EH_CUDA(cudaMemsetAsync(per.p, 0, ((size_t)t->n_head + 1) * 4, s));
+  EH_CUDA(cudaMemsetAsync(cnt.p, 0, 48, s));
+  // direction counts and the keys of a relation that goes up, in one pass; the
+  // mirror search only when it goes neither way
+  row_pass_kernel<<<row_pass_grid(t->rows), kRowThreads, 0, s>>>(t->view(), 0, t->rows, seg.p, t->n_nodes, sentinel,
+                                                                 keys.p, rowid.p, per.p, (unsigned int*)(cnt.p + 5),
+                                                                 cnt.p);
   EH_CHECK_LAUNCH();
-  unsigned long long c[4];
-  EH_CUDA(cudaMemcpyAsync(c, cnt.p, 32, cudaMemcpyDeviceToHost, s));
+  unsigned long long c[5];
+  EH_CUDA(cudaMemcpyAsync(c, cnt.p, 40, cudaMemcpyDeviceToHost, s));
   EH_CUDA(cudaStreamSynchronize(s));
+  t->total_wedges = c[4];
   if (c[0] == 0) {
     t->dir = DIR_UP;
   } else if (c[1] == 0) {
     t->dir = DIR_DOWN;
   } else {
-    EH_CUDA(cudaMemsetAsync(cnt.p, 0, 32, s));
-    direction_kernel<true><<<grid, 256, 0, s>>>(t->view(), seg.p, cnt.p);
+    mirror_kernel<<<grid, 256, 0, s>>>(t->view(), seg.p, cnt.p);
     EH_CHECK_LAUNCH();
-    EH_CUDA(cudaMemcpyAsync(c, cnt.p, 32, cudaMemcpyDeviceToHost, s));
+    EH_CUDA(cudaMemcpyAsync(c + 2, cnt.p + 2, 8, cudaMemcpyDeviceToHost, s));
     EH_CUDA(cudaStreamSynchronize(s));
     // a symmetric relation takes the oriented schedule (each undirected
     // triangle once, times 3!) only without self-loops
@@ -771,18 +920,12 @@ void trie_build_reverse(eh_context* ctx, eh_trie* t) {
     up_kernel<<<grid, 256, 0, s>>>(t->view(), t->up.p);
     EH_CHECK_LAUNCH();
   }
-  // group the rows a->b the plans read by b (stable: row order within b);
-  // head positions are below 2^32, so 32-bit keys on bits_for(n_head) bits
-  const int bh = bits_for(t->n_head);
-  const uint32_t sentinel = (uint32_t)((1ull << bh) - 1);  // above every head position
-  DevBuf<uint32_t> keys(t->rows, s), ktmp(t->rows, s);
-  DevBuf<uint32_t> rowid(t->rows, s), vtmp(t->rows, s);
-  DevBuf<uint32_t> per(t->n_head + 1, s);
-  EH_CUDA(cudaMemsetAsync(per.p, 0, (t->n_head + 1) * 4, s));
-  TracePhase ph_key("reverse.keys", s);
-  rev_key_kernel<<<grid, 256, 0, s>>>(t->view(), seg.p, t->dir, sentinel, keys.p, rowid.p, per.p);
-  EH_CHECK_LAUNCH();
-  ph_key.end();
+  if (t->dir != DIR_UP) {
+    TracePhase ph_key("reverse.keys", s);
+    EH_CUDA(cudaMemsetAsync(per.p, 0, ((size_t)t->n_head + 1) * 4, s));
+    rev_key_kernel<<<grid, 256, 0, s>>>(t->view(), seg.p, t->dir, sentinel, keys.p, rowid.p, per.p);
+    EH_CHECK_LAUNCH();
+  }
   reverse_from_keys(ctx, t, seg, keys, ktmp, rowid, vtmp, per);
 }
 
@@ -833,45 +976,6 @@ static void reverse_from_keys(eh_context* ctx, eh_trie* t, DevBuf<uint32_t>& seg
     EH_CUDA(cudaMemcpyAsync(&t->rev_pairs, t->rev_wpre.p + n, 8, cudaMemcpyDeviceToHost, s));
   }
   EH_CUDA(cudaStreamSynchronize(s));
-}
-
-// Rows [r0, r1) of a CSR whose values have just arrived from the host: the
-// largest value, the direction counts (rows not going up, not going down,
-// self-loops), and the reverse level's keys as if every row went up (the
-// common case; trie_build_from_host_csr recomputes them when it is not).
-// Values at or above n_alloc are outside the head index and match no head
-// entry.
-__global__ void host_chunk_kernel(TrieView t, uint64_t r0, uint64_t r1, const uint32_t* __restrict__ seg,
-                                  uint32_t n_alloc, uint32_t sentinel, uint32_t* __restrict__ keys,
-                                  uint32_t* __restrict__ rowid, uint32_t* __restrict__ per,
-                                  unsigned int* __restrict__ vmax, unsigned long long* __restrict__ cnt) {
-  unsigned int mx = 0;
-  unsigned long long not_up = 0, not_down = 0, loops = 0;
-  for (uint64_t e = r0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < r1;
-       e += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t ha = seg[e];
-    const uint32_t a = t.head[ha], b = t.vals[e];
-    mx = max(mx, b);
-    not_up += b <= a;
-    not_down += b >= a;
-    loops += a == b;
-    const int32_t hb = b < n_alloc ? t.head_index[b] : -1;
-    const bool keep = hb >= 0 && e + 1 < t.off[ha + 1];
-    keys[e] = keep ? (uint32_t)hb : sentinel;
-    rowid[e] = (uint32_t)e;
-    if (keep) atomicAdd(&per[hb], 1u);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(kFull, mx, o));
-  not_up = warp_sum(not_up);
-  not_down = warp_sum(not_down);
-  loops = warp_sum(loops);
-  if (lane_id() == 0) {
-    atomicMax(vmax, mx);
-    atomicAdd(&cnt[0], not_up);
-    atomicAdd(&cnt[1], not_down);
-    atomicAdd(&cnt[3], loops);
-  }
 }
 
 // A trie from a CSR in host memory (head[n_head] sorted distinct values,
@@ -934,22 +1038,22 @@ void trie_build_from_host_csr(eh_context* ctx, eh_trie* t, const uint32_t* head,
   const uint32_t sentinel = (uint32_t)((1ull << bh) - 1);
   DevBuf<uint32_t> keys(t->rows, s), ktmp(t->rows, s), rowid(t->rows, s), vtmp(t->rows, s);
   DevBuf<uint32_t> per(t->n_head + 1, s);
-  DevBuf<unsigned long long> cnt(4, s);
+  DevBuf<unsigned long long> cnt(5, s);
   DevBuf<unsigned int> vmax(1, s);
   EH_CUDA(cudaMemsetAsync(per.p, 0, ((size_t)t->n_head + 1) * 4, s));
-  EH_CUDA(cudaMemsetAsync(cnt.p, 0, 32, s));
+  EH_CUDA(cudaMemsetAsync(cnt.p, 0, 40, s));
   EH_CUDA(cudaMemsetAsync(vmax.p, 0, 4, s));
   for (int i = 0; i < kChunks; i++) {
     EH_CUDA(cudaStreamWaitEvent(s, ev[i], 0));
     if (bound[i + 1] > bound[i]) {
-      host_chunk_kernel<<<grid, 256, 0, s>>>(t->view(), bound[i], bound[i + 1], seg.p, n_alloc, sentinel, keys.p,
-                                             rowid.p, per.p, vmax.p, cnt.p);
+      row_pass_kernel<<<row_pass_grid(bound[i + 1] - bound[i]), kRowThreads, 0, s>>>(
+          t->view(), bound[i], bound[i + 1], seg.p, n_alloc, sentinel, keys.p, rowid.p, per.p, vmax.p, cnt.p);
       EH_CHECK_LAUNCH();
     }
   }
-  unsigned long long c[4];
+  unsigned long long c[5];
   unsigned int vm = 0;
-  EH_CUDA(cudaMemcpyAsync(c, cnt.p, 32, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaMemcpyAsync(c, cnt.p, 40, cudaMemcpyDeviceToHost, s));
   EH_CUDA(cudaMemcpyAsync(&vm, vmax.p, 4, cudaMemcpyDeviceToHost, s));
   EH_CUDA(cudaStreamSynchronize(s));
   if (vm >= n_alloc) {  // a value beyond the hint and the head: the whole domain again
@@ -963,6 +1067,7 @@ void trie_build_from_host_csr(eh_context* ctx, eh_trie* t, const uint32_t* head,
   TracePhase ph("build.reverse", s);
   if (vm < n_alloc && c[0] == 0) {  // every row goes up: the keys stand
     t->dir = DIR_UP;
+    t->total_wedges = c[4];
     t->rev_off.alloc(t->n_head + 1, s);
     reverse_from_keys(ctx, t, seg, keys, ktmp, rowid, vtmp, per);
   } else {
