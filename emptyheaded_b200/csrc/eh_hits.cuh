@@ -46,49 +46,39 @@ __device__ __forceinline__ uint32_t hits_stride(uint32_t q, uint32_t W, uint32_t
   return q + 1 < W ? 32u : (d - 32u * q + 7) & ~7u;
 }
 
-// probe() for bit words, on their 32-bit halves: the pass is bound by
-// instruction issue, and a 64-bit variable shift takes several
-template <int P>
-__device__ __forceinline__ bool hit(const Staged& st, uint32_t w) {
-  if (P == P_SBITS || P == P_GBITS) {
-    const uint32_t idx = (w >> 5) - 2 * st.start;
-    if (idx >= 2 * st.n) return false;  // also below the first word (wraps)
-    const uint32_t* h = reinterpret_cast<const uint32_t*>(st.words) + idx;
-    return ((P == P_SBITS ? *h : __ldg(h)) >> (w & 31)) & 1u;
-  }
-  if (P == P_ZBITS) {
-    const uint32_t idx = (w >> 6) - st.start;
-    if (idx >= st.n) return false;
-    const uint2 g = st.pz[idx >> 5];
-    const uint32_t up = g.x >> (idx & 31);
-    if (!(up & 1u)) return false;
-    const uint32_t pos = g.y + __popc(g.x ^ (up << (idx & 31)));
-    return (reinterpret_cast<const uint32_t*>(st.words)[2 * pos + ((w >> 5) & 1u)] >> (w & 31)) & 1u;
-  }
-  return probe<P>(st, w) != 0;
-}
-
 // One batch of 32 rows at a time, a row per lane.  Rows of at least kTripRow
 // candidates run as trips: a trip is one mask word of one row, a bit per lane,
-// and the trips of all the batch's rows form one list, taken four at a time
-// (so a row need not fill four) with the four trips' candidates loaded before
-// any is probed.  Lane t keeps the word of trip t and writes it after 32
+// and the trips of all the batch's rows form one list, taken kHitTrips at a
+// time (so a row need not fill them) with their candidates loaded before any is
+// probed.  Lane t keeps the word of trip t and writes it after 32
 // trips.  Shorter rows are flattened over the lanes, and each lane cuts its
 // row's bits out of the trip's ballot (a short row's candidates lie in at most
 // two words).  Only non-zero words are written.
 constexpr uint32_t kTripRow = 24;  // at most 32: a short row's hits are one register
+constexpr int kHitTrips = 8;  // divides 32; 4-clique R-MAT-20 4.13 -> 4.06 ms against four
 template <int P>
 __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, const RevView& r, uint32_t kb,
                                          uint32_t ke, const uint32_t* __restrict__ moff,
                                          uint32_t* __restrict__ mask, uint32_t shard_index, uint32_t shard_count) {
   const uint32_t lane = lane_id();
   const uint32_t step = r.dir == DIR_DOWN ? 0xffffffffu : 1u;  // from one candidate's element to the next's
+  uint32_t next_lo = 0, next_hi = 0, next_src = 0;  // the next batch's rows, loaded a batch ahead
+  if (kb + lane < ke) {
+    next_lo = __ldg(r.rev_lo + kb + lane);
+    next_hi = __ldg(r.rev_hi + kb + lane);
+    next_src = __ldg(r.rev_src + kb + lane);
+  }
   for (uint32_t k0 = kb; k0 < ke; k0 += 32) {
     const uint32_t k = k0 + lane;
+    const uint32_t lo = next_lo, hi = next_hi, src = next_src;
+    if (k + 32 < ke) {
+      next_lo = __ldg(r.rev_lo + k + 32);
+      next_hi = __ldg(r.rev_hi + k + 32);
+      next_src = __ldg(r.rev_src + k + 32);
+    }
     uint32_t len = 0, fe = 0;               // candidates; the element of the first one
     uint32_t skip = 0, base = 0, rs = 0;    // bit of the first candidate in the row's words, first word, stride
     if (k < ke) {
-      const uint32_t lo = __ldg(r.rev_lo + k), hi = __ldg(r.rev_hi + k), src = __ldg(r.rev_src + k);
       // shards split the heads a: each rank builds and reads the matrices of its own
       if (shard_count == 1 || src % shard_count == shard_index) {
         const StagedRange pr = staged_range(t, src);
@@ -113,10 +103,10 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
       const uint32_t elem0 = fe - step * skip;       // bit p of the row is element elem0 + step * p
       for (uint32_t t0 = 0; t0 < total; t0 += 32) {
         uint32_t mine = 0;
-        for (uint32_t u0 = 0; u0 < 32 && t0 + u0 < total; u0 += 4) {
-          uint32_t v[4];
+        for (uint32_t u0 = 0; u0 < 32 && t0 + u0 < total; u0 += kHitTrips) {
+          uint32_t v[kHitTrips];
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
+          for (int u = 0; u < kHitTrips; u++) {
             const uint32_t x = min(t0 + u0 + u, total - 1);
             const int j = __popc(__ballot_sync(kFull, incl <= x));
             const uint32_t ej = __shfl_sync(kFull, elem0, j), lj = __shfl_sync(kFull, end, j);
@@ -124,7 +114,7 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
             v[u] = __ldg(t.vals + (ej + step * min(p, lj - 1)));  // bits outside the row are masked off below
           }
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
+          for (int u = 0; u < kHitTrips; u++) {
             const uint32_t b = __ballot_sync(kFull, hit<P>(st, v[u]));
             if (lane == u0 + u) mine = b;
           }
@@ -172,7 +162,11 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
   }
 }
 
-__global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const TrieView* __restrict__ views, const RevView* __restrict__ revs,
+// kOne: as in triangle_kernel
+template <bool kOne>
+__global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const __grid_constant__ TrieView t1,
+                                                 const __grid_constant__ RevView r1,
+                                                 const TrieView* __restrict__ views, const RevView* __restrict__ revs,
                                                  const Item* __restrict__ items,
                                                  const unsigned int* __restrict__ n_items_p, int cap_words,
                                                  unsigned int* __restrict__ queue, HitsView hv, float* records,
@@ -187,8 +181,14 @@ __global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const TrieView* __restrict__ vi
     it = __shfl_sync(kFull, it, 0);
     if (it >= n_items) break;
     const Item item = items[it];
-    const TrieView t = views[item.g];
-    const RevView r = revs[item.g];
+    TrieView tg;
+    RevView rg;
+    if (!kOne) {
+      tg = views[item.g];
+      rg = revs[item.g];
+    }
+    const TrieView& t = kOne ? t1 : tg;
+    const RevView& r = kOne ? r1 : rg;
     const uint32_t* moff = hv.moff + hv.gstart[item.g];
     long long t0 = 0;
     if (records && lane == 0) t0 = clock64();

@@ -34,7 +34,7 @@ namespace eh {
 #endif
 constexpr int kMaxWarps = EH_TRI_MAX_THREADS / 32;  // per block
 constexpr int kDefaultWarps = kMaxWarps < 8 ? kMaxWarps : 8;
-constexpr uint32_t kDefaultLongRow = 32;  // rows with at least this many candidates run warp-wide
+constexpr uint32_t kDefaultLongRow = 48;  // rows with at least this many candidates run warp-wide
 #ifndef EH_LONG_UNROLL
 #define EH_LONG_UNROLL 4
 #endif
@@ -69,11 +69,12 @@ constexpr int kLongWords = EH_LONG_WORDS;  // word rows with at least this many 
 #define EH_FLAT_CLIQUE 48
 #endif
 constexpr uint32_t kFlatClique = EH_FLAT_CLIQUE;  // 4-clique: S up to this size has its pairs flattened
-// Defaults measured on B200 at R-MAT-22 (4 KB of staging per warp leaves
-// room for 32 resident warps; 32K-probe items amortise staging); the
+// Defaults measured on B200 at R-MAT-22 (5 KB of staging per warp leaves
+// room for 32 resident warps; 1024 words 7.18 ms against 7.06); the
 // autotuner (emptyheaded_b200/autotune.py) re-picks them per trie.
-constexpr int kDefaultSmemWords = 1024;  // per warp
-constexpr int kDefaultChunk = 32768;
+constexpr int kDefaultSmemWords = 1280;  // per warp
+constexpr int kDefaultChunk = 32768;     // where it is not derived from the work (records, noalloc)
+constexpr uint64_t kMaxChunk = 131072;   // larger items amortise staging: 7.03 ms against 7.18 at 32768
 constexpr uint64_t kMinChunk = 4096;  // the smallest item the planner cuts by itself
 
 struct RevView {
@@ -865,6 +866,179 @@ __device__ __forceinline__ uint64_t stream_rows(const Staged& st, const TrieView
   return cnt;
 }
 
+// probe() for bit words, on their 32-bit halves: these passes are bound by
+// instruction issue, and a 64-bit variable shift takes several
+template <int P>
+__device__ __forceinline__ bool hit(const Staged& st, uint32_t w) {
+  if (P == P_SBITS || P == P_GBITS) {
+    const uint32_t idx = (w >> 5) - 2 * st.start;
+    if (idx >= 2 * st.n) return false;  // also below the first word (wraps)
+    const uint32_t* h = reinterpret_cast<const uint32_t*>(st.words) + idx;
+    return ((P == P_SBITS ? *h : __ldg(h)) >> (w & 31)) & 1u;
+  }
+  if (P == P_ZBITS) {
+    const uint32_t idx = (w >> 6) - st.start;
+    if (idx >= st.n) return false;
+    const uint2 g = st.pz[idx >> 5];
+    const uint32_t up = g.x >> (idx & 31);
+    if (!(up & 1u)) return false;
+    const uint32_t pos = g.y + __popc(g.x ^ (up << (idx & 31)));
+    return (reinterpret_cast<const uint32_t*>(st.words)[2 * pos + ((w >> 5) & 1u)] >> (w & 31)) & 1u;
+  }
+  return probe<P>(st, w) != 0;
+}
+
+// stream_rows for the plain COUNT.  A batch of 32 rows, a row per lane; each
+// row is counted in one of four ways:
+//   word trips     both sets are range bitsets and their common words are fewer
+//                  than the candidates (weighted as in stream_rows), at least
+//                  kTripWords of them: 32 words per trip
+//   word pairs     fewer words: flattened (row, word) pairs over the lanes
+//   element trips  at least long_row candidates: 32 candidates per trip
+//   element pairs  fewer: flattened (row, candidate) pairs over the lanes
+// The trips of all rows of a batch form one list, taken kTrips at a time with
+// their loads issued before the first is used, so that a row need not fill
+// them; the trip's row is found by one ballot.  A word row needs no masks: what
+// N(a) holds outside the candidates is at or before b (after, on a relation
+// that goes down), where N(b) holds nothing -- or, on a symmetric relation, the
+// staged copy of N(b) had it cleared -- so neither its first nor its last
+// candidate is read.
+// Measured (triangle kernel, R-MAT-22 / R-MAT-20, ms): stream_rows 8.49 / 1.43;
+// trips of four 8.10 / 1.21; views as kernel parameters and the next batch's
+// rows loaded ahead 7.76 / 1.14; element trips by eight 7.18 / 1.13 (by six
+// 7.29, word trips by three 7.40, by six 7.39).  48 registers and five blocks per
+// SM 7.84, 80 and three 9.41.
+constexpr int kTrips = 8, kWTrips = 4;
+constexpr uint32_t kTripWords = 16;
+template <int P>
+__device__ __forceinline__ uint64_t count_rows(const Staged& st, const TrieView& t, const RevView& r, uint32_t kb,
+                                               uint32_t ke, uint32_t long_row) {
+  const uint32_t lane = lane_id();
+  // unstaged words of a symmetric N(b) are not cleared: element rows only
+  const bool words_ok = P == P_SBITS || (P == P_GBITS && !t.up);
+  const uint64_t pol_keep = l2_policy_last();
+  constexpr bool kWords = P == P_SBITS || P == P_GBITS;
+  uint64_t total_hits = 0;
+  uint32_t next_lo = 0, next_hi = 0, next_src = 0;  // the next batch's rows, loaded a batch ahead
+  if (kb + lane < ke) {
+    next_lo = __ldg(r.rev_lo + kb + lane);
+    next_hi = __ldg(r.rev_hi + kb + lane);
+    if (kWords) next_src = __ldg(r.rev_src + kb + lane);
+  }
+  for (uint32_t k0 = kb; k0 < ke; k0 += 32) {
+    const uint32_t lo = next_lo, src = next_src;
+    uint32_t len = next_hi - next_lo;
+    next_lo = next_hi = 0;
+    if (k0 + 32 + lane < ke) {
+      next_lo = __ldg(r.rev_lo + k0 + 32 + lane);
+      next_hi = __ldg(r.rev_hi + k0 + 32 + lane);
+      if (kWords) next_src = __ldg(r.rev_src + k0 + 32 + lane);
+    }
+    uint32_t cnt = 0;
+    uint32_t nw = 0, ws = 0;   // words of a word row; its first one, from N(b)'s start
+    uint64_t wbase = 0;        // and in the pool
+    if (kWords && words_ok && len && __ldg(t.layout + src) == EH_LAYOUT_RANGE_BITSET) {
+      const SetAux aa = t.aux[src];
+      const uint32_t lo_w = max(aa.start, st.start);
+      const uint32_t hi_w = min(aa.start + aa.n, st.start + st.n);
+      const uint32_t words = hi_w > lo_w ? hi_w - lo_w : 0;
+      if (words * kWordRowNum < len * kWordRowDen) {
+        len = 0;
+        nw = words;
+        ws = lo_w - st.start;
+        wbase = aa.off + (lo_w - aa.start);
+      }
+    }
+    if (kWords) {
+      const uint32_t nt = nw >= kTripWords ? (nw + 31) >> 5 : 0;
+      const uint32_t incl = warp_incl_scan(nt);
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      if (total) {
+        const uint32_t first = 32 * (incl - nt);  // word q of the list is word q - first of its row
+        const uint64_t pool = wbase - first;
+        const uint32_t staged = ws - first, end = nw + first;
+        for (uint32_t t0 = 0; t0 < total; t0 += kWTrips) {
+          uint64_t x[kWTrips], y[kWTrips];
+#pragma unroll
+          for (int u = 0; u < kWTrips; u++) {
+            const uint32_t trip = min(t0 + u, total - 1);
+            const int j = __popc(__ballot_sync(kFull, incl <= trip));
+            const uint32_t q = 32 * trip + lane;
+            const uint64_t pj = __shfl_sync(kFull, pool, j);
+            const uint32_t sj = __shfl_sync(kFull, staged, j), ej = __shfl_sync(kFull, end, j);
+            const bool in = q < ej && t0 + u < total;
+            x[u] = in ? ld64_hint(t.bs_words + (pj + q), pol_keep) : 0ull;
+            y[u] = in ? ((P == P_SBITS) ? st.words[sj + q] : __ldg(st.words + (sj + q))) : 0ull;
+          }
+#pragma unroll
+          for (int u = 0; u < kWTrips; u++) cnt += __popcll(x[u] & y[u]);
+        }
+        if (nt) nw = 0;
+      }
+      const uint32_t wincl = warp_incl_scan(nw);
+      const uint32_t wtotal = __shfl_sync(kFull, wincl, 31);
+      const uint32_t wfirst = wincl - nw;
+      const uint64_t wpool = wbase - wfirst;
+      const uint32_t wstaged = ws - wfirst;
+      for (uint32_t p = 0; p < wtotal; p += 64) {
+        uint64_t x[2], y[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const uint32_t q = p + 32 * u + lane;
+          const uint32_t j = owner_lane(wincl, min(q, wtotal - 1));
+          const uint64_t pj = __shfl_sync(kFull, wpool, j);
+          const uint32_t sj = __shfl_sync(kFull, wstaged, j);
+          x[u] = q < wtotal ? ld64_hint(t.bs_words + (pj + q), pol_keep) : 0ull;
+          y[u] = q < wtotal ? ((P == P_SBITS) ? st.words[sj + q] : __ldg(st.words + (sj + q))) : 0ull;
+        }
+        cnt += __popcll(x[0] & y[0]) + __popcll(x[1] & y[1]);
+      }
+    }
+    {
+      const uint32_t nt = len >= long_row ? (len + 31) >> 5 : 0;
+      const uint32_t incl = warp_incl_scan(nt);
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      if (total) {
+        const uint32_t first = 32 * (incl - nt);
+        const uint32_t elem = lo - first, end = len + first;
+        for (uint32_t t0 = 0; t0 < total; t0 += kTrips) {
+          uint32_t v[kTrips];
+          bool in[kTrips];
+#pragma unroll
+          for (int u = 0; u < kTrips; u++) {
+            const uint32_t trip = min(t0 + u, total - 1);
+            const int j = __popc(__ballot_sync(kFull, incl <= trip));
+            const uint32_t q = 32 * trip + lane;
+            const uint32_t ej = __shfl_sync(kFull, elem, j);
+            in[u] = q < __shfl_sync(kFull, end, j) && t0 + u < total;
+            v[u] = in[u] ? __ldg(t.vals + (ej + q)) : 0u;
+          }
+#pragma unroll
+          for (int u = 0; u < kTrips; u++) cnt += in[u] && hit<P>(st, v[u]);
+        }
+        if (nt) len = 0;
+      }
+    }
+    const uint32_t incl = warp_incl_scan(len);
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    const uint32_t elem = lo - (incl - len);
+    for (uint32_t p = 0; p < total; p += 32 * kShortUnroll) {
+      uint32_t v[kShortUnroll];
+#pragma unroll
+      for (int u = 0; u < kShortUnroll; u++) {
+        const uint32_t q = p + 32 * u + lane;
+        const uint32_t j = owner_lane(incl, min(q, total - 1));
+        const uint32_t ej = __shfl_sync(kFull, elem, j);
+        v[u] = q < total ? __ldg(t.vals + (ej + q)) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < kShortUnroll; u++) cnt += p + 32 * u + lane < total && hit<P>(st, v[u]);
+    }
+    total_hits += cnt;  // a batch's hits per lane stay far below 2^32
+  }
+  return total_hits;
+}
+
 // Stage N(b) in the warp's shared region according to its layout; returns
 // the probe mode.
 __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_t* sm, int cap_words, Staged& st,
@@ -882,6 +1056,10 @@ __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_
       uint64_t* sw = reinterpret_cast<uint64_t*>(sm);
       for (uint32_t j = lane; j < a.n; j += 32) sw[j] = __ldg(t.bs_words + a.off + j);
       __syncwarp();
+      if (t.up) {  // the first word without the elements before the staged part
+        if (lane == 0) sw[0] &= ~0ull << (__ldg(t.vals + s0) & 63);
+        __syncwarp();
+      }
       st.words = sw;
       return P_SBITS;
     }
@@ -1028,7 +1206,11 @@ __device__ __forceinline__ int stage_set_block(const TrieView& t, uint32_t hb, u
     st.n = a.n;
     if (2 * a.n <= (uint32_t)cap_words) {
       uint64_t* sw = reinterpret_cast<uint64_t*>(sm);
-      for (uint32_t j = threadIdx.x; j < a.n; j += blockDim.x) sw[j] = __ldg(t.bs_words + a.off + j);
+      for (uint32_t j = threadIdx.x; j < a.n; j += blockDim.x) {
+        uint64_t w = __ldg(t.bs_words + a.off + j);
+        if (t.up && j == 0) w &= ~0ull << (__ldg(t.vals + s0) & 63);  // as in stage_set
+        sw[j] = w;
+      }
       st.words = sw;
       return P_SBITS;
     }
@@ -1054,13 +1236,24 @@ __device__ __forceinline__ int stage_set_block(const TrieView& t, uint32_t hb, u
 template <int kMode>
 __device__ __forceinline__ uint64_t rows_of(int mode, const Staged& st, const TrieView& t, const RevView& r,
                                             uint32_t kb, uint32_t ke, uint32_t long_row, const Sink& sk) {
+  if (kMode == MODE_COUNT) {
+    switch (mode) {
+      case P_SBITS: return count_rows<P_SBITS>(st, t, r, kb, ke, long_row);
+      case P_GBITS: return count_rows<P_GBITS>(st, t, r, kb, ke, long_row);
+      case P_SLIST: return count_rows<P_SLIST>(st, t, r, kb, ke, long_row);
+      case P_GLIST: return count_rows<P_GLIST>(st, t, r, kb, ke, long_row);
+      case P_ZBITS: return count_rows<P_ZBITS>(st, t, r, kb, ke, long_row);
+      default: return count_rows<P_GBLOCK>(st, t, r, kb, ke, long_row);
+    }
+  }
+  constexpr int kSum = kMode == MODE_COUNT ? MODE_MAT : kMode;  // no COUNT form of stream_rows
   switch (mode) {
-    case P_SBITS: return stream_rows<P_SBITS, kMode>(st, t, r, kb, ke, long_row, sk);
-    case P_GBITS: return stream_rows<P_GBITS, kMode>(st, t, r, kb, ke, long_row, sk);
-    case P_SLIST: return stream_rows<P_SLIST, kMode>(st, t, r, kb, ke, long_row, sk);
-    case P_GLIST: return stream_rows<P_GLIST, kMode>(st, t, r, kb, ke, long_row, sk);
-    case P_ZBITS: return stream_rows<P_ZBITS, kMode>(st, t, r, kb, ke, long_row, sk);
-    default: return stream_rows<P_GBLOCK, kMode>(st, t, r, kb, ke, long_row, sk);
+    case P_SBITS: return stream_rows<P_SBITS, kSum>(st, t, r, kb, ke, long_row, sk);
+    case P_GBITS: return stream_rows<P_GBITS, kSum>(st, t, r, kb, ke, long_row, sk);
+    case P_SLIST: return stream_rows<P_SLIST, kSum>(st, t, r, kb, ke, long_row, sk);
+    case P_GLIST: return stream_rows<P_GLIST, kSum>(st, t, r, kb, ke, long_row, sk);
+    case P_ZBITS: return stream_rows<P_ZBITS, kSum>(st, t, r, kb, ke, long_row, sk);
+    default: return stream_rows<P_GBLOCK, kSum>(st, t, r, kb, ke, long_row, sk);
   }
 }
 
@@ -1082,8 +1275,12 @@ struct QueryOut {
   uint32_t gcap;               //   shared memory), gcap words each; null: S in shared memory
 };
 
-template <int kMode>
-__global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict__ views,
+// kOne: one trie, whose views are the kernel's parameters -- operands from the
+// constant bank, where copies of a batch's views take two dozen registers.
+template <int kMode, bool kOne>
+__global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ TrieView t1,
+                                                        const __grid_constant__ RevView r1,
+                                                        const TrieView* __restrict__ views,
                                                         const RevView* __restrict__ revs,
                                                         const Item* __restrict__ items, int cap_words,
                                                         QueryOut out) {
@@ -1137,8 +1334,14 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict_
       acc = 0;
       cur_g = item.g;
     }
-    const TrieView t = views[item.g];
-    const RevView r = revs[item.g];
+    TrieView tg;
+    RevView rg;
+    if (!kOne) {
+      tg = views[item.g];
+      rg = revs[item.g];
+    }
+    const TrieView& t = kOne ? t1 : tg;
+    const RevView& r = kOne ? r1 : rg;
     long long t0 = 0;
     if (out.records && lane == 0) t0 = clock64();
     Sink sk{out.annot, out.ma, out.mb, out.mc, 0, &slot[wid], 0, hot, hot_acc, nullptr, 0, nullptr, nullptr,
@@ -1170,11 +1373,10 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const TrieView* __restrict_
         sk.wstart = st.start;
         if (mode == P_SBITS) {
           uint32_t* rk = sm + 2 * st.n;
-          // ranks within the staged part (the first word's may be negative,
-          // mod 2^32: it can hold elements before that part)
+          // ranks within the staged part (none before its first word)
           const uint32_t* grk = t.bs_rank + staged_bits(t, item.hb, sr).off;
           const uint32_t before = (uint32_t)(sr.s0 - t.off[item.hb]);
-          for (uint32_t j = lane; j < st.n; j += 32) rk[j] = __ldg(grk + j) - before;
+          for (uint32_t j = lane; j < st.n; j += 32) rk[j] = j ? __ldg(grk + j) - before : 0u;
           sk.wrank = rk;
         }
         sk.wcnt = sm + used;
@@ -1604,7 +1806,8 @@ struct Prepared {
   DevBuf<unsigned char> own;      // device arrays of a launch that outlives the call (a batch) or is large
   Control* ctl = nullptr;         // control block, results, views, items: one piece of device memory
   unsigned long long* total = nullptr;  // [n] results
-  TrieView view0{};               // the first trie's view
+  TrieView view0{};               // the first trie's views
+  RevView rev0{};
   TrieView* dv = nullptr;
   RevView* dr = nullptr;
   Item* items = nullptr;          // warp items, at most cap_w
@@ -1692,15 +1895,15 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   P.threads = 32 * ep.warps;
   P.smem = (size_t)ep.smem_words * 4 * ep.warps;
   const void* kfn;
-  if (hits) kfn = (const void*)hits_kernel;
+  if (hits) kfn = n == 1 ? (const void*)hits_kernel<true> : (const void*)hits_kernel<false>;
   else if (query == EH_QUERY_CLIQUE4) kfn = (const void*)clique4_kernel;
-  else if (annot) kfn = (const void*)triangle_kernel<MODE_ANNOT>;
-  else kfn = (const void*)triangle_kernel<MODE_COUNT>;
+  else if (annot) kfn = (const void*)triangle_kernel<MODE_ANNOT, true>;
+  else kfn = n == 1 ? (const void*)triangle_kernel<MODE_COUNT, true> : (const void*)triangle_kernel<MODE_COUNT, false>;
   {
     size_t room = dynamic_smem_room(kfn);
     // the materializing pass launches MODE_MAT with the same shape
     if (!hits && !annot && query != EH_QUERY_CLIQUE4)
-      room = std::min(room, dynamic_smem_room((const void*)triangle_kernel<MODE_MAT>));
+      room = std::min(room, dynamic_smem_room((const void*)triangle_kernel<MODE_MAT, true>));
     if (P.smem > room) {
       // shrink the per-warp region to what a block may hold (a staged set
       // that no longer fits is probed in global memory instead)
@@ -1709,17 +1912,17 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
       P.smem = (size_t)ep.smem_words * 4 * ep.warps;
     }
   }
-  if (hits) set_smem_attr(hits_kernel, P.smem);
+  if (hits) set_smem_attr(n == 1 ? hits_kernel<true> : hits_kernel<false>, P.smem);
   else if (query == EH_QUERY_CLIQUE4) set_smem_attr(clique4_kernel, P.smem);
-  else if (annot) set_smem_attr(triangle_kernel<MODE_ANNOT>, P.smem);
-  else set_smem_attr(triangle_kernel<MODE_COUNT>, P.smem);
+  else if (annot) set_smem_attr(triangle_kernel<MODE_ANNOT, true>, P.smem);
+  else if (n == 1) set_smem_attr(triangle_kernel<MODE_COUNT, true>, P.smem);
+  else set_smem_attr(triangle_kernel<MODE_COUNT, false>, P.smem);
   const int per_sm = blocks_per_sm(kfn, P.threads, P.smem);
   // block items only for the plain triangle COUNT
   const bool blocks = block_items && !hits && query == EH_QUERY_TRIANGLE && !annot && ep.warps > 1 &&
                       !ep.no_block_items;
-  // work of all tries, and how finely to cut it: the default item is
-  // kDefaultChunk, and smaller when that would leave resident warps without
-  // work (8 items for each)
+  // work of all tries, and how finely to cut it: 8 items for each resident
+  // warp, of kMinChunk to kMaxChunk
   uint64_t cost = 0, head_items = 0;
   P.n = n;
   for (uint32_t g = 0; g < n; g++) {
@@ -1730,7 +1933,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   }
   if (!ep.chunk_given) {
     const uint64_t slots = (uint64_t)num_sms() * per_sm * ep.warps;
-    ep.chunk = (uint32_t)std::min<uint64_t>(kDefaultChunk, std::max<uint64_t>(kMinChunk, cost / (8 * slots)));
+    ep.chunk = (uint32_t)std::min<uint64_t>(kMaxChunk, std::max<uint64_t>(kMinChunk, cost / (8 * slots)));
   }
   PlanShape shape{ep.chunk, nullptr, 0.0, (uint32_t)ep.smem_words,
                    blocks ? (uint32_t)ep.smem_words * (uint32_t)ep.warps : 0u, (uint32_t)ep.warps};
@@ -1772,7 +1975,10 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     // 16-byte loads at 16-byte aligned indices
     if ((reinterpret_cast<uintptr_t>(v.vals) | reinterpret_cast<uintptr_t>(v.bs_words)) & 15u)
       throw Error{EH_ERR_UNSUPPORTED, "trie arrays are not 16-byte aligned"};
-    if (!g) P.view0 = v;
+    if (!g) {
+      P.view0 = v;
+      P.rev0 = r;
+    }
   }
   EH_CUDA(cudaMemcpyAsync(base, host, head_bytes, cudaMemcpyHostToDevice, s));
   for (uint32_t g = 0; g < n; g++) {
@@ -1823,8 +2029,9 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
     const Hits& H = P.hits;
     const HitsView hv = H.view();
     EH_CUDA(cudaMemsetAsync(H.mask.p, 0, H.words * 4, s));
-    hits_kernel<<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, P.ctl->items, ep.smem_words,
-                                                  P.ctl->queue, hv, d_records, ep.shard_index, ep.shard_count);
+    (P.n == 1 ? hits_kernel<true> : hits_kernel<false>)<<<P.grid, P.threads, P.smem, s>>>(
+        P.view0, P.rev0, P.dv, P.dr, P.items, P.ctl->items, ep.smem_words, P.ctl->queue, hv, d_records,
+        ep.shard_index, ep.shard_count);
     EH_CHECK_LAUNCH();
     if (H.use == HITS_CLIQUE) {
       clique_small_kernel<<<std::min(num_sms() * 8, ceil_div(H.heads, 256)), 256, 0, s>>>(P.dv, hv, d_total);
@@ -1848,9 +2055,14 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
   if (P.query == EH_QUERY_CLIQUE4)
     clique4_kernel<<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, ep.smem_words, out);
   else if (P.annot)
-    triangle_kernel<MODE_ANNOT><<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, ep.smem_words, out);
+    triangle_kernel<MODE_ANNOT, true><<<P.grid, P.threads, P.smem, s>>>(P.view0, P.rev0, P.dv, P.dr, P.items,
+                                                                        ep.smem_words, out);
+  else if (P.n == 1)
+    triangle_kernel<MODE_COUNT, true><<<P.grid, P.threads, P.smem, s>>>(P.view0, P.rev0, P.dv, P.dr, P.items,
+                                                                        ep.smem_words, out);
   else
-    triangle_kernel<MODE_COUNT><<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, ep.smem_words, out);
+    triangle_kernel<MODE_COUNT, false><<<P.grid, P.threads, P.smem, s>>>(P.view0, P.rev0, P.dv, P.dr, P.items,
+                                                                         ep.smem_words, out);
   EH_CHECK_LAUNCH();
 }
 
@@ -2389,7 +2601,7 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   Prepared P;
   const eh_trie* ts[1] = {t};
   prepare(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, false, P);
-  set_smem_attr(triangle_kernel<MODE_MAT>, P.smem);
+  set_smem_attr(triangle_kernel<MODE_MAT, true>, P.smem);
   unsigned int n_items = 0;
   EH_CUDA(cudaMemcpyAsync(&n_items, P.ctl->items, 4, cudaMemcpyDeviceToHost, s));
   EH_CUDA(cudaStreamSynchronize(s));
@@ -2398,7 +2610,8 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   QueryOut out{P.ep.long_row, P.total, nullptr, nullptr, P.ctl->queue, P.ctl->items, P.bitems};
   out.item_counts = counts.p;
   out.count_mult = mult;
-  triangle_kernel<MODE_COUNT><<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, P.ep.smem_words, out);
+  triangle_kernel<MODE_COUNT, true><<<P.grid, P.threads, P.smem, s>>>(P.view0, P.rev0, P.dv, P.dr, P.items,
+                                                                      P.ep.smem_words, out);
   EH_CHECK_LAUNCH();
   exclusive_scan<uint64_t>((const uint64_t*)counts.p, (uint64_t*)offs.p, n_items, (uint64_t*)rows.p, s);
   uint64_t nr = 0;
@@ -2412,7 +2625,8 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   out.mb = mb.p;
   out.mc = mc.p;
   EH_CUDA(cudaMemsetAsync(P.ctl->queue, 0, 8, s));
-  triangle_kernel<MODE_MAT><<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, P.ep.smem_words, out);
+  triangle_kernel<MODE_MAT, true><<<P.grid, P.threads, P.smem, s>>>(P.view0, P.rev0, P.dv, P.dr, P.items,
+                                                                    P.ep.smem_words, out);
   EH_CHECK_LAUNCH();
   // order by (a, b, c): stable sort by c, then stable sort by (a, b)
   const int grid = num_sms() * 8;
@@ -2461,7 +2675,7 @@ void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const 
   // launch shape and shared memory, checked before anything is launched
   const int threads = 32 * ep.warps;
   const size_t smem = (size_t)ep.smem_words * 4 * ep.warps;
-  const void* kfn = clique ? (const void*)clique4_kernel : (const void*)triangle_kernel<MODE_COUNT>;
+  const void* kfn = clique ? (const void*)clique4_kernel : (const void*)triangle_kernel<MODE_COUNT, true>;
   {
     const size_t room = dynamic_smem_room(kfn);
     EH_REQUIRE(smem <= room, EH_ERR_UNSUPPORTED,
@@ -2469,7 +2683,7 @@ void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const 
                    " a block may use");
   }
   if (clique) set_smem_attr(clique4_kernel, smem);
-  else set_smem_attr(triangle_kernel<MODE_COUNT>, smem);
+  else set_smem_attr(triangle_kernel<MODE_COUNT, true>, smem);
   const int per_sm = blocks_per_sm(kfn, threads, smem);
   // carve the scratch
   const uint32_t nh = t->n_head;
@@ -2535,7 +2749,7 @@ void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const 
     if (clique)
       clique4_kernel<<<grid, threads, smem, s>>>(dv, dr, items, ep.smem_words, out);
     else
-      triangle_kernel<MODE_COUNT><<<grid, threads, smem, s>>>(dv, dr, items, ep.smem_words, out);
+      triangle_kernel<MODE_COUNT, true><<<grid, threads, smem, s>>>(hv, hr, dv, dr, items, ep.smem_words, out);
     EH_CHECK_LAUNCH();
   }
   unsigned long long h = 0;
