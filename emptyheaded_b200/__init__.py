@@ -591,12 +591,12 @@ def set_intersect(sets, layouts, pairs, materialize=False, ctx=None):
         out_off = np.zeros(len(pa), np.uint64)
         if len(pa) > 1:
             np.cumsum(room[:-1], out=out_off[1:])
-        out = np.zeros(max(int(room.sum()), 1), np.uint32)
+        out = np.empty(max(int(room.sum()), 1), np.uint32)
     _check(lib().eh_set_intersect_batch(ctx.h, _ptr(elems), _ptr(off), len(sets), _ptr(lay), _ptr(pa), _ptr(pb),
                                         len(pa), _ptr(counts), _ptr(out_off), _ptr(out)))
     counts = counts[: len(pa)]
     if materialize:
-        return counts, [out[int(o): int(o) + int(c)].copy() for o, c in zip(out_off, counts)]
+        return counts, [out[o:e].copy() for o, e in zip(out_off.tolist(), (out_off + counts).tolist())]
     return counts
 
 

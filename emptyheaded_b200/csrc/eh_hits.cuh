@@ -193,7 +193,7 @@ __global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const __grid_constant__ TrieVie
     long long t0 = 0;
     if (records && lane == 0) t0 = clock64();
     Staged st;
-    const int mode = stage_set(t, item.hb, sm, cap_words, st, true);
+    const int mode = stage_set(t, item.hb, sm, cap_words, st, item.ke - item.kb > kListRows);
     switch (mode) {
       case P_SBITS:
         hit_rows<P_SBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);

@@ -65,6 +65,11 @@ constexpr uint32_t kWordRowNum = EH_WORD_ROW_NUM, kWordRowDen = EH_WORD_ROW_DEN;
 #define EH_LONG_WORDS 32
 #endif
 constexpr int kLongWords = EH_LONG_WORDS;  // word rows with at least this many words run warp-wide
+// an item of at most this many rows keeps a uint N(b) as a list: searching it
+// for so few beats building a bitmap (kernel ms, R-MAT-22 6.93 -> 6.85,
+// symmetric Chung-Lu 2^21 2.52 -> 2.21, ER-16K 0.0225 -> 0.0205; at 32 rows
+// R-MAT-22 6.96)
+constexpr uint32_t kListRows = 16;
 #ifndef EH_FLAT_CLIQUE
 #define EH_FLAT_CLIQUE 48
 #endif
@@ -340,8 +345,9 @@ __global__ void __launch_bounds__(256) plan_split_kernel(PlanArgs p) {
   }
 }
 
-// counts -> places in entry order; the totals to places[0..1] of ctl->spare
-__global__ void __launch_bounds__(256) plan_place_kernel(PlanArgs p, unsigned long long* __restrict__ total) {
+// counts -> places in entry order; the total of this trie, and the items so far
+__global__ void __launch_bounds__(256) plan_place_kernel(PlanArgs p, unsigned long long* __restrict__ total,
+                                                         Control* __restrict__ ctl) {
   __shared__ uint64_t s_warp[8], s_before;
   const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
   uint64_t before = 0;  // sums of the tiles before this one
@@ -372,20 +378,23 @@ __global__ void __launch_bounds__(256) plan_place_kernel(PlanArgs p, unsigned lo
     if (b0 + i < p.t.n_head) p.pos[b0 + i] = run;
     run += v[i];
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 255) *total = run;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 255) {
+    *total = run;
+    ctl->items[0] += (uint32_t)run;
+    ctl->items[1] += (uint32_t)(run >> 32);
+  }
 }
 
 // One thread per item (warp items first): item q of a class belongs to the last
 // entry whose place is at or before q (entries without items share the next
 // one's place and are never found), and covers the rows from the first one at
-// its share of the entry's cost to the first one at the next share.  Items are
-// appended after those of the tries before (ctl->items, which the next
-// launch on the stream adds to).
+// its share of the entry's cost to the first one at the next share.  Its items
+// follow those of the tries before.
 __global__ void __launch_bounds__(256) plan_fill_kernel(PlanArgs p, const unsigned long long* __restrict__ total,
                                                         const Control* __restrict__ ctl, Item* __restrict__ items,
                                                         Item* __restrict__ bitems) {
   const uint32_t nw = (uint32_t)*total, nb = (uint32_t)(*total >> 32);
-  const uint32_t w0 = ctl->items[0], b0 = ctl->items[1];
+  const uint32_t w0 = ctl->items[0] - nw, b0 = ctl->items[1] - nb;
   for (uint64_t x = blockIdx.x * 256ull + threadIdx.x; x < (uint64_t)nw + nb; x += gridDim.x * 256ull) {
     const bool cls = x >= nw;
     const uint32_t q = cls ? (uint32_t)(x - nw) : (uint32_t)x;
@@ -407,11 +416,6 @@ __global__ void __launch_bounds__(256) plan_fill_kernel(PlanArgs p, const unsign
     (cls ? bitems + b0 + (nb - 1 - q) : items + w0 + (nw - 1 - q))[0] = Item{b, (uint32_t)kb, (uint32_t)ke, p.g};
   }
 }
-__global__ void plan_append_kernel(const unsigned long long* __restrict__ total, Control* __restrict__ ctl) {
-  ctl->items[0] += (uint32_t)*total;
-  ctl->items[1] += (uint32_t)(*total >> 32);
-}
-
 
 // L2 eviction priority for the word rows' loads of N(a)'s bitset words: the
 // sources of the word rows are the density rule's dense sets (75 MB of words
@@ -1358,7 +1362,7 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ Tri
       mode = stage_set_block(t, item.hb, smem, cap_words * (int)nwarps, st);
       __syncthreads();
     } else {
-      mode = stage_set(t, item.hb, sm, cap_words, st, kMode == MODE_COUNT);
+      mode = stage_set(t, item.hb, sm, cap_words, st, kMode == MODE_COUNT && item.ke - item.kb > kListRows);
     }
     const StagedRange sr = staged_range(t, item.hb);
     const uint32_t blen = sr.len;
@@ -1995,14 +1999,13 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     const int tiles = ceil_div(t->n_head, kPlanTile);
     unsigned long long* total = &P.ctl->spare[1];
     plan_split_kernel<<<tiles, 256, 0, s>>>(pa);
-    plan_place_kernel<<<tiles, 256, 0, s>>>(pa, total);
+    plan_place_kernel<<<tiles, 256, 0, s>>>(pa, total, P.ctl);
     const uint64_t most = std::min<uint64_t>(t->n_head, t->rev_entries) +
                           (t->rev_pairs + kRowCost * t->rev_entries) / ep.chunk;
     plan_fill_kernel<<<(int)std::min<uint64_t>(num_sms() * 8, (most + 255) / 256), 256, 0, s>>>(pa, total, P.ctl,
                                                                                               P.items, P.bitems);
-    plan_append_kernel<<<1, 1, 0, s>>>(total, P.ctl);
     EH_CHECK_LAUNCH();
-    P.plan_launches += 4;
+    P.plan_launches += 3;
   }
   const uint64_t units = P.cap_b + (P.cap_w + ep.warps - 1) / ep.warps;
   P.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * per_sm, units));

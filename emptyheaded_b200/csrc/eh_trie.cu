@@ -184,10 +184,20 @@ __global__ void layout_heuristic_kernel(SetSrc src, uint32_t n_sets, int policy,
   }
 }
 
-// Sets with more than kBigSet elements (the head set, hubs of a symmetric
-// relation) are built by grid-wide passes, one set at a time; the
-// warp-per-set kernels below skip them.
-constexpr uint64_t kBigSet = 8192;
+// How a set's structure is built depends on its size (elements, or bitset words
+// when there are more of them): a warp up to kBigSet, a block up to kHugeSet, and
+// beyond (the head set of a large relation, hubs) grid-wide passes, one set at a
+// time.  (Every set above 8192 elements grid-wide, and wide sparse bitsets by a
+// warp, took 17 big sets of a 512-set batch 0.9 ms of launches and waits and
+// 0.35 ms in the warps.)
+constexpr uint64_t kBigSet = 2048;
+constexpr uint64_t kHugeSet = 1u << 17;
+constexpr int kBigThreads = 512;
+__device__ __forceinline__ uint64_t set_size(const uint32_t* p, uint64_t len, uint8_t layout) {
+  if (layout != EH_LAYOUT_RANGE_BITSET || !len) return len;
+  const uint64_t words = (uint64_t)(p[len - 1] >> 6) - (p[0] >> 6) + 1;
+  return len > words ? len : words;
+}
 
 // sizes of each set's bitset structure: words (range bitset) or blocks
 __global__ void aux_size_kernel(SetSrc src, uint32_t n_sets, const uint8_t* __restrict__ layout,
@@ -238,7 +248,7 @@ __global__ void bitset_fill_kernel(SetSrc src, uint32_t n_sets, const uint8_t* _
     const uint32_t* p;
     uint64_t len;
     src.get(i, p, len);
-    if (!len || len > kBigSet) continue;
+    if (!len || set_size(p, len, EH_LAYOUT_RANGE_BITSET) > kBigSet) continue;
     const SetAux a = aux[i];
     uint64_t* w = words + a.off;
     uint32_t* r = rank + a.off;
@@ -296,17 +306,118 @@ __global__ void block_fill_kernel(SetSrc src, uint32_t n_sets, const uint8_t* __
   }
 }
 
-// ---- grid-wide passes over one big set
+// ---- sets of more than a warp's size
+// lists: count[0] big sets from the front of idx, count[1] huge ones from its end
 __global__ void big_sets_kernel(SetSrc src, uint32_t n_sets, const uint8_t* __restrict__ layout,
                                 uint32_t* __restrict__ idx, unsigned int* __restrict__ count) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_sets; i += gridDim.x * blockDim.x) {
     const uint8_t l = layout[i];
     if (l != EH_LAYOUT_RANGE_BITSET && l != EH_LAYOUT_BLOCK_BITSET) continue;
-    const uint64_t len = i == src.n_head ? src.n_head : src.off[i + 1] - src.off[i];
-    if (len > kBigSet) idx[atomicAdd(count, 1u)] = i;
+    const uint32_t* p;
+    uint64_t len;
+    src.get(i, p, len);
+    const uint64_t size = set_size(p, len, l);
+    if (size > kHugeSet) idx[n_sets - 1 - atomicAdd(count + 1, 1u)] = i;
+    else if (size > kBigSet) idx[atomicAdd(count, 1u)] = i;
   }
 }
 
+// exclusive scan of v over the block; *total its sum
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  const uint32_t incl = warp_incl_scan(v);
+  if (lane == 31) s_warp[wid] = incl;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+  for (uint32_t w = 0; w < kBigThreads / 32; w++) {
+    const uint32_t c = s_warp[w];
+    if (w < wid) before += c;
+    all += c;
+  }
+  __syncthreads();  // s_warp is used again
+  *total = all;
+  return before + incl - v;
+}
+
+// block counts of the big block-bitset sets, a block per set
+__global__ void __launch_bounds__(kBigThreads) big_count_kernel(SetSrc src, const uint8_t* __restrict__ layout,
+                                                                const uint32_t* __restrict__ idx,
+                                                                const unsigned int* __restrict__ count,
+                                                                uint64_t* __restrict__ blocks,
+                                                                SetAux* __restrict__ aux) {
+  __shared__ uint32_t s_warp[kBigThreads / 32];
+  const unsigned int n = *count;
+  for (unsigned int k = blockIdx.x; k < n; k += gridDim.x) {
+    const uint32_t i = idx[k];
+    if (layout[i] != EH_LAYOUT_BLOCK_BITSET) continue;
+    const uint32_t* p;
+    uint64_t len;
+    src.get(i, p, len);
+    uint32_t c = 0;
+    for (uint64_t j = threadIdx.x; j < len; j += kBigThreads) c += j == 0 || (p[j] >> 8) != (p[j - 1] >> 8);
+    uint32_t total;
+    block_scan(c, s_warp, &total);
+    if (threadIdx.x == 0) {
+      blocks[i] = total;
+      aux[i].n = total;
+    }
+  }
+}
+
+// the structures of the big sets, a block per set
+__global__ void __launch_bounds__(kBigThreads) big_fill_kernel(SetSrc src, const uint8_t* __restrict__ layout,
+                                                               const uint32_t* __restrict__ idx,
+                                                               const unsigned int* __restrict__ count,
+                                                               const SetAux* __restrict__ aux,
+                                                               uint64_t* __restrict__ words,
+                                                               uint32_t* __restrict__ rank,
+                                                               uint32_t* __restrict__ bid,
+                                                               uint32_t* __restrict__ brank,
+                                                               uint64_t* __restrict__ bwords) {
+  __shared__ uint32_t s_warp[kBigThreads / 32];
+  const unsigned int n = *count;
+  for (unsigned int k = blockIdx.x; k < n; k += gridDim.x) {
+    const uint32_t i = idx[k];
+    const uint32_t* p;
+    uint64_t len;
+    src.get(i, p, len);
+    const SetAux a = aux[i];
+    uint32_t run = 0, total;
+    if (layout[i] == EH_LAYOUT_RANGE_BITSET) {
+      uint64_t* w = words + a.off;
+      for (uint32_t j = threadIdx.x; j < a.n; j += kBigThreads) w[j] = 0;
+      __syncthreads();
+      for (uint64_t j = threadIdx.x; j < len; j += kBigThreads)
+        atomicOr((unsigned long long*)&w[(p[j] >> 6) - a.start], 1ull << (p[j] & 63));
+      __syncthreads();
+      for (uint32_t j0 = 0; j0 < a.n; j0 += kBigThreads) {
+        const uint32_t j = j0 + threadIdx.x;
+        const uint32_t c = j < a.n ? (uint32_t)__popcll(__ldcg(&w[j])) : 0u;  // the atomics wrote to L2
+        const uint32_t before = block_scan(c, s_warp, &total);
+        if (j < a.n) rank[a.off + j] = run + before;
+        run += total;
+      }
+    } else {
+      for (uint32_t j = threadIdx.x; j < 4 * a.n; j += kBigThreads) bwords[4 * a.off + j] = 0;
+      __syncthreads();
+      for (uint64_t j0 = 0; j0 < len; j0 += kBigThreads) {
+        const uint64_t j = j0 + threadIdx.x;
+        const uint32_t x = j < len ? p[j] : 0;
+        const uint32_t first = j < len && (j == 0 || (x >> 8) != (p[j - 1] >> 8));
+        const uint32_t before = block_scan(first, s_warp, &total);
+        const uint64_t blk = a.off + run + before + first - 1;  // of element j
+        if (first) {
+          bid[blk] = x >> 8;
+          brank[blk] = (uint32_t)j;
+        }
+        if (j < len) atomicOr((unsigned long long*)&bwords[4 * blk + ((x >> 6) & 3)], 1ull << (x & 63));
+        run += total;
+      }
+    }
+  }
+}
+
+// ---- grid-wide passes over one huge set
 // first element of each 256-value block of set i (flag per element)
 __global__ void big_block_flags_kernel(SetSrc src, uint32_t i, uint32_t* __restrict__ flag,
                                        unsigned long long* __restrict__ nblocks) {
@@ -426,20 +537,24 @@ static void build_layout_structs(eh_context* ctx, eh_trie* t) {
   DevBuf<uint64_t> words(n_sets + 1, s), blocks(n_sets + 1, s), tot(2, s);
   aux_size_kernel<<<grid, 256, 0, s>>>(src, n_sets, t->layout.p, t->aux.p, words.p, blocks.p);
   EH_CHECK_LAUNCH();
-  // the big sets, and the block counts of big block-bitset sets
-  std::vector<uint32_t> big;
+  // the big sets (counted here, filled below, by blocks) and the huge ones
+  std::vector<uint32_t> big;  // huge sets
+  DevBuf<uint32_t> idx(n_sets, s);
+  DevBuf<unsigned int> lists(2, s);
+  const int big_grid = num_sms() * 2;
   {
-    DevBuf<uint32_t> idx(n_sets, s);
-    DevBuf<unsigned int> cnt(1, s);
-    EH_CUDA(cudaMemsetAsync(cnt.p, 0, 4, s));
-    big_sets_kernel<<<grid, 256, 0, s>>>(src, n_sets, t->layout.p, idx.p, cnt.p);
+    EH_CUDA(cudaMemsetAsync(lists.p, 0, 8, s));
+    big_sets_kernel<<<grid, 256, 0, s>>>(src, n_sets, t->layout.p, idx.p, lists.p);
+    big_count_kernel<<<big_grid, kBigThreads, 0, s>>>(src, t->layout.p, idx.p, lists.p, blocks.p, t->aux.p);
     EH_CHECK_LAUNCH();
-    unsigned int nb = 0;
-    EH_CUDA(cudaMemcpyAsync(&nb, cnt.p, 4, cudaMemcpyDeviceToHost, s));
+    unsigned int nb[2] = {0, 0};
+    EH_CUDA(cudaMemcpyAsync(nb, lists.p, 8, cudaMemcpyDeviceToHost, s));
     EH_CUDA(cudaStreamSynchronize(s));
-    big.resize(nb);
-    if (nb) EH_CUDA(cudaMemcpyAsync(big.data(), idx.p, nb * 4, cudaMemcpyDeviceToHost, s));
-    EH_CUDA(cudaStreamSynchronize(s));
+    big.resize(nb[1]);
+    if (nb[1]) {
+      EH_CUDA(cudaMemcpyAsync(big.data(), idx.p + n_sets - nb[1], nb[1] * 4, cudaMemcpyDeviceToHost, s));
+      EH_CUDA(cudaStreamSynchronize(s));
+    }
   }
   std::vector<uint8_t> big_layout(big.size());
   std::vector<uint64_t> big_len(big.size());
@@ -488,6 +603,9 @@ static void build_layout_structs(eh_context* ctx, eh_trie* t) {
                                            t->bb_words.p);
     EH_CHECK_LAUNCH();
   }
+  big_fill_kernel<<<big_grid, kBigThreads, 0, s>>>(src, t->layout.p, idx.p, lists.p, t->aux.p, t->bs_words.p,
+                                                   t->bs_rank.p, t->bb_id.p, t->bb_rank.p, t->bb_words.p);
+  EH_CHECK_LAUNCH();
   ph_bfill.end();
   TracePhase ph_big("structs.big_sets", s);
   for (size_t k = 0; k < big.size(); k++) {
