@@ -162,6 +162,78 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
   }
 }
 
+// hit_rows for a merged item: each row's candidates looked up in its own entry's
+// list.  Short rows are flattened as there; a longer one (the item holds 1024
+// candidates at most) runs a mask word at a time.
+__device__ __forceinline__ void hit_merged(const TrieView& t, const RevView& r, uint32_t h0, uint32_t kb, uint32_t ke,
+                                           const uint32_t* __restrict__ moff, uint32_t* __restrict__ mask,
+                                           uint32_t shard_index, uint32_t shard_count) {
+  const uint32_t lane = lane_id();
+  const uint32_t step = r.dir == DIR_DOWN ? 0xffffffffu : 1u;
+  const Merged m(t, r, h0);
+  for (uint32_t k0 = kb; k0 < ke; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    uint32_t len = 0, fe = 0, skip = 0, base = 0, rs = 0;
+    if (k < ke) {
+      const uint32_t src = __ldg(r.rev_src + k);
+      if (shard_count == 1 || src % shard_count == shard_index) {
+        const uint32_t lo = __ldg(r.rev_lo + k), hi = __ldg(r.rev_hi + k);
+        const uint32_t d = staged_range(t, src).len, W = (d + 31) >> 5;
+        len = hi - lo;
+        const uint32_t i = d - 1 - len, q = i >> 5;
+        fe = r.dir == DIR_DOWN ? hi - 1 : lo;
+        skip = (i & 31) + 1;
+        base = __ldg(moff + src) + hits_block(q, W) + (i & 31);
+        rs = hits_stride(q, W, d);
+      }
+    }
+    const uint32_t e = m.entry(min(k, ke - 1));
+    const uint32_t s0 = __shfl_sync(kFull, (uint32_t)m.s0, e), n = __shfl_sync(kFull, m.len, e);
+    uint32_t rows = __ballot_sync(kFull, len > 32);
+    while (rows) {
+      const int j = __ffs(rows) - 1;
+      rows &= rows - 1;
+      const uint32_t sk = __shfl_sync(kFull, skip, j), end = sk + __shfl_sync(kFull, len, j);
+      const uint32_t ej = __shfl_sync(kFull, fe, j) - step * sk, sj = __shfl_sync(kFull, s0, j);
+      const uint32_t nj = __shfl_sync(kFull, n, j), bj = __shfl_sync(kFull, base, j), rj = __shfl_sync(kFull, rs, j);
+      for (uint32_t w = 0; 32 * w < end; w++) {
+        const uint32_t p = 32 * w + lane;
+        const uint32_t b = __ballot_sync(kFull, p >= sk && p < end && list_has(t.vals, sj, nj, __ldg(t.vals + (ej + step * min(max(p, sk), end - 1)))));
+        if (lane == 0 && b) mask[bj + w * rj] = b;
+      }
+    }
+    if (len > 32) len = 0;
+    const uint32_t incl = warp_incl_scan(len);
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    const uint32_t excl = incl - len;
+    const uint32_t elem0 = fe - step * excl;
+    uint32_t acc = 0;
+    for (uint32_t p = 0; p < total; p += 64) {
+      uint32_t w[2], sj[2], nj[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const uint32_t q = min(p + 32 * u + lane, total - 1);
+        const uint32_t j = owner_lane(incl, q);
+        w[u] = __ldg(t.vals + (__shfl_sync(kFull, elem0, j) + step * q));
+        sj[u] = __shfl_sync(kFull, s0, j);
+        nj[u] = __shfl_sync(kFull, n, j);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const uint32_t p0 = p + 32 * u;
+        const uint32_t ball = __ballot_sync(kFull, list_has(t.vals, sj[u], nj[u], w[u]));
+        const uint32_t s = max(excl, p0), x = min(incl, p0 + 32);
+        if (s < x) acc |= ((ball >> (s - p0)) & (0xffffffffu >> (32 - (x - s)))) << (s - excl);
+      }
+    }
+    if (acc) {
+      const uint64_t bits = (uint64_t)acc << skip;
+      if ((uint32_t)bits) mask[base] = (uint32_t)bits;
+      if ((uint32_t)(bits >> 32)) mask[base + rs] = (uint32_t)(bits >> 32);
+    }
+  }
+}
+
 // kOne: as in triangle_kernel
 template <bool kOne>
 __global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const __grid_constant__ TrieView t1,
@@ -192,6 +264,10 @@ __global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const __grid_constant__ TrieVie
     const uint32_t* moff = hv.moff + hv.gstart[item.g];
     long long t0 = 0;
     if (records && lane == 0) t0 = clock64();
+    if (item.hb & kMerged) {
+      hit_merged(t, r, item.hb & ~kMerged, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+      continue;
+    }
     Staged st;
     const int mode = stage_set(t, item.hb, sm, cap_words, st, item.ke - item.kb > kListRows);
     switch (mode) {

@@ -244,6 +244,7 @@ struct PlanShape {
   uint32_t warp_words;   // staging capacity of a warp (u32 words)
   uint32_t block_words;  // staging capacity of a block; 0: no block items
   uint32_t warps;        // warps per block
+  uint32_t merge;        // 1: neighbouring entries with little work share an item
 };
 
 // Cost of a row beside its candidates, in candidates: a row of one candidate
@@ -301,9 +302,34 @@ struct PlanArgs {
 };
 constexpr uint32_t kPlanTile = 2048;
 
+// Neighbouring entries whose work together is small share one item (kMerged):
+// its rows are looked up in their sets' lists where they lie, nothing is
+// staged.  Most entries of a skewed relation end a few rows of a few candidates
+// each, and an item of its own costs one of them a queue turn and a chain of
+// loads of some 5,000 cycles for a hundred cycles of work (96 R-MAT graphs
+// 1.77 -> 1.45 ms, lollipop Chung-Lu 2^21 4.26 -> 3.39).  Groups are aligned:
+// 16 entries, or 8, of at most kMergeRows rows and kMergeElems candidates and
+// elements.
+constexpr uint32_t kMerged = 0x80000000u;
+constexpr uint64_t kMergeRows = 128, kMergeElems = 1024;
+__device__ __forceinline__ bool plan_small(const PlanArgs& p, uint32_t h0, uint32_t span) {
+  if (h0 + span > p.t.n_head) return false;
+  const uint64_t k0 = p.r.rev_off[h0], k1 = p.r.rev_off[h0 + span];
+  return k1 - k0 <= kMergeRows && p.r.rev_wpre[k1] - p.r.rev_wpre[k0] <= kMergeElems &&
+         p.t.off[h0 + span] - p.t.off[h0] <= kMergeElems;
+}
+// entries that share b's item, the first of which has it; 1: none
+__device__ __forceinline__ uint32_t plan_span(const PlanArgs& p, uint32_t b) {
+  if (!p.ps.merge) return 1;
+  if (plan_small(p, b & ~15u, 16)) return 16;
+  return plan_small(p, b & ~7u, 8) ? 8 : 1;
+}
+
 // items of entry b over all shards
 __device__ __forceinline__ uint32_t plan_items(const PlanArgs& p, uint32_t b, uint64_t k0, uint64_t k1, bool& blk) {
   blk = false;
+  const uint32_t span = plan_span(p, b);
+  if (span > 1) return (b & (span - 1)) == 0 && p.r.rev_off[b + span] > k0 ? 1 : 0;
   if (k1 <= k0) return 0;
   const uint64_t w = p.r.rev_wpre[k1] - p.r.rev_wpre[k0];
   if (p.ps.block_words && w >= kMinBlockWork) {
@@ -410,6 +436,11 @@ __global__ void __launch_bounds__(256) plan_fill_kernel(PlanArgs p, const unsign
     bool blk;
     const uint64_t m = plan_items(p, b, k0, k1, blk);
     const uint64_t i = plan_first(p, b) + (uint64_t)(q - (cls ? (uint32_t)(v >> 32) : (uint32_t)v)) * p.shard_count;
+    const uint32_t span = plan_span(p, b);
+    if (span > 1) {
+      items[w0 + (nw - 1 - q)] = Item{b | kMerged, (uint32_t)k0, (uint32_t)p.r.rev_off[b + span], p.g};
+      continue;
+    }
     const uint64_t wp = p.r.rev_wpre[k0], W = p.r.rev_wpre[k1] - wp + kRowCost * (k1 - k0);
     const uint64_t kb = i ? row_at_cost(p.r.rev_wpre, k0, k1, wp, (W * i) / m) : k0;
     const uint64_t ke = i + 1 < m ? row_at_cost(p.r.rev_wpre, k0, k1, wp, (W * (i + 1)) / m) : k1;
@@ -1043,6 +1074,75 @@ __device__ __forceinline__ uint64_t count_rows(const Staged& st, const TrieView&
   return total_hits;
 }
 
+// Entries of a merged item: lane i <= 15 holds entry h0 + i's first row and its
+// staged range (entries past the item's last row are never asked for).
+struct Merged {
+  uint64_t s0;
+  uint32_t len, row;
+  __device__ __forceinline__ Merged(const TrieView& t, const RevView& r, uint32_t h0) {
+    const uint32_t i = lane_id() & 15u;
+    const uint32_t h = min(h0 + i, t.n_head - 1);
+    const StagedRange sr = staged_range(t, h);
+    s0 = sr.s0;
+    len = sr.len;
+    row = h0 + i < t.n_head ? (uint32_t)__ldg(r.rev_off + h) : 0xffffffffu;
+  }
+  // which entry row k belongs to: the last one that starts at or before it
+  __device__ __forceinline__ uint32_t entry(uint32_t k) const {
+    uint32_t e = 0;
+#pragma unroll
+    for (int step = 8; step; step >>= 1) {
+      const uint32_t v = __shfl_sync(kFull, row, e + step);
+      if (v <= k) e += step;
+    }
+    return e;
+  }
+};
+__device__ __forceinline__ bool list_has(const uint32_t* __restrict__ vals, uint32_t s0, uint32_t n, uint32_t w) {
+  const uint32_t* p = vals + s0;  // n >= 1: an entry with rows has a staged part
+  while (n > 1) {
+    const uint32_t half = n >> 1;
+    if (__ldg(p + half) <= w) p += half;
+    n -= half;
+  }
+  return __ldg(p) == w;
+}
+// the hits of a merged item: flattened (row, candidate) pairs, each looked up in
+// its own entry's list
+__device__ __forceinline__ uint32_t count_merged(const TrieView& t, const RevView& r, uint32_t h0, uint32_t kb,
+                                                 uint32_t ke) {
+  const uint32_t lane = lane_id();
+  const Merged m(t, r, h0);
+  uint32_t cnt = 0;
+  for (uint32_t k0 = kb; k0 < ke; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    uint32_t lo = 0, len = 0;
+    if (k < ke) {
+      lo = __ldg(r.rev_lo + k);
+      len = __ldg(r.rev_hi + k) - lo;
+    }
+    const uint32_t e = m.entry(min(k, ke - 1));
+    const uint32_t s0 = __shfl_sync(kFull, (uint32_t)m.s0, e), n = __shfl_sync(kFull, m.len, e);
+    const uint32_t incl = warp_incl_scan(len);
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    const uint32_t elem = lo - (incl - len);
+    for (uint32_t p = 0; p < total; p += 64) {
+      uint32_t w[2], sj[2], nj[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const uint32_t q = min(p + 32 * u + lane, total - 1);
+        const uint32_t j = owner_lane(incl, q);
+        w[u] = __ldg(t.vals + (__shfl_sync(kFull, elem, j) + q));
+        sj[u] = __shfl_sync(kFull, s0, j);
+        nj[u] = __shfl_sync(kFull, n, j);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++) cnt += p + 32 * u + lane < total && list_has(t.vals, sj[u], nj[u], w[u]);
+    }
+  }
+  return cnt;
+}
+
 // Stage N(b) in the warp's shared region according to its layout; returns
 // the probe mode.
 __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_t* sm, int cap_words, Staged& st,
@@ -1309,6 +1409,11 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ Tri
   // time from a block counter.  Then each warp pulls warp items on its own.
   __shared__ unsigned int s_q, s_next;
   const uint32_t nwarps = blockDim.x >> 5;
+  // a batch's current views, per warp: read where they are used instead of
+  // held in two dozen registers
+  __shared__ TrieView s_view[kOne ? 1 : kMaxWarps];
+  __shared__ RevView s_rev[kOne ? 1 : kMaxWarps];
+  uint32_t view_g = 0xffffffffu;
   const uint32_t n_witems = __ldg(out.n_items), n_bitems = kMode == MODE_COUNT ? __ldg(out.n_items + 1) : 0u;
   bool block_phase = n_bitems != 0;
   for (;;) {
@@ -1338,14 +1443,17 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ Tri
       acc = 0;
       cur_g = item.g;
     }
-    TrieView tg;
-    RevView rg;
-    if (!kOne) {
-      tg = views[item.g];
-      rg = revs[item.g];
+    if (!kOne && item.g != view_g) {
+      view_g = item.g;
+      __syncwarp();
+      if (lane == 0) {
+        s_view[wid] = views[item.g];
+        s_rev[wid] = revs[item.g];
+      }
+      __syncwarp();
     }
-    const TrieView& t = kOne ? t1 : tg;
-    const RevView& r = kOne ? r1 : rg;
+    const TrieView& t = kOne ? t1 : s_view[kOne ? 0 : wid];
+    const RevView& r = kOne ? r1 : s_rev[kOne ? 0 : wid];
     long long t0 = 0;
     if (out.records && lane == 0) t0 = clock64();
     Sink sk{out.annot, out.ma, out.mb, out.mc, 0, &slot[wid], 0, hot, hot_acc, nullptr, 0, nullptr, nullptr,
@@ -1358,13 +1466,16 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ Tri
     }
     Staged st;
     int mode;
-    if (block_phase) {
+    const bool merged = kMode == MODE_COUNT && (item.hb & kMerged);
+    if (merged) {
+      mode = P_GLIST;
+    } else if (block_phase) {
       mode = stage_set_block(t, item.hb, smem, cap_words * (int)nwarps, st);
       __syncthreads();
     } else {
       mode = stage_set(t, item.hb, sm, cap_words, st, kMode == MODE_COUNT && item.ke - item.kb > kListRows);
     }
-    const StagedRange sr = staged_range(t, item.hb);
+    const StagedRange sr = kMode == MODE_ANNOT ? staged_range(t, item.hb) : StagedRange{0, 0};
     const uint32_t blen = sr.len;
     if (kMode == MODE_ANNOT && r.dir == DIR_SYM && (mode == P_SLIST || mode == P_SBITS)) {
       // per-element counters after the staged structure, if they fit
@@ -1389,7 +1500,9 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ Tri
       }
     }
     uint64_t c = 0;
-    if (block_phase) {
+    if (kMode == MODE_COUNT && merged) {
+      c = count_merged(t, r, item.hb & ~kMerged, item.kb, item.ke);
+    } else if (block_phase) {
       for (;;) {
         uint32_t batch = 0;
         if (lane == 0) batch = atomicAdd(&s_next, 1u);
@@ -1879,9 +1992,11 @@ static void size_clique_staging(ExecParams& ep, uint32_t max_set) {
 }
 
 // hits_use: run the plan on hit masks when they can be had (HITS_*; -1: never).
-// keep: the launch outlives the call, so its device memory is its own.
+// keep: the launch outlives the call, so its device memory is its own.  merge:
+// entries with little work may share items.
 static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query, ExecParams ep, bool annot,
-                    Prepared& P, bool block_items = false, int hits_use = -1, bool keep = false) {
+                    Prepared& P, bool block_items = false, int hits_use = -1, bool keep = false,
+                    bool merge = true) {
   cudaStream_t s = ctx->stream;
   P.query = query;
   P.annot = annot;
@@ -1923,6 +2038,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   else set_smem_attr(triangle_kernel<MODE_COUNT, false>, P.smem);
   const int per_sm = blocks_per_sm(kfn, P.threads, P.smem);
   // block items only for the plain triangle COUNT
+  const bool blocks_query = query == EH_QUERY_TRIANGLE && !annot;
   const bool blocks = block_items && !hits && query == EH_QUERY_TRIANGLE && !annot && ep.warps > 1 &&
                       !ep.no_block_items;
   // work of all tries, and how finely to cut it: 8 items for each resident
@@ -1935,12 +2051,12 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     cost += tries[g]->rev_pairs + kRowCost * tries[g]->rev_entries;
     head_items += std::min<uint64_t>(tries[g]->n_head, tries[g]->rev_entries);
   }
+  const uint64_t slots = (uint64_t)num_sms() * per_sm * ep.warps;  // resident warps
   if (!ep.chunk_given) {
-    const uint64_t slots = (uint64_t)num_sms() * per_sm * ep.warps;
     ep.chunk = (uint32_t)std::min<uint64_t>(kMaxChunk, std::max<uint64_t>(kMinChunk, cost / (8 * slots)));
   }
   PlanShape shape{ep.chunk, nullptr, 0.0, (uint32_t)ep.smem_words,
-                   blocks ? (uint32_t)ep.smem_words * (uint32_t)ep.warps : 0u, (uint32_t)ep.warps};
+                   blocks ? (uint32_t)ep.smem_words * (uint32_t)ep.warps : 0u, (uint32_t)ep.warps, 0u};
   // items: at most one per entry with rows and one per chunk of work (with
   // predicted costs: per chunk of probes, the sum of rounded-up shares; the
   // slack covers their rounding)
@@ -1989,6 +2105,10 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     const eh_trie* t = tries[g];
     if (!t->rev_entries) continue;
     // every shard of a plan on hit masks runs all the items: the masks split by head entry
+    // records are per entry, only these kernels look rows up, and few entries
+    // are better spread over the warps (ER-16K, three entries a warp: 77 us a
+    // query against 87 with shared items)
+    shape.merge = merge && (hits || blocks_query) && t->n_head < kMerged && head_items > 4 * slots;
     PlanArgs pa{t->view(), rev_view(t), shape, g, hits ? 0 : ep.shard_index, hits ? 1 : ep.shard_count,
                 reinterpret_cast<uint64_t*>(base + o_pos), nullptr};
     pa.tiles = pa.pos + t->n_head;
@@ -2080,7 +2200,7 @@ static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n
     TracePhase ph("query.prepare", s);
     // selections weight cliques by their members: they run without masks
     const int use = sel ? -1 : query == EH_QUERY_CLIQUE4 ? HITS_CLIQUE : annot ? HITS_ANNOT : -1;
-    prepare(ctx, tries, n, query, ep, annot, P, true, use);
+    prepare(ctx, tries, n, query, ep, annot, P, true, use, false, d_records == nullptr);
   }
   P.sel = sel;
   L.launches = P.plan_launches;
@@ -2603,7 +2723,7 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   ep.shard_count = 1;
   Prepared P;
   const eh_trie* ts[1] = {t};
-  prepare(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, false, P);
+  prepare(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, false, P, false, -1, false, false);
   set_smem_attr(triangle_kernel<MODE_MAT, true>, P.smem);
   unsigned int n_items = 0;
   EH_CUDA(cudaMemcpyAsync(&n_items, P.ctl->items, 4, cudaMemcpyDeviceToHost, s));
