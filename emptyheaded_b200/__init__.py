@@ -138,6 +138,8 @@ def lib():
                                       ctypes.POINTER(QueryStats)],
             "eh_query_materialize": [_P, _P, ctypes.c_int, ctypes.POINTER(ExecConfig), ctypes.c_int, _P, _P, _P,
                                      ctypes.c_uint64, _u64p],
+            "eh_query_materialize_rows": [_P, _P, ctypes.c_int, ctypes.POINTER(ExecConfig), _P, ctypes.c_uint64,
+                                          _u64p],
             "eh_query_count_batched": [_P, _P, ctypes.c_uint32, ctypes.c_int, ctypes.POINTER(ExecConfig), _P,
                                        ctypes.POINTER(QueryStats)],
             "eh_triangle_annotation": [_P, _P, ctypes.POINTER(ExecConfig), _P],
@@ -458,20 +460,25 @@ class Trie:
     def materialize(self, query="triangle", project=False):
         """Rows of Triangle(a,b,c) sorted by (a,b,c) as an (n, 3) uint32
         array; project=True gives TriangleProj(a,b), an (n, 2) array."""
-        cols = 2 if project else 3
         e = _exec_cfg()
         n = ctypes.c_uint64()
-        # the device builds the rows once to size them, then fills
-        _check(lib().eh_query_materialize(self.ctx.h, self.h, QUERIES[query], ctypes.byref(e), cols, None, None,
-                                          None, 0, ctypes.byref(n)))
+        # the device counts the rows to size them, then fills
+        if not project:
+            fill = lib().eh_query_materialize_rows
+            _check(fill(self.ctx.h, self.h, QUERIES[query], ctypes.byref(e), None, 0, ctypes.byref(n)))
+            out = np.empty((n.value, 3), np.uint32)
+            if n.value:
+                _check(fill(self.ctx.h, self.h, QUERIES[query], ctypes.byref(e), _ptr(out), n.value, ctypes.byref(n)))
+            return out
+        _check(lib().eh_query_materialize(self.ctx.h, self.h, QUERIES[query], ctypes.byref(e), 2, None, None, None, 0,
+                                          ctypes.byref(n)))
         rows = n.value
         a = np.empty(max(rows, 1), np.uint32)
         b = np.empty(max(rows, 1), np.uint32)
         c = np.empty(max(rows, 1), np.uint32)
-        _check(lib().eh_query_materialize(self.ctx.h, self.h, QUERIES[query], ctypes.byref(e), cols, _ptr(a),
-                                          _ptr(b), _ptr(c), rows, ctypes.byref(n)))
-        out = [a[:rows], b[:rows]] + ([] if project else [c[:rows]])
-        return np.stack(out, 1)
+        _check(lib().eh_query_materialize(self.ctx.h, self.h, QUERIES[query], ctypes.byref(e), 2, _ptr(a), _ptr(b),
+                                          _ptr(c), rows, ctypes.byref(n)))
+        return np.stack([a[:rows], b[:rows]], 1)
 
     def weighted_root(self, query, z):
         """Root bag of lollipop / barbell over an annotation z given by node

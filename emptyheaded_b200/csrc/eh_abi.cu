@@ -598,6 +598,15 @@ eh_status eh_query_materialize(eh_context* ctx, const eh_trie* trie, int query, 
   });
 }
 
+eh_status eh_query_materialize_rows(eh_context* ctx, const eh_trie* trie, int query, const eh_exec_config* cfg,
+                                    uint32_t* rows, uint64_t cap, uint64_t* n_rows) {
+  return guarded([&] {
+    need(ctx && trie && n_rows, "null argument");
+    set_device(ctx);
+    query_materialize(ctx, trie, query, cfg, 3, nullptr, nullptr, nullptr, cap, n_rows, rows);
+  });
+}
+
 eh_status eh_batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n_tries, int query,
                           const eh_exec_config* cfg, eh_batch** out) {
   return guarded([&] {

@@ -79,6 +79,11 @@ __global__ void order_keys_kernel(const void* __restrict__ col, uint64_t n, int 
     keys[i] = order_key(col, i, type, bad);
 }
 
+__global__ void add_kernel(const uint64_t* in, uint64_t n, uint64_t x, uint64_t* out) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    out[i] = in[i] + x;
+}
+
 __global__ void minmax_u64_kernel(const uint64_t* __restrict__ a, uint64_t n, unsigned long long* __restrict__ mm) {
   unsigned long long lo = ~0ull, hi = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -198,12 +203,20 @@ eh_encoding* encoding_build(eh_context* ctx, const void* const* cols, const uint
       EH_CUDA(cudaStreamSynchronize(s));
       EH_REQUIRE(hb == 0, EH_ERR_INVALID, "NaN in a float column (no order to encode it by)");
       const uint64_t lo = h[0], hi = h[1];
-      radix_sort_u64(keys.p, tmp.p, total, bits_for_u64(hi), s);
+      // sorted as offsets from the smallest key where that takes fewer 8-bit
+      // passes (signed values set the top bit: 42-bit ids 8 -> 6)
+      const uint64_t base = (bits_for_u64(hi - lo) + 7) / 8 < (bits_for_u64(hi) + 7) / 8 ? lo : 0;
+      if (base) {
+        add_kernel<<<grid, 256, 0, s>>>(keys.p, total, 0 - base, keys.p);
+        EH_CHECK_LAUNCH();
+      }
+      radix_sort_u64(keys.p, tmp.p, total, bits_for_u64(hi - base), s);
       const uint64_t d = unique_sorted_u64(keys.p, tmp.p, total, s);
       EH_REQUIRE(d <= 0xfffffffeull, EH_ERR_UNSUPPORTED, "more than 2^32 - 2 distinct values");
       e->n_distinct = d;
       e->dict.alloc(d, s);
-      EH_CUDA(cudaMemcpyAsync(e->dict.p, tmp.p, d * 8, cudaMemcpyDeviceToDevice, s));
+      add_kernel<<<grid, 256, 0, s>>>(tmp.p, d, base, e->dict.p);
+      EH_CHECK_LAUNCH();
       const uint64_t span = hi - lo + 1;  // hi >= lo; span 0 means the full 2^64 range
       if (span != 0 && span <= 4 * d + (1ull << 20)) {
         e->lo = lo;

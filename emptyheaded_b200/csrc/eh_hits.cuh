@@ -551,7 +551,7 @@ __global__ void hits_row_count_kernel(TrieView t, int dir, HitsView hv, const ui
 __global__ void __launch_bounds__(256) hits_row_write_kernel(TrieView t, int dir, HitsView hv,
                                                              const uint32_t* __restrict__ seg,
                                                              const uint64_t* __restrict__ pos, uint64_t total,
-                                                             uint32_t* __restrict__ oa, uint32_t* __restrict__ ob,
+                                                             int stride, uint32_t* __restrict__ oa, uint32_t* __restrict__ ob,
                                                              uint32_t* __restrict__ oc) {
   const uint32_t lane = lane_id();
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(256) hits_row_write_kernel(TrieView t, int dir
         if ((x >> lane) & 1u) {
           const uint32_t bit = dir == DIR_DOWN ? 31 - lane : lane;
           const uint32_t j = 32 * (q + k) + bit;
-          const uint64_t o = out + __popc(x & lanemask_lt());
+          const uint64_t o = (out + __popc(x & lanemask_lt())) * stride;
           oa[o] = va;
           ob[o] = vb;
           oc[o] = __ldg(t.vals + pr.s0 + (dir == DIR_DOWN ? d - 1 - j : j));

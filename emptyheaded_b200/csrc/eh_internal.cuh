@@ -198,7 +198,8 @@ void batch_free(eh_batch* b);
 void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const eh_exec_config* cfg,
                             unsigned char* scratch, size_t bytes, uint64_t* result);
 void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_exec_config* cfg, int n_cols,
-                       uint32_t* a, uint32_t* b, uint32_t* c, uint64_t cap, uint64_t* n_rows);
+                       uint32_t* a, uint32_t* b, uint32_t* c, uint64_t cap, uint64_t* n_rows,
+                       uint32_t* rows_out = nullptr);
 
 // rules (eh_rule.cu): the EH_QUERY_* of a rule body, and its relation
 int rule_match(const eh_rule* rule, uint32_t* relation);

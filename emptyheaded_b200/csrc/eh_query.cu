@@ -2601,12 +2601,15 @@ __global__ void ab_key_kernel(const uint32_t* __restrict__ a, const uint32_t* __
     vals[i] = (uint32_t)csorted[i];
   }
 }
-__global__ void split_ab_kernel(const uint64_t* __restrict__ keys, uint64_t n, int bb, uint32_t* __restrict__ a,
-                                uint32_t* __restrict__ b) {
+// triangle i at out[i * stride], its next value `next` further
+__global__ void split_abc_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ c, uint64_t n, int bb,
+                                 int stride, uint64_t next, uint32_t* __restrict__ out) {
   const uint64_t mask = (1ull << bb) - 1;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    a[i] = (uint32_t)(keys[i] >> bb);
-    b[i] = (uint32_t)(keys[i] & mask);
+    uint32_t* o = out + i * stride;
+    o[0] = (uint32_t)(keys[i] >> bb);
+    o[next] = (uint32_t)(keys[i] & mask);
+    o[2 * next] = c[i];
   }
 }
 
@@ -2659,11 +2662,28 @@ static void query_project_ab(eh_context* ctx, const eh_trie* t, uint32_t* ha, ui
   EH_CUDA(cudaStreamSynchronize(s));
 }
 
+// Where materialized triangles go on the host: three columns, or rows of three.
+struct HostRows {
+  uint32_t *a, *b, *c;
+  uint32_t* rows;  // null: the columns
+  bool given() const { return rows || (a && b && c); }
+  void take(const uint32_t* dev, uint64_t n, cudaStream_t s) const {  // n triangles, laid out the same way
+    if (rows) {
+      EH_CUDA(cudaMemcpyAsync(rows, dev, 3 * n * 4, cudaMemcpyDeviceToHost, s));
+    } else {
+      EH_CUDA(cudaMemcpyAsync(a, dev, n * 4, cudaMemcpyDeviceToHost, s));
+      EH_CUDA(cudaMemcpyAsync(b, dev + n, n * 4, cudaMemcpyDeviceToHost, s));
+      EH_CUDA(cudaMemcpyAsync(c, dev + 2 * n, n * 4, cudaMemcpyDeviceToHost, s));
+    }
+    EH_CUDA(cudaStreamSynchronize(s));
+  }
+};
+
 // Oriented relations: the hit masks hold every triangle at its place in the
 // order (a, b, c), so the rows are counted per relation row, placed by a scan
 // and written in order; nothing is sorted.  false: no masks for this relation.
-static bool materialize_hits(eh_context* ctx, const eh_trie* t, const eh_exec_config* cfg, uint32_t* ha, uint32_t* hb,
-                             uint32_t* hc, uint64_t cap, uint64_t* n_rows) {
+static bool materialize_hits(eh_context* ctx, const eh_trie* t, const eh_exec_config* cfg, const HostRows& host,
+                             uint64_t cap, uint64_t* n_rows) {
   cudaStream_t s = ctx->stream;
   ExecParams ep = exec_params(cfg);
   ep.shard_index = 0;
@@ -2690,18 +2710,16 @@ static bool materialize_hits(eh_context* ctx, const eh_trie* t, const eh_exec_co
   EH_REQUIRE(cap >= n, EH_ERR_INVALID, "output columns hold fewer rows than the result");
   EH_REQUIRE(n < (1ull << 32), EH_ERR_UNSUPPORTED, "materialized results hold fewer than 2^32 rows");
   DevBuf<uint32_t> out(3 * n, s);
-  hits_row_write_kernel<<<grid, 256, 0, s>>>(t->view(), t->dir, P.hits.view(), seg.p, pos.p, n, out.p, out.p + n,
-                                             out.p + 2 * n);
+  const uint64_t next = host.rows ? 1 : n;  // from a row's one value to its next
+  hits_row_write_kernel<<<grid, 256, 0, s>>>(t->view(), t->dir, P.hits.view(), seg.p, pos.p, n, host.rows ? 3 : 1,
+                                             out.p, out.p + next, out.p + 2 * next);
   EH_CHECK_LAUNCH();
-  EH_CUDA(cudaMemcpyAsync(ha, out.p, n * 4, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaMemcpyAsync(hb, out.p + n, n * 4, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaMemcpyAsync(hc, out.p + 2 * n, n * 4, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaStreamSynchronize(s));
+  host.take(out.p, n, s);
   return true;
 }
 
 void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_exec_config* cfg, int n_cols,
-                       uint32_t* ha, uint32_t* hb, uint32_t* hc, uint64_t cap, uint64_t* n_rows) {
+                       uint32_t* ha, uint32_t* hb, uint32_t* hc, uint64_t cap, uint64_t* n_rows, uint32_t* rows_out) {
   cudaStream_t s = ctx->stream;
   EH_REQUIRE(query == EH_QUERY_TRIANGLE, EH_ERR_UNSUPPORTED, "materialized output is built for the triangle plan");
   EH_REQUIRE(n_cols == 2 || n_cols == 3, EH_ERR_INVALID, "n_cols must be 3 (a,b,c) or 2 (projection on a,b)");
@@ -2711,11 +2729,12 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
     query_project_ab(ctx, t, ha, hb, cap, n_rows);
     return;
   }
-  if (ha && hb && hc && t->dir != DIR_SYM && materialize_hits(ctx, t, cfg, ha, hb, hc, cap, n_rows)) return;
+  const HostRows host{ha, hb, hc, rows_out};
+  if (host.given() && t->dir != DIR_SYM && materialize_hits(ctx, t, cfg, host, cap, n_rows)) return;
   uint64_t n = 0;
   query_count(ctx, t, EH_QUERY_TRIANGLE, cfg, &n, nullptr);
   *n_rows = n;
-  if (n == 0 || !ha || !hb || !hc) return;  // the row count is the triangle count
+  if (n == 0 || !host.given()) return;  // the row count is the triangle count
   EH_REQUIRE(cap >= n, EH_ERR_INVALID, "output columns hold fewer rows than the result");
   EH_REQUIRE(n < (1ull << 32), EH_ERR_UNSUPPORTED, "materialized results hold fewer than 2^32 rows");
   ExecParams ep = exec_params(cfg);
@@ -2765,12 +2784,10 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   ab_key_kernel<<<grid, 256, 0, s>>>(ma.p, mb.p, idx.p, k1.p, n, bb, k2.p, v2.p);
   EH_CHECK_LAUNCH();
   radix_sort_kv(k2.p, k1t.p, v2.p, idxt.p, n, 2 * bb, s);
-  split_ab_kernel<<<grid, 256, 0, s>>>(k2.p, n, bb, ma.p, mb.p);
+  DevBuf<uint32_t> sorted(3 * n, s);
+  split_abc_kernel<<<grid, 256, 0, s>>>(k2.p, v2.p, n, bb, rows_out ? 3 : 1, rows_out ? 1 : n, sorted.p);
   EH_CHECK_LAUNCH();
-  EH_CUDA(cudaMemcpyAsync(ha, ma.p, n * 4, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaMemcpyAsync(hb, mb.p, n * 4, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaMemcpyAsync(hc, v2.p, n * 4, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaStreamSynchronize(s));
+  host.take(sorted.p, n, s);
 }
 
 // One triangle / 4-clique COUNT of one trie with every piece of device

@@ -343,6 +343,12 @@ eh_status eh_rule_count(eh_context* ctx, const eh_trie* const* relations, uint32
 eh_status eh_query_materialize(eh_context* ctx, const eh_trie* trie, int query, const eh_exec_config* cfg,
                                int n_cols, uint32_t* a, uint32_t* b, uint32_t* c, uint64_t cap, uint64_t* n_rows);
 
+/* The same triangles as rows of three values, rows[3 * i ..]: what a caller
+ * that wants them as a matrix would otherwise put together from the columns.
+ * rows == NULL: only *n_rows. */
+eh_status eh_query_materialize_rows(eh_context* ctx, const eh_trie* trie, int query, const eh_exec_config* cfg,
+                                    uint32_t* rows, uint64_t cap, uint64_t* n_rows);
+
 /* Same plan over many tries in one persistent launch; results[g] per
  * trie. */
 eh_status eh_query_count_batched(eh_context* ctx, const eh_trie* const* tries, uint32_t n_tries, int query,
