@@ -603,7 +603,7 @@ def set_intersect(sets, layouts, pairs, materialize=False, ctx=None):
                                         len(pa), _ptr(counts), _ptr(out_off), _ptr(out)))
     counts = counts[: len(pa)]
     if materialize:
-        return counts, [out[o:e].copy() for o, e in zip(out_off.tolist(), (out_off + counts).tolist())]
+        return counts, [out[o:e] for o, e in zip(out_off.tolist(), (out_off + counts).tolist())]
     return counts
 
 

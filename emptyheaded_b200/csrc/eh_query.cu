@@ -348,8 +348,12 @@ __device__ __forceinline__ uint32_t plan_first(const PlanArgs& p, uint32_t b) {
   return p.shard_count > 1 ? (p.shard_index + p.shard_count - (b + p.g) % p.shard_count) % p.shard_count : 0;
 }
 
-__global__ void __launch_bounds__(256) plan_split_kernel(PlanArgs p) {
+// zero: bytes of the control block and results to clear (a single trie, whose
+// control block no copy sets up)
+__global__ void __launch_bounds__(256) plan_split_kernel(PlanArgs p, Control* __restrict__ ctl, uint32_t zero) {
   __shared__ uint64_t s_warp[8];
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < zero / 4; i += 256) reinterpret_cast<uint32_t*>(ctl)[i] = 0;
   uint64_t sum = 0;
   for (uint32_t x = threadIdx.x; x < kPlanTile; x += 256) {
     const uint64_t b = (uint64_t)blockIdx.x * kPlanTile + x;
@@ -1792,10 +1796,29 @@ static RevView rev_view(const eh_trie* t) {
   return RevView{t->rev_off.p, t->rev_lo.p, t->rev_hi.p, t->rev_src.p, t->rev_wpre.p, t->dir};
 }
 
-static int blocks_per_sm(const void* kernel, int threads, size_t smem) {
-  int b = 0;
-  EH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, smem));
-  return std::max(1, b);
+// What a kernel may use and how many of its blocks an SM holds are constants of
+// the device: asked of the runtime once per kernel (and launch shape), not on
+// every query (some 8 us of a small one).  A kernel's dynamic shared memory limit
+// is raised to all it may use the first time.
+struct KernelShapes {
+  std::mutex mu;
+  struct Room {
+    const void* kernel;
+    int device;
+    size_t bytes;
+  };
+  struct Blocks {
+    const void* kernel;
+    int device, threads;
+    size_t smem;
+    int blocks;
+  };
+  std::vector<Room> rooms;
+  std::vector<Blocks> blocks;
+};
+static KernelShapes& kernel_shapes() {
+  static KernelShapes k;
+  return k;
 }
 
 // dynamic shared memory a block of `kernel` may use: the device's opt-in
@@ -1803,15 +1826,32 @@ static int blocks_per_sm(const void* kernel, int threads, size_t smem) {
 static size_t dynamic_smem_room(const void* kernel) {
   int dev = 0, optin = 0;
   EH_CUDA(cudaGetDevice(&dev));
+  KernelShapes& k = kernel_shapes();
+  std::lock_guard<std::mutex> l(k.mu);
+  for (const auto& r : k.rooms)
+    if (r.kernel == kernel && r.device == dev) return r.bytes;
   EH_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   cudaFuncAttributes fa;
   EH_CUDA(cudaFuncGetAttributes(&fa, kernel));
-  return (size_t)optin > fa.sharedSizeBytes ? (size_t)optin - fa.sharedSizeBytes : 0;
+  const size_t room = (size_t)optin > fa.sharedSizeBytes ? (size_t)optin - fa.sharedSizeBytes : 0;
+  EH_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+  k.rooms.push_back({kernel, dev, room});
+  return room;
 }
-
-template <typename K>
-static void set_smem_attr(K kernel, size_t smem) {
-  EH_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+// after dynamic_smem_room(kernel)
+static int blocks_per_sm(const void* kernel, int threads, size_t smem) {
+  int dev = 0, b = 0;
+  EH_CUDA(cudaGetDevice(&dev));
+  KernelShapes& k = kernel_shapes();
+  std::lock_guard<std::mutex> l(k.mu);
+  for (const auto& x : k.blocks)
+    if (x.kernel == kernel && x.device == dev && x.threads == threads && x.smem == smem) return x.blocks;
+  EH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, smem));
+  b = std::max(1, b);
+  // 4-cliques without masks size their staging by the largest set: the oldest shapes go
+  if (k.blocks.size() >= 64) k.blocks.erase(k.blocks.begin());
+  k.blocks.push_back({kernel, dev, threads, smem, b});
+  return b;
 }
 
 // Small device and pinned host memory of a context, kept from call to call (a
@@ -1858,8 +1898,12 @@ struct Hits {
   int use = 0;
   uint64_t words = 0;
   uint32_t units = 0, heads = 0, n = 0;
-  DevBuf<uint32_t> mask, moff, upre, gstart;
-  HitsView view() const { return HitsView{mask.p, moff.p, upre.p, gstart.p, n, heads}; }
+  DevBuf<uint32_t> mask;
+  DevBuf<uint32_t> plan;  // [heads] mask offsets, [heads + 1] units before, [n + 1] graph starts, sums
+  uint32_t* moff() const { return plan.p; }
+  uint32_t* upre() const { return plan.p + heads; }
+  uint32_t* gstart() const { return upre() + heads + 1; }
+  HitsView view() const { return HitsView{mask.p, moff(), upre(), gstart(), n, heads}; }
 };
 // Masks hold a bit per candidate, so a relation in degree order needs far less
 // than its trie (R-MAT-22: 1.2 GB); past this many words (8 GB: a set of 300 K
@@ -1883,26 +1927,25 @@ static bool plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
   H.use = use;
   H.n = n;
   H.heads = (uint32_t)heads;
-  H.moff.alloc(heads, s);
-  H.upre.alloc(heads + 1, s);
-  H.gstart.alloc(n + 1, s);
-  DevBuf<unsigned long long> sums(2, s);
-  EH_CUDA(cudaMemsetAsync(sums.p, 0, 16, s));
-  EH_CUDA(cudaMemsetAsync(H.upre.p + heads, 0, 4, s));
-  EH_CUDA(cudaMemcpyAsync(H.gstart.p, gstart.data(), (n + 1) * 4, cudaMemcpyHostToDevice, s));
+  const size_t o_sums = (2 * heads + 1 + n + 1 + 1) & ~(size_t)1;  // two 64-bit sums
+  H.plan.alloc(o_sums + 4, s);
+  unsigned long long* sums = reinterpret_cast<unsigned long long*>(H.plan.p + o_sums);
+  EH_CUDA(cudaMemsetAsync(sums, 0, 16, s));
+  EH_CUDA(cudaMemsetAsync(H.upre() + heads, 0, 4, s));
+  EH_CUDA(cudaMemcpyAsync(H.gstart(), gstart.data(), (n + 1) * 4, cudaMemcpyHostToDevice, s));
   for (uint32_t g = 0; g < n; g++) {
     const uint32_t nh = tries[g]->n_head;
     if (!nh) continue;
     const int grid = std::min(num_sms() * 4, ceil_div(nh, 256));
-    hits_size_kernel<<<grid, 256, 0, s>>>(tries[g]->view(), use, H.moff.p + gstart[g], H.upre.p + gstart[g], sums.p);
+    hits_size_kernel<<<grid, 256, 0, s>>>(tries[g]->view(), use, H.moff() + gstart[g], H.upre() + gstart[g], sums);
     EH_CHECK_LAUNCH();
   }
   unsigned long long h[2];
-  EH_CUDA(cudaMemcpyAsync(h, sums.p, 16, cudaMemcpyDeviceToHost, s));
+  EH_CUDA(cudaMemcpyAsync(h, sums, 16, cudaMemcpyDeviceToHost, s));
   EH_CUDA(cudaStreamSynchronize(s));
   if (h[0] > kMaxHitWords || h[1] >= kMaxHitWords) return false;
-  exclusive_scan<uint32_t>(H.moff.p, H.moff.p, heads, nullptr, s);
-  exclusive_scan<uint32_t>(H.upre.p, H.upre.p, heads + 1, nullptr, s);
+  exclusive_scan<uint32_t>(H.moff(), H.moff(), heads, nullptr, s);
+  exclusive_scan<uint32_t>(H.upre(), H.upre(), heads + 1, nullptr, s);
   try {
     H.mask.alloc(h[0] ? h[0] : 1, s);
   } catch (const Error& e) {
@@ -2031,11 +2074,6 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
       P.smem = (size_t)ep.smem_words * 4 * ep.warps;
     }
   }
-  if (hits) set_smem_attr(n == 1 ? hits_kernel<true> : hits_kernel<false>, P.smem);
-  else if (query == EH_QUERY_CLIQUE4) set_smem_attr(clique4_kernel, P.smem);
-  else if (annot) set_smem_attr(triangle_kernel<MODE_ANNOT, true>, P.smem);
-  else if (n == 1) set_smem_attr(triangle_kernel<MODE_COUNT, true>, P.smem);
-  else set_smem_attr(triangle_kernel<MODE_COUNT, false>, P.smem);
   const int per_sm = blocks_per_sm(kfn, P.threads, P.smem);
   // block items only for the plain triangle COUNT
   const bool blocks_query = query == EH_QUERY_TRIANGLE && !annot;
@@ -2100,7 +2138,10 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
       P.rev0 = r;
     }
   }
-  EH_CUDA(cudaMemcpyAsync(base, host, head_bytes, cudaMemcpyHostToDevice, s));
+  // a single trie's views are kernel parameters (not the clique passes'), and
+  // the planner clears its control block: no copy
+  const bool copied = n > 1 || !tries[0]->rev_entries || query == EH_QUERY_CLIQUE4 || (annot && !hits);
+  if (copied) EH_CUDA(cudaMemcpyAsync(base, host, head_bytes, cudaMemcpyHostToDevice, s));
   for (uint32_t g = 0; g < n; g++) {
     const eh_trie* t = tries[g];
     if (!t->rev_entries) continue;
@@ -2118,7 +2159,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     }
     const int tiles = ceil_div(t->n_head, kPlanTile);
     unsigned long long* total = &P.ctl->spare[1];
-    plan_split_kernel<<<tiles, 256, 0, s>>>(pa);
+    plan_split_kernel<<<tiles, 256, 0, s>>>(pa, P.ctl, copied ? 0 : (uint32_t)P.ctl_bytes());
     plan_place_kernel<<<tiles, 256, 0, s>>>(pa, total, P.ctl);
     const uint64_t most = std::min<uint64_t>(t->n_head, t->rev_entries) +
                           (t->rev_pairs + kRowCost * t->rev_entries) / ep.chunk;
@@ -2743,7 +2784,7 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
   Prepared P;
   const eh_trie* ts[1] = {t};
   prepare(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, false, P, false, -1, false, false);
-  set_smem_attr(triangle_kernel<MODE_MAT, true>, P.smem);
+  dynamic_smem_room((const void*)triangle_kernel<MODE_MAT, true>);
   unsigned int n_items = 0;
   EH_CUDA(cudaMemcpyAsync(&n_items, P.ctl->items, 4, cudaMemcpyDeviceToHost, s));
   EH_CUDA(cudaStreamSynchronize(s));
@@ -2822,8 +2863,6 @@ void query_count_in_scratch(eh_context* ctx, const eh_trie* t, int query, const 
                "shared staging of " + std::to_string(smem) + " bytes per block is above the " + std::to_string(room) +
                    " a block may use");
   }
-  if (clique) set_smem_attr(clique4_kernel, smem);
-  else set_smem_attr(triangle_kernel<MODE_COUNT, true>, smem);
   const int per_sm = blocks_per_sm(kfn, threads, smem);
   // carve the scratch
   const uint32_t nh = t->n_head;
