@@ -89,7 +89,11 @@ void trim_device_pool(int device);
 // (the bitset ranks of an R-MAT-22 layout: 2 ms every call, up to hundreds of
 // ms at random calls; end to end 28.2 ms with spikes against 24.7 ms steady
 // when each free waits for its stream), so a free waits for its stream,
-// except while the stream is being captured into a graph.
+// except while the stream is being captured into a graph.  Small blocks do not
+// hold up large requests, and waiting for theirs left the device idle between
+// kernels (load R-MAT-20 5.45 -> 5.32 ms, barbell Chung-Lu 2^16 0.28 -> 0.26, no
+// spikes over 25 calls of each): they are not waited for.
+constexpr size_t kSettleBytes = 1u << 20;
 inline void settle_free(cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) cudaStreamSynchronize(s);
@@ -132,7 +136,7 @@ struct DevBuf {
   void release() {
     if (p) {
       cudaFreeAsync(p, s);
-      settle_free(s);
+      if (n * sizeof(T) >= kSettleBytes) settle_free(s);
     }
     p = nullptr;
     n = 0;

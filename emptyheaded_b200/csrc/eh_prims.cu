@@ -328,7 +328,10 @@ static uint32_t* radix_sort_impl(K* keys, K* tmp, uint32_t* vals, uint32_t* vtmp
   if (n < 2) return vals;
   EH_REQUIRE(n < (1ull << 32), EH_ERR_UNSUPPORTED, "radix sort supports fewer than 2^32 keys");
   const uint32_t tiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
-  DevBuf<uint32_t> counts((uint64_t)kRadix * tiles, s);
+  // the counters, then the tile sums of their scan: taken once for all passes (a
+  // buffer per scan was freed, and waited for, twice a pass)
+  const uint64_t n_counts = (uint64_t)kRadix * tiles, n_sums = scan_scratch_elems(n_counts);
+  DevBuf<uint32_t> counts(n_counts + n_sums, s);
   set_scatter_smem<K>();
   K* src = keys;
   K* dst = tmp;
@@ -338,7 +341,7 @@ static uint32_t* radix_sort_impl(K* keys, K* tmp, uint32_t* vals, uint32_t* vtmp
     const int write_keys = copy_back || shift + 8 < bits;
     radix_hist_kernel<K><<<tiles, kSortThreads, 0, s>>>(src, n, shift, counts.p, tiles);
     EH_CHECK_LAUNCH();
-    exclusive_scan<uint32_t>(counts.p, counts.p, (uint64_t)kRadix * tiles, nullptr, s);
+    exclusive_scan_scratch<uint32_t>(counts.p, counts.p, n_counts, nullptr, counts.p + n_counts, n_sums, s);
     if (vals)
       radix_scatter_kernel<K, true><<<tiles, kSortThreads, scatter_smem<K>(true), s>>>(
           src, dst, n, shift, counts.p, tiles, vsrc, vdst, write_keys);
