@@ -18,12 +18,12 @@ checked against the first one, so tuning can never change a result.
 import statistics
 
 GRID = {
-    "smem_words": (512, 1024, 1536),
+    "smem_words": (768, 1024, 1280, 1536),
     "chunk": (16384, 32768, 65536, 131072),
-    "long_row": (16, 32, 64, 128),
+    "long_row": (24, 48, 64, 128),
     "warps": (4, 8, 16),
 }
-DEFAULT = {"warps": 8, "smem_words": 1024, "chunk": 32768, "long_row": 32}
+DEFAULT = {"warps": 8, "smem_words": 1280, "chunk": 32768, "long_row": 48}
 
 
 def _time(trie, cfg, query, reps, want):

@@ -82,8 +82,8 @@ eh_status eh_context_stream(eh_context* ctx, void** stream);
  * reference, which allocates from the host heap per call): bytes the pool
  * holds, bytes in use, and the peak in use since the last reserve.  Not
  * counted: the lollipop / barbell COUNT's per-head counters (8 bytes per head
- * entry of the largest trie queried so), a separate device allocation the
- * context keeps until it is destroyed. */
+ * entry of the largest trie queried so) and the queries' work plans (64 MiB at
+ * most), separate device allocations the context keeps until it is destroyed. */
 eh_status eh_context_memory(eh_context* ctx, uint64_t* reserved, uint64_t* used, uint64_t* peak);
 /* Returns the pool's unused memory to the driver and reserves `bytes` as one
  * block that later allocations are carved from, so that calls whose peak fits
@@ -229,14 +229,17 @@ eh_status eh_set_intersect_batch(eh_context* ctx, const uint32_t* elems, const u
 /* ------------------------------------------------------------- queries */
 typedef struct {
   int warps_per_block;   /* 0 = tuned default */
-  int chunk_pairs;       /* target (v,w) pairs per work item; 0 = tuned default */
+  int chunk_pairs;       /* target work per item: (v,w) pairs, a row counted as 8
+                            more; 0 = derived from the work (4096 to 131072) */
   int long_row;          /* size-class boundary: rows with at least this many
                             candidates run warp-wide, shorter ones are
-                            flattened over the lanes; 0 = default (32) */
+                            flattened over the lanes; 0 = default (48) */
   int smem_words;        /* per-warp shared staging capacity in u32 words; 0 = default */
   int record_timings;    /* 1: log per-item device time for the cost model */
-  int shard_index;       /* run work items i with i % shard_count == shard_index */
-  int shard_count;       /* 0 or 1: all items (multi-GPU ranks split the plan) */
+  int shard_index;       /* this rank's share of the plan: item i of head entry b
+                            runs where (b + i) % shard_count == shard_index (the
+                            4-clique's hit masks: head entries a % shard_count) */
+  int shard_count;       /* 0 or 1: everything */
   int no_block_items;    /* 1: stage every N(b) in one warp's region; 0: an N(b)
                             too large for a warp's region but not for the
                             block's is staged block-wide and all the block's
