@@ -569,7 +569,8 @@ static bool small_steps(eh_model* m, const float* x, const float* y, uint32_t ba
     EH_CUDA(cudaMemcpyAsync(base + o_y, y, ny * sizeof(float), cudaMemcpyHostToDevice, s));
   }
   const size_t smem = step_smem(sh);
-  EH_CUDA(cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the most any network takes, so that calls of other contexts never lower it
+  EH_CUDA(cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepMaxSmem));
   for (uint32_t it = 0; it < steps; it++) {
     mlp_step_kernel<<<blocks, 256, smem, s>>>(sh, m->params.p, base, base + o_y, (int)batch, 1.f / (float)batch,
                                               base + o_part, base + o_loss);
