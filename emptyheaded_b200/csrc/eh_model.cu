@@ -98,10 +98,12 @@ __global__ void sgd_kernel(float* __restrict__ p, const float* __restrict__ g, s
 // per-layer kernels took eleven, of which the weight gradients summed the whole
 // batch in one thread per weight (0.87 -> 0.05 ms a step of 2048 samples).
 // Activations are stored sample-fastest: the lanes of a warp are samples of one
-// or two outputs, so a weight is a broadcast and the chain over the inputs runs
-// in the order of the per-layer kernels.  Rows are padded to kStepPitch floats
+// or two outputs, so a weight is a broadcast.  Rows are padded to kStepPitch values
 // (16-byte loads, spread over the banks).
-constexpr int kStepRows = 16, kStepPitch = 20;
+// Everything between the fp32 parameters and the update is computed in 64 bits (an
+// SM does 64 such FMAs a clock, and a step is bound by its launches): a rounded
+// pre-activation near zero would let a whole sample's gradient through, or not.
+constexpr int kStepRows = 16, kStepPitch = 18;
 constexpr int kStepMaxLayers = 8;
 constexpr size_t kStepMaxSmem = 96 * 1024;
 struct StepShape {
@@ -111,43 +113,43 @@ struct StepShape {
   int a_off[kStepMaxLayers + 1];      // first unit of a layer
 };
 static size_t step_smem(const StepShape& sh) {
-  return ((size_t)2 * sh.n_params + (size_t)2 * sh.units * kStepPitch) * sizeof(float);
+  return sh.n_params * (sizeof(double) + sizeof(float)) + (size_t)2 * sh.units * kStepPitch * sizeof(double);
 }
 
 __global__ void __launch_bounds__(256) mlp_step_kernel(StepShape sh, const float* __restrict__ params,
                                                        const float* __restrict__ x, const float* __restrict__ y,
-                                                       int batch, float inv_batch, float* __restrict__ part,
-                                                       float* __restrict__ loss_part) {
-  extern __shared__ __align__(16) float sm[];
-  float* z = sm;                                // [unit][sample] pre-activations, then the input layer as is
-  float* dz = z + sh.units * kStepPitch;
-  float* P = dz + sh.units * kStepPitch;
-  float* G = P + sh.n_params;                   // this block's gradient; entry k belongs to thread k % 256
+                                                       int batch, double inv_batch, double* __restrict__ part,
+                                                       double* __restrict__ loss_part) {
+  extern __shared__ __align__(16) double sm[];
+  double* z = sm;                               // [unit][sample] pre-activations, the input layer as is
+  double* dz = z + sh.units * kStepPitch;
+  double* G = dz + sh.units * kStepPitch;       // this block's gradient; entry k belongs to thread k % 256
+  float* P = reinterpret_cast<float*>(G + sh.n_params);
   const int tid = threadIdx.x, L = sh.n_layers, dL = sh.dims[L];
   for (int k = tid; k < sh.n_params; k += 256) {
     P[k] = params[k];
-    G[k] = 0.f;
+    G[k] = 0.0;
   }
-  float loss = 0.f;
+  double loss = 0.0;
   for (int r0 = blockIdx.x * kStepRows; r0 < batch; r0 += gridDim.x * kStepRows) {
     const int rows = min(kStepRows, batch - r0);
     __syncthreads();
     for (int e = tid; e < sh.dims[0] * kStepRows; e += 256) {
       const int r = e / sh.dims[0], i = e - r * sh.dims[0];
-      z[i * kStepPitch + r] = r < rows ? x[(size_t)r0 * sh.dims[0] + e] : 0.f;
+      z[i * kStepPitch + r] = r < rows ? x[(size_t)r0 * sh.dims[0] + e] : 0.0;
     }
     for (int l = 0; l < L; l++) {
       __syncthreads();
       const int din = sh.dims[l], dout = sh.dims[l + 1];
       const float* W = P + sh.w_off[l];
-      const float* in = z + sh.a_off[l] * kStepPitch;
-      float* out = z + sh.a_off[l + 1] * kStepPitch;
+      const double* in = z + sh.a_off[l] * kStepPitch;
+      double* out = z + sh.a_off[l + 1] * kStepPitch;
       for (int e = tid; e < dout * kStepRows; e += 256) {
         const int o = e / kStepRows, r = e % kStepRows;
-        float s = W[dout * din + o];
+        double s = W[dout * din + o];
         for (int i = 0; i < din; i++) {
-          const float v = in[i * kStepPitch + r];
-          s = fmaf(W[o * din + i], l > 0 && v < 0.f ? 0.f : v, s);
+          const double v = in[i * kStepPitch + r];
+          s = fma((double)W[o * din + i], l > 0 && v < 0.0 ? 0.0 : v, s);
         }
         out[o * kStepPitch + r] = s;
       }
@@ -156,51 +158,49 @@ __global__ void __launch_bounds__(256) mlp_step_kernel(StepShape sh, const float
     for (int e = tid; e < dL * kStepRows; e += 256) {
       const int o = e / kStepRows, r = e % kStepRows;
       const int u = (sh.a_off[L] + o) * kStepPitch + r;
-      const float d = r < rows ? z[u] - y[(size_t)(r0 + r) * dL + o] : 0.f;
+      const double d = r < rows ? z[u] - y[(size_t)(r0 + r) * dL + o] : 0.0;
       dz[u] = d * inv_batch;
-      loss += 0.5f * d * d;
+      loss += 0.5 * d * d;
     }
     for (int l = L - 1; l >= 0; l--) {
       __syncthreads();
       const int din = sh.dims[l], dout = sh.dims[l + 1];
       const float* W = P + sh.w_off[l];
-      const float* in = z + sh.a_off[l] * kStepPitch;
-      const float* g = dz + sh.a_off[l + 1] * kStepPitch;
+      const double* in = z + sh.a_off[l] * kStepPitch;
+      const double* g = dz + sh.a_off[l + 1] * kStepPitch;
       const int w0 = sh.w_off[l], nw = dout * din + dout;
       // parameters k = tid mod 256 of this layer: weights, then biases
       for (int k = w0 + ((tid - w0) % 256 + 256) % 256; k < w0 + nw; k += 256) {
         const int e = k - w0;
         const bool bias = e >= dout * din;
         const int o = bias ? e - dout * din : e / din, i = bias ? 0 : e - o * din;
-        float s = 0.f;
-        for (int r = 0; r < kStepRows; r += 4) {
-          const float4 gg = *reinterpret_cast<const float4*>(g + o * kStepPitch + r);
+        double s = 0.0;
+        for (int r = 0; r < kStepRows; r += 2) {
+          const double2 gg = *reinterpret_cast<const double2*>(g + o * kStepPitch + r);
           if (bias) {
-            s += (gg.x + gg.y) + (gg.z + gg.w);
+            s += gg.x + gg.y;
           } else {
-            const float4 v = *reinterpret_cast<const float4*>(in + i * kStepPitch + r);
-            s = fmaf(gg.x, l > 0 && v.x < 0.f ? 0.f : v.x, s);
-            s = fmaf(gg.y, l > 0 && v.y < 0.f ? 0.f : v.y, s);
-            s = fmaf(gg.z, l > 0 && v.z < 0.f ? 0.f : v.z, s);
-            s = fmaf(gg.w, l > 0 && v.w < 0.f ? 0.f : v.w, s);
+            const double2 v = *reinterpret_cast<const double2*>(in + i * kStepPitch + r);
+            s = fma(gg.x, l > 0 && v.x < 0.0 ? 0.0 : v.x, s);
+            s = fma(gg.y, l > 0 && v.y < 0.0 ? 0.0 : v.y, s);
           }
         }
         G[k] += s;
       }
       if (l > 0) {
-        float* gin = dz + sh.a_off[l] * kStepPitch;
+        double* gin = dz + sh.a_off[l] * kStepPitch;
         for (int e = tid; e < din * kStepRows; e += 256) {
           const int i = e / kStepRows, r = e % kStepRows;
-          float s = 0.f;
-          if (!(in[i * kStepPitch + r] < 0.f))
-            for (int o = 0; o < dout; o++) s = fmaf(W[o * din + i], g[o * kStepPitch + r], s);
+          double s = 0.0;
+          if (!(in[i * kStepPitch + r] < 0.0))
+            for (int o = 0; o < dout; o++) s = fma((double)W[o * din + i], g[o * kStepPitch + r], s);
           gin[i * kStepPitch + r] = s;
         }
       }
     }
   }
   for (int k = tid; k < sh.n_params; k += 256) part[(size_t)blockIdx.x * sh.n_params + k] = G[k];
-  __shared__ float s_loss[8];
+  __shared__ double s_loss[8];
   loss = warp_sum(loss);
   if (lane_id() == 0) s_loss[tid >> 5] = loss;
   __syncthreads();
@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(256) mlp_step_kernel(StepShape sh, const float
 
 // gradient = sum of the blocks' shares; with lr the SGD step, without it the
 // gradient itself to `grads`.  32 parameters per block, 8 threads each.
-__global__ void __launch_bounds__(256) grad_reduce_kernel(const float* __restrict__ part, int blocks, int n_params,
-                                                          const float* __restrict__ loss_part, double inv_batch,
+__global__ void __launch_bounds__(256) grad_reduce_kernel(const double* __restrict__ part, int blocks, int n_params,
+                                                          const double* __restrict__ loss_part, double inv_batch,
                                                           float lr, float* __restrict__ params,
                                                           float* __restrict__ grads, float* __restrict__ loss) {
   __shared__ double s[8][32];
@@ -225,9 +225,8 @@ __global__ void __launch_bounds__(256) grad_reduce_kernel(const float* __restric
   __syncthreads();
   if (w == 0 && k < n_params) {
     for (int i = 1; i < 8; i++) v += s[i][c];
-    const float g = (float)v;
-    if (grads) grads[k] = g;
-    else params[k] -= lr * g;
+    if (grads) grads[k] = (float)v;
+    else params[k] = (float)((double)params[k] - (double)lr * v);
   }
   if (blockIdx.x == 0 && w == 1) {
     double l = 0;
@@ -528,7 +527,7 @@ static bool step_shape(const eh_model* m, StepShape& sh) {
   sh.n_layers = m->n_layers;
   sh.n_params = (int)m->n_params;
   sh.units = 0;
-  if (m->n_layers > kStepMaxLayers || m->n_params > kStepMaxSmem / 8) return false;
+  if (m->n_layers > kStepMaxLayers || m->n_params > kStepMaxSmem / 12) return false;
   for (int l = 0; l <= m->n_layers; l++) {
     sh.dims[l] = m->dims[l];
     sh.a_off[l] = sh.units;
@@ -551,8 +550,8 @@ static bool small_steps(eh_model* m, const float* x, const float* y, uint32_t ba
   const int blocks = (int)std::min<uint64_t>((batch + kStepRows - 1) / kStepRows, 2ull * num_sms());
   const size_t pad = 64;  // floats: keep every piece 256-byte aligned
   const size_t o_y = (nx + pad - 1) / pad * pad, o_part = o_y + (ny + pad - 1) / pad * pad;
-  const size_t o_loss = o_part + ((size_t)blocks * m->n_params + pad - 1) / pad * pad;
-  const size_t o_out = o_loss + (blocks + pad - 1) / pad * pad, total = (o_out + 1) * sizeof(float);
+  const size_t o_loss = o_part + ((size_t)2 * blocks * m->n_params + pad - 1) / pad * pad;  // shares are doubles
+  const size_t o_out = o_loss + (2 * blocks + pad - 1) / pad * pad, total = (o_out + 1) * sizeof(float);
   DevBuf<float> own;
   float* base = reinterpret_cast<float*>(workspace(ctx, total));
   if (!base) {
@@ -572,9 +571,11 @@ static bool small_steps(eh_model* m, const float* x, const float* y, uint32_t ba
   // the most any network takes, so that calls of other contexts never lower it
   EH_CUDA(cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepMaxSmem));
   for (uint32_t it = 0; it < steps; it++) {
-    mlp_step_kernel<<<blocks, 256, smem, s>>>(sh, m->params.p, base, base + o_y, (int)batch, 1.f / (float)batch,
-                                              base + o_part, base + o_loss);
-    grad_reduce_kernel<<<(sh.n_params + 31) / 32, 256, 0, s>>>(base + o_part, blocks, sh.n_params, base + o_loss,
+    double* part = reinterpret_cast<double*>(base + o_part);
+    double* loss_part = reinterpret_cast<double*>(base + o_loss);
+    mlp_step_kernel<<<blocks, 256, smem, s>>>(sh, m->params.p, base, base + o_y, (int)batch, 1.0 / (double)batch,
+                                              part, loss_part);
+    grad_reduce_kernel<<<(sh.n_params + 31) / 32, 256, 0, s>>>(part, blocks, sh.n_params, loss_part,
                                                                1.0 / (double)batch, lr, m->params.p, grads,
                                                                base + o_out);
     EH_CHECK_LAUNCH();
