@@ -269,7 +269,7 @@ __global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const __grid_constant__ TrieVie
       continue;
     }
     Staged st;
-    const int mode = stage_set(t, item.hb, sm, cap_words, st, item.ke - item.kb > kListRows);
+    const int mode = stage_set(t, item.hb, sm, cap_words, st, !few_candidates(r, item));
     switch (mode) {
       case P_SBITS:
         hit_rows<P_SBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
@@ -326,10 +326,12 @@ __device__ __forceinline__ uint64_t hits_units(uint64_t d, int use) {
   return (d + 7) / 8;
 }
 
-// mask words and second-pass units of every head entry; sums over all of them
+// mask words and second-pass units of every head entry; sums over all of them, and
+// the longest part
 __global__ void hits_size_kernel(TrieView t, int use, uint32_t* __restrict__ words, uint32_t* __restrict__ units,
                                  unsigned long long* __restrict__ sums) {
   unsigned long long sw = 0, su = 0;
+  uint32_t most = 0;
   for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < t.n_head; a += gridDim.x * blockDim.x) {
     const uint64_t d = staged_range(t, a).len;
     const uint64_t w = hits_words(d), u = hits_units(d, use);
@@ -337,6 +339,7 @@ __global__ void hits_size_kernel(TrieView t, int use, uint32_t* __restrict__ wor
     units[a] = (uint32_t)u;
     sw += w;
     su += u;
+    most = max(most, (uint32_t)d);
   }
   sw = warp_sum(sw);
   su = warp_sum(su);
@@ -344,6 +347,8 @@ __global__ void hits_size_kernel(TrieView t, int use, uint32_t* __restrict__ wor
     if (sw) atomicAdd(sums, sw);
     if (su) atomicAdd(sums + 1, su);
   }
+  most = __reduce_max_sync(kFull, most);
+  if (lane_id() == 0 && most) atomicMax(sums + 2, (unsigned long long)most);
 }
 
 // 4-cliques whose lowest vertex (highest, on a relation that goes down) has a
@@ -392,6 +397,36 @@ __global__ void __launch_bounds__(256) clique_small_kernel(const TrieView* __res
   if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
 }
 
+// A wide matrix may be nearly empty: then the words to AND for a unit's eight rows
+// are far more than the pairs of their hits, whose bits can be tested one by one.
+// (A star of 2^16 leaves with 2^18 rows among them: 90 ms by words alone, 4.7 with
+// this.)  32 pairs are 32 scattered words and a step of the AND three lines, so they
+// are weighed 8 to 1.
+constexpr uint32_t kSparseWords = 64;  // matrices this wide (2048 neighbours) may be sparse
+constexpr uint32_t kSparseHits = 256;  // hits of a row that are kept and paired
+__device__ __noinline__ bool sparse_rows(const uint32_t* rows, uint32_t ri, uint32_t qi, uint32_t W) {
+  uint32_t h[8] = {0, 0, 0, 0, 0, 0, 0, 0}, steps = 0;
+  for (uint32_t q = qi + lane_id(); q < W; q += 32) {
+    uint32_t any = 0;
+#pragma unroll
+    for (int x = 0; x < 8; x++) {
+      const uint32_t w = __ldg(rows + x + (q - qi) * ri);
+      any |= w;
+      h[x] += __popc(w);
+    }
+    if (any) steps += W - q;
+  }
+  uint32_t most = 0;
+  uint64_t pairs = 0;
+#pragma unroll
+  for (int x = 0; x < 8; x++) {
+    h[x] = __reduce_add_sync(kFull, h[x]);
+    most = max(most, h[x]);
+    pairs += (uint64_t)h[x] * (h[x] + 32);  // 32 pairs a step, at least one step per hit
+  }
+  return most <= kSparseHits && pairs < 4ull * __reduce_add_sync(kFull, steps);
+}
+
 // 4-cliques of the larger parts.  A unit is eight consecutive rows i of one
 // matrix.  For a block q of 32 later positions j, each lane holds the row of
 // one j and ANDs its words with the same words of the eight rows, of each row
@@ -426,6 +461,7 @@ __global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restr
       const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
       const uint32_t i0 = 8 * (u - __ldg(hv.upre + gh)), qi = i0 >> 5, ri = hits_stride(qi, W, d);
       const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
+      if (W > kSparseWords && sparse_rows(rows, ri, qi, W)) continue;  // clique_sparse_kernel's
       uint32_t c = 0;  // below 2^32: masks of 2^31 words hold at most 2^26 (j word, row) steps per lane
       for (uint32_t q = qi; q < W; q++) {
         const uint4 ma = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri));
@@ -455,6 +491,51 @@ __global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restr
   if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
 }
 
+// the units that sparse_rows keeps from clique_big_kernel
+__global__ void __launch_bounds__(256) clique_sparse_kernel(const TrieView* __restrict__ views, HitsView hv,
+                                                            uint32_t n_units,
+                                                            unsigned long long* __restrict__ total) {
+  __shared__ uint32_t s_hits[8][kSparseHits];
+  uint32_t* hits = s_hits[threadIdx.x >> 5];
+  const uint32_t lane = lane_id();
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint64_t u = warp; u < n_units; u += nwarps) {
+    const uint32_t gh = hits_unit_head(hv, (uint32_t)u);
+    const uint32_t g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0;
+    const uint32_t d = staged_range(views[g], gh - hv.gstart[g]).len, W = (d + 31) >> 5;
+    if (W <= kSparseWords) continue;
+    const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
+    const uint32_t i0 = 8 * ((uint32_t)u - __ldg(hv.upre + gh)), qi = i0 >> 5, ri = hits_stride(qi, W, d);
+    const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
+    if (!sparse_rows(rows, ri, qi, W)) continue;
+    unsigned long long acc = 0;
+    for (uint32_t x = 0; x < 8; x++) {
+      uint32_t n = 0;
+      __syncwarp();
+      for (uint32_t q0 = qi; q0 < W; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        uint32_t w = q < W ? __ldg(rows + x + (q - qi) * ri) : 0u;
+        const uint32_t incl = warp_incl_scan((uint32_t)__popc(w));
+        uint32_t at = n + incl - __popc(w);
+        n += __shfl_sync(kFull, incl, 31);
+        for (; w; w &= w - 1) hits[at++] = 32 * q + __ffs(w) - 1;
+      }
+      __syncwarp();
+      for (uint32_t y = 0; y + 1 < n; y++) {
+        const uint32_t j = hits[y], qj = j >> 5, rj = hits_stride(qj, W, d);
+        const uint32_t* jr = m + hits_block(qj, W) + (j & 31);
+        for (uint32_t z = y + 1 + lane; z < n; z += 32) {
+          const uint32_t l = hits[z];
+          acc += (__ldg(jr + ((l >> 5) - qj) * rj) >> (l & 31)) & 1u;
+        }
+      }
+    }
+    acc = warp_sum(acc);
+    if (lane == 0 && acc) atomicAdd(total + g, acc);
+  }
+}
+
 // 32 x 32 bits, row r in lane r's word -> column c in lane c's word
 __device__ __forceinline__ uint32_t transpose32(uint32_t x) {
   const uint32_t lane = lane_id();
@@ -479,6 +560,11 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x) {
 // a few L2 lines.  The last kHubs entries count in shared memory and are added
 // to T once per block.
 constexpr uint32_t kHubs = 4096;
+// kWide: the units of columns kWideColumn on, each of many tiles: one at a time per
+// warp, four tiles' loads in flight (lollipop on a star of 2^17 leaves: 42 ms
+// without, 15); not: the others.
+constexpr uint32_t kWideColumn = 16;
+template <bool kWide>
 __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv, uint32_t n_units,
                                                          unsigned long long* __restrict__ T) {
   __shared__ unsigned int hub[kHubs];
@@ -490,7 +576,7 @@ __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   // runs of consecutive units, so that few searches find the head entries,
   // spread over the warps, so that the long rows of a range of ids are too
-  constexpr uint32_t kRun = 16;
+  constexpr uint32_t kRun = kWide ? 1 : 16;
   uint32_t a = 0;
   for (uint64_t v = 0;; v++) {
     const uint64_t u64 = ((v / kRun) * nwarps + warp) * kRun + v % kRun;
@@ -499,14 +585,30 @@ __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv
     if (v % kRun == 0) a = hits_unit_head(hv, u);
     while (__ldg(hv.upre + a + 1) <= u) a++;
     const uint32_t k = u - __ldg(hv.upre + a);
+    if ((k >= kWideColumn) != kWide) continue;
     const StagedRange pr = staged_range(t, a);
     const uint32_t d = pr.len, W = (d + 31) >> 5;
     const uint32_t* m = hv.mask + __ldg(hv.moff + a);
     uint32_t col = 0, row = 0;
-    for (uint32_t q = 0; q <= k; q++) {
-      const uint32_t rq = hits_stride(q, W, d);
-      const uint32_t x = lane < rq ? __ldg(m + hits_block(q, W) + (k - q) * rq + lane) : 0u;
-      if (__any_sync(kFull, x != 0)) col += __popc(transpose32(x));
+    if (!kWide) {
+      for (uint32_t q = 0; q <= k; q++) {
+        const uint32_t rq = hits_stride(q, W, d);
+        const uint32_t x = lane < rq ? __ldg(m + hits_block(q, W) + (k - q) * rq + lane) : 0u;
+        if (__any_sync(kFull, x != 0)) col += __popc(transpose32(x));
+      }
+    } else {
+      for (uint32_t q0 = 0; q0 <= k; q0 += 4) {
+        uint32_t x[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const uint32_t q = q0 + i;
+          const uint32_t rq = hits_stride(q, W, d);
+          x[i] = q <= k && lane < rq ? __ldg(m + hits_block(q, W) + (k - q) * rq + lane) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (__any_sync(kFull, x[i] != 0)) col += __popc(transpose32(x[i]));
+      }
     }
     const uint32_t rk = hits_stride(k, W, d);
     if (lane < rk)

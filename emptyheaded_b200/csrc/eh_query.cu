@@ -65,11 +65,13 @@ constexpr uint32_t kWordRowNum = EH_WORD_ROW_NUM, kWordRowDen = EH_WORD_ROW_DEN;
 #define EH_LONG_WORDS 32
 #endif
 constexpr int kLongWords = EH_LONG_WORDS;  // word rows with at least this many words run warp-wide
-// an item of at most this many rows keeps a uint N(b) as a list: searching it
-// for so few beats building a bitmap (kernel ms, R-MAT-22 6.93 -> 6.85,
-// symmetric Chung-Lu 2^21 2.52 -> 2.21, ER-16K 0.0225 -> 0.0205; at 32 rows
-// R-MAT-22 6.96)
+// an item of at most this many rows and candidates keeps a uint N(b) as a list:
+// searching it for so few beats building a bitmap (kernel ms, R-MAT-22 6.93 ->
+// 6.85, symmetric Chung-Lu 2^21 2.52 -> 2.21, ER-16K 0.0225 -> 0.0205; at 32 rows
+// R-MAT-22 6.96; without the bound on candidates a star of 2^16 leaves, whose rows
+// hold 32 K of them, took 4.9 ms instead of 2.4)
 constexpr uint32_t kListRows = 16;
+constexpr uint64_t kListCandidates = 2048;
 #ifndef EH_FLAT_CLIQUE
 #define EH_FLAT_CLIQUE 48
 #endif
@@ -1147,6 +1149,11 @@ __device__ __forceinline__ uint32_t count_merged(const TrieView& t, const RevVie
   return cnt;
 }
 
+__device__ __forceinline__ bool few_candidates(const RevView& r, const Item& item) {
+  return item.ke - item.kb <= kListRows &&
+         __ldg(r.rev_wpre + item.ke) - __ldg(r.rev_wpre + item.kb) <= kListCandidates;
+}
+
 // Stage N(b) in the warp's shared region according to its layout; returns
 // the probe mode.
 __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_t* sm, int cap_words, Staged& st,
@@ -1477,7 +1484,7 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ Tri
       mode = stage_set_block(t, item.hb, smem, cap_words * (int)nwarps, st);
       __syncthreads();
     } else {
-      mode = stage_set(t, item.hb, sm, cap_words, st, kMode == MODE_COUNT && item.ke - item.kb > kListRows);
+      mode = stage_set(t, item.hb, sm, cap_words, st, kMode == MODE_COUNT && !few_candidates(r, item));
     }
     const StagedRange sr = kMode == MODE_ANNOT ? staged_range(t, item.hb) : StagedRange{0, 0};
     const uint32_t blen = sr.len;
@@ -1898,6 +1905,7 @@ struct Hits {
   int use = 0;
   uint64_t words = 0;
   uint32_t units = 0, heads = 0, n = 0;
+  uint32_t longest = 0;   // longest part
   DevBuf<uint32_t> mask;
   DevBuf<uint32_t> plan;  // [heads] mask offsets, [heads + 1] units before, [n + 1] graph starts, sums
   uint32_t* moff() const { return plan.p; }
@@ -1927,10 +1935,10 @@ static bool plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
   H.use = use;
   H.n = n;
   H.heads = (uint32_t)heads;
-  const size_t o_sums = (2 * heads + 1 + n + 1 + 1) & ~(size_t)1;  // two 64-bit sums
-  H.plan.alloc(o_sums + 4, s);
+  const size_t o_sums = (2 * heads + 1 + n + 1 + 1) & ~(size_t)1;  // 64-bit sums
+  H.plan.alloc(o_sums + 6, s);
   unsigned long long* sums = reinterpret_cast<unsigned long long*>(H.plan.p + o_sums);
-  EH_CUDA(cudaMemsetAsync(sums, 0, 16, s));
+  EH_CUDA(cudaMemsetAsync(sums, 0, 24, s));
   EH_CUDA(cudaMemsetAsync(H.upre() + heads, 0, 4, s));
   EH_CUDA(cudaMemcpyAsync(H.gstart(), gstart.data(), (n + 1) * 4, cudaMemcpyHostToDevice, s));
   for (uint32_t g = 0; g < n; g++) {
@@ -1940,8 +1948,8 @@ static bool plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
     hits_size_kernel<<<grid, 256, 0, s>>>(tries[g]->view(), use, H.moff() + gstart[g], H.upre() + gstart[g], sums);
     EH_CHECK_LAUNCH();
   }
-  unsigned long long h[2];
-  EH_CUDA(cudaMemcpyAsync(h, sums, 16, cudaMemcpyDeviceToHost, s));
+  unsigned long long h[3];
+  EH_CUDA(cudaMemcpyAsync(h, sums, 24, cudaMemcpyDeviceToHost, s));
   EH_CUDA(cudaStreamSynchronize(s));
   if (h[0] > kMaxHitWords || h[1] >= kMaxHitWords) return false;
   exclusive_scan<uint32_t>(H.moff(), H.moff(), heads, nullptr, s);
@@ -1954,6 +1962,7 @@ static bool plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
   }
   H.words = h[0];
   H.units = (uint32_t)h[1];
+  H.longest = (uint32_t)h[2];
   H.on = true;
   return true;
 }
@@ -2053,7 +2062,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   // the annotated pass stages more of N(b) by default: its matched elements
   // then count in shared memory (measured on Chung-Lu 2^23: 2048 words per
   // warp 234 ms, 1024 245 ms)
-  if (annot && !hits && !ep.smem_given) ep.smem_words = 2 * kDefaultSmemWords;
+  if (annot && !hits && !ep.smem_given) ep.smem_words = 2048;
   P.threads = 32 * ep.warps;
   P.smem = (size_t)ep.smem_words * 4 * ep.warps;
   const void* kfn;
@@ -2204,9 +2213,16 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
         clique_big_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 32)), 256, 0, s>>>(
             P.dv, hv, H.units, P.ctl->queue + 1, d_total);
         EH_CHECK_LAUNCH();
+        if (H.longest > 32 * kSparseWords) {
+          clique_sparse_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 8)), 256, 0, s>>>(P.dv, hv, H.units,
+                                                                                            d_total);
+          EH_CHECK_LAUNCH();
+        }
       }
     } else if (H.use == HITS_ANNOT && H.units) {
-      annot_hits_kernel<<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, d_annot);
+      annot_hits_kernel<false><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, d_annot);
+      if (H.longest > 32 * kWideColumn)
+        annot_hits_kernel<true><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, d_annot);
       EH_CHECK_LAUNCH();
     }
     return;

@@ -72,3 +72,27 @@ def test_batched_cliques(eh, oracle):
         assert b.run().tolist() == want
     assert eh.count_batched(tries, "clique4").tolist() == want
     b.free()
+
+
+@pytest.mark.parametrize("kind", ["up", "down", "sym"])
+@pytest.mark.parametrize("d,extra,core", [(2047, 3000, 0), (2049, 3000, 40), (5000, 20000, 0), (5000, 2000, 300),
+                                          (9000, 40000, 120)])
+def test_wide_sparse_neighbourhoods(eh, oracle, kind, d, extra, core):
+    """Hubs of more than 2048 neighbours (as lowest or highest id) with few
+    edges among them, and with a dense core whose rows pass 256 hits."""
+    rng = np.random.default_rng(d + core)
+    a, b = rng.integers(1, d + 1, extra), rng.integers(1, d + 1, extra)
+    ca, cb = np.triu_indices(core, 1)
+    ids = np.sort(rng.choice(np.arange(1, d + 1), core, replace=False)) if core else np.zeros(0, np.int64)
+    u = np.concatenate([np.zeros(d, np.int64), np.minimum(a, b), ids[ca], np.arange(1, d + 1)])
+    v = np.concatenate([np.arange(1, d + 1), np.maximum(a, b), ids[cb], np.full(d, d + 1)])
+    keep = u != v
+    u, v = _orient(u[keep].astype(np.uint32), v[keep].astype(np.uint32), kind)
+    o = oracle.Trie(u, v)
+    t = eh.Trie(u, v)
+    assert t.count("triangle") == o.triangle()
+    assert t.count("clique4") == o.clique4()
+    assert eh.count_batched([t, t], "clique4").tolist() == [o.clique4()] * 2
+    assert sum(t.count("clique4", shard=(i, 3)) for i in range(3)) == o.clique4()
+    np.testing.assert_array_equal(t.triangle_annotation(), o.triangle_per_vertex())
+    t.free()
