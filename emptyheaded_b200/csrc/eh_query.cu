@@ -666,7 +666,7 @@ __device__ __forceinline__ uint64_t stream_rows(const Staged& st, const TrieView
     if (k < ke) {
       lo = __ldg(r.rev_lo + k);
       len = __ldg(r.rev_hi + k) - lo;
-      if (kMode != MODE_COUNT || kBits) src = __ldg(r.rev_src + k);
+      src = __ldg(r.rev_src + k);
     }
     // ---- word rows
     if (kBits) {
@@ -703,7 +703,7 @@ __device__ __forceinline__ uint64_t stream_rows(const Staged& st, const TrieView
           const uint32_t lo_w = __shfl_sync(kFull, wlo, j), hi_w = __shfl_sync(kFull, whi, j);
           const uint32_t b0 = __shfl_sync(kFull, v0, j), b1 = __shfl_sync(kFull, v1, j);
           const uint64_t base = __shfl_sync(kFull, abase, j);
-          const uint32_t sj = (kMode != MODE_COUNT) ? __shfl_sync(kFull, src, j) : 0u;
+          const uint32_t sj = __shfl_sync(kFull, src, j);
           const uint32_t w_first = b0 >> 6, w_last = b1 >> 6;
           uint32_t row_hits = 0;
           // The row's words lo_w..hi_w are read in pairs from an even pool
@@ -784,7 +784,7 @@ __device__ __forceinline__ uint64_t stream_rows(const Staged& st, const TrieView
           const uint32_t lo_w = __shfl_sync(kFull, wlo, j), ex = __shfl_sync(kFull, wexcl, j);
           const uint32_t b0 = __shfl_sync(kFull, v0, j), b1 = __shfl_sync(kFull, v1, j);
           const uint64_t base = __shfl_sync(kFull, abase, j);
-          sj[u] = (kMode != MODE_COUNT) ? __shfl_sync(kFull, src, j) : 0u;
+          sj[u] = __shfl_sync(kFull, src, j);
           x[u] = 0;
           wv[u] = 0;
           if (q < wtotal) {
@@ -834,11 +834,7 @@ __device__ __forceinline__ uint64_t stream_rows(const Staged& st, const TrieView
         const uint32_t rlo = __shfl_sync(kFull, lo, j), rn = __shfl_sync(kFull, rlen, j);
         const uint32_t rlo2 = __shfl_sync(kFull, lo, j2);
         const uint32_t rn2 = two ? __shfl_sync(kFull, rlen, j2) : 0u;
-        uint32_t src_j = 0, src_j2 = 0;
-        if (kMode != MODE_COUNT) {
-          src_j = __shfl_sync(kFull, src, j);
-          src_j2 = __shfl_sync(kFull, src, j2);
-        }
+        const uint32_t src_j = __shfl_sync(kFull, src, j), src_j2 = __shfl_sync(kFull, src, j2);
         const uint32_t* row = t.vals + rlo;
         const uint32_t* row2 = t.vals + rlo2;
         uint32_t row_hits = 0, row_hits2 = 0;
@@ -855,12 +851,12 @@ __device__ __forceinline__ uint64_t stream_rows(const Staged& st, const TrieView
             if (i + 32 * u < rn) {
               const uint32_t h = probe<P>(st, w[u]);
               row_hits += h;
-              if (kMode != MODE_COUNT && h) on_hit<kMode, true>(t, r, sk, src_j, w[u]);
+              if (h) on_hit<kMode, true>(t, r, sk, src_j, w[u]);
             }
             if (i + 32 * u < rn2) {
               const uint32_t h = probe<P>(st, w2[u]);
               row_hits2 += h;
-              if (kMode != MODE_COUNT && h) on_hit<kMode, true>(t, r, sk, src_j2, w2[u]);
+              if (h) on_hit<kMode, true>(t, r, sk, src_j2, w2[u]);
             }
           }
         }
@@ -886,7 +882,7 @@ __device__ __forceinline__ uint64_t stream_rows(const Staged& st, const TrieView
         const uint32_t q = p + 32 * u + lane;
         const uint32_t j = owner_lane(incl, q);
         const uint32_t loj = __shfl_sync(kFull, lo, j), exj = __shfl_sync(kFull, excl, j);
-        sj[u] = (kMode != MODE_COUNT) ? __shfl_sync(kFull, src, j) : 0u;
+        sj[u] = __shfl_sync(kFull, src, j);
         w[u] = q < total ? __ldg(t.vals + loj + (q - exj)) : 0u;
       }
 #pragma unroll
@@ -900,7 +896,7 @@ __device__ __forceinline__ uint64_t stream_rows(const Staged& st, const TrieView
           const uint32_t hm = __ballot_sync(kFull, h) & grp;
           if (lane == (uint32_t)(__ffs(grp) - 1)) add_src<kMode>(r, sk, sj[u], __popc(hm));
         }
-        if (kMode != MODE_COUNT && h) on_hit<kMode, true>(t, r, sk, sj[u], w[u]);
+        if (h) on_hit<kMode, true>(t, r, sk, sj[u], w[u]);
       }
     }
   }
@@ -1351,7 +1347,7 @@ __device__ __forceinline__ int stage_set_block(const TrieView& t, uint32_t hb, u
 template <int kMode>
 __device__ __forceinline__ uint64_t rows_of(int mode, const Staged& st, const TrieView& t, const RevView& r,
                                             uint32_t kb, uint32_t ke, uint32_t long_row, const Sink& sk) {
-  if (kMode == MODE_COUNT) {
+  if constexpr (kMode == MODE_COUNT) {
     switch (mode) {
       case P_SBITS: return count_rows<P_SBITS>(st, t, r, kb, ke, long_row);
       case P_GBITS: return count_rows<P_GBITS>(st, t, r, kb, ke, long_row);
@@ -1360,15 +1356,15 @@ __device__ __forceinline__ uint64_t rows_of(int mode, const Staged& st, const Tr
       case P_ZBITS: return count_rows<P_ZBITS>(st, t, r, kb, ke, long_row);
       default: return count_rows<P_GBLOCK>(st, t, r, kb, ke, long_row);
     }
-  }
-  constexpr int kSum = kMode == MODE_COUNT ? MODE_MAT : kMode;  // no COUNT form of stream_rows
-  switch (mode) {
-    case P_SBITS: return stream_rows<P_SBITS, kSum>(st, t, r, kb, ke, long_row, sk);
-    case P_GBITS: return stream_rows<P_GBITS, kSum>(st, t, r, kb, ke, long_row, sk);
-    case P_SLIST: return stream_rows<P_SLIST, kSum>(st, t, r, kb, ke, long_row, sk);
-    case P_GLIST: return stream_rows<P_GLIST, kSum>(st, t, r, kb, ke, long_row, sk);
-    case P_ZBITS: return stream_rows<P_ZBITS, kSum>(st, t, r, kb, ke, long_row, sk);
-    default: return stream_rows<P_GBLOCK, kSum>(st, t, r, kb, ke, long_row, sk);
+  } else {
+    switch (mode) {
+      case P_SBITS: return stream_rows<P_SBITS, kMode>(st, t, r, kb, ke, long_row, sk);
+      case P_GBITS: return stream_rows<P_GBITS, kMode>(st, t, r, kb, ke, long_row, sk);
+      case P_SLIST: return stream_rows<P_SLIST, kMode>(st, t, r, kb, ke, long_row, sk);
+      case P_GLIST: return stream_rows<P_GLIST, kMode>(st, t, r, kb, ke, long_row, sk);
+      case P_ZBITS: return stream_rows<P_ZBITS, kMode>(st, t, r, kb, ke, long_row, sk);
+      default: return stream_rows<P_GBLOCK, kMode>(st, t, r, kb, ke, long_row, sk);
+    }
   }
 }
 
