@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kPairThreads) pair_block_kernel(TrieView t, co
     const uint32_t p = big[k], A = pa[p], B = pb[p];
     uint32_t* dst = out.out_off ? out.out + out.out_off[p] : nullptr;
     uint64_t written = 0;
-    // hits of this thread in this round -> its place, and the round's total
+    // hits of this thread in this step -> its place, and the step's total
     auto place = [&](uint32_t c) {
       const uint32_t incl = warp_incl_scan(c);
       if (lane == 31) s_warp[wid] = incl;
