@@ -560,12 +560,16 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x) {
 // a few L2 lines.  The last kHubs entries count in shared memory and are added
 // to T once per block.
 constexpr uint32_t kHubs = 4096;
-// kWide: the units of columns kWideColumn on, each of many tiles: one at a time per
-// warp, four tiles' loads in flight (lollipop on a star of 2^17 leaves: 42 ms
-// without, 15); not: the others.
-constexpr uint32_t kWideColumn = 16;
+// kWide: the units of columns kWideColumn on, each of many tiles: spread over the
+// warps one by one, four tiles' loads in flight (lollipop on a star of 2^17 leaves:
+// 42 ms without, 15); not: the columns before `wide`.  The wide launch looks every
+// unit's entry up, 32 at a time, and pays where a part is longer than kWidePart
+// (launched for every part past column 16, one look-up at a time, the lollipop on
+// Chung-Lu 2^23 took 25.3 ms instead of 17.6).
+constexpr uint32_t kWideColumn = 16, kWidePart = 4096;
 template <bool kWide>
 __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv, uint32_t n_units,
+                                                         uint32_t wide,
                                                          unsigned long long* __restrict__ T) {
   __shared__ unsigned int hub[kHubs];
   for (uint32_t i = threadIdx.x; i < kHubs; i += blockDim.x) hub[i] = 0;
@@ -576,16 +580,36 @@ __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   // runs of consecutive units, so that few searches find the head entries,
   // spread over the warps, so that the long rows of a range of ids are too
-  constexpr uint32_t kRun = kWide ? 1 : 16;
+  constexpr uint32_t kRun = 16;
   uint32_t a = 0;
-  for (uint64_t v = 0;; v++) {
-    const uint64_t u64 = ((v / kRun) * nwarps + warp) * kRun + v % kRun;
-    if (u64 >= n_units) break;
-    const uint32_t u = (uint32_t)u64;
-    if (v % kRun == 0) a = hits_unit_head(hv, u);
-    while (__ldg(hv.upre + a + 1) <= u) a++;
-    const uint32_t k = u - __ldg(hv.upre + a);
-    if ((k >= kWideColumn) != kWide) continue;
+  uint32_t la = 0, lk = 0, todo = 0;  // kWide: each lane's unit, and the units still to do
+  for (uint64_t v = 0;;) {
+    uint32_t k;
+    if (kWide) {
+      if (!todo) {
+        const uint64_t base = 32 * v++ * nwarps + warp;
+        if (base >= n_units) break;
+        const uint64_t u = base + (uint64_t)lane * nwarps;
+        if (u < n_units) {
+          la = hits_unit_head(hv, (uint32_t)u);
+          lk = (uint32_t)u - __ldg(hv.upre + la);
+        }
+        todo = __ballot_sync(kFull, u < n_units && lk >= wide);
+        continue;
+      }
+      const int j = __ffs(todo) - 1;
+      todo &= todo - 1;
+      a = __shfl_sync(kFull, la, j);
+      k = __shfl_sync(kFull, lk, j);
+    } else {
+      const uint64_t u64 = ((v / kRun) * nwarps + warp) * kRun + v % kRun;
+      if (u64 >= n_units) break;
+      const uint32_t u = (uint32_t)u64;
+      if (v++ % kRun == 0) a = hits_unit_head(hv, u);
+      while (__ldg(hv.upre + a + 1) <= u) a++;
+      k = u - __ldg(hv.upre + a);
+      if (k >= wide) continue;
+    }
     const StagedRange pr = staged_range(t, a);
     const uint32_t d = pr.len, W = (d + 31) >> 5;
     const uint32_t* m = hv.mask + __ldg(hv.moff + a);

@@ -2216,9 +2216,10 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
         }
       }
     } else if (H.use == HITS_ANNOT && H.units) {
-      annot_hits_kernel<false><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, d_annot);
-      if (H.longest > 32 * kWideColumn)
-        annot_hits_kernel<true><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, d_annot);
+      const uint32_t wide = H.longest > kWidePart ? kWideColumn : ~0u;
+      annot_hits_kernel<false><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, wide, d_annot);
+      if (H.longest > kWidePart)
+        annot_hits_kernel<true><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, wide, d_annot);
       EH_CHECK_LAUNCH();
     }
     return;
