@@ -314,6 +314,16 @@ __device__ __forceinline__ uint32_t hits_unit_head(const HitsView& hv, uint32_t 
   }
   return lo - 1;
 }
+// head entry of unit u, at or after head entry a.  The next few are looked at
+// one by one (neighbours mostly have units); entries without units can lie in
+// hundreds of thousands between two that have some, so then by search (two
+// Erdos-Renyi graphs of 2^18 nodes, whose 4-clique units lie at the low ids of
+// each: 12.9 ms walking, one load after the other, 0.20 with the search).
+__device__ __forceinline__ uint32_t hits_unit_next(const HitsView& hv, uint32_t a, uint32_t u) {
+  for (uint32_t end = a + 8; a < end; a++)  // unit u exists, so some entry below hv.heads is found
+    if (__ldg(hv.upre + a + 1) > u) return a;
+  return hits_unit_head(hv, u);
+}
 
 // Work units of a head entry in the second pass.
 // 4-clique: eight rows of a part of d > 32 elements; smaller parts are one row
@@ -449,7 +459,7 @@ __global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restr
     const uint32_t u1 = min(u0 + 4, n_units);
     uint32_t gh = hits_unit_head(hv, u0);
     for (uint32_t u = u0; u < u1; u++) {
-      while (__ldg(hv.upre + gh + 1) <= u) gh++;  // entries without units have equal bounds
+      gh = hits_unit_next(hv, gh, u);
       const uint32_t g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0;
       if (g != cur_g) {
         acc = warp_sum(acc);
@@ -606,7 +616,7 @@ __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv
       if (u64 >= n_units) break;
       const uint32_t u = (uint32_t)u64;
       if (v++ % kRun == 0) a = hits_unit_head(hv, u);
-      while (__ldg(hv.upre + a + 1) <= u) a++;
+      a = hits_unit_next(hv, a, u);
       k = u - __ldg(hv.upre + a);
       if (k >= wide) continue;
     }
