@@ -681,9 +681,10 @@ __global__ void hits_row_count_kernel(TrieView t, int dir, HitsView hv, const ui
     cnt[e] = c;
   }
 }
-// a warp per relation row with triangles: word by word, a lane per bit; the
-// relation's rows and the elements of a part are in ascending order, so the
-// triangles come out sorted by (a, b, c)
+// a warp per relation row with triangles: the words that hold some, found 32 at
+// a time, a lane per bit; the relation's rows and the elements of a part are in
+// ascending order, so the triangles come out sorted by (a, b, c).  (All words one
+// after the other: a star of 2^16 leaves with 2^18 rows among them 33 ms.)
 __global__ void __launch_bounds__(256) hits_row_write_kernel(TrieView t, int dir, HitsView hv,
                                                              const uint32_t* __restrict__ seg,
                                                              const uint64_t* __restrict__ pos, uint64_t total,
@@ -711,20 +712,25 @@ __global__ void __launch_bounds__(256) hits_row_write_kernel(TrieView t, int dir
       const uint32_t rs = hits_stride(q, W, d);
       const uint32_t* row = hv.mask + __ldg(hv.moff + a) + hits_block(q, W) + (i & 31);
       const uint32_t va = __ldg(t.head + a), vb = __ldg(t.vals + e);
-      for (uint32_t kk = 0; kk < W - q; kk++) {
+      for (uint32_t k0 = 0; k0 < W - q; k0 += 32) {
         // ascending elements: positions descend on a relation that goes down
-        const uint32_t k = dir == DIR_DOWN ? W - q - 1 - kk : kk;
-        uint32_t x = __ldg(row + k * rs);
-        if (dir == DIR_DOWN) x = __brev(x);
-        if ((x >> lane) & 1u) {
-          const uint32_t bit = dir == DIR_DOWN ? 31 - lane : lane;
-          const uint32_t j = 32 * (q + k) + bit;
-          const uint64_t o = (out + __popc(x & lanemask_lt())) * stride;
-          oa[o] = va;
-          ob[o] = vb;
-          oc[o] = __ldg(t.vals + pr.s0 + (dir == DIR_DOWN ? d - 1 - j : j));
+        const uint32_t kl = dir == DIR_DOWN ? W - q - 1 - (k0 + lane) : k0 + lane;
+        const uint32_t word = k0 + lane < W - q ? __ldg(row + kl * rs) : 0u;
+        for (uint32_t words = __ballot_sync(kFull, word != 0); words; words &= words - 1) {
+          const int j = __ffs(words) - 1;
+          const uint32_t k = __shfl_sync(kFull, kl, j);
+          uint32_t x = __shfl_sync(kFull, word, j);
+          if (dir == DIR_DOWN) x = __brev(x);
+          if ((x >> lane) & 1u) {
+            const uint32_t bit = dir == DIR_DOWN ? 31 - lane : lane;
+            const uint32_t p = 32 * (q + k) + bit;
+            const uint64_t o = (out + __popc(x & lanemask_lt())) * stride;
+            oa[o] = va;
+            ob[o] = vb;
+            oc[o] = __ldg(t.vals + pr.s0 + (dir == DIR_DOWN ? d - 1 - p : p));
+          }
+          out += __popc(x);
         }
-        out += __popc(x);
       }
     }
   }
