@@ -33,12 +33,18 @@ struct HitsView {
   const uint32_t* gstart; // [graphs + 1] first head entry of a graph
   uint32_t n_graphs;
   uint32_t heads;         // of all graphs
+  CliqueShare share;      // 4-clique: the rows of this rank
 };
 
 __host__ __device__ __forceinline__ uint64_t hits_words(uint64_t d) {
   if (d < 2) return 0;
   const uint64_t W = (d + 31) / 32;
   return 32 * (W * (W + 1) / 2 - 1) + ((d - 32 * (W - 1) + 7) & ~7ull);
+}
+// steps of the 4-clique's second pass over a full matrix, up to a factor
+__host__ __device__ __forceinline__ uint64_t hits_work(uint64_t d) {
+  const uint64_t W = (d + 31) / 32;
+  return W * W * W;
 }
 // words before row block q; rows of a block (the stride between two words of a row)
 __device__ __forceinline__ uint32_t hits_block(uint32_t q, uint32_t W) { return 32 * (q * W - q * (q - 1) / 2); }
@@ -59,7 +65,7 @@ constexpr int kHitTrips = 8;  // divides 32; 4-clique R-MAT-20 4.13 -> 4.06 ms a
 template <int P>
 __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, const RevView& r, uint32_t kb,
                                          uint32_t ke, const uint32_t* __restrict__ moff,
-                                         uint32_t* __restrict__ mask, uint32_t shard_index, uint32_t shard_count) {
+                                         uint32_t* __restrict__ mask, const CliqueShare& share) {
   const uint32_t lane = lane_id();
   const uint32_t step = r.dir == DIR_DOWN ? 0xffffffffu : 1u;  // from one candidate's element to the next's
   uint32_t next_lo = 0, next_hi = 0, next_src = 0;  // the next batch's rows, loaded a batch ahead
@@ -79,10 +85,9 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
     uint32_t len = 0, fe = 0;               // candidates; the element of the first one
     uint32_t skip = 0, base = 0, rs = 0;    // bit of the first candidate in the row's words, first word, stride
     if (k < ke) {
-      // shards split the heads a: each rank builds and reads the matrices of its own
-      if (shard_count == 1 || src % shard_count == shard_index) {
-        const StagedRange pr = staged_range(t, src);
-        const uint32_t d = pr.len, W = (d + 31) >> 5;
+      const uint32_t d = staged_range(t, src).len;
+      if (share.builds(src, d)) {
+        const uint32_t W = (d + 31) >> 5;
         len = hi - lo;
         const uint32_t i = d - 1 - len;
         fe = r.dir == DIR_DOWN ? hi - 1 : lo;
@@ -167,7 +172,7 @@ __device__ __forceinline__ void hit_rows(const Staged& st, const TrieView& t, co
 // candidates at most) runs a mask word at a time.
 __device__ __forceinline__ void hit_merged(const TrieView& t, const RevView& r, uint32_t h0, uint32_t kb, uint32_t ke,
                                            const uint32_t* __restrict__ moff, uint32_t* __restrict__ mask,
-                                           uint32_t shard_index, uint32_t shard_count) {
+                                           const CliqueShare& share) {
   const uint32_t lane = lane_id();
   const uint32_t step = r.dir == DIR_DOWN ? 0xffffffffu : 1u;
   const Merged m(t, r, h0);
@@ -176,9 +181,10 @@ __device__ __forceinline__ void hit_merged(const TrieView& t, const RevView& r, 
     uint32_t len = 0, fe = 0, skip = 0, base = 0, rs = 0;
     if (k < ke) {
       const uint32_t src = __ldg(r.rev_src + k);
-      if (shard_count == 1 || src % shard_count == shard_index) {
+      const uint32_t d = staged_range(t, src).len;
+      if (share.builds(src, d)) {
         const uint32_t lo = __ldg(r.rev_lo + k), hi = __ldg(r.rev_hi + k);
-        const uint32_t d = staged_range(t, src).len, W = (d + 31) >> 5;
+        const uint32_t W = (d + 31) >> 5;
         len = hi - lo;
         const uint32_t i = d - 1 - len, q = i >> 5;
         fe = r.dir == DIR_DOWN ? hi - 1 : lo;
@@ -241,8 +247,7 @@ __global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const __grid_constant__ TrieVie
                                                  const TrieView* __restrict__ views, const RevView* __restrict__ revs,
                                                  const Item* __restrict__ items,
                                                  const unsigned int* __restrict__ n_items_p, int cap_words,
-                                                 unsigned int* __restrict__ queue, HitsView hv, float* records,
-                                                 uint32_t shard_index, uint32_t shard_count) {
+                                                 unsigned int* __restrict__ queue, HitsView hv, float* records) {
   extern __shared__ uint32_t smem[];
   const uint32_t lane = lane_id();
   uint32_t* sm = smem + (size_t)(threadIdx.x >> 5) * cap_words;
@@ -265,29 +270,29 @@ __global__ void EH_TRI_LAUNCH_BOUNDS hits_kernel(const __grid_constant__ TrieVie
     long long t0 = 0;
     if (records && lane == 0) t0 = clock64();
     if (item.hb & kMerged) {
-      hit_merged(t, r, item.hb & ~kMerged, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+      hit_merged(t, r, item.hb & ~kMerged, item.kb, item.ke, moff, hv.mask, hv.share);
       continue;
     }
     Staged st;
     const int mode = stage_set(t, item.hb, sm, cap_words, st, !few_candidates(r, item));
     switch (mode) {
       case P_SBITS:
-        hit_rows<P_SBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        hit_rows<P_SBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, hv.share);
         break;
       case P_GBITS:
-        hit_rows<P_GBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        hit_rows<P_GBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, hv.share);
         break;
       case P_SLIST:
-        hit_rows<P_SLIST>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        hit_rows<P_SLIST>(st, t, r, item.kb, item.ke, moff, hv.mask, hv.share);
         break;
       case P_GLIST:
-        hit_rows<P_GLIST>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        hit_rows<P_GLIST>(st, t, r, item.kb, item.ke, moff, hv.mask, hv.share);
         break;
       case P_ZBITS:
-        hit_rows<P_ZBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        hit_rows<P_ZBITS>(st, t, r, item.kb, item.ke, moff, hv.mask, hv.share);
         break;
       default:
-        hit_rows<P_GBLOCK>(st, t, r, item.kb, item.ke, moff, hv.mask, shard_index, shard_count);
+        hit_rows<P_GBLOCK>(st, t, r, item.kb, item.ke, moff, hv.mask, hv.share);
         break;
     }
     __syncwarp();  // the staged region is reused by the next item
@@ -336,26 +341,31 @@ __device__ __forceinline__ uint64_t hits_units(uint64_t d, int use) {
   return (d + 7) / 8;
 }
 
-// mask words and second-pass units of every head entry; sums over all of them, and
-// the longest part
-__global__ void hits_size_kernel(TrieView t, int use, uint32_t* __restrict__ words, uint32_t* __restrict__ units,
-                                 unsigned long long* __restrict__ sums) {
-  unsigned long long sw = 0, su = 0;
+// mask words and second-pass units of every head entry, none for those that only
+// other ranks build; sums over all of them, the longest part, and the sum of their
+// hits_work
+__global__ void hits_size_kernel(TrieView t, int use, CliqueShare share, uint32_t* __restrict__ words,
+                                 uint32_t* __restrict__ units, unsigned long long* __restrict__ sums) {
+  unsigned long long sw = 0, su = 0, work = 0;
   uint32_t most = 0;
   for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < t.n_head; a += gridDim.x * blockDim.x) {
     const uint64_t d = staged_range(t, a).len;
-    const uint64_t w = hits_words(d), u = hits_units(d, use);
+    const bool built = share.builds(a, (uint32_t)d);
+    const uint64_t w = built ? hits_words(d) : 0, u = built ? hits_units(d, use) : 0;
     words[a] = (uint32_t)w;  // meaningful only while the sum stays below 2^32, which the host checks
     units[a] = (uint32_t)u;
     sw += w;
     su += u;
+    if (built) work += hits_work(d);
     most = max(most, (uint32_t)d);
   }
   sw = warp_sum(sw);
   su = warp_sum(su);
+  work = warp_sum(work);
   if (lane_id() == 0) {
     if (sw) atomicAdd(sums, sw);
     if (su) atomicAdd(sums + 1, su);
+    if (work) atomicAdd(sums + 3, work);
   }
   most = __reduce_max_sync(kFull, most);
   if (lane_id() == 0 && most) atomicMax(sums + 2, (unsigned long long)most);
@@ -377,7 +387,9 @@ __global__ void __launch_bounds__(256) clique_small_kernel(const TrieView* __res
     if (gh < hv.heads) {
       g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0;
       const TrieView& t = views[g];
-      d = staged_range(t, gh - hv.gstart[g]).len;
+      const uint32_t a = gh - hv.gstart[g];
+      d = staged_range(t, a).len;
+      if (!hv.share.owns(a, d, 0)) d = 0;
       mo = __ldg(hv.moff + gh);
     }
     uint32_t todo = __ballot_sync(kFull, d >= 3 && d <= 32);
@@ -467,9 +479,10 @@ __global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restr
         acc = 0;
         cur_g = g;
       }
-      const uint32_t d = staged_range(views[g], gh - hv.gstart[g]).len, W = (d + 31) >> 5;
+      const uint32_t a = gh - hv.gstart[g], d = staged_range(views[g], a).len, W = (d + 31) >> 5;
       const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
       const uint32_t i0 = 8 * (u - __ldg(hv.upre + gh)), qi = i0 >> 5, ri = hits_stride(qi, W, d);
+      if (!hv.share.owns(a, d, i0)) continue;
       const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
       if (W > kSparseWords && sparse_rows(rows, ri, qi, W)) continue;  // clique_sparse_kernel's
       uint32_t c = 0;  // below 2^32: masks of 2^31 words hold at most 2^26 (j word, row) steps per lane
@@ -513,10 +526,11 @@ __global__ void __launch_bounds__(256) clique_sparse_kernel(const TrieView* __re
   for (uint64_t u = warp; u < n_units; u += nwarps) {
     const uint32_t gh = hits_unit_head(hv, (uint32_t)u);
     const uint32_t g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0;
-    const uint32_t d = staged_range(views[g], gh - hv.gstart[g]).len, W = (d + 31) >> 5;
+    const uint32_t a = gh - hv.gstart[g], d = staged_range(views[g], a).len, W = (d + 31) >> 5;
     if (W <= kSparseWords) continue;
     const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
     const uint32_t i0 = 8 * ((uint32_t)u - __ldg(hv.upre + gh)), qi = i0 >> 5, ri = hits_stride(qi, W, d);
+    if (!hv.share.owns(a, d, i0)) continue;
     const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
     if (!sparse_rows(rows, ri, qi, W)) continue;
     unsigned long long acc = 0;

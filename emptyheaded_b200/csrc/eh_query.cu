@@ -1368,6 +1368,26 @@ __device__ __forceinline__ uint64_t rows_of(int mode, const Staged& st, const Tr
   }
 }
 
+// A rank's part of the 4-clique of a relation that has an order (up, down,
+// symmetric): the cliques whose lowest vertex (highest, going down) is head entry
+// a belong to the rank of a.  A part so wide that, if it were dense, it would be
+// more than an even share of the work (hits_work) is dealt out instead, eight rows
+// a->b at a time by their position (eh_hits.cuh), and every rank makes its masks:
+// one vertex next to most others would leave the other ranks idle (R-MAT-16 by its
+// own ids in 8 shares: 30.9 ms on one rank, 1 to 6 on the others; so 6.1 to 7.0
+// on each).  The rule asks the relation and
+// the number of ranks alone, so that with or without masks the ranks cut alike.
+struct CliqueShare {
+  uint32_t index = 0, count = 1;
+  uint32_t wide = 0xffffffffu;  // parts of at least this many elements are dealt out; above 32
+  __device__ __forceinline__ bool builds(uint32_t a, uint32_t d) const {
+    return count == 1 || d >= wide || a % count == index;
+  }
+  __device__ __forceinline__ bool owns(uint32_t a, uint32_t d, uint32_t i) const {
+    return count == 1 || (d >= wide ? i >> 3 : a) % count == index;
+  }
+};
+
 struct QueryOut {
   uint32_t long_row;                  // size-class boundary of rows (warp-wide vs flattened)
   unsigned long long* total;   // per graph results (one per trie)
@@ -1384,6 +1404,7 @@ struct QueryOut {
   int32_t hot[kHot];           // MODE_ANNOT on a symmetric relation: largest sets' head entries, -1 if none
   uint32_t* gsbuf;             // 4-clique: per-warp S buffers in global memory (sets too large for
   uint32_t gcap;               //   shared memory), gcap words each; null: S in shared memory
+  CliqueShare share;           // 4-clique without masks of an ordered relation: this rank's rows
 };
 
 // kOne: one trie, whose views are the kernel's parameters -- operands from the
@@ -1591,7 +1612,8 @@ __device__ __forceinline__ uint32_t sel_bit(const uint32_t* sel, uint32_t x) {
 // the members that are selected (the host multiplies by 3!).
 template <int P>
 __device__ uint64_t clique_rows(const Staged& st, const TrieView& t, const RevView& r, uint32_t kb, uint32_t ke,
-                                uint32_t* sbuf, uint32_t cap, const uint32_t* sel, uint32_t wb) {
+                                uint32_t* sbuf, uint32_t cap, const uint32_t* sel, uint32_t wb,
+                                const CliqueShare& share) {
   const uint32_t lane = lane_id();
   const bool up = r.dir != DIR_DOWN;
   const bool general = r.dir == DIR_GENERAL;
@@ -1604,6 +1626,10 @@ __device__ uint64_t clique_rows(const Staged& st, const TrieView& t, const RevVi
       wab = wa + wb;
     }
     const uint32_t lo = __ldg(r.rev_lo + k), hi = __ldg(r.rev_hi + k);
+    if (share.count > 1) {
+      const uint32_t a = __ldg(r.rev_src + k), d = staged_range(t, a).len;
+      if (!share.owns(a, d, d - 1 - (hi - lo))) continue;
+    }
     // S = N(a)[lo, hi) ∩ N(b), compacted in order
     uint32_t ns = 0;
     for (uint32_t base = lo; base < hi; base += 32) {
@@ -1707,12 +1733,12 @@ __global__ void EH_TRI_LAUNCH_BOUNDS clique4_kernel(const TrieView* __restrict__
     const uint32_t wb = out.sel ? sel_bit(out.sel, t.head[item.hb]) : 0u;
     uint64_t c;
     switch (mode) {
-      case P_SBITS: c = clique_rows<P_SBITS>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb); break;
-      case P_GBITS: c = clique_rows<P_GBITS>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb); break;
-      case P_SLIST: c = clique_rows<P_SLIST>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb); break;
-      case P_GLIST: c = clique_rows<P_GLIST>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb); break;
-      case P_ZBITS: c = clique_rows<P_ZBITS>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb); break;
-      default: c = clique_rows<P_GBLOCK>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb); break;
+      case P_SBITS: c = clique_rows<P_SBITS>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb, out.share); break;
+      case P_GBITS: c = clique_rows<P_GBITS>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb, out.share); break;
+      case P_SLIST: c = clique_rows<P_SLIST>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb, out.share); break;
+      case P_GLIST: c = clique_rows<P_GLIST>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb, out.share); break;
+      case P_ZBITS: c = clique_rows<P_ZBITS>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb, out.share); break;
+      default: c = clique_rows<P_GBLOCK>(st, t, r, item.kb, item.ke, sbuf, scap, out.sel, wb, out.share); break;
     }
     acc += warp_sum(c);
     __syncwarp();
@@ -1902,65 +1928,86 @@ struct Hits {
   uint64_t words = 0;
   uint32_t units = 0, heads = 0, n = 0;
   uint32_t longest = 0;   // longest part
+  CliqueShare share;      // HITS_CLIQUE
   DevBuf<uint32_t> mask;
   DevBuf<uint32_t> plan;  // [heads] mask offsets, [heads + 1] units before, [n + 1] graph starts, sums
   uint32_t* moff() const { return plan.p; }
   uint32_t* upre() const { return plan.p + heads; }
   uint32_t* gstart() const { return upre() + heads + 1; }
-  HitsView view() const { return HitsView{mask.p, moff(), upre(), gstart(), n, heads}; }
+  HitsView view() const { return HitsView{mask.p, moff(), upre(), gstart(), n, heads, share}; }
 };
 // Masks hold a bit per candidate, so a relation in degree order needs far less
 // than its trie (R-MAT-22: 1.2 GB); past this many words (8 GB: a set of 300 K
 // elements read whole) the plans run without them.
 constexpr uint64_t kMaxHitWords = 1ull << 31;
 
-// false: the relation is general, or its masks are too large
-static bool plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int use, Hits& H) {
+// parts from this length on have more than a count-th of all the 4-clique's work
+static uint32_t wide_part(uint64_t work, uint32_t longest, uint32_t count) {
+  uint32_t lo = 33, hi = std::max(33u, longest + 1);
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if ((double)hits_work(mid) * count > (double)work) hi = mid; else lo = mid + 1;
+  }
+  return lo;
+}
+
+// Sizes and allocates the masks.  H.on: they are there.  H.share: how ranks share
+// a 4-clique of this relation, with its masks or (no memory for them) without; of
+// one rank if the relation is general or its masks are too large for any.
+static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int use, const ExecParams& ep,
+                      Hits& H) {
   cudaStream_t s = ctx->stream;
   uint64_t heads = 0;
   std::vector<uint32_t> gstart(n + 1, 0);
   for (uint32_t g = 0; g < n; g++) {
     const int dir = tries[g]->dir;
-    if (dir == DIR_GENERAL || (use == HITS_ANNOT && dir != DIR_SYM) || (use == HITS_ROWS && dir == DIR_SYM))
-      return false;
+    if (dir == DIR_GENERAL || (use == HITS_ANNOT && dir != DIR_SYM) || (use == HITS_ROWS && dir == DIR_SYM)) return;
     heads += tries[g]->n_head;
-    if (heads >= (1ull << 32) - 1) return false;
+    if (heads >= (1ull << 32) - 1) return;
     gstart[g + 1] = (uint32_t)heads;
   }
-  if (!heads) return false;
+  if (!heads) return;
   H.use = use;
   H.n = n;
   H.heads = (uint32_t)heads;
   const size_t o_sums = (2 * heads + 1 + n + 1 + 1) & ~(size_t)1;  // 64-bit sums
-  H.plan.alloc(o_sums + 6, s);
+  H.plan.alloc(o_sums + 8, s);
   unsigned long long* sums = reinterpret_cast<unsigned long long*>(H.plan.p + o_sums);
-  EH_CUDA(cudaMemsetAsync(sums, 0, 24, s));
   EH_CUDA(cudaMemsetAsync(H.upre() + heads, 0, 4, s));
   EH_CUDA(cudaMemcpyAsync(H.gstart(), gstart.data(), (n + 1) * 4, cudaMemcpyHostToDevice, s));
-  for (uint32_t g = 0; g < n; g++) {
-    const uint32_t nh = tries[g]->n_head;
-    if (!nh) continue;
-    const int grid = std::min(num_sms() * 4, ceil_div(nh, 256));
-    hits_size_kernel<<<grid, 256, 0, s>>>(tries[g]->view(), use, H.moff() + gstart[g], H.upre() + gstart[g], sums);
-    EH_CHECK_LAUNCH();
+  // of the head entries that `share` builds: mask words, units, longest part, bound of the 4-clique's work
+  unsigned long long h[4];
+  auto size = [&](const CliqueShare& share) {
+    EH_CUDA(cudaMemsetAsync(sums, 0, 32, s));
+    for (uint32_t g = 0; g < n; g++) {
+      const uint32_t nh = tries[g]->n_head;
+      if (!nh) continue;
+      const int grid = std::min(num_sms() * 4, ceil_div(nh, 256));
+      hits_size_kernel<<<grid, 256, 0, s>>>(tries[g]->view(), use, share, H.moff() + gstart[g], H.upre() + gstart[g],
+                                            sums);
+      EH_CHECK_LAUNCH();
+    }
+    EH_CUDA(cudaMemcpyAsync(h, sums, 32, cudaMemcpyDeviceToHost, s));
+    EH_CUDA(cudaStreamSynchronize(s));
+  };
+  size(CliqueShare{});
+  if (h[0] > kMaxHitWords || h[1] >= kMaxHitWords) return;
+  H.longest = (uint32_t)h[2];
+  if (use == HITS_CLIQUE && ep.shard_count > 1) {
+    H.share = CliqueShare{ep.shard_index, ep.shard_count, wide_part(h[3], H.longest, ep.shard_count)};
+    size(H.share);
   }
-  unsigned long long h[3];
-  EH_CUDA(cudaMemcpyAsync(h, sums, 24, cudaMemcpyDeviceToHost, s));
-  EH_CUDA(cudaStreamSynchronize(s));
-  if (h[0] > kMaxHitWords || h[1] >= kMaxHitWords) return false;
   exclusive_scan<uint32_t>(H.moff(), H.moff(), heads, nullptr, s);
   exclusive_scan<uint32_t>(H.upre(), H.upre(), heads + 1, nullptr, s);
   try {
     H.mask.alloc(h[0] ? h[0] : 1, s);
   } catch (const Error& e) {
     if (e.code != EH_ERR_OOM) throw;
-    return false;
+    return;
   }
   H.words = h[0];
   H.units = (uint32_t)h[1];
-  H.longest = (uint32_t)h[2];
   H.on = true;
-  return true;
 }
 
 // Runs the intersection kernel of `query` over the concatenated plans of
@@ -2048,7 +2095,8 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   cudaStream_t s = ctx->stream;
   P.query = query;
   P.annot = annot;
-  const bool hits = hits_use >= 0 && plan_hits(ctx, tries, n, hits_use, P.hits);
+  if (hits_use >= 0) plan_hits(ctx, tries, n, hits_use, ep, P.hits);
+  const bool hits = P.hits.on;
   if (query == EH_QUERY_CLIQUE4 && !hits) {
     uint32_t mx = 0;
     for (uint32_t g = 0; g < n; g++) mx = std::max(mx, tries[g]->info.max_set);
@@ -2150,12 +2198,13 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   for (uint32_t g = 0; g < n; g++) {
     const eh_trie* t = tries[g];
     if (!t->rev_entries) continue;
-    // every shard of a plan on hit masks runs all the items: the masks split by head entry
+    // every shard of a 4-clique that is split by rows (CliqueShare) runs all the items
+    const bool by_rows = hits || P.hits.share.count > 1;
     // records are per entry, only these kernels look rows up, and few entries
     // are better spread over the warps (ER-16K, three entries a warp: 77 us a
     // query against 87 with shared items)
     shape.merge = merge && (hits || blocks_query) && t->n_head < kMerged && head_items > 4 * slots;
-    PlanArgs pa{t->view(), rev_view(t), shape, g, hits ? 0 : ep.shard_index, hits ? 1 : ep.shard_count,
+    PlanArgs pa{t->view(), rev_view(t), shape, g, by_rows ? 0 : ep.shard_index, by_rows ? 1 : ep.shard_count,
                 reinterpret_cast<uint64_t*>(base + o_pos), nullptr};
     pa.tiles = pa.pos + t->n_head;
     if (t->work_pred.p && t->pred_per_probe > 0) {
@@ -2199,8 +2248,7 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
     const HitsView hv = H.view();
     EH_CUDA(cudaMemsetAsync(H.mask.p, 0, H.words * 4, s));
     (P.n == 1 ? hits_kernel<true> : hits_kernel<false>)<<<P.grid, P.threads, P.smem, s>>>(
-        P.view0, P.rev0, P.dv, P.dr, P.items, P.ctl->items, ep.smem_words, P.ctl->queue, hv, d_records,
-        ep.shard_index, ep.shard_count);
+        P.view0, P.rev0, P.dv, P.dr, P.items, P.ctl->items, ep.smem_words, P.ctl->queue, hv, d_records);
     EH_CHECK_LAUNCH();
     if (H.use == HITS_CLIQUE) {
       clique_small_kernel<<<std::min(num_sms() * 8, ceil_div(H.heads, 256)), 256, 0, s>>>(P.dv, hv, d_total);
@@ -2229,6 +2277,7 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
   for (int k = 0; k < kHot; k++) out.hot[k] = P.hot[k];
   out.gsbuf = ep.s_cap ? P.gs.p : nullptr;
   out.gcap = ep.s_cap;
+  out.share = P.hits.share;
   if (P.query == EH_QUERY_CLIQUE4)
     clique4_kernel<<<P.grid, P.threads, P.smem, s>>>(P.dv, P.dr, P.items, ep.smem_words, out);
   else if (P.annot)

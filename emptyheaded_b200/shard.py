@@ -2,9 +2,10 @@
 
 Every rank holds the whole trie (0.3-1.3 GB at the benchmark sizes; HBM is
 180 GB) and runs its share of the heaviest-first plan: item i of head entry b
-where (b + i) % world == rank, for the 4-clique the head entries a with
-a % world == rank (eh_exec_config.shard_index / shard_count).  The only
-exchange is the final sum: one 8-byte all-reduce.  Counts are modulo 2^64
+where (b + i) % world == rank; for the 4-clique of an up, down or symmetric
+relation the cliques of the head entries a with a % world == rank, those of the
+widest entries by eight rows (eh_exec_config.shard_index / shard_count).  The
+only exchange is the final sum: one 8-byte all-reduce.  Counts are modulo 2^64
 like the reference's signed long, so the sum is taken on int64 tensors and
 read back as uint64 bit patterns.  The reference's own parallelism is the
 same split over threads (par::for_range + par::reducer,

@@ -237,8 +237,12 @@ typedef struct {
   int smem_words;        /* per-warp shared staging capacity in u32 words; 0 = default */
   int record_timings;    /* 1: log per-item device time for the cost model */
   int shard_index;       /* this rank's share of the plan: item i of head entry b
-                            runs where (b + i) % shard_count == shard_index (the
-                            4-clique's hit masks: head entries a % shard_count) */
+                            runs where (b + i) % shard_count == shard_index; of
+                            the 4-clique of an up, down or symmetric relation
+                            the cliques whose lowest (going down: highest)
+                            vertex is head entry a, a % shard_count, the widest
+                            entries' by eight rows.  Every rank gives the same
+                            configuration but for shard_index */
   int shard_count;       /* 0 or 1: everything */
   int no_block_items;    /* 1: stage every N(b) in one warp's region; 0: an N(b)
                             too large for a warp's region but not for the
