@@ -423,8 +423,9 @@ class Trie:
     def count(self, query="triangle", warps=0, chunk=0, smem_words=0, record=False, stats=False, shard=(0, 1),
               long_row=0, config=None, block_items=True):
         """Run a named COUNT plan; returns the count (and stats if asked).
-        shard=(i, n) runs the i-th of n round-robin shares of the work items
-        (the partial counts of the n shares sum to the count).  `config`
+        shard=(i, n) runs the i-th of n shares of the work (emptyheaded_b200.shard;
+        the partial counts of the n shares sum to the count, every share run with
+        the same schedule).  `config`
         (a dict from emptyheaded_b200.autotune) supplies the schedule knobs."""
         if config:
             warps = config.get("warps", warps)

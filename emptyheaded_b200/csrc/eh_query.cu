@@ -83,6 +83,7 @@ constexpr int kDefaultSmemWords = 1280;  // per warp
 constexpr int kDefaultChunk = 32768;     // where it is not derived from the work (records, noalloc)
 constexpr uint64_t kMaxChunk = 131072;   // larger items amortise staging: 7.03 ms against 7.18 at 32768
 constexpr uint64_t kMinChunk = 4096;  // the smallest item the planner cuts by itself
+constexpr uint32_t kShareWarps = 148 * 32;  // resident warps of a B200 at the default schedule
 
 struct RevView {
   const uint64_t* rev_off;
@@ -293,7 +294,8 @@ struct Control {
 // items come last.  (Reserving the places by atomics in one launch put heavy
 // blocks behind light ones: triangle R-MAT-20 1.43 -> 1.7-2.5 ms.)
 // Shards take the items i of entry b with (b + i + g) % shard_count ==
-// shard_index.
+// shard_index; of shared items (kMerged), which begin at multiples of 8 or 16, the
+// group's number counts in place of b.
 struct PlanArgs {
   TrieView t;
   RevView r;
@@ -327,10 +329,11 @@ __device__ __forceinline__ uint32_t plan_span(const PlanArgs& p, uint32_t b) {
   return plan_small(p, b & ~7u, 8) ? 8 : 1;
 }
 
-// items of entry b over all shards
-__device__ __forceinline__ uint32_t plan_items(const PlanArgs& p, uint32_t b, uint64_t k0, uint64_t k1, bool& blk) {
+// items of entry b over all shards; span: plan_span
+__device__ __forceinline__ uint32_t plan_items(const PlanArgs& p, uint32_t b, uint64_t k0, uint64_t k1, bool& blk,
+                                               uint32_t& span) {
   blk = false;
-  const uint32_t span = plan_span(p, b);
+  span = plan_span(p, b);
   if (span > 1) return (b & (span - 1)) == 0 && p.r.rev_off[b + span] > k0 ? 1 : 0;
   if (k1 <= k0) return 0;
   const uint64_t w = p.r.rev_wpre[k1] - p.r.rev_wpre[k0];
@@ -346,8 +349,8 @@ __device__ __forceinline__ uint32_t plan_items(const PlanArgs& p, uint32_t b, ui
   return (uint32_t)((w + kRowCost * (k1 - k0) + p.ps.chunk * mult - 1) / (p.ps.chunk * mult));
 }
 // this shard's first item of entry b
-__device__ __forceinline__ uint32_t plan_first(const PlanArgs& p, uint32_t b) {
-  return p.shard_count > 1 ? (p.shard_index + p.shard_count - (b + p.g) % p.shard_count) % p.shard_count : 0;
+__device__ __forceinline__ uint32_t plan_first(const PlanArgs& p, uint32_t b, uint32_t span) {
+  return p.shard_count > 1 ? (p.shard_index + p.shard_count - (b / span + p.g) % p.shard_count) % p.shard_count : 0;
 }
 
 // zero: bytes of the control block and results to clear (a single trie, whose
@@ -361,8 +364,9 @@ __global__ void __launch_bounds__(256) plan_split_kernel(PlanArgs p, Control* __
     const uint64_t b = (uint64_t)blockIdx.x * kPlanTile + x;
     if (b >= p.t.n_head) break;
     bool blk;
-    const uint32_t n = plan_items(p, (uint32_t)b, p.r.rev_off[b], p.r.rev_off[b + 1], blk);
-    const uint32_t first = plan_first(p, (uint32_t)b);
+    uint32_t span;
+    const uint32_t n = plan_items(p, (uint32_t)b, p.r.rev_off[b], p.r.rev_off[b + 1], blk, span);
+    const uint32_t first = plan_first(p, (uint32_t)b, span);
     const uint64_t mine = n > first ? (n - first + p.shard_count - 1) / p.shard_count : 0;
     const uint64_t v = blk ? mine << 32 : mine;
     p.pos[b] = v;
@@ -440,9 +444,10 @@ __global__ void __launch_bounds__(256) plan_fill_kernel(PlanArgs p, const unsign
     const uint64_t v = p.pos[b];
     const uint64_t k0 = p.r.rev_off[b], k1 = p.r.rev_off[b + 1];
     bool blk;
-    const uint64_t m = plan_items(p, b, k0, k1, blk);
-    const uint64_t i = plan_first(p, b) + (uint64_t)(q - (cls ? (uint32_t)(v >> 32) : (uint32_t)v)) * p.shard_count;
-    const uint32_t span = plan_span(p, b);
+    uint32_t span;
+    const uint64_t m = plan_items(p, b, k0, k1, blk, span);
+    const uint64_t i =
+        plan_first(p, b, span) + (uint64_t)(q - (cls ? (uint32_t)(v >> 32) : (uint32_t)v)) * p.shard_count;
     if (span > 1) {
       items[w0 + (nw - 1 - q)] = Item{b | kMerged, (uint32_t)k0, (uint32_t)p.r.rev_off[b + span], p.g};
       continue;
@@ -2133,7 +2138,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   const bool blocks = block_items && !hits && query == EH_QUERY_TRIANGLE && !annot && ep.warps > 1 &&
                       !ep.no_block_items;
   // work of all tries, and how finely to cut it: 8 items for each resident
-  // warp, of kMinChunk to kMaxChunk
+  // warp (of every rank), of kMinChunk to kMaxChunk
   uint64_t cost = 0, head_items = 0;
   P.n = n;
   for (uint32_t g = 0; g < n; g++) {
@@ -2142,7 +2147,9 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     cost += tries[g]->rev_pairs + kRowCost * tries[g]->rev_entries;
     head_items += std::min<uint64_t>(tries[g]->n_head, tries[g]->rev_entries);
   }
-  const uint64_t slots = (uint64_t)num_sms() * per_sm * ep.warps;  // resident warps
+  // ranks that share a query cut the same items, whatever they run on
+  const uint64_t resident = (uint64_t)num_sms() * per_sm * ep.warps;
+  const uint64_t slots = ep.shard_count > 1 ? (uint64_t)kShareWarps * ep.shard_count : resident;
   if (!ep.chunk_given) {
     ep.chunk = (uint32_t)std::min<uint64_t>(kMaxChunk, std::max<uint64_t>(kMinChunk, cost / (8 * slots)));
   }

@@ -2,7 +2,8 @@
 
 Every rank holds the whole trie (0.3-1.3 GB at the benchmark sizes; HBM is
 180 GB) and runs its share of the heaviest-first plan: item i of head entry b
-where (b + i) % world == rank; for the 4-clique of an up, down or symmetric
+where (b + i) % world == rank (of an item that a group of 8 or 16 neighbouring
+entries share, the group's number in place of b); for the 4-clique of an up, down or symmetric
 relation the cliques of the head entries a with a % world == rank, those of the
 widest entries by eight rows (eh_exec_config.shard_index / shard_count).  The
 only exchange is the final sum: one 8-byte all-reduce.  Counts are modulo 2^64
@@ -39,6 +40,7 @@ def max_over_ranks(x, device="cpu", group=None):
     return float(t.item())
 
 
-def owned(n_items, rank, world):
-    """Indices of the work items a rank runs (host mirror of the device rule)."""
-    return range(rank, n_items, world)
+def owned(n_items, rank, world, entry=0):
+    """Indices i of the n_items items of a head entry that a rank runs:
+    (entry + i) % world == rank, the device's rule."""
+    return range((rank - entry) % world, n_items, world)
