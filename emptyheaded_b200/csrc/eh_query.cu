@@ -1933,6 +1933,7 @@ struct Hits {
   uint64_t words = 0;
   uint32_t units = 0, heads = 0, n = 0;
   uint32_t longest = 0;   // longest part
+  uint32_t launches = 0;  // kernels of the mask plan
   CliqueShare share;      // HITS_CLIQUE
   DevBuf<uint32_t> mask;
   DevBuf<uint32_t> plan;  // [heads] mask offsets, [heads + 1] units before, [n + 1] graph starts, sums
@@ -1991,6 +1992,7 @@ static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
       hits_size_kernel<<<grid, 256, 0, s>>>(tries[g]->view(), use, share, H.moff() + gstart[g], H.upre() + gstart[g],
                                             sums);
       EH_CHECK_LAUNCH();
+      H.launches++;
     }
     EH_CUDA(cudaMemcpyAsync(h, sums, 32, cudaMemcpyDeviceToHost, s));
     EH_CUDA(cudaStreamSynchronize(s));
@@ -2004,6 +2006,7 @@ static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
   }
   exclusive_scan<uint32_t>(H.moff(), H.moff(), heads, nullptr, s);
   exclusive_scan<uint32_t>(H.upre(), H.upre(), heads + 1, nullptr, s);
+  H.launches += scan_launches(heads) + scan_launches(heads + 1);
   try {
     H.mask.alloc(h[0] ? h[0] : 1, s);
   } catch (const Error& e) {
@@ -2059,16 +2062,19 @@ __global__ void top_set_kernel(const uint64_t* __restrict__ off, uint32_t nh, In
   if (lane_id() == 0 && m) atomicMax(best, m);
 }
 
-// the kHot head entries with the largest sets of a trie (-1 where fewer)
-static void hot_sets(eh_context* ctx, const eh_trie* t, int32_t* hot) {
+// the kHot head entries with the largest sets of a trie (-1 where fewer); the
+// kernels launched
+static uint32_t hot_sets(eh_context* ctx, const eh_trie* t, int32_t* hot) {
   cudaStream_t s = ctx->stream;
   Int4 ex{{-1, -1, -1, -1}};
   DevBuf<unsigned long long> best(1, s);
+  uint32_t launches = 0;
   for (int k = 0; k < kHot; k++) hot[k] = -1;
   for (int k = 0; k < kHot && (uint32_t)k < t->n_head; k++) {
     EH_CUDA(cudaMemsetAsync(best.p, 0, 8, s));
     top_set_kernel<<<num_sms() * 4, 256, 0, s>>>(t->off.p, t->n_head, ex, best.p);
     EH_CHECK_LAUNCH();
+    launches++;
     unsigned long long h = 0;
     EH_CUDA(cudaMemcpyAsync(&h, best.p, 8, cudaMemcpyDeviceToHost, s));
     EH_CUDA(cudaStreamSynchronize(s));
@@ -2076,6 +2082,7 @@ static void hot_sets(eh_context* ctx, const eh_trie* t, int32_t* hot) {
     hot[k] = (int32_t)(h & 0xffffffffu);
     ex.v[k] = hot[k];
   }
+  return launches;
 }
 
 // 4-clique without hit masks: the warp's shared region holds the staged N(b) and S
@@ -2101,6 +2108,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   P.query = query;
   P.annot = annot;
   if (hits_use >= 0) plan_hits(ctx, tries, n, hits_use, ep, P.hits);
+  P.plan_launches += P.hits.launches;
   const bool hits = P.hits.on;
   if (query == EH_QUERY_CLIQUE4 && !hits) {
     uint32_t mx = 0;
@@ -2231,7 +2239,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   }
   const uint64_t units = P.cap_b + (P.cap_w + ep.warps - 1) / ep.warps;
   P.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * per_sm, units));
-  if (annot && !hits && n == 1 && tries[0]->dir == DIR_SYM) hot_sets(ctx, tries[0], P.hot);
+  if (annot && !hits && n == 1 && tries[0]->dir == DIR_SYM) P.plan_launches += hot_sets(ctx, tries[0], P.hot);
   if (query == EH_QUERY_CLIQUE4 && !hits && ep.s_cap) {
     // one S buffer per resident warp, at most 2 GiB in all
     const uint64_t per_block = (uint64_t)ep.warps * ep.s_cap * 4;
@@ -2243,11 +2251,11 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
 
 // Enqueue one run of a prepared launch; the first follows prepare directly, a
 // later one resets the queues.  No host synchronisation: capturable in a CUDA
-// graph.
-static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, unsigned long long* d_annot,
+// graph.  Returns the kernels launched.
+static uint32_t launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, unsigned long long* d_annot,
                    float* d_records, bool again = false) {
   cudaStream_t s = ctx->stream;
-  if (!P.entries) return;
+  if (!P.entries) return 0;
   if (again) EH_CUDA(cudaMemsetAsync(P.ctl->queue, 0, 8, s));
   const ExecParams& ep = P.ep;
   if (P.hits.on) {
@@ -2257,27 +2265,33 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
     (P.n == 1 ? hits_kernel<true> : hits_kernel<false>)<<<P.grid, P.threads, P.smem, s>>>(
         P.view0, P.rev0, P.dv, P.dr, P.items, P.ctl->items, ep.smem_words, P.ctl->queue, hv, d_records);
     EH_CHECK_LAUNCH();
+    uint32_t launches = 1;
     if (H.use == HITS_CLIQUE) {
       clique_small_kernel<<<std::min(num_sms() * 8, ceil_div(H.heads, 256)), 256, 0, s>>>(P.dv, hv, d_total);
       EH_CHECK_LAUNCH();
+      launches++;
       if (H.units) {
         clique_big_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 32)), 256, 0, s>>>(
             P.dv, hv, H.units, P.ctl->queue + 1, d_total);
         EH_CHECK_LAUNCH();
+        launches++;
         if (H.longest > 32 * kSparseWords) {
           clique_sparse_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 8)), 256, 0, s>>>(P.dv, hv, H.units,
                                                                                             d_total);
           EH_CHECK_LAUNCH();
+          launches++;
         }
       }
     } else if (H.use == HITS_ANNOT && H.units) {
-      const uint32_t wide = H.longest > kWidePart ? kWideColumn : ~0u;
+      const bool wide_parts = H.longest > kWidePart;
+      const uint32_t wide = wide_parts ? kWideColumn : ~0u;
       annot_hits_kernel<false><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, wide, d_annot);
-      if (H.longest > kWidePart)
+      if (wide_parts)
         annot_hits_kernel<true><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, wide, d_annot);
       EH_CHECK_LAUNCH();
+      launches += wide_parts ? 2 : 1;
     }
-    return;
+    return launches;
   }
   QueryOut out{ep.long_row, d_total, d_annot, d_records, P.ctl->queue, P.ctl->items, P.bitems};
   out.sel = P.sel;
@@ -2297,6 +2311,7 @@ static void launch(eh_context* ctx, Prepared& P, unsigned long long* d_total, un
     triangle_kernel<MODE_COUNT, false><<<P.grid, P.threads, P.smem, s>>>(P.view0, P.rev0, P.dv, P.dr, P.items,
                                                                          ep.smem_words, out);
   EH_CHECK_LAUNCH();
+  return 1;
 }
 
 // Plan and run; nothing is waited for.  ev1 and ev2 bracket the intersection
@@ -2317,10 +2332,9 @@ static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n
   EH_CUDA(cudaEventRecord(ctx->ev1, s));
   {
     TracePhase ph("query.kernel", s);
-    launch(ctx, P, spare ? P.ctl->spare : d_total ? d_total : P.total, d_annot, d_records);
+    L.launches += launch(ctx, P, spare ? P.ctl->spare : d_total ? d_total : P.total, d_annot, d_records);
   }
   EH_CUDA(cudaEventRecord(ctx->ev2, s));
-  if (P.entries) L.launches += P.hits.on ? (P.hits.use == HITS_CLIQUE && P.hits.units ? 3 : 2) : 1;
   return L;
 }
 
@@ -3021,6 +3035,7 @@ struct eh_batch {
   std::vector<int> dirs;
   uint32_t n = 0;
   uint64_t items = 0;
+  uint32_t launches = 0;  // kernels of a run
   int query = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -3059,7 +3074,7 @@ eh_batch* batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n,
     cudaError_t cap = cudaSuccess;
     try {
       EH_CUDA(cudaMemsetAsync(b->P.total, 0, n * 8, s));
-      launch(ctx, b->P, b->P.total, nullptr, nullptr, true);
+      b->launches = launch(ctx, b->P, b->P.total, nullptr, nullptr, true);
       EH_CUDA(cudaMemcpyAsync(b->host, b->P.total, n * 8, cudaMemcpyDeviceToHost, s));
     } catch (...) {
       cudaGraph_t g = nullptr;
@@ -3095,7 +3110,7 @@ void batch_run(eh_context* ctx, eh_batch* b, uint64_t* results, eh_query_stats* 
   if (stats) {
     stats->query_ms = ms;
     stats->kernel_ms = ms;
-    stats->launches = 1;
+    stats->launches = b->launches;
     stats->work_items = b->items;
     stats->wedges = b->P.pairs;
     stats->algorithmic_bytes = 0;
