@@ -342,30 +342,36 @@ __device__ __forceinline__ uint64_t hits_units(uint64_t d, int use) {
 }
 
 // mask words and second-pass units of every head entry, none for those that only
-// other ranks build; sums over all of them, the longest part, and the sum of their
-// hits_work
+// other ranks build; the sums over all entries, their longest part and the sum of
+// their hits_work, and the sums over the entries built here
 __global__ void hits_size_kernel(TrieView t, int use, CliqueShare share, uint32_t* __restrict__ words,
                                  uint32_t* __restrict__ units, unsigned long long* __restrict__ sums) {
-  unsigned long long sw = 0, su = 0, work = 0;
+  unsigned long long sw = 0, su = 0, work = 0, bw = 0, bu = 0;
   uint32_t most = 0;
   for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < t.n_head; a += gridDim.x * blockDim.x) {
     const uint64_t d = staged_range(t, a).len;
+    const uint64_t w = hits_words(d), u = hits_units(d, use);
     const bool built = share.builds(a, (uint32_t)d);
-    const uint64_t w = built ? hits_words(d) : 0, u = built ? hits_units(d, use) : 0;
-    words[a] = (uint32_t)w;  // meaningful only while the sum stays below 2^32, which the host checks
-    units[a] = (uint32_t)u;
+    words[a] = built ? (uint32_t)w : 0u;  // meaningful only while the sum stays below 2^32, which the host checks
+    units[a] = built ? (uint32_t)u : 0u;
     sw += w;
     su += u;
-    if (built) work += hits_work(d);
+    bw += built ? w : 0;
+    bu += built ? u : 0;
+    work += hits_work(d);
     most = max(most, (uint32_t)d);
   }
   sw = warp_sum(sw);
   su = warp_sum(su);
   work = warp_sum(work);
+  bw = warp_sum(bw);
+  bu = warp_sum(bu);
   if (lane_id() == 0) {
     if (sw) atomicAdd(sums, sw);
     if (su) atomicAdd(sums + 1, su);
     if (work) atomicAdd(sums + 3, work);
+    if (bw) atomicAdd(sums + 4, bw);
+    if (bu) atomicAdd(sums + 5, bu);
   }
   most = __reduce_max_sync(kFull, most);
   if (lane_id() == 0 && most) atomicMax(sums + 2, (unsigned long long)most);

@@ -1946,6 +1946,13 @@ struct Hits {
 // than its trie (R-MAT-22: 1.2 GB); past this many words (8 GB: a set of 300 K
 // elements read whole) the plans run without them.
 constexpr uint64_t kMaxHitWords = 1ull << 31;
+// A 4-clique of few rows with small sets runs without: its pairs are few too, and the
+// mask plan (sizes, two scans, clearing, two passes) would be most of it.  Sets of at
+// most 32, us without masks / with: K_24 74 / 115, 64 of them in a batch 58 / 71;
+// Erdos-Renyi of 4096 nodes and degree 8, 74 / 139, 3 in a batch 46 / 58; 64 of 1024
+// nodes (200 K rows) 83 / 58.  Above: K_48 156 / 131, in a batch 132 / 70.
+constexpr uint64_t kFewRows = 65536;
+constexpr uint32_t kSmallSet = 32;
 
 // parts from this length on have more than a count-th of all the 4-clique's work
 static uint32_t wide_part(uint64_t work, uint32_t longest, uint32_t count) {
@@ -1959,32 +1966,37 @@ static uint32_t wide_part(uint64_t work, uint32_t longest, uint32_t count) {
 
 // Sizes and allocates the masks.  H.on: they are there.  H.share: how ranks share
 // a 4-clique of this relation, with its masks or (no memory for them) without; of
-// one rank if the relation is general or its masks are too large for any.
+// one rank if the relation is general, its masks are too large for any, or it has
+// no or few rows: all facts of the relation, the same on every rank.
 static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int use, const ExecParams& ep,
                       Hits& H) {
   cudaStream_t s = ctx->stream;
-  uint64_t heads = 0;
+  uint64_t heads = 0, entries = 0;
+  uint32_t max_set = 0;
   std::vector<uint32_t> gstart(n + 1, 0);
   for (uint32_t g = 0; g < n; g++) {
     const int dir = tries[g]->dir;
     if (dir == DIR_GENERAL || (use == HITS_ANNOT && dir != DIR_SYM) || (use == HITS_ROWS && dir == DIR_SYM)) return;
     heads += tries[g]->n_head;
+    entries += tries[g]->rev_entries;
+    max_set = std::max(max_set, tries[g]->info.max_set);
     if (heads >= (1ull << 32) - 1) return;
     gstart[g + 1] = (uint32_t)heads;
   }
-  if (!heads) return;
+  if (!entries || (use == HITS_CLIQUE && entries <= kFewRows && max_set <= kSmallSet)) return;
   H.use = use;
   H.n = n;
   H.heads = (uint32_t)heads;
   const size_t o_sums = (2 * heads + 1 + n + 1 + 1) & ~(size_t)1;  // 64-bit sums
-  H.plan.alloc(o_sums + 8, s);
+  H.plan.alloc(o_sums + 12, s);
   unsigned long long* sums = reinterpret_cast<unsigned long long*>(H.plan.p + o_sums);
   EH_CUDA(cudaMemsetAsync(H.upre() + heads, 0, 4, s));
   EH_CUDA(cudaMemcpyAsync(H.gstart(), gstart.data(), (n + 1) * 4, cudaMemcpyHostToDevice, s));
-  // of the head entries that `share` builds: mask words, units, longest part, bound of the 4-clique's work
-  unsigned long long h[4];
+  // mask words, units and longest part of all head entries, bound of the 4-clique's work on them; words and
+  // units of the head entries that `share` builds
+  unsigned long long h[6];
   auto size = [&](const CliqueShare& share) {
-    EH_CUDA(cudaMemsetAsync(sums, 0, 32, s));
+    EH_CUDA(cudaMemsetAsync(sums, 0, sizeof(h), s));
     for (uint32_t g = 0; g < n; g++) {
       const uint32_t nh = tries[g]->n_head;
       if (!nh) continue;
@@ -1994,27 +2006,28 @@ static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
       EH_CHECK_LAUNCH();
       H.launches++;
     }
-    EH_CUDA(cudaMemcpyAsync(h, sums, 32, cudaMemcpyDeviceToHost, s));
+    EH_CUDA(cudaMemcpyAsync(h, sums, sizeof(h), cudaMemcpyDeviceToHost, s));
     EH_CUDA(cudaStreamSynchronize(s));
   };
-  size(CliqueShare{});
+  const bool shared = use == HITS_CLIQUE && ep.shard_count > 1;
+  size(shared ? CliqueShare{ep.shard_index, ep.shard_count} : CliqueShare{});
   if (h[0] > kMaxHitWords || h[1] >= kMaxHitWords) return;
   H.longest = (uint32_t)h[2];
-  if (use == HITS_CLIQUE && ep.shard_count > 1) {
+  if (shared) {
     H.share = CliqueShare{ep.shard_index, ep.shard_count, wide_part(h[3], H.longest, ep.shard_count)};
-    size(H.share);
+    if (H.longest >= H.share.wide) size(H.share);  // once more with the wide ones
   }
   exclusive_scan<uint32_t>(H.moff(), H.moff(), heads, nullptr, s);
   exclusive_scan<uint32_t>(H.upre(), H.upre(), heads + 1, nullptr, s);
   H.launches += scan_launches(heads) + scan_launches(heads + 1);
   try {
-    H.mask.alloc(h[0] ? h[0] : 1, s);
+    H.mask.alloc(h[4] ? h[4] : 1, s);
   } catch (const Error& e) {
     if (e.code != EH_ERR_OOM) throw;
     return;
   }
-  H.words = h[0];
-  H.units = (uint32_t)h[1];
+  H.words = h[4];
+  H.units = (uint32_t)h[5];
   H.on = true;
 }
 
@@ -2239,7 +2252,8 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   }
   const uint64_t units = P.cap_b + (P.cap_w + ep.warps - 1) / ep.warps;
   P.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * per_sm, units));
-  if (annot && !hits && n == 1 && tries[0]->dir == DIR_SYM) P.plan_launches += hot_sets(ctx, tries[0], P.hot);
+  if (P.entries && annot && !hits && n == 1 && tries[0]->dir == DIR_SYM)
+    P.plan_launches += hot_sets(ctx, tries[0], P.hot);
   if (query == EH_QUERY_CLIQUE4 && !hits && ep.s_cap) {
     // one S buffer per resident warp, at most 2 GiB in all
     const uint64_t per_block = (uint64_t)ep.warps * ep.s_cap * 4;
