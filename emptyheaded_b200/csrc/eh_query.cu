@@ -1946,13 +1946,6 @@ struct Hits {
 // than its trie (R-MAT-22: 1.2 GB); past this many words (8 GB: a set of 300 K
 // elements read whole) the plans run without them.
 constexpr uint64_t kMaxHitWords = 1ull << 31;
-// A 4-clique of few rows with small sets runs without: its pairs are few too, and the
-// mask plan (sizes, two scans, clearing, two passes) would be most of it.  Sets of at
-// most 32, us without masks / with: K_24 74 / 115, 64 of them in a batch 58 / 71;
-// Erdos-Renyi of 4096 nodes and degree 8, 74 / 139, 3 in a batch 46 / 58; 64 of 1024
-// nodes (200 K rows) 83 / 58.  Above: K_48 156 / 131, in a batch 132 / 70.
-constexpr uint64_t kFewRows = 65536;
-constexpr uint32_t kSmallSet = 32;
 
 // parts from this length on have more than a count-th of all the 4-clique's work
 static uint32_t wide_part(uint64_t work, uint32_t longest, uint32_t count) {
@@ -1966,24 +1959,22 @@ static uint32_t wide_part(uint64_t work, uint32_t longest, uint32_t count) {
 
 // Sizes and allocates the masks.  H.on: they are there.  H.share: how ranks share
 // a 4-clique of this relation, with its masks or (no memory for them) without; of
-// one rank if the relation is general, its masks are too large for any, or it has
-// no or few rows: all facts of the relation, the same on every rank.
+// one rank if the relation is general, its masks are too large for any, or no row
+// has candidates: all facts of the relation, the same on every rank.
 static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int use, const ExecParams& ep,
                       Hits& H) {
   cudaStream_t s = ctx->stream;
   uint64_t heads = 0, entries = 0;
-  uint32_t max_set = 0;
   std::vector<uint32_t> gstart(n + 1, 0);
   for (uint32_t g = 0; g < n; g++) {
     const int dir = tries[g]->dir;
     if (dir == DIR_GENERAL || (use == HITS_ANNOT && dir != DIR_SYM) || (use == HITS_ROWS && dir == DIR_SYM)) return;
     heads += tries[g]->n_head;
     entries += tries[g]->rev_entries;
-    max_set = std::max(max_set, tries[g]->info.max_set);
     if (heads >= (1ull << 32) - 1) return;
     gstart[g + 1] = (uint32_t)heads;
   }
-  if (!entries || (use == HITS_CLIQUE && entries <= kFewRows && max_set <= kSmallSet)) return;
+  if (!entries) return;
   H.use = use;
   H.n = n;
   H.heads = (uint32_t)heads;
@@ -2281,7 +2272,8 @@ static uint32_t launch(eh_context* ctx, Prepared& P, unsigned long long* d_total
     EH_CHECK_LAUNCH();
     uint32_t launches = 1;
     if (H.use == HITS_CLIQUE) {
-      clique_small_kernel<<<std::min(num_sms() * 8, ceil_div(H.heads, 256)), 256, 0, s>>>(P.dv, hv, d_total);
+      const uint32_t most = num_sms() * 8, span = std::min(32u, std::max(1u, H.heads / (8 * most)));
+      clique_small_kernel<<<std::min<int>(most, ceil_div(H.heads, 8 * span)), 256, 0, s>>>(P.dv, hv, span, d_total);
       EH_CHECK_LAUNCH();
       launches++;
       if (H.units) {

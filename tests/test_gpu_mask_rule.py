@@ -1,7 +1,7 @@
 """Which relations run on hit masks.  Without rows that have candidates nothing but
-the plan's bookkeeping runs; a 4-clique of few rows with small sets runs without
-masks, and gives the same counts on both sides of the rule's lines (sets of 32 and
-33 elements, 65,536 rows), in shares and batches; against the oracle, exact."""
+the plan's bookkeeping runs.  Small neighbourhoods (up to 32 elements: a row per
+lane) around that line, few of them and more than there are warps for one at a
+time, in shares and batches; against the oracle, exact."""
 import numpy as np
 import pytest
 
@@ -55,12 +55,11 @@ def test_small_sets(eh, oracle, kind, n):
 
 
 @pytest.mark.parametrize("kind", ["up", "down", "sym"])
-def test_few_rows(eh, oracle, kind):
-    """Groups of five vertices: 10 rows each, of which 6 have candidates (3 in
-    each of a symmetric relation's directions count once): 10,000 groups are below
-    65,536 such rows, 12,000 above."""
+def test_many_small_neighbourhoods(eh, oracle, kind):
+    """Groups of five vertices, a 4-clique's neighbourhoods among them: up to 4,
+    and more than 8 head entries for each warp of the device."""
     a, b = np.triu_indices(5, 1)
-    for groups in (10_000, 12_000):
+    for groups in (1, 3, 2_000, 40_000):
         base = 5 * np.arange(groups)[:, None]
         u, v = (base + a).ravel().astype(np.uint32), (base + b).ravel().astype(np.uint32)
         u, v = _orient(u, v, kind)
