@@ -1946,6 +1946,13 @@ struct Hits {
 // than its trie (R-MAT-22: 1.2 GB); past this many words (8 GB: a set of 300 K
 // elements read whole) the plans run without them.
 constexpr uint64_t kMaxHitWords = 1ull << 31;
+// Every rank that shares a 4-clique makes the masks of the widest parts (CliqueShare).
+// Where the widest is so wide that the relation's rows can fill no more than a
+// kSparseHub-th of its matrix, making it is nearly all of the query, and the plan
+// without masks splits better (slowest of 8 shares, without / with, ms: star of 2^16
+// leaves with 2^18 rows among them, filled to a 6500th at most, 1.3 / 3.4; of 2^13,
+// an 800th, 0.23 / 0.27; R-MAT-16 by its own ids, a 50th, 134 / 7.6).
+constexpr double kSparseHub = 1024;
 
 // parts from this length on have more than a count-th of all the 4-clique's work
 static uint32_t wide_part(uint64_t work, uint32_t longest, uint32_t count) {
@@ -1959,18 +1966,20 @@ static uint32_t wide_part(uint64_t work, uint32_t longest, uint32_t count) {
 
 // Sizes and allocates the masks.  H.on: they are there.  H.share: how ranks share
 // a 4-clique of this relation, with its masks or (no memory for them) without; of
-// one rank if the relation is general, its masks are too large for any, or no row
-// has candidates: all facts of the relation, the same on every rank.
+// one rank (they share by items) if the relation is general, its masks are too large
+// for any or not worth it for ranks, or no row has candidates: all facts of the
+// relation, the same on every rank.
 static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int use, const ExecParams& ep,
                       Hits& H) {
   cudaStream_t s = ctx->stream;
-  uint64_t heads = 0, entries = 0;
+  uint64_t heads = 0, entries = 0, rows = 0;
   std::vector<uint32_t> gstart(n + 1, 0);
   for (uint32_t g = 0; g < n; g++) {
     const int dir = tries[g]->dir;
     if (dir == DIR_GENERAL || (use == HITS_ANNOT && dir != DIR_SYM) || (use == HITS_ROWS && dir == DIR_SYM)) return;
     heads += tries[g]->n_head;
     entries += tries[g]->rev_entries;
+    rows += tries[g]->rows;
     if (heads >= (1ull << 32) - 1) return;
     gstart[g + 1] = (uint32_t)heads;
   }
@@ -2004,6 +2013,7 @@ static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
   size(shared ? CliqueShare{ep.shard_index, ep.shard_count} : CliqueShare{});
   if (h[0] > kMaxHitWords || h[1] >= kMaxHitWords) return;
   H.longest = (uint32_t)h[2];
+  if (shared && 0.5 * H.longest * H.longest > kSparseHub * rows) return;
   if (shared) {
     H.share = CliqueShare{ep.shard_index, ep.shard_count, wide_part(h[3], H.longest, ep.shard_count)};
     if (H.longest >= H.share.wide) size(H.share);  // once more with the wide ones

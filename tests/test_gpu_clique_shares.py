@@ -9,14 +9,15 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _hub(d, extra, core, kind="up", seed=3):
-    """Vertex 0 next to 1..d; `extra` random edges among those, and a clique of `core`."""
+def _hub(d, extra, core, kind="up", seed=3, hubs=1):
+    """`hubs` vertices, each next to d others; `extra` random edges among those, and
+    a clique of `core`."""
     rng = np.random.default_rng(seed)
-    a, b = rng.integers(1, d + 1, extra), rng.integers(1, d + 1, extra)
+    a, b = rng.integers(0, d, extra) + hubs, rng.integers(0, d, extra) + hubs
     ca, cb = np.triu_indices(core, 1)
-    ids = np.sort(rng.choice(np.arange(1, d + 1), core, replace=False))
-    u = np.concatenate([np.zeros(d, np.int64), np.minimum(a, b), ids[ca]])
-    v = np.concatenate([np.arange(1, d + 1), np.maximum(a, b), ids[cb]])
+    ids = np.sort(rng.choice(np.arange(hubs, d + hubs), core, replace=False))
+    u = np.concatenate([np.repeat(np.arange(hubs), d), np.minimum(a, b), ids[ca]])
+    v = np.concatenate([np.tile(np.arange(hubs, d + hubs), hubs), np.maximum(a, b), ids[cb]])
     keep = u != v
     u, v = u[keep].astype(np.uint32), v[keep].astype(np.uint32)
     if kind == "down":
@@ -46,9 +47,9 @@ class _FillTo:
 
 @pytest.mark.parametrize("kind", ["up", "down", "sym"])
 def test_a_rank_without_memory_counts_the_same_share(eh, ctx, oracle, kind):
-    # masks of 300,000^2 / 64 words are 5.6 GB; the plan without them takes
-    # 2 GiB of buffers at most
-    u, v = _hub(300_000, 20_000, 60, kind)
+    # masks of 56 * 40,000^2 / 64 words are 5.6 GB, on a rank of three a third of
+    # the hubs' ones 1.9; the plan without them takes 0.9 GB
+    u, v = _hub(40_000, 20_000, 60, kind, hubs=56)
     t = eh.Trie(u, v, ctx=ctx)
     want = oracle.Trie(u, v).clique4()
     assert want >= 60 * 59 * 58 * 57 // 24
@@ -56,7 +57,7 @@ def test_a_rank_without_memory_counts_the_same_share(eh, ctx, oracle, kind):
     shares = [t.count("clique4", shard=(r, 3)) for r in range(3)]
     assert sum(shares) == want
     for r in range(3):
-        with _FillTo(ctx, 4 << 30):
+        with _FillTo(ctx, 1500 << 20):
             assert t.count("clique4", shard=(r, 3)) == shares[r], r
     t.free()
 
@@ -69,6 +70,31 @@ def test_shares_of_a_hub(eh, oracle, kind, d, extra, core):
     want = oracle.Trie(u, v).clique4()
     for world in (2, 3, 8, 37):
         assert sum(t.count("clique4", shard=(r, world)) for r in range(world)) == want, world
+    t.free()
+
+
+@pytest.mark.parametrize("kind", ["up", "down", "sym"])
+@pytest.mark.parametrize("rows", [-40, 0, 40])
+def test_shares_at_the_hub_rule(eh, oracle, kind, rows):
+    """A part of d elements around the line where the rows fill a 1024th of its matrix."""
+    d = 4400
+    u, v = _hub(d, 4950 + rows, 30, kind)
+    t = eh.Trie(u, v)
+    want = oracle.Trie(u, v).clique4()
+    for world in (2, 5):
+        assert sum(t.count("clique4", shard=(r, world)) for r in range(world)) == want, world
+    t.free()
+
+
+def test_shares_of_a_star_are_even(eh):
+    """2^16 vertices next to vertex 0 and few rows among them: no rank takes over
+    half as long as the whole."""
+    t = eh.Trie(*_hub(1 << 16, 1 << 18, 4))
+
+    def ms(**kw):
+        return min(t.count("clique4", stats=True, **kw)[1]["kernel_ms"] for _ in range(4))
+
+    assert max(ms(shard=(r, 8)) for r in range(8)) < 0.5 * ms()
     t.free()
 
 
