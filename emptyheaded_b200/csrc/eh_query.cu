@@ -108,6 +108,8 @@ struct ExecParams {
   bool smem_given; // the caller chose smem_words
   bool chunk_given;  // the caller chose chunk
   bool no_block_items;  // stage every N(b) per warp (no block items)
+  bool masks = true;      // hit masks may be made
+  bool* held = nullptr;   // set once they are
 };
 
 static ExecParams exec_params(const eh_exec_config* cfg) {
@@ -2018,6 +2020,7 @@ static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
     H.share = CliqueShare{ep.shard_index, ep.shard_count, wide_part(h[3], H.longest, ep.shard_count)};
     if (H.longest >= H.share.wide) size(H.share);  // once more with the wide ones
   }
+  if (!ep.masks) return;
   exclusive_scan<uint32_t>(H.moff(), H.moff(), heads, nullptr, s);
   exclusive_scan<uint32_t>(H.upre(), H.upre(), heads + 1, nullptr, s);
   H.launches += scan_launches(heads) + scan_launches(heads + 1);
@@ -2030,6 +2033,25 @@ static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
   H.words = h[4];
   H.units = (uint32_t)h[5];
   H.on = true;
+  if (ep.held) *ep.held = true;
+}
+
+// Masks are up to 8 GB.  A call that has them and then finds no memory for the rest
+// of what it needs (a fine plan, materialized rows) gives them back and runs once
+// more without: f(ExecParams) is the whole call, and holds its memory itself.
+template <typename F>
+static void with_or_without_masks(eh_context* ctx, ExecParams ep, F f) {
+  bool held = false;
+  ep.held = &held;
+  try {
+    f(ep);
+    return;
+  } catch (const Error& e) {
+    if (e.code != EH_ERR_OOM || !held) throw;
+  }
+  EH_CUDA(cudaStreamSynchronize(ctx->stream));  // the first try's work; pinned memory is written again
+  ep.masks = false;
+  f(ep);
 }
 
 // Runs the intersection kernel of `query` over the concatenated plans of
@@ -2262,6 +2284,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     P.gs.alloc((size_t)P.grid * ep.warps * ep.s_cap, s);
   }
   P.ep = ep;
+  P.ep.held = nullptr;
 }
 
 // Enqueue one run of a prepared launch; the first follows prepare directly, a
@@ -2503,23 +2526,12 @@ static unsigned long long* annot_buffer(eh_context* ctx, size_t n) {
   return ctx->annot;
 }
 
-void query_count_batched(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query,
-                         const eh_exec_config* cfg, uint64_t* results, eh_query_stats* stats) {
+static void run_count(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query, bool record, ExecParams ep,
+                      uint64_t* results, eh_query_stats* stats) {
   cudaStream_t s = ctx->stream;
-  EH_REQUIRE(query >= EH_QUERY_TRIANGLE && query <= EH_QUERY_BARBELL, EH_ERR_INVALID, "unknown query");
-  EH_REQUIRE(n > 0, EH_ERR_INVALID, "no tries");
-  for (uint32_t g = 0; g < n; g++) {
-    EH_REQUIRE(tries[g] != nullptr, EH_ERR_INVALID, "null trie");
-    EH_REQUIRE(tries[g]->ctx == ctx, EH_ERR_INVALID, "trie belongs to another context");
-  }
-  ExecParams ep = exec_params(cfg);
-  Call call(ctx);
-  TracePhase ph_all("query.total", s);
-  EH_CUDA(cudaEventRecord(ctx->ev0, s));
   Prepared P;
   Launch L;
   DevBuf<float> rec;
-  const bool record = cfg && cfg->record_timings && n == 1;
   if (record) {
     // one record per item; the plan size is known only after planning, so
     // size for the worst case, as prepare does for the items; fixed chunks
@@ -2561,6 +2573,22 @@ void query_count_batched(eh_context* ctx, const eh_trie* const* tries, uint32_t 
   fill_stats(stats, got.query_ms, got.kernel_ms, L.launches, got.items, P.pairs, alg);
 }
 
+void query_count_batched(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query,
+                         const eh_exec_config* cfg, uint64_t* results, eh_query_stats* stats) {
+  EH_REQUIRE(query >= EH_QUERY_TRIANGLE && query <= EH_QUERY_BARBELL, EH_ERR_INVALID, "unknown query");
+  EH_REQUIRE(n > 0, EH_ERR_INVALID, "no tries");
+  for (uint32_t g = 0; g < n; g++) {
+    EH_REQUIRE(tries[g] != nullptr, EH_ERR_INVALID, "null trie");
+    EH_REQUIRE(tries[g]->ctx == ctx, EH_ERR_INVALID, "trie belongs to another context");
+  }
+  const ExecParams ep = exec_params(cfg);
+  const bool record = cfg && cfg->record_timings && n == 1;
+  Call call(ctx);
+  TracePhase ph_all("query.total", ctx->stream);
+  EH_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
+  with_or_without_masks(ctx, ep, [&](const ExecParams& p) { run_count(ctx, tries, n, query, record, p, results, stats); });
+}
+
 void query_count(eh_context* ctx, const eh_trie* t, int query, const eh_exec_config* cfg, uint64_t* result,
                  eh_query_stats* stats) {
   const eh_trie* ts[1] = {t};
@@ -2573,12 +2601,14 @@ void triangle_annotation(eh_context* ctx, const eh_trie* t, const eh_exec_config
   ep.shard_index = 0;
   ep.shard_count = 1;
   Call call(ctx);
-  EH_CUDA(cudaMemsetAsync(annot_dev, 0, (t->n_head ? t->n_head : 1) * 8, s));
   const eh_trie* ts[1] = {t};
-  Prepared P;
-  run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, true, P, nullptr, (unsigned long long*)annot_dev, nullptr, nullptr,
-            true);
-  EH_CUDA(cudaStreamSynchronize(s));
+  with_or_without_masks(ctx, ep, [&](const ExecParams& p) {
+    EH_CUDA(cudaMemsetAsync(annot_dev, 0, (t->n_head ? t->n_head : 1) * 8, s));
+    Prepared P;
+    run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, p, true, P, nullptr, (unsigned long long*)annot_dev, nullptr, nullptr,
+              true);
+    EH_CUDA(cudaStreamSynchronize(s));
+  });
 }
 
 // ------------------------------------------------------------ selections
@@ -2692,18 +2722,20 @@ void query_count_select(eh_context* ctx, const eh_trie* t, int query, uint32_t v
       if (t->dir == DIR_SYM) v *= 6ull;  // 3! orderings start at each selected member
     } else if (hv >= 0) {
       DevBuf<unsigned long long> T(t->n_head, s);
-      EH_CUDA(cudaMemsetAsync(T.p, 0, (size_t)t->n_head * 8, s));
-      EH_CUDA(cudaMemsetAsync(sums.p, 0, 32, s));
-      Prepared P;
-      const Launch K = run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, true, P, nullptr, T.p, nullptr, nullptr, true);
-      select_partners_kernel<<<sgrid, 256, 0, s>>>(t->view(), value, nullptr, T.p, sums.p);
-      EH_CHECK_LAUNCH();
-      L.launches += K.launches + 1;
-      EH_CUDA(cudaMemcpyAsync(h, sums.p, 32, cudaMemcpyDeviceToHost, s));
-      const Returned got = finish(ctx, P);
-      items = got.items;
-      pairs = P.pairs;
-      kernel_ms = got.kernel_ms;
+      with_or_without_masks(ctx, ep, [&](const ExecParams& p) {
+        EH_CUDA(cudaMemsetAsync(T.p, 0, (size_t)t->n_head * 8, s));
+        EH_CUDA(cudaMemsetAsync(sums.p, 0, 32, s));
+        Prepared P;
+        const Launch K = run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, p, true, P, nullptr, T.p, nullptr, nullptr, true);
+        select_partners_kernel<<<sgrid, 256, 0, s>>>(t->view(), value, nullptr, T.p, sums.p);
+        EH_CHECK_LAUNCH();
+        L.launches += K.launches + 1;
+        EH_CUDA(cudaMemcpyAsync(h, sums.p, 32, cudaMemcpyDeviceToHost, s));
+        const Returned got = finish(ctx, P);
+        items = got.items;
+        pairs = P.pairs;
+        kernel_ms = got.kernel_ms;
+      });
       v = (uint64_t)h[0] * (uint64_t)h[1];
     }
   }
@@ -2822,12 +2854,9 @@ struct HostRows {
 // Oriented relations: the hit masks hold every triangle at its place in the
 // order (a, b, c), so the rows are counted per relation row, placed by a scan
 // and written in order; nothing is sorted.  false: no masks for this relation.
-static bool materialize_hits(eh_context* ctx, const eh_trie* t, const eh_exec_config* cfg, const HostRows& host,
+static bool materialize_hits(eh_context* ctx, const eh_trie* t, const ExecParams& ep, const HostRows& host,
                              uint64_t cap, uint64_t* n_rows) {
   cudaStream_t s = ctx->stream;
-  ExecParams ep = exec_params(cfg);
-  ep.shard_index = 0;
-  ep.shard_count = 1;
   Prepared P;
   const eh_trie* ts[1] = {t};
   prepare(ctx, ts, 1, EH_QUERY_TRIANGLE, ep, false, P, false, HITS_ROWS);
@@ -2870,7 +2899,16 @@ void query_materialize(eh_context* ctx, const eh_trie* t, int query, const eh_ex
     return;
   }
   const HostRows host{ha, hb, hc, rows_out};
-  if (host.given() && t->dir != DIR_SYM && materialize_hits(ctx, t, cfg, host, cap, n_rows)) return;
+  if (host.given() && t->dir != DIR_SYM) {
+    ExecParams ep = exec_params(cfg);
+    ep.shard_index = 0;
+    ep.shard_count = 1;
+    bool done = false;
+    with_or_without_masks(ctx, ep, [&](const ExecParams& p) {
+      done = p.masks && materialize_hits(ctx, t, p, host, cap, n_rows);
+    });
+    if (done) return;
+  }
   uint64_t n = 0;
   query_count(ctx, t, EH_QUERY_TRIANGLE, cfg, &n, nullptr);
   *n_rows = n;
@@ -3064,16 +3102,9 @@ struct eh_batch {
 
 namespace eh {
 
-eh_batch* batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query,
-                       const eh_exec_config* cfg) {
+static eh_batch* make_batch(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query,
+                            const ExecParams& ep) {
   cudaStream_t s = ctx->stream;
-  EH_REQUIRE(n > 0, EH_ERR_INVALID, "no tries");
-  EH_REQUIRE(query == EH_QUERY_TRIANGLE || query == EH_QUERY_CLIQUE4, EH_ERR_UNSUPPORTED,
-             "batches run the triangle or 4-clique plan");
-  ExecParams ep = exec_params(cfg);
-  for (uint32_t g = 0; g < n; g++)
-    EH_REQUIRE(tries[g] && tries[g]->ctx == ctx, EH_ERR_INVALID, "null trie or trie of another context");
-  Call call(ctx);
   auto* b = new eh_batch();
   try {
     b->ctx = ctx;
@@ -3105,6 +3136,20 @@ eh_batch* batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n,
     delete b;
     throw;
   }
+  return b;
+}
+
+eh_batch* batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query,
+                       const eh_exec_config* cfg) {
+  EH_REQUIRE(n > 0, EH_ERR_INVALID, "no tries");
+  EH_REQUIRE(query == EH_QUERY_TRIANGLE || query == EH_QUERY_CLIQUE4, EH_ERR_UNSUPPORTED,
+             "batches run the triangle or 4-clique plan");
+  const ExecParams ep = exec_params(cfg);
+  for (uint32_t g = 0; g < n; g++)
+    EH_REQUIRE(tries[g] && tries[g]->ctx == ctx, EH_ERR_INVALID, "null trie or trie of another context");
+  Call call(ctx);
+  eh_batch* b = nullptr;
+  with_or_without_masks(ctx, ep, [&](const ExecParams& p) { b = make_batch(ctx, tries, n, query, p); });
   return b;
 }
 

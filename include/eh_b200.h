@@ -266,7 +266,11 @@ typedef struct {
  * loop nest (storage_engine/include/TrieBuilder.hpp:117-165,
  * storage_engine/src/TrieBuilder.cpp:451-578) and par::reducer
  * (storage_engine/include/utils/parallel.hpp:8-34).  The result is the
- * count modulo 2^64 (the reference's signed long, bit for bit). */
+ * count modulo 2^64 (the reference's signed long, bit for bit).
+ * The 4-clique of an up, down or symmetric relation, the lollipop, barbell and
+ * annotation of a symmetric one and the triangles of an up or down one keep a bit
+ * per candidate while they run: 8 GB at most, and where there is no memory for
+ * that, or not for the rest of the call beside it, they run without. */
 eh_status eh_query_count(eh_context* ctx, const eh_trie* trie, int query, const eh_exec_config* cfg,
                          uint64_t* result, eh_query_stats* stats);
 
@@ -365,7 +369,8 @@ eh_status eh_query_count_batched(eh_context* ctx, const eh_trie* const* tries, u
  * concatenated once into one queue, and the step (zero the results and the
  * queue, the persistent kernel over every trie's items, the results to
  * host) captured in a CUDA graph.  eh_batch_run replays the graph: one
- * launch for the whole batch.  Same results as eh_query_count per trie.
+ * launch for the whole batch.  Same results as eh_query_count per trie.  A
+ * 4-clique's bits (eh_query_count) stay allocated as long as the batch.
  * The tries must outlive the batch and not be re-laid-out while it exists. */
 typedef struct eh_batch eh_batch;
 eh_status eh_batch_create(eh_context* ctx, const eh_trie* const* tries, uint32_t n_tries, int query,
