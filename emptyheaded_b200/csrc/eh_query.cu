@@ -933,11 +933,13 @@ __device__ __forceinline__ bool hit(const Staged& st, uint32_t w) {
 }
 
 // stream_rows for the plain COUNT.  A batch of 32 rows, a row per lane; each
-// row is counted in one of four ways:
+// row is counted in one of five ways:
 //   word trips     both sets are range bitsets and their common words are fewer
 //                  than the candidates (weighted as in stream_rows), at least
 //                  kTripWords of them: 32 words per trip
 //   word pairs     fewer words: flattened (row, word) pairs over the lanes
+//   wide rows      at least kWideRow candidates: the warp runs along the row, no trip
+//                  to be looked up
 //   element trips  at least long_row candidates: 32 candidates per trip
 //   element pairs  fewer: flattened (row, candidate) pairs over the lanes
 // The trips of all rows of a batch form one list, taken kTrips at a time with
@@ -951,9 +953,13 @@ __device__ __forceinline__ bool hit(const Staged& st, uint32_t w) {
 // trips of four 8.10 / 1.21; views as kernel parameters and the next batch's
 // rows loaded ahead 7.76 / 1.14; element trips by eight 7.18 / 1.13 (by six
 // 7.29, word trips by three 7.40, by six 7.39).  48 registers and five blocks per
-// SM 7.84, 80 and three 9.41.
+// SM 7.84, 80 and three 9.41.  Wide rows apart from 128 / 256 / 512 / 1024 candidates
+// or never: R-MAT-22 6.95 / 6.59 / 6.67 / 6.67 / 6.67, Chung-Lu 2^18 by descending
+// degree 5.35 / 5.36 / 5.43 / 5.57 / 7.85, Chung-Lu 2^21 1.66 / 1.65 / 1.70 / 1.70 /
+// 1.70 (a trip costs a ballot and two shuffles per 32 candidates: a star's rows ran
+// at 2.35 instead of 1.23).
 constexpr int kTrips = 8, kWTrips = 4;
-constexpr uint32_t kTripWords = 16;
+constexpr uint32_t kTripWords = 16, kWideRow = 256;
 template <int P>
 __device__ __forceinline__ uint64_t count_rows(const Staged& st, const TrieView& t, const RevView& r, uint32_t kb,
                                                uint32_t ke, uint32_t long_row) {
@@ -1037,6 +1043,21 @@ __device__ __forceinline__ uint64_t count_rows(const Staged& st, const TrieView&
         }
         cnt += __popcll(x[0] & y[0]) + __popcll(x[1] & y[1]);
       }
+    }
+    for (uint32_t rows = __ballot_sync(kFull, len >= kWideRow); rows; rows &= rows - 1) {
+      const int j = __ffs(rows) - 1;
+      const uint32_t* row = t.vals + __shfl_sync(kFull, lo, j);
+      const uint32_t n = __shfl_sync(kFull, len, j);
+      uint32_t i = lane;
+      for (; i + 32 * (kTrips - 1) < n; i += 32 * kTrips) {
+        uint32_t v[kTrips];
+#pragma unroll
+        for (int u = 0; u < kTrips; u++) v[u] = __ldg(row + (i + 32 * u));
+#pragma unroll
+        for (int u = 0; u < kTrips; u++) cnt += hit<P>(st, v[u]);
+      }
+      for (; i < n; i += 32) cnt += hit<P>(st, __ldg(row + i));
+      if (lane == j) len = 0;
     }
     {
       const uint32_t nt = len >= long_row ? (len + 31) >> 5 : 0;
