@@ -2207,7 +2207,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   const bool blocks = block_items && !hits && query == EH_QUERY_TRIANGLE && !annot && ep.warps > 1 &&
                       !ep.no_block_items;
   // work of all tries, and how finely to cut it: 8 items for each resident
-  // warp (of every rank), of kMinChunk to kMaxChunk
+  // warp (of every rank), of kMinChunk to kMaxChunk at most
   uint64_t cost = 0, head_items = 0;
   P.n = n;
   for (uint32_t g = 0; g < n; g++) {
@@ -2220,7 +2220,10 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   const uint64_t resident = (uint64_t)num_sms() * per_sm * ep.warps;
   const uint64_t slots = ep.shard_count > 1 ? (uint64_t)kShareWarps * ep.shard_count : resident;
   if (!ep.chunk_given) {
-    ep.chunk = (uint32_t)std::min<uint64_t>(kMaxChunk, std::max<uint64_t>(kMinChunk, cost / (8 * slots)));
+    // a 4-clique without masks does far more per row than the plan weighs (selection
+    // on R-MAT-18 going down by degree 548 ms; cut up to kMaxChunk 902)
+    const uint64_t most = query == EH_QUERY_CLIQUE4 && !hits ? kDefaultChunk : kMaxChunk;
+    ep.chunk = (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(kMinChunk, cost / (8 * slots)));
   }
   PlanShape shape{ep.chunk, nullptr, 0.0, (uint32_t)ep.smem_words,
                    blocks ? (uint32_t)ep.smem_words * (uint32_t)ep.warps : 0u, (uint32_t)ep.warps, 0u};
