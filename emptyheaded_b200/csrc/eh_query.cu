@@ -1246,8 +1246,7 @@ __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_
   // shared atomics, ranks by a warp scan, each element's bit OR-ed into its
   // non-zero word) when that fits: two shared loads per probe in place of a
   // ~8-step binary search (R-MAT-22, density rule: 49.8 -> 28.7 warp-cycles
-  // per probe including the build, kernel 9.91 -> 8.19 ms).  The annotated
-  // pass keeps the list: its per-element counters are indexed by position in it.
+  // per probe including the build, kernel 9.91 -> 8.19 ms).
   if (zlist && len >= 2) {
     const uint32_t first = __ldg(t.vals + s0), last = __ldg(t.vals + s0 + len - 1);
     const uint32_t W = (last >> 6) - (first >> 6) + 1;
@@ -1529,7 +1528,12 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ Tri
       mode = stage_set_block(t, item.hb, smem, cap_words * (int)nwarps, st);
       __syncthreads();
     } else {
-      mode = stage_set(t, item.hb, sm, cap_words, st, kMode == MODE_COUNT && !few_candidates(r, item));
+      // bitmaps for the annotation of an ordered or general relation too (kernel ms, star
+      // of 2^16 leaves 5.4 -> 3.3, R-MAT-18 going down by degree 15.2 -> 7.0, R-MAT-20
+      // 2.45 -> 1.87); a symmetric one's per-element counters are indexed by position in
+      // the list
+      const bool bitmap = kMode == MODE_COUNT || (kMode == MODE_ANNOT && r.dir != DIR_SYM);
+      mode = stage_set(t, item.hb, sm, cap_words, st, bitmap && !few_candidates(r, item));
     }
     const StagedRange sr = kMode == MODE_ANNOT ? staged_range(t, item.hb) : StagedRange{0, 0};
     const uint32_t blen = sr.len;
@@ -2177,10 +2181,12 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     size_clique_staging(ep, mx);
   }
   // the launch shape first: the plan's classes depend on the staging capacity
-  // the annotated pass stages more of N(b) by default: its matched elements
-  // then count in shared memory (measured on Chung-Lu 2^23: 2048 words per
-  // warp 234 ms, 1024 245 ms)
-  if (annot && !hits && !ep.smem_given) ep.smem_words = 2048;
+  // the annotated pass of a symmetric relation stages more of N(b) by default: its
+  // matched elements then count in shared memory (measured on Chung-Lu 2^23: 2048
+  // words per warp 234 ms, 1024 245 ms)
+  bool sym = false;
+  for (uint32_t g = 0; g < n; g++) sym |= tries[g]->dir == DIR_SYM;
+  if (annot && sym && !hits && !ep.smem_given) ep.smem_words = 2048;
   P.threads = 32 * ep.warps;
   P.smem = (size_t)ep.smem_words * 4 * ep.warps;
   const void* kfn;
