@@ -593,91 +593,113 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x) {
 // a few L2 lines.  The last kHubs entries count in shared memory and are added
 // to T once per block.
 constexpr uint32_t kHubs = 4096;
-// kWide: the units of columns kWideColumn on, each of many tiles: spread over the
-// warps one by one, four tiles' loads in flight (lollipop on a star of 2^17 leaves:
-// 42 ms without, 15); not: the columns before `wide`.  The wide launch looks every
-// unit's entry up, 32 at a time, and pays where a part is longer than kWidePart
-// (launched for every part past column 16, one look-up at a time, the lollipop on
-// Chung-Lu 2^23 took 25.3 ms instead of 17.6).
-constexpr uint32_t kWideColumn = 16, kWidePart = 4096;
+// A unit of a part of W words is a chain of W + 1 loads and some.  kWide: the units of
+// parts of more than kWidePart elements, each shared by up to the eight warps of a
+// block; every unit's entry is looked up, a thread each.  Otherwise the units of the
+// other parts.  (Split by column instead, the row sums of a wide part's first columns
+// stayed on one warp: lollipop on a star of 2^16 leaves with 2^18 rows among them 10.5
+// ms, so 2.9; without masks 6.6.  Kernels, ms, wide from 1024 / 4096 elements: star of
+// 2^12 0.06 / 0.10, R-MAT-16 by its own ids 0.86 / 0.97, Chung-Lu 2^23, where the look-up
+// is paid for little, 16.8 / 16.7, and from 512 17.6.)
+constexpr uint32_t kWidePart = 4096;
+constexpr uint32_t kWideShare = 64;  // words of a part per warp that shares its units
+
+// slice s of S of unit k of entry a's matrix: the column sums of column k's tiles and
+// the row sums of block k's words, added to T and the block's hubs
+template <bool kWide>
+__device__ __forceinline__ void annot_column(const TrieView& t, const HitsView& hv, uint32_t a, uint32_t k,
+                                             uint32_t s, uint32_t S, uint32_t hub0, unsigned int* hub,
+                                             unsigned long long* __restrict__ T) {
+  const uint32_t lane = lane_id();
+  const StagedRange pr = staged_range(t, a);
+  const uint32_t d = pr.len, W = (d + 31) >> 5;
+  const uint32_t* m = hv.mask + __ldg(hv.moff + a);
+  uint32_t col = 0, row = 0;
+  const uint32_t rk = hits_stride(k, W, d);
+  const uint32_t* mk = m + hits_block(k, W) + lane;
+  if (!kWide) {
+    for (uint32_t q = 0; q <= k; q++) {
+      const uint32_t rq = hits_stride(q, W, d);
+      const uint32_t x = lane < rq ? __ldg(m + hits_block(q, W) + (k - q) * rq + lane) : 0u;
+      if (__any_sync(kFull, x != 0)) col += __popc(transpose32(x));
+    }
+    if (lane < rk)
+      for (uint32_t w = k; w < W; w++) row += __popc(__ldg(mk + (w - k) * rk));
+  } else {
+    for (uint32_t q0 = 4 * s; q0 <= k; q0 += 4 * S) {
+      uint32_t x[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const uint32_t q = q0 + i;
+        const uint32_t rq = hits_stride(q, W, d);
+        x[i] = q <= k && lane < rq ? __ldg(m + hits_block(q, W) + (k - q) * rq + lane) : 0u;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (__any_sync(kFull, x[i] != 0)) col += __popc(transpose32(x[i]));
+    }
+    if (lane < rk)
+#pragma unroll 4
+      for (uint32_t w = k + s; w < W; w += S) row += __popc(__ldg(mk + (w - k) * rk));
+  }
+  if (col + row) {  // so the position is below d
+    const uint32_t h = (uint32_t)__ldg(t.head_index + __ldg(t.vals + pr.s0 + 32 * k + lane));
+    const uint32_t v = col + row;
+    if (h < hub0) atomicAdd(T + h, 2ull * v);
+    else if (atomicAdd(hub + (h - hub0), v) > 0xffffffffu - v) atomicAdd(T + h, 2ull << 32);  // wrapped
+  }
+  const uint32_t all = warp_sum(row);
+  if (lane == 0 && all) atomicAdd(T + a, 2ull * all);
+}
+
 template <bool kWide>
 __global__ void __launch_bounds__(256) annot_hits_kernel(TrieView t, HitsView hv, uint32_t n_units,
-                                                         uint32_t wide,
+                                                         uint32_t run,
                                                          unsigned long long* __restrict__ T) {
   __shared__ unsigned int hub[kHubs];
   for (uint32_t i = threadIdx.x; i < kHubs; i += blockDim.x) hub[i] = 0;
   __syncthreads();
   const uint32_t hub0 = t.n_head > kHubs ? t.n_head - kHubs : 0;
-  const uint32_t lane = lane_id();
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  // runs of consecutive units, so that few searches find the head entries,
-  // spread over the warps, so that the long rows of a range of ids are too
-  constexpr uint32_t kRun = 16;
-  uint32_t a = 0;
-  uint32_t la = 0, lk = 0, todo = 0;  // kWide: each lane's unit, and the units still to do
-  for (uint64_t v = 0;;) {
-    uint32_t k;
-    if (kWide) {
-      if (!todo) {
-        const uint64_t base = 32 * v++ * nwarps + warp;
-        if (base >= n_units) break;
-        const uint64_t u = base + (uint64_t)lane * nwarps;
-        if (u < n_units) {
-          la = hits_unit_head(hv, (uint32_t)u);
-          lk = (uint32_t)u - __ldg(hv.upre + la);
+  if (kWide) {
+    __shared__ uint32_t s_a[256], s_k[256];  // the wide units among the block's 256
+    __shared__ unsigned int s_n;
+    const uint32_t wid = threadIdx.x >> 5;
+    for (uint64_t base = 0; base < n_units; base += 256ull * gridDim.x) {  // the same on every thread
+      if (threadIdx.x == 0) s_n = 0;
+      __syncthreads();
+      const uint64_t u = base + (uint64_t)threadIdx.x * gridDim.x + blockIdx.x;
+      if (u < n_units) {
+        const uint32_t a = hits_unit_head(hv, (uint32_t)u), k = (uint32_t)u - __ldg(hv.upre + a);
+        if (staged_range(t, a).len > kWidePart) {
+          const uint32_t i = atomicAdd(&s_n, 1u);
+          s_a[i] = a;
+          s_k[i] = k;
         }
-        todo = __ballot_sync(kFull, u < n_units && lk >= wide);
-        continue;
       }
-      const int j = __ffs(todo) - 1;
-      todo &= todo - 1;
-      a = __shfl_sync(kFull, la, j);
-      k = __shfl_sync(kFull, lk, j);
-    } else {
-      const uint64_t u64 = ((v / kRun) * nwarps + warp) * kRun + v % kRun;
-      if (u64 >= n_units) break;
-      const uint32_t u = (uint32_t)u64;
-      if (v++ % kRun == 0) a = hits_unit_head(hv, u);
-      a = hits_unit_next(hv, a, u);
-      k = u - __ldg(hv.upre + a);
-      if (k >= wide) continue;
+      __syncthreads();
+      const uint32_t n = s_n;
+      for (uint32_t i = 0; i < n; i++) {
+        const uint32_t a = s_a[i];
+        const uint32_t S = min(8u, 1 + (staged_range(t, a).len >> 5) / kWideShare), s = (wid + i) & 7;
+        if (s < S) annot_column<true>(t, hv, a, s_k[i], s, S, hub0, hub, T);
+      }
+      __syncthreads();
     }
-    const StagedRange pr = staged_range(t, a);
-    const uint32_t d = pr.len, W = (d + 31) >> 5;
-    const uint32_t* m = hv.mask + __ldg(hv.moff + a);
-    uint32_t col = 0, row = 0;
-    if (!kWide) {
-      for (uint32_t q = 0; q <= k; q++) {
-        const uint32_t rq = hits_stride(q, W, d);
-        const uint32_t x = lane < rq ? __ldg(m + hits_block(q, W) + (k - q) * rq + lane) : 0u;
-        if (__any_sync(kFull, x != 0)) col += __popc(transpose32(x));
-      }
-    } else {
-      for (uint32_t q0 = 0; q0 <= k; q0 += 4) {
-        uint32_t x[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const uint32_t q = q0 + i;
-          const uint32_t rq = hits_stride(q, W, d);
-          x[i] = q <= k && lane < rq ? __ldg(m + hits_block(q, W) + (k - q) * rq + lane) : 0u;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-          if (__any_sync(kFull, x[i] != 0)) col += __popc(transpose32(x[i]));
+  } else {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    // runs of consecutive units, so that few searches find the head entries,
+    // spread over the warps, so that the long rows of a range of ids are too
+    uint32_t a = 0;
+    for (uint64_t u0 = (uint64_t)warp * run; u0 < n_units; u0 += (uint64_t)nwarps * run) {
+      const uint32_t u1 = (uint32_t)min(u0 + run, (uint64_t)n_units);
+      a = hits_unit_head(hv, (uint32_t)u0);
+      for (uint32_t u = (uint32_t)u0; u < u1; u++) {
+        a = hits_unit_next(hv, a, u);
+        if (staged_range(t, a).len <= kWidePart)
+          annot_column<false>(t, hv, a, u - __ldg(hv.upre + a), 0, 1, hub0, hub, T);
       }
     }
-    const uint32_t rk = hits_stride(k, W, d);
-    if (lane < rk)
-      for (uint32_t w = k; w < W; w++) row += __popc(__ldg(m + hits_block(k, W) + (w - k) * rk + lane));
-    if (col + row) {  // so the position is below d
-      const uint32_t h = (uint32_t)__ldg(t.head_index + __ldg(t.vals + pr.s0 + 32 * k + lane));
-      const uint32_t v = col + row;
-      if (h < hub0) atomicAdd(T + h, 2ull * v);
-      else if (atomicAdd(hub + (h - hub0), v) > 0xffffffffu - v) atomicAdd(T + h, 2ull << 32);  // wrapped
-    }
-    const uint32_t all = warp_sum(row);
-    if (lane == 0 && all) atomicAdd(T + a, 2ull * all);
   }
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < kHubs; i += blockDim.x)

@@ -2357,10 +2357,9 @@ static uint32_t launch(eh_context* ctx, Prepared& P, unsigned long long* d_total
       }
     } else if (H.use == HITS_ANNOT && H.units) {
       const bool wide_parts = H.longest > kWidePart;
-      const uint32_t wide = wide_parts ? kWideColumn : ~0u;
-      annot_hits_kernel<false><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, wide, d_annot);
-      if (wide_parts)
-        annot_hits_kernel<true><<<num_sms() * 8, 256, 0, s>>>(P.view0, hv, H.units, wide, d_annot);
+      const uint32_t blocks = num_sms() * 8, run = std::min(16u, std::max(1u, H.units / (8 * blocks)));
+      annot_hits_kernel<false><<<blocks, 256, 0, s>>>(P.view0, hv, H.units, run, d_annot);
+      if (wide_parts) annot_hits_kernel<true><<<blocks, 256, 0, s>>>(P.view0, hv, H.units, run, d_annot);
       EH_CHECK_LAUNCH();
       launches += wide_parts ? 2 : 1;
     }
