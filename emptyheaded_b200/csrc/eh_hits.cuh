@@ -464,20 +464,28 @@ __device__ __noinline__ bool sparse_rows(const uint32_t* rows, uint32_t ri, uint
 // i whose bit j is set.  Row j's word is one line per warp and serves all eight
 // rows, whose own words are two 16-byte loads, the same for all lanes; that
 // leaves AND, popcount and add per (i, j word) and makes the popcounts (16
-// lanes per clock) the bound.  A warp takes the four units of one row block in
-// a row: its L1 then holds the matrix.
-__global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restrict__ views, HitsView hv,
-                                                         uint32_t n_units, unsigned int* __restrict__ queue,
+// lanes per clock) the bound.  A warp takes `grab` units in a row, the four of one
+// row block where there are units enough: its L1 then holds the matrix.  Where there
+// are fewer than warps, `slices` warps share a unit, each every so many of its blocks
+// q (all four units of a block on one warp always, kernels, ms: star of 2^11 leaves
+// 0.54, so 0.075, without masks 0.035; R-MAT-13 by its own ids 1.25 -> 0.51; Chung-Lu
+// 2^15 26.8 -> 14.2).  Six blocks per SM: R-MAT-20 3.87, four 3.97.
+template <bool kSlices>
+__global__ void __launch_bounds__(256, 6) clique_big_kernel(const TrieView* __restrict__ views, HitsView hv,
+                                                         uint32_t n_units, uint32_t grab, uint32_t slices,
+                                                         unsigned int* __restrict__ queue,
                                                          unsigned long long* __restrict__ total) {
   const uint32_t lane = lane_id();
   unsigned long long acc = 0;
   uint32_t cur_g = 0;
   for (;;) {
-    uint32_t u0 = 0;
-    if (lane == 0) u0 = atomicAdd(queue, 4u);
-    u0 = __shfl_sync(kFull, u0, 0);
+    uint32_t x0 = 0;
+    if (lane == 0) x0 = atomicAdd(queue, grab);
+    x0 = __shfl_sync(kFull, x0, 0);
+    const uint32_t u0 = kSlices ? x0 / slices : x0;
+    const uint32_t slice = kSlices ? x0 - u0 * slices : 0;
     if (u0 >= n_units) break;
-    const uint32_t u1 = min(u0 + 4, n_units);
+    const uint32_t u1 = min(u0 + grab, n_units);
     uint32_t gh = hits_unit_head(hv, u0);
     for (uint32_t u = u0; u < u1; u++) {
       gh = hits_unit_next(hv, gh, u);
@@ -494,8 +502,10 @@ __global__ void __launch_bounds__(256) clique_big_kernel(const TrieView* __restr
       if (!hv.share.owns(a, d, i0)) continue;
       const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
       if (W > kSparseWords && sparse_rows(rows, ri, qi, W)) continue;  // clique_sparse_kernel's
-      uint32_t c = 0;  // below 2^32: masks of 2^31 words hold at most 2^26 (j word, row) steps per lane
-      for (uint32_t q = qi; q < W; q++) {
+      // below 2^29: the masks of all entries are 2^31 words at most, which bounds the
+      // sum of all d^2 by 2^37, and a lane's j, at most 2^13, add up to 8 d_j each
+      uint32_t c = 0;
+      for (uint32_t q = qi + slice; q < W; q += kSlices ? slices : 1) {
         const uint4 ma = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri));
         const uint4 mb = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri + 4));
         if (!(ma.x | ma.y | ma.z | ma.w | mb.x | mb.y | mb.z | mb.w)) continue;

@@ -2344,8 +2344,12 @@ static uint32_t launch(eh_context* ctx, Prepared& P, unsigned long long* d_total
       EH_CHECK_LAUNCH();
       launches++;
       if (H.units) {
-        clique_big_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 32)), 256, 0, s>>>(
-            P.dv, hv, H.units, P.ctl->queue + 1, d_total);
+        const uint32_t warps = 8 * most, grab = std::min(4u, std::max(1u, H.units / warps));
+        const uint32_t slices = std::min(8u, std::max(1u, warps / H.units));
+        const uint64_t turns = (uint64_t)H.units * slices / grab + 1;
+        (slices > 1 ? clique_big_kernel<true> : clique_big_kernel<false>)<<<
+            (int)std::min<uint64_t>(most, ceil_div(turns, 8)), 256, 0, s>>>(P.dv, hv, H.units, grab, slices,
+                                                                           P.ctl->queue + 1, d_total);
         EH_CHECK_LAUNCH();
         launches++;
         if (H.longest > 32 * kSparseWords) {
