@@ -2175,6 +2175,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   if (hits_use >= 0) plan_hits(ctx, tries, n, hits_use, ep, P.hits);
   P.plan_launches += P.hits.launches;
   const bool hits = P.hits.on;
+  if (hits_use == HITS_ROWS && !hits) return;  // rows come from masks, or from a plan made for them
   if (query == EH_QUERY_CLIQUE4 && !hits) {
     uint32_t mx = 0;
     for (uint32_t g = 0; g < n; g++) mx = std::max(mx, tries[g]->info.max_set);
@@ -2788,10 +2789,11 @@ void query_count_select(eh_context* ctx, const eh_trie* t, int query, uint32_t v
 // Triangle(a,b,c) :- Edge(a,b),Edge(b,c),Edge(a,c) as tuples sorted by
 // (a,b,c): the rows Trie::foreach (Trie.cpp:130-160) yields on the
 // reference's materialized output trie (TrieBuilder::build_set /
-// allocate_next / set_level, TrieBuilder.cpp:44-221, 376-410).  One counting
-// run sizes every work item's slice, a second run writes the tuples into
-// the slices, and two stable key-value radix sorts (by c, then by (a,b))
-// order them.
+// allocate_next / set_level, TrieBuilder.cpp:44-221, 376-410).  An up or down
+// relation's come in order from its hit masks (materialize_hits).  Of a symmetric or
+// general one, and where there is no memory for masks, one counting run sizes every
+// work item's slice, a second run writes the tuples into the slices, and two stable
+// key-value radix sorts (by c, then by (a,b)) order them.
 __global__ void iota_kernel(uint32_t* __restrict__ v, uint64_t n) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
     v[i] = (uint32_t)i;
