@@ -2392,10 +2392,10 @@ static uint32_t launch(eh_context* ctx, Prepared& P, unsigned long long* d_total
 }
 
 // Plan and run; nothing is waited for.  ev1 and ev2 bracket the intersection
-// kernels.  Results go to d_total (null: P.total; spare: nowhere that is read).
+// kernels.  Results go to P.total (spare: nowhere that is read).
 static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query, ExecParams ep,
-                        bool annot, Prepared& P, unsigned long long* d_total, unsigned long long* d_annot,
-                        float* d_records, const uint32_t* sel = nullptr, bool spare = false) {
+                        bool annot, Prepared& P, unsigned long long* d_annot, float* d_records,
+                        const uint32_t* sel = nullptr, bool spare = false) {
   cudaStream_t s = ctx->stream;
   Launch L;
   {
@@ -2409,7 +2409,7 @@ static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n
   EH_CUDA(cudaEventRecord(ctx->ev1, s));
   {
     TracePhase ph("query.kernel", s);
-    L.launches += launch(ctx, P, spare ? P.ctl->spare : d_total ? d_total : P.total, d_annot, d_records);
+    L.launches += launch(ctx, P, spare ? P.ctl->spare : P.total, d_annot, d_records);
   }
   EH_CUDA(cudaEventRecord(ctx->ev2, s));
   return L;
@@ -2578,7 +2578,7 @@ static void run_count(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
     rec.alloc(8 * (tries[0]->n_head + 2 * (cost / ep.chunk + cost / ep.chunk / 32) + 256), s);
   }
   if (query == EH_QUERY_TRIANGLE || query == EH_QUERY_CLIQUE4) {
-    L = run_plans(ctx, tries, n, query, ep, false, P, nullptr, nullptr, rec.p);
+    L = run_plans(ctx, tries, n, query, ep, false, P, nullptr, rec.p);
   } else {
     EH_REQUIRE(n == 1, EH_ERR_UNSUPPORTED, "batched lollipop/barbell is not supported");
     const eh_trie* t = tries[0];
@@ -2586,7 +2586,7 @@ static void run_count(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
     unsigned long long* T = annot_buffer(ctx, t->n_head ? t->n_head : 1);
     EH_CUDA(cudaMemsetAsync(T, 0, (t->n_head ? t->n_head : 1) * 8, s));
     // the annotated pass (recorded), then the root bag over T into P.total
-    L = run_plans(ctx, tries, 1, EH_QUERY_TRIANGLE, ep, true, P, nullptr, T, rec.p, nullptr, true);
+    L = run_plans(ctx, tries, 1, EH_QUERY_TRIANGLE, ep, true, P, T, rec.p, nullptr, true);
     L.launches += root_bag(ctx, t, query, T, nullptr, P.total);
   }
   const Returned got = finish(ctx, P);
@@ -2643,8 +2643,7 @@ void triangle_annotation(eh_context* ctx, const eh_trie* t, const eh_exec_config
   with_or_without_masks(ctx, ep, [&](const ExecParams& p) {
     EH_CUDA(cudaMemsetAsync(annot_dev, 0, (t->n_head ? t->n_head : 1) * 8, s));
     Prepared P;
-    run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, p, true, P, nullptr, (unsigned long long*)annot_dev, nullptr, nullptr,
-              true);
+    run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, p, true, P, (unsigned long long*)annot_dev, nullptr, nullptr, true);
     EH_CUDA(cudaStreamSynchronize(s));
   });
 }
@@ -2751,7 +2750,7 @@ void query_count_select(eh_context* ctx, const eh_trie* t, int query, uint32_t v
   if (h[2] > 0) {  // no partners: the selected bag is empty and so is the join
     if (clique) {
       Prepared P;
-      L.launches += run_plans(ctx, ts, 1, EH_QUERY_CLIQUE4, ep, false, P, nullptr, nullptr, nullptr, bits.p).launches;
+      L.launches += run_plans(ctx, ts, 1, EH_QUERY_CLIQUE4, ep, false, P, nullptr, nullptr, bits.p).launches;
       const Returned got = finish(ctx, P);
       items = got.items;
       pairs = P.pairs;
@@ -2764,7 +2763,7 @@ void query_count_select(eh_context* ctx, const eh_trie* t, int query, uint32_t v
         EH_CUDA(cudaMemsetAsync(T.p, 0, (size_t)t->n_head * 8, s));
         EH_CUDA(cudaMemsetAsync(sums.p, 0, 32, s));
         Prepared P;
-        const Launch K = run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, p, true, P, nullptr, T.p, nullptr, nullptr, true);
+        const Launch K = run_plans(ctx, ts, 1, EH_QUERY_TRIANGLE, p, true, P, T.p, nullptr, nullptr, true);
         select_partners_kernel<<<sgrid, 256, 0, s>>>(t->view(), value, nullptr, T.p, sums.p);
         EH_CHECK_LAUNCH();
         L.launches += K.launches + 1;
