@@ -80,7 +80,7 @@ constexpr uint32_t kFlatClique = EH_FLAT_CLIQUE;  // 4-clique: S up to this size
 // room for 32 resident warps; 1024 words 7.18 ms against 7.06); the
 // autotuner (emptyheaded_b200/autotune.py) re-picks them per trie.
 constexpr int kDefaultSmemWords = 1280;  // per warp
-constexpr int kDefaultChunk = 32768;     // where it is not derived from the work (records, noalloc)
+constexpr int kDefaultChunk = 32768;     // where it is not derived from the work (noalloc); 4-clique without masks: at most
 constexpr uint64_t kMaxChunk = 131072;   // larger items amortise staging: 7.03 ms against 7.18 at 32768
 constexpr uint64_t kMinChunk = 4096;  // the smallest item the planner cuts by itself
 constexpr uint32_t kShareWarps = 148 * 32;  // resident warps of a B200 at the default schedule
@@ -2392,9 +2392,11 @@ static uint32_t launch(eh_context* ctx, Prepared& P, unsigned long long* d_total
 }
 
 // Plan and run; nothing is waited for.  ev1 and ev2 bracket the intersection
-// kernels.  Results go to P.total (spare: nowhere that is read).
+// kernels.  Results go to P.total (spare: nowhere that is read).  rec: one record per
+// item, of the plan that runs otherwise but for items that entries share (a record is
+// one set's).
 static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n, int query, ExecParams ep,
-                        bool annot, Prepared& P, unsigned long long* d_annot, float* d_records,
+                        bool annot, Prepared& P, unsigned long long* d_annot, DevBuf<float>* rec = nullptr,
                         const uint32_t* sel = nullptr, bool spare = false) {
   cudaStream_t s = ctx->stream;
   Launch L;
@@ -2402,14 +2404,15 @@ static Launch run_plans(eh_context* ctx, const eh_trie* const* tries, uint32_t n
     TracePhase ph("query.prepare", s);
     // selections weight cliques by their members: they run without masks
     const int use = sel ? -1 : query == EH_QUERY_CLIQUE4 ? HITS_CLIQUE : annot ? HITS_ANNOT : -1;
-    prepare(ctx, tries, n, query, ep, annot, P, true, use, false, d_records == nullptr);
+    prepare(ctx, tries, n, query, ep, annot, P, true, use, false, rec == nullptr);
   }
+  if (rec) rec->alloc(8 * (P.cap_w + P.cap_b), s);
   P.sel = sel;
   L.launches = P.plan_launches;
   EH_CUDA(cudaEventRecord(ctx->ev1, s));
   {
     TracePhase ph("query.kernel", s);
-    L.launches += launch(ctx, P, spare ? P.ctl->spare : P.total, d_annot, d_records);
+    L.launches += launch(ctx, P, spare ? P.ctl->spare : P.total, d_annot, rec ? rec->p : nullptr);
   }
   EH_CUDA(cudaEventRecord(ctx->ev2, s));
   return L;
@@ -2570,15 +2573,9 @@ static void run_count(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
   Prepared P;
   Launch L;
   DevBuf<float> rec;
-  if (record) {
-    // one record per item; the plan size is known only after planning, so
-    // size for the worst case, as prepare does for the items; fixed chunks
-    ep.chunk_given = true;
-    const uint64_t cost = tries[0]->rev_pairs + kRowCost * tries[0]->rev_entries;
-    rec.alloc(8 * (tries[0]->n_head + 2 * (cost / ep.chunk + cost / ep.chunk / 32) + 256), s);
-  }
+  DevBuf<float>* recorded = record ? &rec : nullptr;
   if (query == EH_QUERY_TRIANGLE || query == EH_QUERY_CLIQUE4) {
-    L = run_plans(ctx, tries, n, query, ep, false, P, nullptr, rec.p);
+    L = run_plans(ctx, tries, n, query, ep, false, P, nullptr, recorded);
   } else {
     EH_REQUIRE(n == 1, EH_ERR_UNSUPPORTED, "batched lollipop/barbell is not supported");
     const eh_trie* t = tries[0];
@@ -2586,7 +2583,7 @@ static void run_count(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
     unsigned long long* T = annot_buffer(ctx, t->n_head ? t->n_head : 1);
     EH_CUDA(cudaMemsetAsync(T, 0, (t->n_head ? t->n_head : 1) * 8, s));
     // the annotated pass (recorded), then the root bag over T into P.total
-    L = run_plans(ctx, tries, 1, EH_QUERY_TRIANGLE, ep, true, P, T, rec.p, nullptr, true);
+    L = run_plans(ctx, tries, 1, EH_QUERY_TRIANGLE, ep, true, P, T, recorded, nullptr, true);
     L.launches += root_bag(ctx, t, query, T, nullptr, P.total);
   }
   const Returned got = finish(ctx, P);
