@@ -7,7 +7,8 @@ inside the engine, eh_query_stats.kernel_ms):
   warps        warps per block of the persistent kernel
   smem_words   shared staging per warp (u32 words): the tile width a staged
                N(b) may have before it is probed in global memory
-  chunk        probes per work item (work-chunk size of the queue)
+  chunk        probes per work item (work-chunk size of the queue); 0: derived
+               from the work, as every query without a schedule has it
   long_row     size-class boundary: rows with at least this many candidates
                run warp-wide, shorter rows are flattened over the lanes
 
@@ -19,11 +20,11 @@ import statistics
 
 GRID = {
     "smem_words": (768, 1024, 1280, 1536),
-    "chunk": (16384, 32768, 65536, 131072),
+    "chunk": (0, 16384, 32768, 65536, 131072),
     "long_row": (24, 48, 64, 128),
     "warps": (4, 8, 16),
 }
-DEFAULT = {"warps": 8, "smem_words": 1280, "chunk": 32768, "long_row": 48}
+DEFAULT = {"warps": 8, "smem_words": 1280, "chunk": 0, "long_row": 48}
 
 
 def _time(trie, cfg, query, reps, want):
