@@ -1179,9 +1179,10 @@ __device__ __forceinline__ bool few_candidates(const RevView& r, const Item& ite
 }
 
 // Stage N(b) in the warp's shared region according to its layout; returns
-// the probe mode.
+// the probe mode.  zlist: lists as bitmaps; blocks_too: block bitsets that fit as lists
+// as well, by their elements.
 __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_t* sm, int cap_words, Staged& st,
-                                         bool zlist = false) {
+                                         bool zlist = false, bool blocks_too = false) {
   const uint32_t lane = lane_id();
   const uint8_t layout = t.layout[hb];
   const StagedRange sr = staged_range(t, hb);
@@ -1234,7 +1235,7 @@ __device__ __forceinline__ int stage_set(const TrieView& t, uint32_t hb, uint32_
     st.words = t.bs_words + a.off;
     return P_GBITS;
   }
-  if (layout == EH_LAYOUT_BLOCK_BITSET) {
+  if (layout == EH_LAYOUT_BLOCK_BITSET && !(blocks_too && len <= (uint32_t)cap_words)) {
     st.ids = t.bb_id + a.off;
     st.bwords = t.bb_words + 4 * a.off;
     st.n = a.n;
