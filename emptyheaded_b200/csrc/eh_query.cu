@@ -2204,7 +2204,7 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
     if (P.smem > room) {
       // shrink the per-warp region to what a block may hold (a staged set
       // that no longer fits is probed in global memory instead)
-      EH_REQUIRE(hits || query != EH_QUERY_CLIQUE4, EH_ERR_UNSUPPORTED, "4-clique staging exceeds shared memory");
+      EH_REQUIRE(query != EH_QUERY_CLIQUE4, EH_ERR_UNSUPPORTED, "4-clique staging exceeds shared memory");
       ep.smem_words = (int)((room / 4 / ep.warps) & ~(size_t)1);
       P.smem = (size_t)ep.smem_words * 4 * ep.warps;
     }
