@@ -331,6 +331,7 @@ __device__ __forceinline__ uint32_t plan_span(const PlanArgs& p, uint32_t b) {
   return plan_small(p, b & ~7u, 8) ? 8 : 1;
 }
 
+constexpr uint64_t kPredTrust = 4;
 // items of entry b over all shards; span: plan_span
 __device__ __forceinline__ uint32_t plan_items(const PlanArgs& p, uint32_t b, uint64_t k0, uint64_t k1, bool& blk,
                                                uint32_t& span) {
@@ -344,11 +345,15 @@ __device__ __forceinline__ uint32_t plan_items(const PlanArgs& p, uint32_t b, ui
     blk = sw > p.ps.warp_words && sw <= p.ps.block_words;
   }
   const uint64_t mult = blk ? p.ps.warps : 1;
+  const uint64_t cost = w + kRowCost * (k1 - k0);
   if (p.ps.pred) {
+    // whatever the model predicts, no item of more than kPredTrust chunks: one that
+    // misjudges a hub would leave it to one warp (Chung-Lu 2^20, untrained: 4.6 ms,
+    // so 0.95, by chunks alone 0.70)
     const uint64_t m = (uint64_t)ceil((double)p.ps.pred[b] / (p.ps.unit * (double)mult));
-    return (uint32_t)max((uint64_t)1, min(m, (w + 63) / 64));
+    return (uint32_t)max(max((uint64_t)1, min(m, (w + 63) / 64)), cost / (kPredTrust * p.ps.chunk * mult));
   }
-  return (uint32_t)((w + kRowCost * (k1 - k0) + p.ps.chunk * mult - 1) / (p.ps.chunk * mult));
+  return (uint32_t)((cost + p.ps.chunk * mult - 1) / (p.ps.chunk * mult));
 }
 // this shard's first item of entry b
 __device__ __forceinline__ uint32_t plan_first(const PlanArgs& p, uint32_t b, uint32_t span) {
@@ -2235,13 +2240,14 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   }
   PlanShape shape{ep.chunk, nullptr, 0.0, (uint32_t)ep.smem_words,
                    blocks ? (uint32_t)ep.smem_words * (uint32_t)ep.warps : 0u, (uint32_t)ep.warps, 0u};
-  // items: at most one per entry with rows and one per chunk of work (with
-  // predicted costs: per chunk of probes, the sum of rounded-up shares; the
-  // slack covers their rounding)
-  P.cap_w = head_items + (cost / ep.chunk) + cost / ep.chunk / 64 + 64;
-  P.cap_b = blocks ? std::min<uint64_t>(P.cap_w, cost / ((uint64_t)ep.chunk * ep.warps) + cost / kMinBlockWork +
-                                                     cost / ep.chunk / 64 + 64)
-                   : 0;
+  // items: at most one per entry with rows and one per chunk of work; with predicted
+  // costs one per chunk of predicted cycles (the sum of rounded-up shares; the slack
+  // covers their rounding) and one per kPredTrust chunks of work
+  bool pred = false;
+  for (uint32_t g = 0; g < n; g++) pred |= tries[g]->work_pred.p != nullptr;
+  const uint64_t chunks = cost / ep.chunk + (pred ? cost / (kPredTrust * ep.chunk) : 0);
+  P.cap_w = head_items + chunks + chunks / 64 + 64;
+  P.cap_b = blocks ? std::min<uint64_t>(P.cap_w, chunks / ep.warps + cost / kMinBlockWork + chunks / 64 + 64) : 0;
   EH_REQUIRE(P.cap_w < (1ull << 32), EH_ERR_UNSUPPORTED, "work plan of 2^32 items or more");
   const size_t o_views = (P.ctl_bytes() + 127) & ~(size_t)127;
   const size_t o_rev = o_views + n * sizeof(TrieView);
