@@ -430,34 +430,42 @@ __global__ void __launch_bounds__(256) clique_small_kernel(const TrieView* __res
   if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
 }
 
-// A wide matrix may be nearly empty: then the words to AND for a unit's eight rows
-// are far more than the pairs of their hits, whose bits can be tested one by one.
-// (A star of 2^16 leaves with 2^18 rows among them: 90 ms by words alone, 4.7 with
-// this.)  32 pairs are 32 scattered words and a step of the AND three lines, so they
-// are weighed 8 to 1.
-constexpr uint32_t kSparseWords = 64;  // matrices this wide (2048 neighbours) may be sparse
-constexpr uint32_t kSparseHits = 256;  // hits of a row that are kept and paired
-__device__ __noinline__ bool sparse_rows(const uint32_t* rows, uint32_t ri, uint32_t qi, uint32_t W) {
-  uint32_t h[8] = {0, 0, 0, 0, 0, 0, 0, 0}, steps = 0;
-  for (uint32_t q = qi + lane_id(); q < W; q += 32) {
-    uint32_t any = 0;
-#pragma unroll
-    for (int x = 0; x < 8; x++) {
-      const uint32_t w = __ldg(rows + x + (q - qi) * ri);
-      any |= w;
-      h[x] += __popc(w);
+// parts of more words than this (2048 neighbours) are clique_wide_kernel's
+constexpr uint32_t kSparseWords = 64;
+
+// A unit of the 4-clique: the eight rows at `rows` of row block qi of the matrix m (W
+// words wide, d elements) against the blocks q0, q0 + step, ... of later positions.  A
+// function of its own, or its caller's state takes registers from the loop (4-clique
+// R-MAT-20, ms, so / inlined: at eight blocks per SM 3.78 / -, at six 3.98 / 3.99, at
+// four 3.93 / 3.96).
+__device__ __noinline__ uint32_t clique_dense(const uint32_t* m, const uint32_t* rows, uint32_t ri, uint32_t qi,
+                                                 uint32_t W, uint32_t d, uint32_t q0, uint32_t step) {
+  const uint32_t lane = lane_id();
+  // below 2^29: the masks of all entries are 2^31 words at most, which bounds the
+  // sum of all d^2 by 2^37, and a lane's j, at most 2^13, add up to 8 d_j each
+  uint32_t c = 0;
+  for (uint32_t q = q0; q < W; q += step) {
+    const uint4 ma = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri));
+    const uint4 mb = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri + 4));
+    if (!(ma.x | ma.y | ma.z | ma.w | mb.x | mb.y | mb.z | mb.w)) continue;
+    // all ones where the lane's position j = 32 q + lane is a hit of the row
+    const uint32_t on[8] = {0u - ((ma.x >> lane) & 1u), 0u - ((ma.y >> lane) & 1u), 0u - ((ma.z >> lane) & 1u),
+                            0u - ((ma.w >> lane) & 1u), 0u - ((mb.x >> lane) & 1u), 0u - ((mb.y >> lane) & 1u),
+                            0u - ((mb.z >> lane) & 1u), 0u - ((mb.w >> lane) & 1u)};
+    const uint32_t rq = hits_stride(q, W, d);
+    const uint32_t* jw = m + hits_block(q, W) + lane;
+    const bool has = lane < rq;
+#pragma unroll 2
+    for (uint32_t k = q; k < W; k++) {
+      const uint32_t y = has ? __ldg(jw + (k - q) * rq) : 0u;
+      const uint4 xa = __ldg(reinterpret_cast<const uint4*>(rows + (k - qi) * ri));
+      const uint4 xb = __ldg(reinterpret_cast<const uint4*>(rows + (k - qi) * ri + 4));
+      c += __popc(xa.x & y & on[0]) + __popc(xa.y & y & on[1]) + __popc(xa.z & y & on[2]) +
+           __popc(xa.w & y & on[3]) + __popc(xb.x & y & on[4]) + __popc(xb.y & y & on[5]) +
+           __popc(xb.z & y & on[6]) + __popc(xb.w & y & on[7]);
     }
-    if (any) steps += W - q;
   }
-  uint32_t most = 0;
-  uint64_t pairs = 0;
-#pragma unroll
-  for (int x = 0; x < 8; x++) {
-    h[x] = __reduce_add_sync(kFull, h[x]);
-    most = max(most, h[x]);
-    pairs += (uint64_t)h[x] * (h[x] + 32);  // 32 pairs a step, at least one step per hit
-  }
-  return most <= kSparseHits && pairs < 4ull * __reduce_add_sync(kFull, steps);
+  return c;
 }
 
 // 4-cliques of the larger parts.  A unit is eight consecutive rows i of one
@@ -470,10 +478,9 @@ __device__ __noinline__ bool sparse_rows(const uint32_t* rows, uint32_t ri, uint
 // row block where there are units enough: its L1 then holds the matrix.  Where there
 // are fewer than warps, `slices` warps share a unit, each every so many of its blocks
 // q (all four units of a block on one warp always, kernels, ms: star of 2^11 leaves
-// 0.54, so 0.075, without masks 0.035; R-MAT-13 by its own ids 1.25 -> 0.51; Chung-Lu
-// 2^15 26.8 -> 14.2).  Six blocks per SM: R-MAT-20 3.87, four 3.97.
+// 0.54, so 0.09, without masks 0.04; R-MAT-13 by its own ids 1.25 -> 0.25).
 template <bool kSlices>
-__global__ void __launch_bounds__(256, 6) clique_big_kernel(const TrieView* __restrict__ views, HitsView hv,
+__global__ void __launch_bounds__(256, 8) clique_big_kernel(const TrieView* __restrict__ views, HitsView hv,
                                                          uint32_t n_units, uint32_t grab, uint32_t slices,
                                                          unsigned int* __restrict__ queue,
                                                          unsigned long long* __restrict__ total) {
@@ -501,83 +508,181 @@ __global__ void __launch_bounds__(256, 6) clique_big_kernel(const TrieView* __re
       const uint32_t a = gh - hv.gstart[g], d = staged_range(views[g], a).len, W = (d + 31) >> 5;
       const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
       const uint32_t i0 = 8 * (u - __ldg(hv.upre + gh)), qi = i0 >> 5, ri = hits_stride(qi, W, d);
-      if (!hv.share.owns(a, d, i0)) continue;
+      if (W > kSparseWords || !hv.share.owns(a, d, i0)) continue;
       const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
-      if (W > kSparseWords && sparse_rows(rows, ri, qi, W)) continue;  // clique_sparse_kernel's
-      // below 2^29: the masks of all entries are 2^31 words at most, which bounds the
-      // sum of all d^2 by 2^37, and a lane's j, at most 2^13, add up to 8 d_j each
-      uint32_t c = 0;
-      for (uint32_t q = qi + slice; q < W; q += kSlices ? slices : 1) {
-        const uint4 ma = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri));
-        const uint4 mb = __ldg(reinterpret_cast<const uint4*>(rows + (q - qi) * ri + 4));
-        if (!(ma.x | ma.y | ma.z | ma.w | mb.x | mb.y | mb.z | mb.w)) continue;
-        // all ones where the lane's position j = 32 q + lane is a hit of the row
-        const uint32_t on[8] = {0u - ((ma.x >> lane) & 1u), 0u - ((ma.y >> lane) & 1u), 0u - ((ma.z >> lane) & 1u),
-                                0u - ((ma.w >> lane) & 1u), 0u - ((mb.x >> lane) & 1u), 0u - ((mb.y >> lane) & 1u),
-                                0u - ((mb.z >> lane) & 1u), 0u - ((mb.w >> lane) & 1u)};
-        const uint32_t rq = hits_stride(q, W, d);
-        const uint32_t* jw = m + hits_block(q, W) + lane;
-        const bool has = lane < rq;
-#pragma unroll 2
-        for (uint32_t k = q; k < W; k++) {
-          const uint32_t y = has ? __ldg(jw + (k - q) * rq) : 0u;
-          const uint4 xa = __ldg(reinterpret_cast<const uint4*>(rows + (k - qi) * ri));
-          const uint4 xb = __ldg(reinterpret_cast<const uint4*>(rows + (k - qi) * ri + 4));
-          c += __popc(xa.x & y & on[0]) + __popc(xa.y & y & on[1]) + __popc(xa.z & y & on[2]) +
-               __popc(xa.w & y & on[3]) + __popc(xb.x & y & on[4]) + __popc(xb.y & y & on[5]) +
-               __popc(xb.z & y & on[6]) + __popc(xb.w & y & on[7]);
-        }
-      }
-      acc += c;
+      acc += clique_dense(m, rows, ri, qi, W, d, qi + slice, kSlices ? slices : 1);
     }
   }
   acc = warp_sum(acc);
   if (lane == 0 && acc) atomicAdd(total + cur_g, acc);
 }
 
-// the units that sparse_rows keeps from clique_big_kernel
-__global__ void __launch_bounds__(256) clique_sparse_kernel(const TrieView* __restrict__ views, HitsView hv,
-                                                            uint32_t n_units,
-                                                            unsigned long long* __restrict__ total) {
-  __shared__ uint32_t s_hits[8][kSparseHits];
-  uint32_t* hits = s_hits[threadIdx.x >> 5];
+// 4-cliques of one row of a wide, nearly empty matrix: the non-zero words of row x of
+// the unit, at most kRowWords of them at a time in `list` (word, bits), are ANDed with
+// the same words of the row of each of its hits, every mw-th of them from `sub` on.
+constexpr uint32_t kRowWords = 256;
+__device__ __forceinline__ unsigned long long clique_sparse_row(const uint32_t* m, const uint32_t* row, uint32_t ri,
+                                                                uint32_t qi, uint32_t W, uint32_t d, uint32_t sub,
+                                                                uint32_t mw, uint2* list) {
   const uint32_t lane = lane_id();
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint64_t u = warp; u < n_units; u += nwarps) {
-    const uint32_t gh = hits_unit_head(hv, (uint32_t)u);
-    const uint32_t g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0;
-    const uint32_t a = gh - hv.gstart[g], d = staged_range(views[g], a).len, W = (d + 31) >> 5;
-    if (W <= kSparseWords) continue;
-    const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
-    const uint32_t i0 = 8 * ((uint32_t)u - __ldg(hv.upre + gh)), qi = i0 >> 5, ri = hits_stride(qi, W, d);
-    if (!hv.share.owns(a, d, i0)) continue;
-    const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
-    if (!sparse_rows(rows, ri, qi, W)) continue;
-    unsigned long long acc = 0;
-    for (uint32_t x = 0; x < 8; x++) {
-      uint32_t n = 0;
-      __syncwarp();
-      for (uint32_t q0 = qi; q0 < W; q0 += 32) {
-        const uint32_t q = q0 + lane;
-        uint32_t w = q < W ? __ldg(rows + x + (q - qi) * ri) : 0u;
-        const uint32_t incl = warp_incl_scan((uint32_t)__popc(w));
-        uint32_t at = n + incl - __popc(w);
-        n += __shfl_sync(kFull, incl, 31);
-        for (; w; w &= w - 1) hits[at++] = 32 * q + __ffs(w) - 1;
-      }
-      __syncwarp();
-      for (uint32_t y = 0; y + 1 < n; y++) {
-        const uint32_t j = hits[y], qj = j >> 5, rj = hits_stride(qj, W, d);
-        const uint32_t* jr = m + hits_block(qj, W) + (j & 31);
-        for (uint32_t z = y + 1 + lane; z < n; z += 32) {
-          const uint32_t l = hits[z];
-          acc += (__ldg(jr + ((l >> 5) - qj) * rj) >> (l & 31)) & 1u;
+  unsigned long long acc = 0;
+  for (uint32_t next = qi; next < W;) {
+    uint32_t n = 0;
+    __syncwarp();
+    for (; next < W && n <= kRowWords - 32; next += 32) {
+      const uint32_t q = next + lane;
+      const uint32_t w = q < W ? __ldg(row + (q - qi) * ri) : 0u;
+      const uint32_t set = __ballot_sync(kFull, w != 0);
+      if (w) list[n + __popc(set & lanemask_lt())] = make_uint2(q, w);
+      n += __popc(set);
+    }
+    __syncwarp();
+    if (!n) continue;
+    uint32_t first = 0, hit = 0;  // first word of the list at or after the hit's; hits so far
+    for (uint32_t q0 = qi; q0 < next; q0 += 32) {
+      const uint32_t q = q0 + lane;
+      const uint32_t w = q < W ? __ldg(row + (q - qi) * ri) : 0u;
+      for (uint32_t set = __ballot_sync(kFull, w != 0); set; set &= set - 1) {
+        const uint32_t qj = q0 + __ffs(set) - 1;
+        while (first < n && list[first].x < qj) first++;
+        const uint32_t rj = hits_stride(qj, W, d);
+        const uint32_t* jw = m + hits_block(qj, W);
+        for (uint32_t bits = __shfl_sync(kFull, w, qj - q0); bits; bits &= bits - 1) {
+          if (hit++ % mw != sub) continue;
+          const uint32_t* jr = jw + (__ffs(bits) - 1);
+          uint32_t c = 0;
+          for (uint32_t e = first + lane; e < n; e += 32) c += __popc(list[e].y & __ldg(jr + (list[e].x - qj) * rj));
+          acc += c;
         }
       }
     }
+  }
+  return acc;
+}
+
+// 4-cliques of parts of more than kSparseWords words (ids not in degree order: a hub
+// next to many).  One unit's AND can be millions of steps there, and its matrix nearly
+// empty.  The warps of a block share a unit.  Each first weighs one of the eight rows:
+// where the words of their hits' rows are few against the words to AND (32 scattered
+// words against a step of three lines for eight rows, weighed 16 to 1) a warp takes one
+// row by its non-zero words, else the warps take the blocks q in turn.
+// Units of more than kHeavySteps steps go to a list that blocks work off in
+// kHeavySlices pieces once they have seen their own units.  Nobody waits: a block
+// leaves when it finds the list worked off or its next entry not yet written, and
+// whoever is still writing one works the list off after that.
+// (4-clique, kernels, ms, without masks / a warp per unit, sparse ones by pairs of at
+// most 256 hits / so: Chung-Lu 2^20 of exponent 2.6 by its own ids 52 / 307 / 9.4, 2^15
+// of 2.1 63 / 27 / 1.5, R-MAT-16 by its own ids 140 / 31 / 5.3, star of 2^17 leaves with
+// 2^20 rows among them 32 / 15 / 13.8.  Heavy units shared by up to 17 blocks that each
+// weigh them instead of the list: the star 110.)
+constexpr uint32_t kHeavySteps = 16384, kHeavySlices = 32, kHeavySparse = 0x80000000u, kHeavyNone = 0xffffffffu;
+struct HeavyUnits {
+  unsigned int* count;  // [2] entries, pieces taken
+  unsigned int* unit;   // [cap] unit, with kHeavySparse if it runs by its rows' words; kHeavyNone: not written
+  uint32_t cap;
+};
+__global__ void __launch_bounds__(256, 4) clique_wide_kernel(const TrieView* __restrict__ views, HitsView hv,
+                                                             uint32_t n_units, HeavyUnits heavy,
+                                                             unsigned long long* __restrict__ total) {
+  __shared__ uint2 s_list[8][kRowWords];
+  __shared__ uint32_t s_unit[256];  // the wide units among the block's 256
+  __shared__ uint32_t s_hits[8], s_words[8], s_steps[8];
+  __shared__ unsigned int s_n;
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  // slice s of S of unit u; weigh: decide how, and whether it is for the list
+  auto run = [&](uint32_t u, bool weigh, bool sparse, uint32_t s, uint32_t S) {
+    const uint32_t gh = hits_unit_head(hv, u);
+    const uint32_t g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0, a = gh - hv.gstart[g];
+    const uint32_t d = staged_range(views[g], a).len, W = (d + 31) >> 5;
+    const uint32_t* m = hv.mask + __ldg(hv.moff + gh);
+    const uint32_t i0 = 8 * (u - __ldg(hv.upre + gh)), qi = i0 >> 5, ri = hits_stride(qi, W, d);
+    const uint32_t* rows = m + hits_block(qi, W) + (i0 & 31);
+    if (weigh) {
+      uint32_t h = 0, nz = 0, steps = 0;  // steps: of an AND of this row alone
+      for (uint32_t q = qi + lane; q < W; q += 32) {
+        const uint32_t w = __ldg(rows + wid + (q - qi) * ri);
+        if (w) {
+          h += __popc(w);
+          nz++;
+          steps += W - q;
+        }
+      }
+      h = __reduce_add_sync(kFull, h);
+      nz = __reduce_add_sync(kFull, nz);
+      steps = __reduce_add_sync(kFull, steps);
+      if (lane == 0) {
+        s_hits[wid] = h;
+        s_words[wid] = nz;
+        s_steps[wid] = steps;
+      }
+      __syncthreads();
+      uint64_t pairs = 0;  // (hit, word) pairs, at least one step of 32 per hit
+      const float full = 0.5f * (float)(W - qi) * (float)(W - qi + 1);
+      float empty = 1.f;  // share of the steps that no row needs, if their words lie independently
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        pairs += (uint64_t)s_hits[r] * (s_words[r] + 32);
+        empty *= 1.f - (float)s_steps[r] / full;
+      }
+      if (!pairs) return;  // the same on every thread, as all that follows from these numbers
+      const float dense = full * (1.f - empty);
+      sparse = (float)pairs < 4.f * dense;
+      if ((sparse ? (float)pairs / 64.f : dense) > (float)kHeavySteps) {
+        if (threadIdx.x == 0) {
+          const uint32_t i = atomicAdd(heavy.count, 1u);
+          if (i < heavy.cap) atomicExch(heavy.unit + i, sparse ? u | kHeavySparse : u);
+          s_n = i < heavy.cap;  // the block's units are counted out already
+        }
+        __syncthreads();
+        if (s_n) return;
+      }
+    }
+    unsigned long long acc;
+    if (sparse) acc = clique_sparse_row(m, rows + wid, ri, qi, W, d, s, S, s_list[wid]);
+    else acc = clique_dense(m, rows, ri, qi, W, d, qi + 8 * s + wid, 8 * S);
     acc = warp_sum(acc);
     if (lane == 0 && acc) atomicAdd(total + g, acc);
+  };
+  for (uint64_t base = 0; base < n_units; base += 256ull * gridDim.x) {  // the same on every thread
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const uint64_t u = base + (uint64_t)threadIdx.x * gridDim.x + blockIdx.x;
+    if (u < n_units) {
+      const uint32_t gh = hits_unit_head(hv, (uint32_t)u);
+      const uint32_t g = hv.n_graphs > 1 ? hits_graph(hv, gh) : 0, a = gh - hv.gstart[g];
+      const uint32_t d = staged_range(views[g], a).len;
+      if (d > 32 * kSparseWords && hv.share.owns(a, d, 8 * ((uint32_t)u - __ldg(hv.upre + gh))))
+        s_unit[atomicAdd(&s_n, 1u)] = (uint32_t)u;
+    }
+    __syncthreads();
+    const uint32_t n = s_n;
+    for (uint32_t x = 0; x < n; x++) {
+      run(s_unit[x], true, false, 0, 1);
+      __syncthreads();  // the rows' numbers are the next unit's
+    }
+    __syncthreads();  // everybody has seen n
+  }
+  for (;;) {
+    if (threadIdx.x == 0) {
+      s_n = 0;
+      unsigned int piece = atomicAdd(heavy.count + 1, 0u);
+      while (piece / kHeavySlices < heavy.cap) {
+        const unsigned int code = atomicAdd(heavy.unit + piece / kHeavySlices, 0u);
+        if (code == kHeavyNone) break;
+        const unsigned int seen = atomicCAS(heavy.count + 1, piece, piece + 1);
+        if (seen == piece) {
+          s_n = 1;
+          s_unit[0] = code;
+          s_unit[1] = piece % kHeavySlices;
+          break;
+        }
+        piece = seen;  // another block took it: the next one
+      }
+    }
+    __syncthreads();
+    if (!s_n) break;
+    run(s_unit[0] & ~kHeavySparse, false, (s_unit[0] & kHeavySparse) != 0, s_unit[1], kHeavySlices);
+    __syncthreads();
   }
 }
 

@@ -1974,6 +1974,7 @@ struct Hits {
   CliqueShare share;      // HITS_CLIQUE
   DevBuf<uint32_t> mask;
   DevBuf<uint32_t> plan;  // [heads] mask offsets, [heads + 1] units before, [n + 1] graph starts, sums
+  DevBuf<uint32_t> heavy; // 4-clique with wide parts: HeavyUnits, the two counters first
   uint32_t* moff() const { return plan.p; }
   uint32_t* upre() const { return plan.p + heads; }
   uint32_t* gstart() const { return upre() + heads + 1; }
@@ -2061,6 +2062,9 @@ static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
   H.launches += scan_launches(heads) + scan_launches(heads + 1);
   try {
     H.mask.alloc(h[4] ? h[4] : 1, s);
+    // a wide part has 4 (W + 1) mask words per unit
+    if (use == HITS_CLIQUE && H.longest > 32 * kSparseWords)
+      H.heavy.alloc(2 + std::min<uint64_t>(h[5], h[4] / (4 * kSparseWords)) + 1, s);
   } catch (const Error& e) {
     if (e.code != EH_ERR_OOM) throw;
     return;
@@ -2361,8 +2365,10 @@ static uint32_t launch(eh_context* ctx, Prepared& P, unsigned long long* d_total
         EH_CHECK_LAUNCH();
         launches++;
         if (H.longest > 32 * kSparseWords) {
-          clique_sparse_kernel<<<std::min(num_sms() * 8, ceil_div(H.units, 8)), 256, 0, s>>>(P.dv, hv, H.units,
-                                                                                            d_total);
+          EH_CUDA(cudaMemsetAsync(H.heavy.p, 0, 8, s));
+          EH_CUDA(cudaMemsetAsync(H.heavy.p + 2, 0xff, (H.heavy.n - 2) * 4, s));
+          const HeavyUnits heavy{H.heavy.p, H.heavy.p + 2, (uint32_t)H.heavy.n - 2};
+          clique_wide_kernel<<<num_sms() * 4, 256, 0, s>>>(P.dv, hv, H.units, heavy, d_total);
           EH_CHECK_LAUNCH();
           launches++;
         }
