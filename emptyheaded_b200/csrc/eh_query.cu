@@ -80,7 +80,7 @@ constexpr uint32_t kFlatClique = EH_FLAT_CLIQUE;  // 4-clique: S up to this size
 // room for 32 resident warps; 1024 words 7.18 ms against 7.06); the
 // autotuner (emptyheaded_b200/autotune.py) re-picks them per trie.
 constexpr int kDefaultSmemWords = 1280;  // per warp
-constexpr int kDefaultChunk = 32768;     // where it is not derived from the work (noalloc); 4-clique without masks: at most
+constexpr int kDefaultChunk = 32768;     // where it is not derived from the work (noalloc); 4-clique and annotation without masks: at most
 constexpr uint64_t kMaxChunk = 131072;   // larger items amortise staging: 7.03 ms against 7.18 at 32768
 constexpr uint64_t kMinChunk = 4096;  // the smallest item the planner cuts by itself
 constexpr uint32_t kShareWarps = 148 * 32;  // resident warps of a B200 at the default schedule
@@ -1183,6 +1183,16 @@ __device__ __forceinline__ bool few_candidates(const RevView& r, const Item& ite
          __ldg(r.rev_wpre + item.ke) - __ldg(r.rev_wpre + item.kb) <= kListCandidates;
 }
 
+// The annotated pass's rows run longer on a list than count_rows', so a bitmap has to
+// serve more of them (kernel ms, from 1,000 / 3,000 / 10,000 candidates, lists always:
+// R-MAT-20 of edge factor 4 by its own ids, down 2.94 / 3.00 / 2.62, 2.65, general 9.4 /
+// 9.3 / 9.0, 8.5; Chung-Lu 2^20 of exponent 2.6, general 8.0 / 8.0 / 7.3, 7.4; R-MAT-16,
+// general 1.37 / 1.42 / 1.88, 1.95).
+constexpr uint64_t kAnnotCandidates = 10000;
+__device__ __forceinline__ bool many_candidates(const RevView& r, const Item& item) {
+  return __ldg(r.rev_wpre + item.ke) - __ldg(r.rev_wpre + item.kb) >= kAnnotCandidates;
+}
+
 // Stage N(b) in the warp's shared region according to its layout; returns
 // the probe mode.  zlist: lists as bitmaps; blocks_too: block bitsets that fit as lists
 // as well, by their elements.
@@ -1536,10 +1546,11 @@ __global__ void EH_TRI_LAUNCH_BOUNDS triangle_kernel(const __grid_constant__ Tri
     } else {
       // bitmaps for the annotation of an ordered or general relation too (kernel ms, star
       // of 2^16 leaves 5.4 -> 3.3, R-MAT-18 going down by degree 15.2 -> 7.0, R-MAT-20
-      // 2.45 -> 1.87); a symmetric one's per-element counters are indexed by position in
+      // 2.45 -> 2.0); a symmetric one's per-element counters are indexed by position in
       // the list
-      const bool bitmap = kMode == MODE_COUNT || (kMode == MODE_ANNOT && r.dir != DIR_SYM);
-      mode = stage_set(t, item.hb, sm, cap_words, st, bitmap && !few_candidates(r, item));
+      const bool bitmap = kMode == MODE_COUNT ? !few_candidates(r, item)
+                                              : kMode == MODE_ANNOT && r.dir != DIR_SYM && many_candidates(r, item);
+      mode = stage_set(t, item.hb, sm, cap_words, st, bitmap);
     }
     const StagedRange sr = kMode == MODE_ANNOT ? staged_range(t, item.hb) : StagedRange{0, 0};
     const uint32_t blen = sr.len;
@@ -2238,8 +2249,9 @@ static void prepare(eh_context* ctx, const eh_trie* const* tries, uint32_t n, in
   const uint64_t slots = ep.shard_count > 1 ? (uint64_t)kShareWarps * ep.shard_count : resident;
   if (!ep.chunk_given) {
     // a 4-clique without masks does far more per row than the plan weighs (selection
-    // on R-MAT-18 going down by degree 548 ms; cut up to kMaxChunk 902)
-    const uint64_t most = query == EH_QUERY_CLIQUE4 && !hits ? kDefaultChunk : kMaxChunk;
+    // on R-MAT-18 going down by degree 548 ms; cut up to kMaxChunk 902), an annotation
+    // without masks somewhat more
+    const uint64_t most = (query == EH_QUERY_CLIQUE4 || annot) && !hits ? kDefaultChunk : kMaxChunk;
     ep.chunk = (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(kMinChunk, cost / (8 * slots)));
   }
   PlanShape shape{ep.chunk, nullptr, 0.0, (uint32_t)ep.smem_words,

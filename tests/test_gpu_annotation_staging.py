@@ -8,10 +8,10 @@ pytestmark = pytest.mark.gpu
 
 
 def _relation(span, kind):
-    """60 low vertices next to most of each other and to a few hundred of `span` ids,
+    """100 low vertices next to most of each other and to a few hundred of `span` ids,
     of which some meet a few more."""
     rng = np.random.default_rng(span)
-    n = 60
+    n = 100
     far = n + np.unique(rng.integers(0, span, 400))
     u, v = [np.repeat(np.arange(n), n)], [np.tile(np.arange(n), n)]
     for a in range(n):
@@ -42,7 +42,7 @@ def test_annotation(eh, oracle, kind, span):
             continue  # bitsets of the whole span for every set
         t = eh.Trie(u, v, policy=policy, forced=forced, max_bitset_bytes=1 << 40)
         np.testing.assert_array_equal(t.triangle_annotation(), per)
-        for kw in (dict(), dict(smem_words=64), dict(smem_words=400, warps=3), dict(chunk=50), dict(long_row=1)):
+        for kw in (dict(), dict(chunk=1 << 20), dict(smem_words=64), dict(smem_words=400, warps=3), dict(chunk=50), dict(long_row=1)):
             assert t.count("lollipop", **kw) == lollipop, (policy, forced, kw)
         assert t.count("barbell") == barbell
         t.free()
