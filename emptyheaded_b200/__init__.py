@@ -579,7 +579,9 @@ def set_intersect(sets, layouts, pairs, materialize=False, ctx=None):
 
     sets: list of sorted uint32 arrays; layouts: per-set layout codes;
     pairs: (k, 2) array of set indices.  Returns counts (and the
-    materialized intersections as a list when asked)."""
+    materialized intersections as a list when asked: views of one buffer that
+    has room for the smaller set of every pair, so a program that keeps a few of
+    them for long copies those)."""
     ctx = ctx or default_context()
     sizes = np.array([len(s) for s in sets], np.uint64)
     off = np.zeros(len(sets) + 1, np.uint64)

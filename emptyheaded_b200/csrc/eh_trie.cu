@@ -3,8 +3,9 @@
 // Reference: Trie<A,M>::Trie (storage_engine/src/Trie.cpp:380-510) sorts row
 // indices with a column-chasing comparator, finds distinct head values and
 // per-head runs, and builds each set with hybrid::build.  Here:
-//   rows -> packed 64-bit keys (col0 << b | col1) -> LSD radix sort ->
-//   unique -> head flags + scan -> head[], off[], vals[] (CSR) ->
+//   rows, unless they lie in order -> packed 64-bit keys (col0 << b | col1) ->
+//   LSD radix sort; tiles' counts of new rows and heads + scan ->
+//   head[], off[], vals[] (CSR) ->
 //   head_index[] (value -> head position, the dense form of the reference's
 //   NextLevel array, trie/TrieBlock.hpp:26-48) -> per-set layout ->
 //   range-bitset words + per-word ranks, block-bitset blocks.
