@@ -2078,6 +2078,7 @@ static void plan_hits(eh_context* ctx, const eh_trie* const* tries, uint32_t n, 
       H.heavy.alloc(2 + std::min<uint64_t>(h[5], h[4] / (4 * kSparseWords)) + 1, s);
   } catch (const Error& e) {
     if (e.code != EH_ERR_OOM) throw;
+    H.mask.release();
     return;
   }
   H.words = h[4];
